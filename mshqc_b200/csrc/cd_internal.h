@@ -88,6 +88,7 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf pair_sum;      // per-pair energies
     mshqc_cd::DevBuf totals;        // scalar results
     mshqc_cd::DevBuf flag;          // error / NaN flags
+    mshqc_cd::DevBuf gemm_ws;       // split-K partials of the FP64 products
     mshqc_cd::DevBuf pace;          // wave-pacing progress counters of the persistent tile kernels
     mshqc_cd::DevBuf amp;           // backward: staged amplitudes
     mshqc_cd::DevBuf gam[2];        // backward: Gamma per spin
@@ -104,7 +105,7 @@ struct mshqc_cd_ctx {
     bool H_set = false;
     mshqc_cd::DevBuf opdm;          // OMP2: OPDM blocks, densities, Fock matrices
     mshqc_cd::DevBuf omp2_ws;       // OMP2: split-K partials, rotation work matrices
-    mshqc_cd::DevBuf Zt;            // OMP2: P L^Q for every Q (M*N*N)
+    mshqc_cd::DevBuf Zt;            // Fock builds: P L^Q of a chunk of vectors
     mshqc_cd::DevBuf oz_a, oz_b;    // int8 slices of the transform operands (orbitals, vectors)
     mshqc_cd::DevBuf oz_ea, oz_eb;  // their row exponents
     mshqc_cd::DevBuf oz_flag;       // int8-slice product error flag
@@ -141,7 +142,7 @@ struct mshqc_cd_ctx {
         for (const auto& s : spin)
             b += s.C.bytes + s.eps.bytes + s.B64.bytes + s.Bhi.bytes + s.Blo.bytes + s.expo.bytes +
                  s.diag.bytes + s.norms.bytes;
-        b += diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
+        b += gemm_ws.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
         for (const auto& g : gam) b += g.bytes;
         for (const auto& g : grad) b += g.bytes;
         return b;
@@ -158,6 +159,7 @@ struct mshqc_cd_ctx {
         pair_sum.release();
         totals.release();
         flag.release();
+        gemm_ws.release();
         pace.release();
         amp.release();
         BT.release();

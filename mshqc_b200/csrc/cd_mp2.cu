@@ -26,16 +26,6 @@ namespace mshqc_cd {
 
 namespace {
 
-// out[k] = alpha * sum_s parts[s * n + k], in a fixed order
-__global__ void sum_partials_kernel(const double* __restrict__ parts, int S, int64_t n, double alpha,
-                                    double* __restrict__ out) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    double acc = 0.0;
-    for (int s = 0; s < S; ++s) acc += parts[(int64_t)s * n + k];
-    out[k] = alpha * acc;
-}
-
 // Partitioned backward: whether the next unit (block pair, or occupied block
 // of an FP64 pass) belongs to this context's share.  Units beyond the plan
 // (which a mismatch between plan_partition and the passes would produce)
@@ -202,8 +192,7 @@ int transform_f64(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
         g1.B = Lc;  g1.ldb = N;  g1.sB = 0;
         g1.C = ctx->Y.as<double>() + Q0 * N;  g1.ldc = M * N;  g1.sC = 0;
         g1.alpha = 1.0;  g1.beta = 0.0;
-        CD_CUDA(gemm_f64(g1, true, true, ctx->stream));
-        ctx->launches++;
+        CD_RC(gemm_run(ctx, g1, true, true));
     }
     // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu]
     GemmF64Args g2{};
@@ -215,8 +204,7 @@ int transform_f64(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
     g2.B = ctx->Y.as<double>();  g2.ldb = N;  g2.sB = M * N;
     g2.C = s.B64.as<double>() + lo * vp * Mp;  g2.ldc = Mp;  g2.sC = vp * Mp;
     g2.alpha = 1.0;  g2.beta = 0.0;
-    CD_CUDA(gemm_f64(g2, true, true, ctx->stream));
-    ctx->launches++;
+    CD_RC(gemm_run(ctx, g2, true, true));
     return MSHQC_CD_OK;
 }
 
@@ -766,15 +754,17 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int spin, double scale, double* dC)
     const double* C = s.C.as<double>();
     const double* Gm = ctx->gam[spin].as<double>();
     // dC[nu, o+a] = scale sum_{i,Q} Gamma[i][a][Q] Y[i][Q][nu]   (row-major [a][nu] == column-major dC)
-    for (int64_t i = lo; i < hi; ++i) {
+    // one product over the composite K = (i, Q): v x N output tiles alone
+    // leave most SMs idle at small v
+    {
         GemmF64Args g{};
         g.M = (int)v;  g.N = (int)N;  g.K = (int)M;  g.batch = 1;
-        g.A = Gm + i * vp * Mp;  g.lda = Mp;  g.sA = 0;
-        g.B = ctx->Y.as<double>() + (i - lo) * M * N;  g.ldb = N;  g.sB = 0;
+        g.kb = (int)ni;
+        g.A = Gm + lo * vp * Mp;  g.lda = Mp;  g.skA = vp * Mp;
+        g.B = ctx->Y.as<double>();  g.ldb = N;  g.skB = M * N;
         g.C = dC + o * N;  g.ldc = N;  g.sC = 0;
-        g.alpha = scale;  g.beta = i == lo ? 0.0 : 1.0;
-        CD_CUDA(gemm_f64(g, true, false, ctx->stream));
-        ctx->launches++;
+        g.alpha = scale;  g.beta = 0.0;
+        CD_RC(gemm_run(ctx, g, true, false));
     }
     // W[i][Q][nu] = sum_a Gamma[i][a][Q] C[nu, o+a]   (into the Y buffer)
     {
@@ -784,59 +774,23 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int spin, double scale, double* dC)
         g.B = C + o * N;  g.ldb = N;  g.sB = 0;
         g.C = ctx->Y.as<double>();  g.ldc = N;  g.sC = M * N;
         g.alpha = 1.0;  g.beta = 0.0;
-        CD_CUDA(gemm_f64(g, false, false, ctx->stream));
-        ctx->launches++;
+        CD_RC(gemm_run(ctx, g, false, false));
         ctx->Y_spin = -1;
     }
-    // dC[mu, i] = scale sum_{(Q,nu)} W[i][(Q,nu)] L[(Q,nu)][mu]
-    if (ctx->L_gen) {
-        // generated vectors: one GEMM per chunk of Q, accumulated in order
-        const int64_t qc = vectors_chunk_size(ctx);
-        for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
-            const int64_t mc = std::min(qc, M - Q0);
-            const double* Lc = nullptr;
-            CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
-            GemmF64Args g{};
-            g.M = (int)ni;  g.N = (int)N;  g.K = (int)(mc * N);  g.batch = 1;
-            g.A = ctx->Y.as<double>() + Q0 * N;  g.lda = M * N;  g.sA = 0;
-            g.B = Lc;  g.ldb = N;  g.sB = 0;
-            g.C = dC + lo * N;  g.ldc = N;  g.sC = 0;
-            g.alpha = scale;  g.beta = Q0 == 0 ? 0.0 : 1.0;
-            CD_CUDA(gemm_f64(g, true, false, ctx->stream));
-            ctx->launches++;
-        }
-        return MSHQC_CD_OK;
-    }
-    // stored vectors: only o rows, so the long K = M*N is split over S
-    // independent partial products (batched GEMM) that a deterministic
-    // reduction adds up
-    {
-        const int64_t K = M * N;
-        const int64_t tiles = cdiv(ni, 64) * cdiv(N, 64);
-        const int64_t S = std::max<int64_t>(1, std::min<int64_t>(256, cdiv(4 * ctx->num_sms, tiles)));
-        const int64_t Kc = (K / S) / 16 * 16, Krem = K - S * Kc;   // even chunks keep 16-byte copies
-        CD_ALLOC(ctx->W, sizeof(double) * (size_t)(S * ni * N), false);
+    // dC[mu, i] = scale sum_{(Q,nu)} W[i][(Q,nu)] L[(Q,nu)][mu], one chunk of
+    // vectors at a time (only ni rows: K is what fills the GPU)
+    const int64_t qc = vectors_chunk_size(ctx);
+    for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
+        const int64_t mc = std::min(qc, M - Q0);
+        const double* Lc = nullptr;
+        CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
         GemmF64Args g{};
-        g.M = (int)ni;  g.N = (int)N;  g.K = (int)Kc;  g.batch = (int)S;
-        g.A = ctx->Y.as<double>();  g.lda = M * N;  g.sA = Kc;
-        g.B = ctx->L.as<double>();  g.ldb = N;  g.sB = Kc * N;
-        g.C = ctx->W.as<double>();  g.ldc = N;  g.sC = ni * N;
-        g.alpha = 1.0;  g.beta = 0.0;
-        CD_CUDA(gemm_f64(g, true, false, ctx->stream));
-        ctx->launches++;
-        if (Krem > 0) {
-            GemmF64Args t = g;
-            t.K = (int)Krem;  t.batch = 1;
-            t.A = ctx->Y.as<double>() + S * Kc;
-            t.B = ctx->L.as<double>() + S * Kc * N;
-            t.beta = 1.0;
-            CD_CUDA(gemm_f64(t, true, false, ctx->stream));
-            ctx->launches++;
-        }
-        sum_partials_kernel<<<(unsigned)cdiv(ni * N, 256), 256, 0, ctx->stream>>>(
-            ctx->W.as<double>(), (int)S, ni * N, scale, dC + lo * N);
-        CD_CUDA(cudaGetLastError());
-        ctx->launches++;
+        g.M = (int)ni;  g.N = (int)N;  g.K = (int)(mc * N);  g.batch = 1;
+        g.A = ctx->Y.as<double>() + Q0 * N;  g.lda = M * N;  g.sA = 0;
+        g.B = Lc;  g.ldb = N;  g.sB = 0;
+        g.C = dC + lo * N;  g.ldc = N;  g.sC = 0;
+        g.alpha = scale;  g.beta = Q0 == 0 ? 0.0 : 1.0;
+        CD_RC(gemm_run(ctx, g, true, false));
     }
     return MSHQC_CD_OK;
 }
@@ -1057,9 +1011,9 @@ int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* ahi, const uint16_t* alo, in
 int reduce_deps(mshqc_cd_ctx* ctx, const double* prow, const double* pcol, const double* pocc, int64_t ox,
                 int64_t oy, int64_t rsx, int64_t ksy, int64_t vx, int64_t vy, double* deps_x, double* deps_y) {
     const int64_t npairs = ox * oy;
-    deps_rows_kernel<<<(unsigned)cdiv(vx, 128), 128, 0, ctx->stream>>>(prow, npairs, (int)rsx, (int)vx,
+    deps_rows_kernel<<<(unsigned)cdiv(vx, 16), 1024, 0, ctx->stream>>>(prow, npairs, (int)rsx, (int)vx,
                                                                        deps_x + ox);
-    deps_rows_kernel<<<(unsigned)cdiv(vy, 128), 128, 0, ctx->stream>>>(pcol, npairs, (int)ksy, (int)vy,
+    deps_rows_kernel<<<(unsigned)cdiv(vy, 16), 1024, 0, ctx->stream>>>(pcol, npairs, (int)ksy, (int)vy,
                                                                        deps_y + oy);
     deps_occ_kernel<<<(unsigned)cdiv(std::max(ox, oy), 128), 128, 0, ctx->stream>>>(pocc, (int)ox, (int)oy,
                                                                                     deps_x, deps_y);
@@ -1214,8 +1168,8 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
 // The FP64 counterpart of tc_backward_pass, over the same block pairs: S =
 // B_x[I] B_y[J]^T and the Gamma products as FP64 DMMA GEMMs around the
 // element-wise pass.  A diagonal block pair of the symmetric modes forms S
-// for j >= i only (one GEMM per row i), and the element-wise pass completes
-// the amplitude block with the transposes.
+// for j >= i only (GemmF64Args::tri), and the element-wise pass completes the
+// amplitude block with the transposes.
 template <int MODE>
 int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double* deps_y, double* partial) {
     constexpr bool kSym = MODE != AMP_OPPOSITE_SPIN;
@@ -1253,16 +1207,14 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             const double* YJ = Y.B64.as<double>() + J0 * dy.vp * Mp;
             // S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q]
             begin_stage(ctx, ST_AMPLITUDE);
-            for (int r = 0; r < (tri ? nI : 1); ++r) {
-                GemmF64Args g{};
-                g.M = (int)((tri ? 1 : nI) * dx.vp);  g.N = (int)((nJ - r) * dy.vp);  g.K = (int)Mp;  g.batch = 1;
-                g.A = XI + (int64_t)r * dx.vp * Mp;  g.lda = Mp;  g.sA = 0;
-                g.B = YJ + (int64_t)r * dy.vp * Mp;  g.ldb = Mp;  g.sB = 0;
-                g.C = S + (int64_t)r * dx.vp * ldS + (int64_t)r * dy.vp;  g.ldc = ldS;  g.sC = 0;
-                g.alpha = 1.0;  g.beta = 0.0;
-                CD_CUDA(gemm_f64(g, true, true, ctx->stream));
-                ctx->launches++;
-            }
+            GemmF64Args g{};
+            g.M = (int)(nI * dx.vp);  g.N = (int)ldS;  g.K = (int)Mp;  g.batch = 1;
+            g.A = XI;  g.lda = Mp;  g.sA = 0;
+            g.B = YJ;  g.ldb = Mp;  g.sB = 0;
+            g.C = S;  g.ldc = ldS;  g.sC = 0;
+            g.alpha = 1.0;  g.beta = 0.0;
+            g.tri = tri ? (int)dx.vp : 0;
+            CD_RC(gemm_run(ctx, g, true, true));
             end_stage(ctx);
             AmpElemArgs e{};
             e.S = S;
@@ -1306,8 +1258,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             h.B = YJ;  h.ldb = Mp;  h.sB = 0;
             h.C = ctx->gam[sx].as<double>() + I0 * dx.vp * Mp;  h.ldc = Mp;  h.sC = 0;
             h.alpha = 1.0;  h.beta = 1.0;
-            CD_CUDA(gemm_f64(h, true, false, ctx->stream));
-            ctx->launches++;
+            CD_RC(gemm_run(ctx, h, true, false));
             if (mirror) {
                 // Gamma_y[(j,b)][Q] += sum_{(i,a) in I} t[(i,a)][(j,b)] X[(i,a)][Q]
                 GemmF64Args k{};
@@ -1316,8 +1267,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
                 k.B = XI;  k.ldb = Mp;  k.sB = 0;
                 k.C = ctx->gam[sy].as<double>() + J0 * dy.vp * Mp;  k.ldc = Mp;  k.sC = 0;
                 k.alpha = 1.0;  k.beta = 1.0;
-                CD_CUDA(gemm_f64(k, false, false, ctx->stream));
-                ctx->launches++;
+                CD_RC(gemm_run(ctx, k, false, false));
             }
             end_stage(ctx);
         }

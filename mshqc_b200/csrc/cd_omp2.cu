@@ -11,8 +11,15 @@
 //   column Gram  Gvv_x[a][b] += c * sum_i sum_(j,c) A[(i,a)][(j,c)] A[(i,b)][(j,c)]
 //   row Gram     Goo_y[i][j] += c * sum_(k,a) sum_b A[(k,a)][(i,b)] A[(k,a)][(j,b)]
 // Same-spin blocks give both blocks of their own spin (c = +1/2, -1/2, using
-// t[i,k,a,b] = t[k,i,b,a]); the opposite-spin pass with alpha rows gives
-// Gvv_alpha and Goo_beta, the one with beta rows Gvv_beta and Goo_alpha.
+// t[i,k,a,b] = t[k,i,b,a]).  An opposite-spin block that holds every alpha row
+// gives all four blocks (the other two Grams contract its columns); when
+// memory splits the rows, a second pass with beta rows gives Gvv_beta and
+// Goo_alpha.  Each Gram is one product over a composite K (a batch index and a
+// contiguous index, GemmF64Args::kb) with the tiles below the diagonal
+// mirrored: few output tiles and a K of 10^4 .. 10^6, so the split of K over
+// CTAs is what fills the GPU.  At N = 180, o = 18 the earlier form (one GEMM
+// per occupied orbital, 9 CTAs each) took 14 ms per iteration for the column
+// Grams, this one 0.5 ms.
 // The generalized Fock matrix (:331-369) uses the Cholesky J and K:
 //   J = sum_Q <L^Q, P_tot> L^Q,   K_s = sum_Q L^Q P_s L^Q,
 // with Z^Q = P_s L^Q for all Q as one batched GEMM and K_s as one GEMM over
@@ -34,28 +41,6 @@
 namespace mshqc_cd {
 namespace {
 
-// out[k] += alpha * sum_s parts[s * n + k], in a fixed order
-__global__ void sum_parts_acc_kernel(const double* __restrict__ parts, int S, int64_t n, double alpha,
-                                     double* __restrict__ out) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    double acc = 0.0;
-    for (int s = 0; s < S; ++s) acc += parts[(int64_t)s * n + k];
-    out[k] += alpha * acc;
-}
-
-// X[(c * R + r) * w + b] = A[r * ldA + c * w + b]: column blocks of width w
-// become rows, so that a row Gram is an ordinary GEMM over K = (r, b)
-__global__ void regroup_kernel(const double* __restrict__ A, int64_t ldA, int64_t R, int64_t nc, int64_t w,
-                               double* __restrict__ X) {
-    const int64_t total = R * nc * w;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = t % w, rest = t / w, r = rest % R, c = rest / R;
-        X[t] = A[r * ldA + c * w + b];
-    }
-}
-
 // out[q] = sum_k L[q * n + k] P[k] (one CTA per q, fixed-order tree)
 __global__ void dot_rows_kernel(const double* __restrict__ L, int64_t n, const double* __restrict__ P,
                                 double* __restrict__ out) {
@@ -70,6 +55,30 @@ __global__ void dot_rows_kernel(const double* __restrict__ L, int64_t n, const d
         __syncthreads();
     }
     if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+}
+
+// parts[s][k] = sum over the s-th share of the vectors of coef[q] L[q * n + k]:
+// the Coulomb matrix of one pass over the vectors.  HBM bound (8 bytes per
+// multiply-add), so one thread per element and, when n alone does not fill
+// the GPU, the vectors split over blockIdx.y; gemm_reduce_kernel adds the
+// shares in order.  N = 400, M = 1600: 1.02 ms as a GEMM with one row, 0.37 ms
+// here (5.5 TB/s).
+__global__ void __launch_bounds__(256) coulomb_kernel(const double* __restrict__ L, int64_t n, int M, int per,
+                                                      const double* __restrict__ coef, double* __restrict__ parts) {
+    const int64_t k = blockIdx.x * 256LL + threadIdx.x;
+    if (k >= n) return;
+    const int q0 = blockIdx.y * per, q1 = min(M, q0 + per);
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    int q = q0;
+    for (; q + 4 <= q1; q += 4) {
+        const double* l = L + (int64_t)q * n + k;
+        s0 = fma(coef[q], l[0], s0);
+        s1 = fma(coef[q + 1], l[n], s1);
+        s2 = fma(coef[q + 2], l[2 * n], s2);
+        s3 = fma(coef[q + 3], l[3 * n], s3);
+    }
+    for (; q < q1; ++q) s0 = fma(coef[q], L[(int64_t)q * n + k], s0);
+    parts[(int64_t)blockIdx.y * n + k] = (s0 + s1) + (s2 + s3);
 }
 
 // G (N x N) = blockdiag(Goo (o x o), Gvv (v x v, row stride vp)), zero elsewhere
@@ -91,44 +100,21 @@ __global__ void axpy_kernel(const double* __restrict__ a, double s, const double
     if (t < n) out[t] = a[t] + s * b[t];
 }
 
-__global__ void identity_kernel(double* __restrict__ A, int64_t N) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < N * N) A[t] = (t / N == t % N) ? 1.0 : 0.0;
-}
-
 unsigned blocks_for(int64_t n, int threads = 256) { return (unsigned)cdiv(n, threads); }
 
-// C (+)= alpha * sum_k X[m][k] X[n][k] for the o x o Gram of X (o rows of
-// length K), split over K so that enough CTAs run; partials go to `ws`.
-int gram_rows_splitk(mshqc_cd_ctx* ctx, const double* X, int64_t o, int64_t K, double alpha, double* C,
-                     mshqc_cd::DevBuf& ws) {
-    const int64_t tiles = cdiv(o, 64) * cdiv(o, 64);
-    const int64_t S = std::max<int64_t>(1, std::min<int64_t>(512, cdiv(4 * ctx->num_sms, tiles)));
-    const int64_t Kc = (K / S) / 16 * 16, Krem = K - S * Kc;
-    CD_ALLOC(ws, sizeof(double) * (size_t)(S * o * o), false);
-    GemmF64Args g{};
-    g.M = (int)o;  g.N = (int)o;  g.K = (int)Kc;  g.batch = (int)S;
-    g.A = X;  g.lda = K;  g.sA = Kc;
-    g.B = X;  g.ldb = K;  g.sB = Kc;
-    g.C = ws.as<double>();  g.ldc = o;  g.sC = o * o;
-    g.alpha = 1.0;  g.beta = 0.0;
-    if (Kc > 0) {
-        CD_CUDA(gemm_f64(g, true, true, ctx->stream));
-        ctx->launches++;
-    } else {
-        CD_CUDA(cudaMemsetAsync(ws.p, 0, sizeof(double) * (size_t)(S * o * o), ctx->stream));
-    }
-    if (Krem > 0) {
-        GemmF64Args t = g;
-        t.K = (int)Krem;  t.batch = 1;
-        t.A = X + S * Kc;  t.B = X + S * Kc;
-        t.beta = Kc > 0 ? 1.0 : 0.0;
-        CD_CUDA(gemm_f64(t, true, true, ctx->stream));
-        ctx->launches++;
-    }
-    sum_parts_acc_kernel<<<blocks_for(o * o), 256, 0, ctx->stream>>>(ws.as<double>(), (int)S, o * o, alpha, C);
+// J = beta * J + sum_q coef[q] L[q] over mc vectors of n elements
+int coulomb(mshqc_cd_ctx* ctx, const double* L, int64_t n, int64_t mc, const double* coef, double beta, double* J) {
+    const int64_t want = std::max<int64_t>(1, 8LL * ctx->num_sms / cdiv(n, 256));
+    const int per = (int)std::max<int64_t>(4, cdiv(mc, want));
+    const int S = (int)cdiv(mc, per);
+    CD_ALLOC(ctx->gemm_ws, sizeof(double) * (size_t)(S * n), false);
+    coulomb_kernel<<<dim3(blocks_for(n), (unsigned)S), 256, 0, ctx->stream>>>(L, n, (int)mc, per, coef,
+                                                                              ctx->gemm_ws.as<double>());
     CD_CUDA(cudaGetLastError());
-    ctx->launches++;
+    gemm_reduce_kernel<<<dim3((unsigned)cdiv(n, 64), 1), 256, 0, ctx->stream>>>(ctx->gemm_ws.as<double>(), S, 1, (int)n,
+                                                                                1.0, beta, J, n, 0, 0);
+    CD_CUDA(cudaGetLastError());
+    ctx->launches += 2;
     return MSHQC_CD_OK;
 }
 
@@ -137,12 +123,26 @@ struct OpdmOut {
     double* Gvv[2];   // vp_s x vp_s (padded)
 };
 
+// G (+)= coef * sum_h sum_k A_h[m][k] A_h[n][k]  (n x n, symmetric)
+int gram(mshqc_cd_ctx* ctx, const double* A, bool a_k, int64_t n, int64_t K, int64_t ld, int64_t kb, int64_t skb,
+         double coef, double* G, int64_t ldg) {
+    GemmF64Args g{};
+    g.M = g.N = (int)n;  g.K = (int)K;  g.batch = 1;
+    g.A = g.B = A;  g.lda = g.ldb = ld;
+    g.kb = (int)kb;  g.skA = g.skB = skb;
+    g.C = G;  g.ldc = ldg;
+    g.alpha = coef;  g.beta = 1.0;
+    g.sym = 1;
+    return gemm_run(ctx, g, a_k, a_k);
+}
+
 // One amplitude pass: rows i of spin sx (blocks), columns every j of spin sy.
-// Gvv_sx += col_coef * column Gram, Goo_sy += row_coef * row Gram; tile
-// energies to `partial` when it is not null.
+// Gvv_sx += col_coef * column Gram, Goo_sy += row_coef * row Gram; pair
+// energies to `partial` when it is not null.  With `both` (opposite spin) and
+// all rows in one block, Gvv_sy and Goo_sx are added too and *both is set.
 template <int MODE>
 int opdm_pass(mshqc_cd_ctx* ctx, int sx, int sy, double col_coef, double row_coef, const OpdmOut& out,
-              double* partial) {
+              double* partial, bool* both) {
     SpinState& X = ctx->spin[sx];
     SpinState& Y = ctx->spin[sy];
     const int64_t N = ctx->N, Mp = ctx->Mp;
@@ -152,7 +152,8 @@ int opdm_pass(mshqc_cd_ctx* ctx, int sx, int sy, double col_coef, double row_coe
     size_t free_b = 0, total_b = 0;
     CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t per_i = 2 * sizeof(double) * (size_t)vpx * ldS;
-    const size_t budget = std::max<size_t>(per_i, std::min<size_t>(free_b / 4, size_t(24) << 30));
+    const size_t held = ctx->W.bytes + ctx->amp.bytes;
+    const size_t budget = std::max<size_t>(per_i, std::min<size_t>((free_b + held) / 4, size_t(24) << 30));
     const int bi = (int)std::max<int64_t>(1, std::min<int64_t>(ox, (int64_t)(budget / per_i)));
     CD_ALLOC(ctx->W, per_i / 2 * bi, false);
     CD_ALLOC(ctx->amp, per_i / 2 * bi, false);
@@ -161,18 +162,20 @@ int opdm_pass(mshqc_cd_ctx* ctx, int sx, int sy, double col_coef, double row_coe
         CD_ALLOC(ctx->pair_sum, sizeof(double) * (size_t)(ox * oy), false);
         partial = ctx->pair_sum.as<double>();
     }
+    const double* A = ctx->amp.as<double>();
     for (int i0 = 0; i0 < ox; i0 += bi) {
         const int nbi = (int)std::min<int64_t>(bi, ox - i0);
         const int64_t R = (int64_t)nbi * vpx;
-        // S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q]
+        // S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q]; a same-spin block of
+        // all rows is symmetric
         GemmF64Args g{};
         g.M = (int)R;  g.N = (int)ldS;  g.K = (int)Mp;  g.batch = 1;
         g.A = X.B64.as<double>() + (int64_t)i0 * vpx * Mp;  g.lda = Mp;  g.sA = 0;
         g.B = Y.B64.as<double>();  g.ldb = Mp;  g.sB = 0;
         g.C = ctx->W.as<double>();  g.ldc = ldS;  g.sC = 0;
         g.alpha = 1.0;  g.beta = 0.0;
-        CD_CUDA(gemm_f64(g, true, true, ctx->stream));
-        ctx->launches++;
+        g.sym = sx == sy && nbi == ox ? 1 : 0;
+        CD_RC(gemm_run(ctx, g, true, true));
         AmpElemArgs e{};
         e.S = ctx->W.as<double>();
         e.ldS = ldS;
@@ -186,23 +189,17 @@ int opdm_pass(mshqc_cd_ctx* ctx, int sx, int sy, double col_coef, double row_coe
         amp_elem_kernel<MODE, false><<<(unsigned)(nbi * oy), 256, 0, ctx->stream>>>(e);
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
-        // column Gram: Gvv_x[a][b] += c * sum_K A[(i,a)][K] A[(i,b)][K], one GEMM per i
-        for (int ii = 0; ii < nbi; ++ii) {
-            GemmF64Args h{};
-            h.M = (int)vpx;  h.N = (int)vpx;  h.K = (int)ldS;  h.batch = 1;
-            h.A = ctx->amp.as<double>() + (int64_t)ii * vpx * ldS;  h.lda = ldS;  h.sA = 0;
-            h.B = h.A;  h.ldb = ldS;  h.sB = 0;
-            h.C = out.Gvv[sx];  h.ldc = vpx;  h.sC = 0;
-            h.alpha = col_coef;  h.beta = 1.0;
-            CD_CUDA(gemm_f64(h, true, true, ctx->stream));
-            ctx->launches++;
+        // column Gram: K batches i, K = (j, c)
+        CD_RC(gram(ctx, A, true, vpx, ldS, ldS, nbi, vpx * ldS, col_coef, out.Gvv[sx], vpx));
+        // row Gram: K batches (k, a), K = b
+        CD_RC(gram(ctx, A, true, oy, vpy, vpy, R, ldS, row_coef, out.Goo[sy], oy));
+        if (both && nbi == ox) {
+            // the same amplitudes as rows of spin sy: K batches j, K = (i, a)
+            CD_RC(gram(ctx, A, false, vpy, R, ldS, oy, vpy, col_coef, out.Gvv[sy], vpy));
+            // and K batches a, K = (j, b)
+            CD_RC(gram(ctx, A, true, ox, ldS, vpx * ldS, vpx, ldS, row_coef, out.Goo[sx], ox));
+            *both = true;
         }
-        // row Gram: regroup the columns j of A into rows, then an o_y x o_y Gram
-        regroup_kernel<<<(unsigned)std::min<int64_t>(cdiv(R * ldS, 256), (int64_t)ctx->num_sms * 32), 256, 0,
-                         ctx->stream>>>(ctx->amp.as<double>(), ldS, R, oy, vpy, ctx->W.as<double>());
-        CD_CUDA(cudaGetLastError());
-        ctx->launches++;
-        CD_RC(gram_rows_splitk(ctx, ctx->W.as<double>(), oy, R * vpy, row_coef, out.Goo[sy], ctx->omp2_ws));
     }
     return MSHQC_CD_OK;
 }
@@ -221,11 +218,13 @@ int omp2_buffers(mshqc_cd_ctx* ctx, Omp2Buffers& b) {
     const int64_t N = ctx->N, M = ctx->M;
     const int64_t o0 = ctx->spin[0].nocc, o1 = ctx->spin[1].nocc;
     const int64_t vp0 = round_up(N - o0, 64), vp1 = round_up(N - o1, 64);
-    const int64_t n = o0 * o0 + o1 * o1 + vp0 * vp0 + vp1 * vp1 + 9 * N * N + M + 2 * N;
+    // the blocks before the matrices padded to an even count: 16-byte rows for even N
+    const int64_t noo = round_up(o0 * o0 + o1 * o1, 2);
+    const int64_t n = noo + vp0 * vp0 + vp1 * vp1 + 9 * N * N + M + 2 * N;
     CD_ALLOC(ctx->opdm, sizeof(double) * (size_t)n, false);
     double* p = ctx->opdm.as<double>();
     b.Goo[0] = p;  p += o0 * o0;
-    b.Goo[1] = p;  p += o1 * o1;
+    b.Goo[1] = p;  p += noo - o0 * o0;
     b.Gvv[0] = p;  p += vp0 * vp0;
     b.Gvv[1] = p;  p += vp1 * vp1;
     b.P[0] = p;  p += N * N;
@@ -251,8 +250,7 @@ int occupied_density(mshqc_cd_ctx* ctx, const double* C, int64_t o, double* P) {
     g.B = C;  g.ldb = N;  g.sB = 0;
     g.C = P;  g.ldc = N;  g.sC = 0;
     g.alpha = 1.0;  g.beta = 0.0;
-    CD_CUDA(gemm_f64(g, false, false, ctx->stream));
-    ctx->launches++;
+    CD_RC(gemm_run(ctx, g, false, false));
     return MSHQC_CD_OK;
 }
 
@@ -266,7 +264,7 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     const int64_t o0 = ctx->spin[0].nocc, o1 = ctx->spin[1].nocc;
     const int64_t vp0 = ctx->spin[0].vp, vp1 = ctx->spin[1].vp;
     // OPDM blocks start at zero
-    CD_CUDA(cudaMemsetAsync(b.Goo[0], 0, sizeof(double) * (size_t)(o0 * o0 + o1 * o1 + vp0 * vp0 + vp1 * vp1),
+    CD_CUDA(cudaMemsetAsync(b.Goo[0], 0, sizeof(double) * (size_t)(round_up(o0 * o0 + o1 * o1, 2) + vp0 * vp0 + vp1 * vp1),
                             ctx->stream));
     CD_ALLOC(ctx->totals, sizeof(double) * 16, false);
     const int64_t n0 = o0 * o0, n1 = o1 * o1, n2 = o0 * o1;   // one energy per pair
@@ -274,10 +272,11 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     double* part = ctx->partial.as<double>();
     OpdmOut out{{b.Goo[0], b.Goo[1]}, {b.Gvv[0], b.Gvv[1]}};
     begin_stage(ctx, ST_AMPLITUDE);
-    CD_RC(opdm_pass<AMP_SAME_SPIN>(ctx, 0, 0, 0.5, -0.5, out, part));
-    CD_RC(opdm_pass<AMP_SAME_SPIN>(ctx, 1, 1, 0.5, -0.5, out, part + n0));
-    CD_RC(opdm_pass<AMP_OPPOSITE_SPIN>(ctx, 0, 1, 1.0, -1.0, out, part + n0 + n1));
-    CD_RC(opdm_pass<AMP_OPPOSITE_SPIN>(ctx, 1, 0, 1.0, -1.0, out, nullptr));
+    CD_RC(opdm_pass<AMP_SAME_SPIN>(ctx, 0, 0, 0.5, -0.5, out, part, nullptr));
+    CD_RC(opdm_pass<AMP_SAME_SPIN>(ctx, 1, 1, 0.5, -0.5, out, part + n0, nullptr));
+    bool both = false;
+    CD_RC(opdm_pass<AMP_OPPOSITE_SPIN>(ctx, 0, 1, 1.0, -1.0, out, part + n0 + n1, &both));
+    if (!both) CD_RC(opdm_pass<AMP_OPPOSITE_SPIN>(ctx, 1, 0, 1.0, -1.0, out, nullptr, nullptr));
     end_stage(ctx);
     const int64_t offs[3] = {0, n0, n0 + n1}, cnt[3] = {n0, n1, n2};
     for (int k = 0; k < 3; ++k) {
@@ -300,28 +299,22 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
         g.M = (int)N;  g.N = (int)N;  g.K = (int)N;  g.batch = 1;
         g.A = C;  g.lda = N;  g.B = b.G;  g.ldb = N;  g.C = b.T;  g.ldc = N;
         g.alpha = 1.0;  g.beta = 0.0;
-        CD_CUDA(gemm_f64(g, false, false, ctx->stream));
+        CD_RC(gemm_run(ctx, g, false, false));
         // P = T C^T + Pref
         CD_CUDA(cudaMemcpyAsync(b.P[s], Pref[s], sizeof(double) * NN, cudaMemcpyDeviceToDevice, ctx->stream));
         GemmF64Args h{};
         h.M = (int)N;  h.N = (int)N;  h.K = (int)N;  h.batch = 1;
         h.A = b.T;  h.lda = N;  h.B = C;  h.ldb = N;  h.C = b.P[s];  h.ldc = N;
         h.alpha = 1.0;  h.beta = 1.0;
-        CD_CUDA(gemm_f64(h, true, false, ctx->stream));
-        ctx->launches += 3;
+        CD_RC(gemm_run(ctx, h, true, false));
+        ctx->launches++;
     }
     // J = sum_Q <L^Q, P_a + P_b> L^Q
     axpy_kernel<<<blocks_for(NN), 256, 0, ctx->stream>>>(b.P[0], 1.0, b.P[1], NN, b.G);
     dot_rows_kernel<<<(unsigned)M, 256, 0, ctx->stream>>>(ctx->L.as<double>(), NN, b.G, b.coef);
     CD_CUDA(cudaGetLastError());
-    {
-        GemmF64Args g{};
-        g.M = 1;  g.N = (int)NN;  g.K = (int)M;  g.batch = 1;
-        g.A = b.coef;  g.lda = M;  g.B = ctx->L.as<double>();  g.ldb = NN;  g.C = b.J;  g.ldc = NN;
-        g.alpha = 1.0;  g.beta = 0.0;
-        CD_CUDA(gemm_f64(g, true, false, ctx->stream));
-        ctx->launches += 3;
-    }
+    ctx->launches += 2;
+    CD_RC(coulomb(ctx, ctx->L.as<double>(), NN, M, b.coef, 0.0, b.J));
     CD_ALLOC(ctx->Zt, sizeof(double) * (size_t)(M * NN), false);
     for (int s = 0; s < 2; ++s) {
         const double* C = ctx->spin[s].C.as<double>();
@@ -332,7 +325,7 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
         z.B = ctx->L.as<double>();  z.ldb = N;  z.sB = NN;
         z.C = ctx->Zt.as<double>();  z.ldc = N;  z.sC = NN;
         z.alpha = 1.0;  z.beta = 0.0;
-        CD_CUDA(gemm_f64(z, true, false, ctx->stream));
+        CD_RC(gemm_run(ctx, z, true, false));
         // K[mu][lam] = sum_{(Q,nu)} L^Q(mu,nu) Z^Q(nu,lam)
         GemmF64Args k{};
         k.M = (int)N;  k.N = (int)N;  k.K = (int)(M * N);  k.batch = 1;
@@ -340,7 +333,7 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
         k.B = ctx->Zt.as<double>();  k.ldb = N;
         k.C = b.K;  k.ldc = N;
         k.alpha = 1.0;  k.beta = 0.0;
-        CD_CUDA(gemm_f64(k, false, false, ctx->stream));
+        CD_RC(gemm_run(ctx, k, false, false));
         // F_ao = H + J - K
         axpy_kernel<<<blocks_for(NN), 256, 0, ctx->stream>>>(ctx->Hcore.as<double>(), 1.0, b.J, NN, b.Fao);
         axpy_kernel<<<blocks_for(NN), 256, 0, ctx->stream>>>(b.Fao, -1.0, b.K, NN, b.Fao);
@@ -350,13 +343,13 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
         t.M = (int)N;  t.N = (int)N;  t.K = (int)N;  t.batch = 1;
         t.A = b.Fao;  t.lda = N;  t.B = C;  t.ldb = N;  t.C = b.T;  t.ldc = N;
         t.alpha = 1.0;  t.beta = 0.0;
-        CD_CUDA(gemm_f64(t, true, true, ctx->stream));
+        CD_RC(gemm_run(ctx, t, true, true));
         GemmF64Args f{};
         f.M = (int)N;  f.N = (int)N;  f.K = (int)N;  f.batch = 1;
         f.A = b.T;  f.lda = N;  f.B = C;  f.ldb = N;  f.C = b.F[s];  f.ldc = N;
         f.alpha = 1.0;  f.beta = 0.0;
-        CD_CUDA(gemm_f64(f, false, true, ctx->stream));
-        ctx->launches += 6;
+        CD_RC(gemm_run(ctx, f, false, true));
+        ctx->launches += 2;
     }
     end_stage(ctx);
     CD_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -364,11 +357,23 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     return MSHQC_CD_OK;
 }
 
+// W = c0 I + c1 A + c2 A2 + c3 A3 (N x N)
+__global__ void poly3_kernel(const double* __restrict__ A, const double* __restrict__ A2,
+                             const double* __restrict__ A3, int64_t N, double c0, double c1, double c2, double c3,
+                             double* __restrict__ W) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t < N * N) W[t] = fma(c3, A3[t], fma(c2, A2[t], fma(c1, A[t], t / N == t % N ? c0 : 0.0)));
+}
+
 // exp(A) for a real N x N matrix (row-major) of 1-norm norm1, by scaling and
-// squaring with a degree-18 Taylor polynomial in Horner form: with
-// ||A / 2^s||_1 <= 1/2 the truncation error is below 1e-22.  E and W are work
-// matrices; *result points at whichever holds exp(A).
-int expm_device(mshqc_cd_ctx* ctx, const double* A, double norm1, double* E, double* W, const double** result) {
+// squaring with the degree-19 Taylor polynomial: with ||A / 2^s||_1 <= 1/2 the
+// truncation error is below 1e-24.  The polynomial in four-term groups of
+// powers of A^4 (Paterson and Stockmeyer) takes 7 products where Horner's form
+// in A takes 19; each is a latency-bound chain of small tiles.  E, W and
+// pw (3 N^2: the powers) are work matrices; *result points at whichever of E
+// and W holds exp(A).
+int expm_device(mshqc_cd_ctx* ctx, double* A, double norm1, double* E, double* W, double* pw,
+                const double** result) {
     const int64_t N = ctx->N, NN = N * N;
     int s = 0;
     while (norm1 > 0.5 && s < 60) {
@@ -376,27 +381,33 @@ int expm_device(mshqc_cd_ctx* ctx, const double* A, double norm1, double* E, dou
         ++s;
     }
     const double scale = std::ldexp(1.0, -s);
-    identity_kernel<<<blocks_for(NN), 256, 0, ctx->stream>>>(E, N);
-    CD_CUDA(cudaGetLastError());
-    for (int k = 18; k >= 1; --k) {
-        // W = I + (scale / k) A E
-        identity_kernel<<<blocks_for(NN), 256, 0, ctx->stream>>>(W, N);
+    // Z = alpha X Y + beta Z
+    auto mul = [&](const double* X, const double* Y, double alpha, double beta, double* Z) {
         GemmF64Args g{};
         g.M = (int)N;  g.N = (int)N;  g.K = (int)N;  g.batch = 1;
-        g.A = A;  g.lda = N;  g.B = E;  g.ldb = N;  g.C = W;  g.ldc = N;
-        g.alpha = scale / k;  g.beta = 1.0;
-        CD_CUDA(gemm_f64(g, true, false, ctx->stream));
+        g.A = X;  g.lda = N;  g.B = Y;  g.ldb = N;  g.C = Z;  g.ldc = N;
+        g.alpha = alpha;  g.beta = beta;
+        return gemm_run(ctx, g, true, false);
+    };
+    double *A2 = pw, *A3 = pw + NN, *A4 = pw + 2 * NN;   // powers of scale * A
+    CD_RC(mul(A, A, scale * scale, 0.0, A2));
+    CD_RC(mul(A, A2, scale, 0.0, A3));
+    CD_RC(mul(A2, A2, 1.0, 0.0, A4));
+    double c[20];
+    c[0] = 1.0;
+    for (int k = 1; k < 20; ++k) c[k] = c[k - 1] / k;
+    for (int h = 4; h >= 0; --h) {
+        // W = B_h + A4 E, E the higher groups
+        poly3_kernel<<<blocks_for(NN), 256, 0, ctx->stream>>>(A, A2, A3, N, c[4 * h], c[4 * h + 1] * scale,
+                                                              c[4 * h + 2], c[4 * h + 3], W);
+        CD_CUDA(cudaGetLastError());
+        ctx->launches++;
+        if (h < 4) CD_RC(mul(A4, E, 1.0, 1.0, W));
         std::swap(E, W);
-        ctx->launches += 2;
     }
     for (int q = 0; q < s; ++q) {
-        GemmF64Args g{};
-        g.M = (int)N;  g.N = (int)N;  g.K = (int)N;  g.batch = 1;
-        g.A = E;  g.lda = N;  g.B = E;  g.ldb = N;  g.C = W;  g.ldc = N;
-        g.alpha = 1.0;  g.beta = 0.0;
-        CD_CUDA(gemm_f64(g, true, false, ctx->stream));
+        CD_RC(mul(E, E, 1.0, 0.0, W));
         std::swap(E, W);
-        ctx->launches++;
     }
     *result = E;
     return MSHQC_CD_OK;
@@ -424,22 +435,22 @@ int rotate_spin(mshqc_cd_ctx* ctx, int spin, const std::vector<double>& F_host) 
         for (int64_t r = 0; r < N; ++r) col += std::abs(A[r * N + c]);
         norm1 = std::max(norm1, col);
     }
-    CD_ALLOC(ctx->omp2_ws, sizeof(double) * (size_t)(4 * NN), false);
+    CD_ALLOC(ctx->omp2_ws, sizeof(double) * (size_t)(7 * NN), false);
     double* dA = ctx->omp2_ws.as<double>();
     double* E0 = dA + NN;
     double* E1 = E0 + NN;
     double* Cn = E1 + NN;
+    double* pw = Cn + NN;
     CD_CUDA(cudaMemcpyAsync(dA, A.data(), sizeof(double) * NN, cudaMemcpyHostToDevice, ctx->stream));
     const double* E = nullptr;
-    CD_RC(expm_device(ctx, dA, norm1, E0, E1, &E));
+    CD_RC(expm_device(ctx, dA, norm1, E0, E1, pw, &E));
     // column-major C_new = C E: as row-major arrays C_new^T = E^T C^T
     double* C = ctx->spin[spin].C.as<double>();
     GemmF64Args g{};
     g.M = (int)N;  g.N = (int)N;  g.K = (int)N;  g.batch = 1;
     g.A = E;  g.lda = N;  g.B = C;  g.ldb = N;  g.C = Cn;  g.ldc = N;
     g.alpha = 1.0;  g.beta = 0.0;
-    CD_CUDA(gemm_f64(g, false, false, ctx->stream));
-    ctx->launches++;
+    CD_RC(gemm_run(ctx, g, false, false));
     CD_CUDA(cudaMemcpyAsync(C, Cn, sizeof(double) * NN, cudaMemcpyDeviceToDevice, ctx->stream));
     return invalidate_spin(ctx, spin);
 }
@@ -489,12 +500,13 @@ __global__ void row_norm2_kernel(const double* __restrict__ L, int64_t n, double
 }
 
 // Z^q = 0 for the vectors whose Frobenius norm is at most `thr` (the
-// exchange screening of src/scf/cholesky_rhf.cc:120-126); norm2[q] = |L^q|^2
-__global__ void screen_slabs_kernel(double* __restrict__ Z, const double* __restrict__ norm2, int64_t nn,
-                                    double thr) {
+// exchange screening of src/scf/cholesky_rhf.cc:120-126); norm2[q] = |L^q|^2.
+// Row z of vector q: N elements at Z + q * sq + z * ldz (grid: N, vectors, rows)
+__global__ void screen_slabs_kernel(double* __restrict__ Z, const double* __restrict__ norm2, int64_t N, int64_t sq,
+                                    int64_t ldz, double thr) {
     if (norm2[blockIdx.y] > thr * thr) return;
-    double* z = Z + (int64_t)blockIdx.y * nn;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn; t += (int64_t)gridDim.x * blockDim.x)
+    double* z = Z + (int64_t)blockIdx.y * sq + (int64_t)blockIdx.z * ldz;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N; t += (int64_t)gridDim.x * blockDim.x)
         z[t] = 0.0;
 }
 
@@ -502,9 +514,10 @@ __global__ void screen_slabs_kernel(double* __restrict__ Z, const double* __rest
 //   J = sum_Q <L^Q, P_tot> L^Q,   K_s = sum_Q L^Q P_s L^Q,
 // P_tot = P[0] (nspin 1) or P[0] + P[1] (nspin 2), over chunks of vectors
 // (stored or generated): per chunk the coefficients <L^Q, P_tot> (one dot
-// product per vector), J += coef . L as one GEMM, Z^Q = P_s L^Q as one batched
-// GEMM and K_s += L . Z as one GEMM over the composite index (Q, nu).  All
-// matrices are N x N and symmetric; device pointers on the context stream.
+// product per vector) and J += coef . L, Z^Q = P_s L^Q as one batched GEMM and
+// K_s += L . Z over the composite index (Q, nu).  All matrices are N x N and
+// symmetric; device pointers on the context stream.  UHF, N = 400, M = 1600:
+// 85.9 ms before (the K product ran on 49 CTAs), 27 ms with K split.
 int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], bool screen, double* J,
                        double* const K[2], double* work) {
     const int64_t N = ctx->N, NN = N * N, M = ctx->M;
@@ -518,13 +531,15 @@ int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], b
     CD_CUDA(cudaMemsetAsync(J, 0, sizeof(double) * NN, ctx->stream));
     for (int s = 0; s < nspin; ++s) CD_CUDA(cudaMemsetAsync(K[s], 0, sizeof(double) * NN, ctx->stream));
     // vectors per chunk: the generator's chunk, and at most 2 GB of Z
+    const int64_t per_q = NN;
     const int64_t mc_max = std::max<int64_t>(
-        1, std::min<int64_t>({vectors_chunk_size(ctx), (int64_t)((size_t(2) << 30) / (sizeof(double) * NN)),
+        1, std::min<int64_t>({vectors_chunk_size(ctx), (int64_t)((size_t(2) << 30) / (sizeof(double) * per_q)),
                               (int64_t)65535}));
-    CD_ALLOC(ctx->Zt, sizeof(double) * (size_t)(mc_max * NN), false);
+    CD_ALLOC(ctx->Zt, sizeof(double) * (size_t)(mc_max * per_q), false);
     CD_ALLOC(ctx->omp2_ws, sizeof(double) * (size_t)(2 * mc_max), false);
     double* coef = ctx->omp2_ws.as<double>();
     double* norm2 = coef + mc_max;
+    double* Z = ctx->Zt.as<double>();
     for (int64_t Q0 = 0; Q0 < M; Q0 += mc_max) {
         const int64_t mc = std::min<int64_t>(mc_max, M - Q0);
         const double* Lc = nullptr;
@@ -532,40 +547,38 @@ int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], b
         dot_rows_kernel<<<(unsigned)mc, 256, 0, ctx->stream>>>(Lc, NN, Ptot, coef);
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
-        GemmF64Args g{};
-        g.M = 1;  g.N = (int)NN;  g.K = (int)mc;  g.batch = 1;
-        g.A = coef;  g.lda = mc;  g.B = Lc;  g.ldb = NN;  g.C = J;  g.ldc = NN;
-        g.alpha = 1.0;  g.beta = 1.0;
-        CD_CUDA(gemm_f64(g, true, false, ctx->stream));
-        ctx->launches++;
+        CD_RC(coulomb(ctx, Lc, NN, mc, coef, 1.0, J));
         if (screen) {
             row_norm2_kernel<<<(unsigned)mc, 256, 0, ctx->stream>>>(Lc, NN, norm2);
             CD_CUDA(cudaGetLastError());
             ctx->launches++;
         }
-        for (int s = 0; s < nspin; ++s) {
+        // Z (rows x [Q][N], row stride ldz between factor rows or N): A_rows L^Q per vector
+        auto left_product = [&](const double* A, int64_t rows, int64_t ldz, int64_t sz) -> int {
             GemmF64Args z{};
-            z.M = (int)N;  z.N = (int)N;  z.K = (int)N;  z.batch = (int)mc;
-            z.A = P[s];  z.lda = N;  z.sA = 0;
+            z.M = (int)rows;  z.N = (int)N;  z.K = (int)N;  z.batch = (int)mc;
+            z.A = A;  z.lda = N;  z.sA = 0;
             z.B = Lc;  z.ldb = N;  z.sB = NN;
-            z.C = ctx->Zt.as<double>();  z.ldc = N;  z.sC = NN;
+            z.C = Z;  z.ldc = ldz;  z.sC = sz;
             z.alpha = 1.0;  z.beta = 0.0;
-            CD_CUDA(gemm_f64(z, true, false, ctx->stream));
-            ctx->launches++;
+            CD_RC(gemm_run(ctx, z, true, false));
             if (screen) {
-                dim3 grid((unsigned)std::min<int64_t>(cdiv(NN, 256), 1024), (unsigned)mc);
-                screen_slabs_kernel<<<grid, 256, 0, ctx->stream>>>(ctx->Zt.as<double>(), norm2, NN, 1e-8);
+                dim3 grid((unsigned)std::min<int64_t>(cdiv(N, 256), 1024), (unsigned)mc, (unsigned)rows);
+                screen_slabs_kernel<<<grid, 256, 0, ctx->stream>>>(Z, norm2, N, sz, ldz, 1e-8);
                 CD_CUDA(cudaGetLastError());
                 ctx->launches++;
             }
+            return MSHQC_CD_OK;
+        };
+        for (int s = 0; s < nspin; ++s) {
+            CD_RC(left_product(P[s], N, N, NN));
             GemmF64Args k{};
             k.M = (int)N;  k.N = (int)N;  k.K = (int)(mc * N);  k.batch = 1;
             k.A = Lc;  k.lda = N;
-            k.B = ctx->Zt.as<double>();  k.ldb = N;
+            k.B = Z;  k.ldb = N;
             k.C = K[s];  k.ldc = N;
             k.alpha = 1.0;  k.beta = 1.0;
-            CD_CUDA(gemm_f64(k, false, false, ctx->stream));
-            ctx->launches++;
+            CD_RC(gemm_run(ctx, k, false, false));
         }
     }
     return MSHQC_CD_OK;

@@ -71,8 +71,7 @@ extern "C" MSHQC_CD_API int mshqc_cd_get_t2_block(mshqc_cd_ctx* ctx, int block, 
         a.B = Y.B64.as<double>() + j0 * Y.vp * Mp;  a.ldb = Mp;  a.sB = Y.vp * Mp;
         a.C = dst + ii * nj * vx * vy;  a.ldc = vy;  a.sC = vx * vy;
         a.alpha = 1.0;  a.beta = 0.0;
-        CD_CUDA(gemm_f64(a, true, true, ctx->stream));
-        ctx->launches++;
+        CD_RC(gemm_run(ctx, a, true, true));
     }
     const double* ex = X.eps.as<double>();
     const double* ey = Y.eps.as<double>();

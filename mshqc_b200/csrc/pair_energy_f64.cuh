@@ -256,19 +256,22 @@ static __global__ void reduce_pairs_kernel(const double* __restrict__ partial, i
 }
 
 // ... and of per-pair sums into one total (single CTA of 256 threads, fixed
-// order: strided per-thread sums, then a fixed tree).
+// order: strided per-thread sums, a tree in each warp, the 8 warps in order).
 static __global__ void reduce_total_kernel(const double* __restrict__ x, int n, double* __restrict__ out) {
-    __shared__ double ss[256], sc[256];
+    __shared__ double ss[8], sc[8];
     KSum s;
     s.init();
     for (int k = threadIdx.x; k < n; k += 256) s.add(x[k]);
-    ss[threadIdx.x] = s.s;
-    sc[threadIdx.x] = s.c;
+    warp_reduce_ksum(s);
+    if ((threadIdx.x & 31) == 0) {
+        ss[threadIdx.x >> 5] = s.s;
+        sc[threadIdx.x >> 5] = s.c;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         KSum t;
         t.init();
-        for (int k = 0; k < 256; ++k) {
+        for (int k = 0; k < 8; ++k) {
             t.add(ss[k]);
             t.c += sc[k];
         }
