@@ -105,7 +105,8 @@ struct mshqc_cd_ctx {
     bool H_set = false;
     mshqc_cd::DevBuf opdm;          // OMP2: OPDM blocks, densities, Fock matrices
     mshqc_cd::DevBuf omp2_ws;       // OMP2: split-K partials, rotation work matrices
-    mshqc_cd::DevBuf Zt;            // Fock builds: P L^Q of a chunk of vectors
+    mshqc_cd::DevBuf Zt;            // Fock builds: P L^Q (or the factored density's L^Q X) of a chunk of vectors
+    mshqc_cd::DevBuf dens_x;        // Fock builds: Cholesky factors of the densities
     mshqc_cd::DevBuf oz_a, oz_b;    // int8 slices of the transform operands (orbitals, vectors)
     mshqc_cd::DevBuf oz_ea, oz_eb;  // their row exponents
     mshqc_cd::DevBuf oz_flag;       // int8-slice product error flag
@@ -142,7 +143,7 @@ struct mshqc_cd_ctx {
         for (const auto& s : spin)
             b += s.C.bytes + s.eps.bytes + s.B64.bytes + s.Bhi.bytes + s.Blo.bytes + s.expo.bytes +
                  s.diag.bytes + s.norms.bytes;
-        b += gemm_ws.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
+        b += gemm_ws.bytes + dens_x.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
         for (const auto& g : gam) b += g.bytes;
         for (const auto& g : grad) b += g.bytes;
         return b;
@@ -187,6 +188,7 @@ struct mshqc_cd_ctx {
         opdm.release();
         omp2_ws.release();
         Zt.release();
+        dens_x.release();
         oz_a.release();
         oz_b.release();
         oz_ea.release();

@@ -510,14 +510,168 @@ __global__ void screen_slabs_kernel(double* __restrict__ Z, const double* __rest
         z[t] = 0.0;
 }
 
+// Pivoted Cholesky factor of a density matrix P (N x N) for the exchange
+// build: X[k][n], k < rank, with P ~ sum_k X[k] X[k]^T.  One CTA; step k takes
+// the largest remaining diagonal, forms the column left-looking (thread per
+// row, X[k] contiguous in n) and updates the diagonal.  Stops when the largest
+// remaining diagonal is at rounding level of the first one, or after rmax
+// vectors.  Latency bound: about 3 us a step at N = 400.  D is N doubles of
+// work; out: [0] rank.
+__global__ void __launch_bounds__(1024) density_factor_kernel(const double* __restrict__ P, int64_t N, int rmax,
+                                                              double* __restrict__ X, double* __restrict__ D,
+                                                              int* __restrict__ rank) {
+    __shared__ double sv[32];
+    __shared__ int si[32];
+    __shared__ double best_v;
+    __shared__ int best_i;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int64_t n = tid; n < N; n += 1024) D[n] = P[n * N + n];
+    double first = 0.0;
+    int k = 0;
+    for (; k < rmax; ++k) {
+        __syncthreads();
+        double v = -1.0;
+        int idx = 0;
+        for (int64_t n = tid; n < N; n += 1024)
+            if (D[n] > v) {
+                v = D[n];
+                idx = (int)n;
+            }
+#pragma unroll
+        for (int off = 16; off; off >>= 1) {
+            const double ov = __shfl_xor_sync(0xffffffffu, v, off);
+            const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
+            if (ov > v || (ov == v && oi < idx)) {
+                v = ov;
+                idx = oi;
+            }
+        }
+        if (lane == 0) {
+            sv[warp] = v;
+            si[warp] = idx;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < 32; ++w)
+                if (sv[w] > v || (sv[w] == v && si[w] < idx)) {
+                    v = sv[w];
+                    idx = si[w];
+                }
+            best_v = v;
+            best_i = idx;
+        }
+        __syncthreads();
+        const double dp = best_v;
+        const int64_t p = best_i;
+        if (k == 0) first = dp;
+        if (!(dp > 0x1p-50 * first)) break;
+        const double inv = 1.0 / sqrt(dp);
+        for (int64_t n = tid; n < N; n += 1024) {
+            double a0 = P[p * N + n], a1 = 0.0, a2 = 0.0, a3 = 0.0;
+            int h = 0;
+            for (; h + 4 <= k; h += 4) {
+                const double* x = X + (int64_t)h * N;
+                a0 = fma(-x[n], x[p], a0);
+                a1 = fma(-x[N + n], x[N + p], a1);
+                a2 = fma(-x[2 * N + n], x[2 * N + p], a2);
+                a3 = fma(-x[3 * N + n], x[3 * N + p], a3);
+            }
+            for (; h < k; ++h) a0 = fma(-X[(int64_t)h * N + n], X[(int64_t)h * N + p], a0);
+            const double x = ((a0 + a1) + (a2 + a3)) * inv;
+            X[(int64_t)k * N + n] = x;
+            D[n] = n == p ? 0.0 : fma(-x, x, D[n]);
+        }
+    }
+    if (tid == 0) *rank = k;
+}
+
+// bits[0] = max |P|, bits[1] = max |P - sum_k X[k] X[k]^T| (bit patterns of
+// non-negative doubles order like unsigned integers; NaN ends up largest)
+__global__ void __launch_bounds__(256) density_residual_kernel(const double* __restrict__ P, int64_t N,
+                                                               const double* __restrict__ X,
+                                                               const int* __restrict__ rank,
+                                                               unsigned long long* __restrict__ bits) {
+    const int r = *rank;
+    unsigned long long mp = 0, mr = 0;
+    for (int64_t t = blockIdx.x * 256LL + threadIdx.x; t < N * N; t += (int64_t)gridDim.x * 256) {
+        const int64_t i = t / N, j = t % N;
+        double d = P[t];
+        mp = max(mp, (unsigned long long)__double_as_longlong(fabs(d)));
+        for (int k = 0; k < r; ++k) d = fma(-X[(int64_t)k * N + i], X[(int64_t)k * N + j], d);
+        mr = max(mr, (unsigned long long)__double_as_longlong(fabs(d)));
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) {
+        mp = max(mp, __shfl_xor_sync(0xffffffffu, mp, off));
+        mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, off));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(bits, mp);
+        atomicMax(bits + 1, mr);
+    }
+}
+
+// Factors of the densities of an exchange build in ctx->dens_x (X[s] there,
+// rank[s] vectors each, the two spins' one after the other), or rank[s] = 0
+// where P[s] is not represented by at most N / 4 vectors to rounding: max |P - X^T X| <= (4 + r / 8) 2^-52 max |P|,
+// checked on every element (so an indefinite or unsymmetric P is refused too).
+// The exchange then takes 4 M N^2 r operations instead of 4 M N^3.
+constexpr int64_t kDensityFactorMinN = 96;   // below, the full products are as fast as finding the factors
+int density_factors(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], const double* X[2], int rank[2]) {
+    const int64_t N = ctx->N;
+    const int rmax = (int)(N / 4);
+    rank[0] = rank[1] = 0;
+    X[0] = X[1] = nullptr;
+    if (N < kDensityFactorMinN) return MSHQC_CD_OK;
+    CD_ALLOC(ctx->dens_x, sizeof(double) * (size_t)((2 * (rmax + 1) + rmax) * N + 8), false);
+    double* base = ctx->dens_x.as<double>();
+    unsigned long long* tail = reinterpret_cast<unsigned long long*>(base + 2 * (rmax + 1) * N);   // [spin][P, R, rank]
+    CD_CUDA(cudaMemsetAsync(tail, 0, 6 * sizeof(unsigned long long), ctx->stream));
+    for (int s = 0; s < nspin; ++s) {
+        double* x = base + (int64_t)s * (rmax + 1) * N;
+        int* rk = reinterpret_cast<int*>(tail + 3 * s + 2);
+        density_factor_kernel<<<1, 1024, 0, ctx->stream>>>(P[s], N, rmax, x, x + (int64_t)rmax * N, rk);
+        CD_CUDA(cudaGetLastError());
+        density_residual_kernel<<<(unsigned)std::min<int64_t>(cdiv(N * N, 256), 8LL * ctx->num_sms), 256, 0,
+                                  ctx->stream>>>(P[s], N, x, rk, tail + 3 * s);
+        CD_CUDA(cudaGetLastError());
+        ctx->launches += 2;
+        X[s] = x;
+    }
+    unsigned long long h[6];
+    CD_CUDA(cudaMemcpyAsync(h, tail, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    CD_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int s = 0; s < nspin; ++s) {
+        double mp, mr;
+        std::memcpy(&mp, &h[3 * s], sizeof(double));
+        std::memcpy(&mr, &h[3 * s + 1], sizeof(double));
+        const int r = (int)(h[3 * s + 2] & 0xffffffffull);
+        if (r > 0 && mr <= (4.0 + r / 8.0) * 0x1p-52 * mp) rank[s] = r;
+    }
+    if (rank[0] > 0 && rank[1] > 0) {
+        // the second spin's rows right after the first's (never overlapping: rank <= N / 4)
+        double* x1 = base + rank[0] * N;
+        CD_CUDA(cudaMemcpyAsync(ctx->dens_x.as<double>() + 2 * (rmax + 1) * N + 8, X[1],
+                                sizeof(double) * (size_t)(rank[1] * N), cudaMemcpyDeviceToDevice, ctx->stream));
+        CD_CUDA(cudaMemcpyAsync(x1, ctx->dens_x.as<double>() + 2 * (rmax + 1) * N + 8,
+                                sizeof(double) * (size_t)(rank[1] * N), cudaMemcpyDeviceToDevice, ctx->stream));
+        X[1] = x1;
+    }
+    return MSHQC_CD_OK;
+}
+
 // Cholesky Coulomb and exchange matrices of the SCF Fock builds,
 //   J = sum_Q <L^Q, P_tot> L^Q,   K_s = sum_Q L^Q P_s L^Q,
 // P_tot = P[0] (nspin 1) or P[0] + P[1] (nspin 2), over chunks of vectors
 // (stored or generated): per chunk the coefficients <L^Q, P_tot> (one dot
-// product per vector) and J += coef . L, Z^Q = P_s L^Q as one batched GEMM and
+// product per vector) and J += coef . L.  Exchange of a density of low rank
+// (an SCF density has the rank of its occupied orbitals): V_k^Q = L^Q X_k and
+// K_s += V V^T over the composite index (k, Q), of which the tiles on and above
+// the diagonal are computed; otherwise Z^Q = P_s L^Q as one batched GEMM and
 // K_s += L . Z over the composite index (Q, nu).  All matrices are N x N and
-// symmetric; device pointers on the context stream.  UHF, N = 400, M = 1600:
-// 85.9 ms before (the K product ran on 49 CTAs), 27 ms with K split.
+// symmetric; device pointers on the context stream.  UHF, N = 400, M = 1600,
+// 40 and 38 electrons: 85.9 ms before (the K product ran on 49 CTAs), 27 ms
+// with the full products and K split, 4 ms with the factors.
 int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], bool screen, double* J,
                        double* const K[2], double* work) {
     const int64_t N = ctx->N, NN = N * N, M = ctx->M;
@@ -528,10 +682,18 @@ int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], b
         ctx->launches++;
         Ptot = work;
     }
+    const double* X[2];
+    int rank[2];
+    CD_RC(density_factors(ctx, nspin, P, X, rank));
     CD_CUDA(cudaMemsetAsync(J, 0, sizeof(double) * NN, ctx->stream));
     for (int s = 0; s < nspin; ++s) CD_CUDA(cudaMemsetAsync(K[s], 0, sizeof(double) * NN, ctx->stream));
-    // vectors per chunk: the generator's chunk, and at most 2 GB of Z
-    const int64_t per_q = NN;
+    // factored spins first: their V in one product over all factor rows
+    const int rtot = rank[0] + rank[1];
+    const double* Xall = rank[0] > 0 ? X[0] : X[1];
+    bool dense = false;
+    for (int s = 0; s < nspin; ++s) dense = dense || rank[s] == 0;
+    // vectors per chunk: the generator's chunk, and at most 2 GB of Z (or V)
+    const int64_t per_q = std::max<int64_t>((int64_t)rtot * N, dense ? NN : 1);
     const int64_t mc_max = std::max<int64_t>(
         1, std::min<int64_t>({vectors_chunk_size(ctx), (int64_t)((size_t(2) << 30) / (sizeof(double) * per_q)),
                               (int64_t)65535}));
@@ -570,7 +732,24 @@ int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], b
             }
             return MSHQC_CD_OK;
         };
+        if (rtot > 0) {
+            // V[k][Q][mu]; K_s[mu][lam] += sum_{(k,Q)} V V
+            CD_RC(left_product(Xall, rtot, mc * N, N));
+            int64_t k0 = 0;
+            for (int s = 0; s < nspin; ++s) {
+                if (rank[s] == 0) continue;
+                GemmF64Args k{};
+                k.M = k.N = (int)N;  k.K = (int)(rank[s] * mc);  k.batch = 1;
+                k.A = k.B = Z + k0 * mc * N;  k.lda = k.ldb = N;
+                k.C = K[s];  k.ldc = N;
+                k.alpha = 1.0;  k.beta = 1.0;
+                k.sym = 1;
+                CD_RC(gemm_run(ctx, k, false, false));
+                k0 += rank[s];
+            }
+        }
         for (int s = 0; s < nspin; ++s) {
+            if (rank[s] > 0) continue;
             CD_RC(left_product(P[s], N, N, NN));
             GemmF64Args k{};
             k.M = (int)N;  k.N = (int)N;  k.K = (int)(mc * N);  k.batch = 1;
