@@ -55,7 +55,14 @@ enum mshqc_cd_status {
 };
 
 enum mshqc_cd_precision {
-    MSHQC_CD_FP64 = 0,    /* FP64 contractions (DMMA)                       */
+    MSHQC_CD_FP64 = 0,    /* FP64 contractions: FP64 tensor pipe (DMMA), or
+                             for larger products int8 slices with all 53 bits
+                             of each element within a binade of its row's
+                             maximum (7 x 8 bits, exact integer sums, error
+                             per term below 2^-54 of the row maxima; smaller
+                             than that of a chain of FP64 FMAs).
+                             MSHQC_CD_FP64_SLICES=off in the environment:
+                             DMMA only, =on: slices at every size           */
     MSHQC_CD_FP16X3 = 1   /* scaled FP16 x3: every MO row in fixed point with
                              one power-of-two scale, integer hi/lo carried in
                              FP16, three products per pair, exact FP32

@@ -14,6 +14,7 @@
 #include "cd_internal.h"
 #include "gemm_f64.cuh"
 #include "pair_energy_f64.cuh"
+#include "pair_energy_s.cuh"
 #include "pair_energy_tc.cuh"
 #include "split_bf16.cuh"
 #include "gamma_tc.cuh"
@@ -161,8 +162,104 @@ int run_collective(mshqc_cd_ctx* ctx, bool gather, double* buf, int64_t count) {
     return MSHQC_CD_OK;
 }
 
+// Bytes of int8 slices one product operand may hold (bounds the vectors
+// sub-chunks of the first product and the orbital batches of the second).
+constexpr size_t kSliceBytes = size_t(2) << 30;
+
+// ---------------------------------------------------------------------------
+// products of int8 slices (ozaki_i8.cuh)
+// ---------------------------------------------------------------------------
+// out[b](x, y) = alpha sum_k X(x, k) Y(y, k) + beta out at out + b cb + x ldc + y.
+// The 128-row operand is the one that pads the tiles less: X, or (sw) Y with
+// the result stored transposed.
+template <class C>
+bool oz_swap(int64_t x, int64_t y) {
+    const double straight = (double)round_up(x, ozaki::BM) * round_up(y, C::BN);
+    const double swapped = (double)round_up(y, ozaki::BM) * round_up(x, C::BN);
+    return swapped < straight;
+}
+template <class C>
+OzakiOperand oz_operand(int64_t rows, int64_t K, bool as_a, int64_t batch) {
+    return ozaki_operand(rows, K, as_a ? ozaki::BM : C::BN, (int)batch);
+}
+template <class C>
+size_t oz_bytes(const OzakiOperand& op) {
+    return ozaki::operand_bytes<C>(op.Rp, op.Kp) * (size_t)op.batch;
+}
+template <class C>
+int oz_mul(mshqc_cd_ctx* ctx, const OzakiOperand& X, bool x_shared, const OzakiOperand& Y, bool y_shared, bool sw,
+           double* out, int64_t ldc, int64_t cb, double alpha, double beta) {
+    OzakiOpts o;
+    o.a_shared = sw ? y_shared : x_shared;
+    o.b_shared = sw ? x_shared : y_shared;
+    o.trans = sw;
+    CD_CUDA(ozaki_gemm<C>(sw ? Y : X, sw ? X : Y, out, ldc, cb, alpha, beta, o, ctx->oz_flag.as<int>(), ctx->num_sms,
+                          ctx->stream));
+    ctx->launches++;
+    return MSHQC_CD_OK;
+}
+// reserves an operand's digits and exponents
+int oz_reserve(mshqc_cd_ctx* ctx, DevBuf& q, DevBuf& e, size_t bytes, OzakiOperand& op) {
+    CD_ALLOC(q, bytes, false);
+    CD_ALLOC(e, sizeof(int) * (size_t)(op.Rp * op.batch), false);
+    op.q = q.as<int8_t>();
+    op.e = e.as<int>();
+    return MSHQC_CD_OK;
+}
+int oz_check(mshqc_cd_ctx* ctx, const char* what) {
+    int herr = 0;
+    CD_CUDA(cudaMemcpyAsync(&herr, ctx->oz_flag.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CD_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (herr)
+        return set_error(MSHQC_CD_ERR_TIMEOUT,
+                         std::string(what) + " gave up waiting (site " + std::to_string(herr) + ")");
+    return MSHQC_CD_OK;
+}
+
+// Second half of the forward transform from Y [i - lo][Q][nu]:
+// B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu], a batch of orbitals i at a time
+template <class C>
+int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
+    SpinState& s = ctx->spin[spin];
+    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, ni = hi - lo, vp = s.vp;
+    const bool sw = oz_swap<C>(v, M);
+    OzakiOperand Av = oz_operand<C>(v, N, !sw, 1);
+    CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<C>(Av), Av));
+    CD_CUDA(ozaki_slice<C>(s.C.as<double>() + o * N, N, 0, Av, ctx->num_sms, ctx->stream));
+    ctx->launches++;
+    const int64_t per_i = (int64_t)oz_bytes<C>(oz_operand<C>(M, N, sw, 1));
+    const int64_t ib = std::max<int64_t>(1, std::min<int64_t>(ni, (int64_t)kSliceBytes / per_i));
+    for (int64_t i0 = lo; i0 < hi; i0 += ib) {
+        const int64_t nb = std::min(ib, hi - i0);
+        OzakiOperand By = oz_operand<C>(M, N, sw, nb);
+        CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, (size_t)(per_i * nb), By));
+        CD_CUDA(ozaki_slice<C>(ctx->Y.as<double>() + (i0 - lo) * M * N, N, M * N, By, ctx->num_sms, ctx->stream));
+        ctx->launches++;
+        CD_RC(oz_mul<C>(ctx, Av, true, By, false, sw, s.B64.as<double>() + i0 * vp * Mp, Mp, vp * Mp, 1.0, 0.0));
+    }
+    return MSHQC_CD_OK;
+}
+
+// FP64 products of at least this many operations run as int8 slices of full
+// accuracy (ozaki::Full) where each sliced element takes part in at least
+// kSlicedMinReuse multiply-adds: slicing costs about 6 ps an element (HBM),
+// the DMMA products 0.06 ps an operation, the sliced ones 0.03.
+// MSHQC_CD_FP64_SLICES=off keeps every FP64 product on the DMMA pipe, =on slices
+// at every size.
+constexpr double kSlicedMinFlops = 4e9;
+constexpr int64_t kSlicedMinReuse = 256;
+bool fp64_slices(double flops, double min_flops, int64_t reuse) {
+    if (const char* env = std::getenv("MSHQC_CD_FP64_SLICES")) {
+        if (std::strcmp(env, "off") == 0) return false;
+        if (std::strcmp(env, "on") == 0) return true;
+    }
+    return flops >= min_flops && reuse >= kSlicedMinReuse;
+}
+
 // FP64 half transform of one spin into the padded [i][a][Q] layout, for the
 // occupied orbitals [lo, hi) (Y holds rows i - lo; B rows outside stay zero).
+// The first half reads every vector once for few occupied orbitals and stays
+// on the DMMA pipe.
 int transform_f64(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
     SpinState& s = ctx->spin[spin];
     const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, ni = hi - lo;
@@ -194,6 +291,12 @@ int transform_f64(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
         g1.alpha = 1.0;  g1.beta = 0.0;
         CD_RC(gemm_run(ctx, g1, true, true));
     }
+    const char* tenv = std::getenv("MSHQC_CD_TRANSFORM");   // f64: DMMA for both halves
+    if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
+        CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
+        CD_RC(second_half_sliced<ozaki::Full>(ctx, spin, lo, hi));
+        return oz_check(ctx, "int8 tensor-core transform");
+    }
     // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu]
     GemmF64Args g2{};
     g2.M = (int)v;
@@ -208,18 +311,14 @@ int transform_f64(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
     return MSHQC_CD_OK;
 }
 
-// Bytes of int8 slices one product operand may hold (bounds the vectors
-// sub-chunks of the first product and the orbital batches of the second).
-constexpr size_t kSliceBytes = size_t(2) << 30;
-
 bool int8_transform_enabled(const mshqc_cd_ctx* ctx) {
-    if (ctx->N > ozaki::kMaxK) return false;
+    if (ctx->N > ozaki::Mixed::MAXK) return false;
     const char* env = std::getenv("MSHQC_CD_TRANSFORM");
     return !(env && std::strcmp(env, "f64") == 0);
 }
 
 // The forward half transform of a mixed request runs on the int8 tensor
-// cores from N = 512 on; below, the FP64 DMMA products are faster (forward
+// cores from N = 512 on; below, the FP64 products are faster (forward
 // transform of the gradient step, one box: N=400 1.8 ms FP64 vs 2.6 ms int8,
 // N=600 8.8 vs 7.6 ms) and their B is exact.  The transposed transforms keep
 // the int8 products at every size (N=400: 3.4 vs 6.8 ms).
@@ -233,12 +332,12 @@ bool int8_forward_enabled(const mshqc_cd_ctx* ctx) {
 }
 
 // The same half transform as transform_f64 with both products on the int8
-// tensor cores (ozaki_i8.cuh): Y = C_occ^T L per vectors chunk, then
+// tensor cores (ozaki::Mixed): Y = C_occ^T L per vectors chunk, then
 // B_i = C_vir^T Y_i^T in batches of occupied orbitals.  Accuracy of the
 // slices (about 2^-33 of the row maxima per term), not FP64 rounding: used by
 // the mixed-precision path only.
 int transform_i8(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
-    using namespace ozaki;
+    using Cfg = ozaki::Mixed;
     SpinState& s = ctx->spin[spin];
     const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, ni = hi - lo;
     const int64_t vp = round_up(v, 64);
@@ -252,20 +351,14 @@ int transform_i8(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
     s.B64_valid = true;
     s.B64_prec = MSHQC_CD_FP16X3;
     if (ni <= 0) return MSHQC_CD_OK;
-    int* err = ctx->oz_flag.as<int>();
-    const double* C = s.C.as<double>();
-    // rows of C^T: occupied orbitals of the slice (first product), virtual orbitals (second)
-    OzakiOperand Ao = ozaki_operand(ni, N, BM, 1), Av = ozaki_operand(v, N, BM, 1);
-    const size_t ao_bytes = operand_bytes(Ao.Rp, Ao.Kp);
-    CD_ALLOC(ctx->oz_a, ao_bytes + operand_bytes(Av.Rp, Av.Kp), false);
-    CD_ALLOC(ctx->oz_ea, sizeof(int) * (size_t)(Ao.Rp + Av.Rp), false);
-    Ao.q = ctx->oz_a.as<int8_t>();  Ao.e = ctx->oz_ea.as<int>();
-    Av.q = Ao.q + ao_bytes;         Av.e = Ao.e + Ao.Rp;
-    CD_CUDA(ozaki_slice(C + lo * N, N, 0, Ao, ctx->num_sms, ctx->stream));
-    CD_CUDA(ozaki_slice(C + o * N, N, 0, Av, ctx->num_sms, ctx->stream));
-    ctx->launches += 2;
-    // Y[i][(Q,nu)] = sum_mu C[mu,i] L[Q][nu*N + mu]
-    const int64_t per_q = (int64_t)operand_bytes(padded_rows(N, BN), padded_k(N));
+    // Y[i][(Q,nu)] = sum_mu C[mu,i] L[Q][nu*N + mu]: rows of C^T (the occupied
+    // orbitals of the slice) against the vectors' rows
+    const bool sw = round_up(ni, Cfg::BN) < round_up(ni, ozaki::BM);
+    OzakiOperand Ao = oz_operand<Cfg>(ni, N, !sw, 1);
+    CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(Ao), Ao));
+    CD_CUDA(ozaki_slice<Cfg>(s.C.as<double>() + lo * N, N, 0, Ao, ctx->num_sms, ctx->stream));
+    ctx->launches++;
+    const int64_t per_q = (int64_t)ozaki::operand_bytes<Cfg>(round_up(N, ozaki::BM), ozaki::padded_k(N));
     const int64_t qs = std::max<int64_t>(1, (int64_t)kSliceBytes / per_q);
     const int64_t qc = vectors_chunk_size(ctx);
     for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
@@ -274,36 +367,67 @@ int transform_i8(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
         CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
         for (int64_t q0 = 0; q0 < mc; q0 += qs) {
             const int64_t ms = std::min(qs, mc - q0);
-            OzakiOperand Bl = ozaki_operand(ms * N, N, BN, 1);
-            CD_ALLOC(ctx->oz_b, operand_bytes(Bl.Rp, Bl.Kp), false);
-            CD_ALLOC(ctx->oz_eb, sizeof(int) * (size_t)Bl.Rp, false);
-            Bl.q = ctx->oz_b.as<int8_t>();  Bl.e = ctx->oz_eb.as<int>();
-            CD_CUDA(ozaki_slice(Lc + q0 * N * N, N, 0, Bl, ctx->num_sms, ctx->stream));
-            CD_CUDA(ozaki_gemm(Ao, true, Bl, false, ctx->Y.as<double>() + (Q0 + q0) * N, M * N, 0, 1.0, 0.0, err,
-                               ctx->num_sms, ctx->stream));
-            ctx->launches += 2;
+            OzakiOperand Bl = oz_operand<Cfg>(ms * N, N, sw, 1);
+            CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Bl), Bl));
+            CD_CUDA(ozaki_slice<Cfg>(Lc + q0 * N * N, N, 0, Bl, ctx->num_sms, ctx->stream));
+            ctx->launches++;
+            CD_RC(oz_mul<Cfg>(ctx, Ao, true, Bl, false, sw, ctx->Y.as<double>() + (Q0 + q0) * N, M * N, 0, 1.0, 0.0));
         }
     }
-    // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu], a batch of orbitals i at a time
-    const int64_t per_i = (int64_t)operand_bytes(padded_rows(M, BN), padded_k(N));
-    const int64_t ib = std::max<int64_t>(1, std::min<int64_t>(ni, (int64_t)kSliceBytes / per_i));
-    for (int64_t i0 = lo; i0 < hi; i0 += ib) {
-        const int64_t nb = std::min(ib, hi - i0);
-        OzakiOperand By = ozaki_operand(M, N, BN, (int)nb);
-        CD_ALLOC(ctx->oz_b, operand_bytes(By.Rp, By.Kp) * (size_t)nb, false);
-        CD_ALLOC(ctx->oz_eb, sizeof(int) * (size_t)(By.Rp * nb), false);
-        By.q = ctx->oz_b.as<int8_t>();  By.e = ctx->oz_eb.as<int>();
-        CD_CUDA(ozaki_slice(ctx->Y.as<double>() + (i0 - lo) * M * N, N, M * N, By, ctx->num_sms, ctx->stream));
-        CD_CUDA(ozaki_gemm(Av, true, By, false, s.B64.as<double>() + i0 * vp * Mp, Mp, vp * Mp, 1.0, 0.0, err,
-                           ctx->num_sms, ctx->stream));
-        ctx->launches += 2;
+    CD_RC(second_half_sliced<Cfg>(ctx, spin, lo, hi));
+    return oz_check(ctx, "int8 tensor-core transform");
+}
+
+// Whether the FP64 integral and Gamma products of blocks of `rows` x `cols`
+// composite virtual rows run as int8 slices of full accuracy.  N = 161 (17
+// occupied): the products 0.19 ms each against 0.16 (half of the tiles) and
+// 0.31 ms DMMA, but the slicing passes take what is gained; from twice that
+// work on the slices win.
+constexpr double kSlicedPairFlops = 1.6e10;
+bool sliced_pairs(const mshqc_cd_ctx* ctx, int64_t rows, int64_t cols) {
+    return fp64_slices(2.0 * rows * cols * ctx->Mp, kSlicedPairFlops, ctx->Mp);
+}
+
+// S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q] of a block pair from int8
+// slices (row length of S: nJ vpy); tri: column orbitals j >= i only
+int sliced_integrals(mshqc_cd_ctx* ctx, const SpinState& X, const SpinState& Y, int64_t I0, int64_t nI, int64_t J0,
+                     int64_t nJ, bool tri, double* S) {
+    using Cfg = ozaki::Full;
+    const int64_t Mp = ctx->Mp;
+    OzakiOperand A = oz_operand<Cfg>(nI * X.vp, Mp, true, 1), B = oz_operand<Cfg>(nJ * Y.vp, Mp, false, 1);
+    CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(A), A));
+    CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(B), B));
+    CD_CUDA(ozaki_slice<Cfg>(X.B64.as<double>() + I0 * X.vp * Mp, Mp, 0, A, ctx->num_sms, ctx->stream));
+    CD_CUDA(ozaki_slice<Cfg>(Y.B64.as<double>() + J0 * Y.vp * Mp, Mp, 0, B, ctx->num_sms, ctx->stream));
+    OzakiOpts o;
+    o.tri = tri ? (int)X.vp : 0;
+    CD_CUDA(ozaki_gemm<Cfg>(A, B, S, nJ * Y.vp, 0, 1.0, 0.0, o, ctx->oz_flag.as<int>(), ctx->num_sms, ctx->stream));
+    ctx->launches += 3;
+    return MSHQC_CD_OK;
+}
+
+// gamma[r][Q] += sum_k A(r, k) B[k][Q] over `rows` amplitude rows and K columns
+// (transposed: A(r, k) = A[k * lda + r]); the amplitudes' slices go to `work`
+int sliced_gamma(mshqc_cd_ctx* ctx, const double* A, int64_t lda, bool transposed, int64_t rows, int64_t K,
+                 const double* B, double* gamma, DevBuf& work) {
+    using Cfg = ozaki::Full;
+    const int64_t Mp = ctx->Mp;
+    OzakiOperand Ta = oz_operand<Cfg>(rows, K, true, 1), Tb = oz_operand<Cfg>(Mp, K, false, 1);
+    CD_RC(oz_reserve(ctx, work, ctx->oz_ea, oz_bytes<Cfg>(Ta), Ta));
+    CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Tb), Tb));
+    if (transposed)
+        CD_CUDA(ozaki_slice_t<Cfg>(A, lda, 0, Ta, ctx->stream));
+    else
+        CD_CUDA(ozaki_slice<Cfg>(A, lda, 0, Ta, ctx->num_sms, ctx->stream));
+    CD_CUDA(ozaki_slice_t<Cfg>(B, Mp, 0, Tb, ctx->stream));
+    OzakiOpts o;
+    if (K > 4096) {
+        // long K: CTAs that share operand slabs are kept together
+        CD_ALLOC(ctx->pace, sizeof(int) * (size_t)ctx->num_sms, false);
+        o.pace = ctx->pace.as<int>();
     }
-    int herr = 0;
-    CD_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (herr)
-        return set_error(MSHQC_CD_ERR_TIMEOUT, "int8 tensor-core transform gave up waiting (site " +
-                                                   std::to_string(herr) + ")");
+    CD_CUDA(ozaki_gemm<Cfg>(Ta, Tb, gamma, Mp, 0, 1.0, 1.0, o, ctx->oz_flag.as<int>(), ctx->num_sms, ctx->stream));
+    ctx->launches += transposed ? 5 : 4;
     return MSHQC_CD_OK;
 }
 
@@ -371,6 +495,10 @@ int reduce_and_collect(mshqc_cd_ctx* ctx, int mode, const UnitTables& t, int64_t
     return MSHQC_CD_OK;
 }
 
+template <int MODE>
+int pair_pass_f64_staged(mshqc_cd_ctx* ctx, int sx, int sy, double* total, std::vector<double>& pair_mat,
+                         double* total_os);
+
 // One FP64 pair-energy pass.  Returns the total in *total and fills the
 // ordered pair-energy matrix (row-major ox*oy) in pair_mat.
 int pair_pass_f64(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
@@ -380,6 +508,11 @@ int pair_pass_f64(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     const int ox = (int)X.nocc, oy = (int)Y.nocc;
     const int vx = (int)(ctx->N - ox), vy = (int)(ctx->N - oy);
     const int nbx = (int)(X.vp / 64), nby = (int)(Y.vp / 64);
+    if (sliced_pairs(ctx, ox * X.vp, oy * Y.vp)) {
+        if (mode == PAIR_RESTRICTED) return pair_pass_f64_staged<PAIR_RESTRICTED>(ctx, sx, sy, total, pair_mat, total_os);
+        if (mode == PAIR_SAME_SPIN) return pair_pass_f64_staged<PAIR_SAME_SPIN>(ctx, sx, sy, total, pair_mat, total_os);
+        return pair_pass_f64_staged<PAIR_OPPOSITE_SPIN>(ctx, sx, sy, total, pair_mat, total_os);
+    }
     UnitTables t = make_tables(mode, ox, oy, nbx, nby);
     const int npairs = (int)t.pairs.size(), nblocks = (int)t.blocks.size();
     pair_mat.assign((size_t)ox * oy, 0.0);
@@ -434,6 +567,63 @@ int pair_pass_f64(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     return MSHQC_CD_OK;
 }
 
+
+// The FP64 pair-energy pass of larger systems: integrals of block pairs into a
+// staging block (int8 slices of full accuracy), energies from there.
+template <int MODE>
+int pair_pass_f64_staged(mshqc_cd_ctx* ctx, int sx, int sy, double* total, std::vector<double>& pair_mat,
+                         double* total_os) {
+    constexpr bool kSym = MODE != PAIR_OPPOSITE_SPIN;
+    const SpinState& X = ctx->spin[sx];
+    const SpinState& Y = ctx->spin[sy];
+    const int64_t ox = X.nocc, oy = Y.nocc;
+    UnitTables t = make_tables(MODE, (int)ox, (int)oy, 0, 0);
+    const int npairs = (int)t.pairs.size();
+    pair_mat.assign((size_t)(ox * oy), 0.0);
+    *total = 0.0;
+    if (npairs == 0) return MSHQC_CD_OK;
+    size_t free_b = 0, total_b = 0;
+    CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t budget = std::min<size_t>((free_b + ctx->W.bytes) / 3, size_t(40) << 30);
+    const int64_t per_row = (int64_t)sizeof(double) * X.vp * Y.vp;   // per (i, j)
+    const int64_t bI = kSym ? std::max<int64_t>(1, std::min<int64_t>(ox, (int64_t)std::sqrt((double)budget / per_row)))
+                            : std::max<int64_t>(1, std::min<int64_t>(ox, (int64_t)(budget / (per_row * oy))));
+    const int64_t bJ = kSym ? bI : oy;
+    // 4 CTAs a pair where the pairs alone do not fill the GPU several times
+    const int nch = npairs < 32 * ctx->num_sms ? 4 : 1;
+    const int64_t units = (int64_t)npairs * nch;
+    CD_ALLOC(ctx->W, (size_t)(bI * bJ * per_row), false);
+    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)units * 2, false);
+    CD_ALLOC(ctx->pair_sum, sizeof(double) * (size_t)npairs * 2, false);
+    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
+    CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
+    begin_stage(ctx, ST_PAIR);
+    for (int64_t I0 = 0; I0 < ox; I0 += bI) {
+        const int64_t nI = std::min(bI, ox - I0);
+        for (int64_t J0 = kSym ? I0 : 0; J0 < oy; J0 += bJ) {
+            const int64_t nJ = std::min(bJ, oy - J0);
+            CD_RC(sliced_integrals(ctx, X, Y, I0, nI, J0, nJ, kSym && I0 == J0, ctx->W.as<double>()));
+            PairStagedArgs p{};
+            p.S = ctx->W.as<double>();
+            p.ldS = nJ * Y.vp;
+            p.vpx = (int)X.vp;  p.vpy = (int)Y.vp;
+            p.vx = (int)(ctx->N - ox);  p.vy = (int)(ctx->N - oy);
+            p.ox = (int)ox;  p.oy = (int)oy;
+            p.i0 = (int)I0;  p.nbi = (int)nI;  p.j0 = (int)J0;  p.nbj = (int)nJ;
+            p.nchunk = nch;
+            p.eox = X.eps.as<double>();  p.evx = p.eox + ox;
+            p.eoy = Y.eps.as<double>();  p.evy = p.eoy + oy;
+            p.partial = ctx->partial.as<double>();
+            p.partial2 = p.partial + units;
+            pair_energy_staged_kernel<MODE><<<(unsigned)(nI * nJ * nch), 256, 0, ctx->stream>>>(p);
+            CD_CUDA(cudaGetLastError());
+            ctx->launches++;
+        }
+    }
+    end_stage(ctx);
+    CD_RC(reduce_and_collect(ctx, MODE, t, units, npairs, nch, (int)ox, (int)oy, total, pair_mat, total_os));
+    return oz_check(ctx, "int8 tensor-core pair integrals");
+}
 
 // ---------------------------------------------------------------------------
 // FP16x3 tensor-core path
@@ -821,7 +1011,7 @@ int sum_batches(mshqc_cd_ctx* ctx, const double* parts, int nb, int64_t n, doubl
 //   dC[mu, i]   = scale sum_Q (W_Q L_Q)[i][mu]             batches of Q per vectors chunk
 // with W_Q[i][nu] = W[i][Q][nu] and L_Q[mu][nu] = L[Q][nu][mu].
 int transposed_transforms_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
-    using namespace ozaki;
+    using Cfg = ozaki::Mixed;
     SpinState& s = ctx->spin[spin];
     const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o;
     int64_t lo = 0, hi = o;
@@ -833,94 +1023,75 @@ int transposed_transforms_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* 
     const double* Gm = ctx->gam[spin].as<double>();
     double* Y = ctx->Y.as<double>();
     CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
-    int* err = ctx->oz_flag.as<int>();
-    // dC[nu, o+a]: A = Gamma_i (rows a, K = Q), B = Y_i^T (rows nu, K = Q, strided by N)
+    // dC[nu, o+a]: Gamma_i (rows a, K = Q) against Y_i^T (rows nu, K = Q, strided by N)
     {
-        const size_t pa = operand_bytes(padded_rows(v, BM), padded_k(M));
-        const size_t pb = operand_bytes(padded_rows(N, BN), padded_k(M));
+        const bool sw = oz_swap<Cfg>(v, N);
+        const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(v, M, !sw, 1));
+        const size_t pb = oz_bytes<Cfg>(oz_operand<Cfg>(N, M, sw, 1));
         const size_t pp = sizeof(double) * (size_t)(v * N);
         const int64_t ib = std::max<int64_t>(1, std::min<int64_t>(ni, (int64_t)(2 * kSliceBytes / (pa + pb + pp))));
-        CD_ALLOC(ctx->oz_a, pa * ib, false);
-        CD_ALLOC(ctx->oz_b, pb * ib, false);
         CD_ALLOC(ctx->oz_p, pp * ib, false);
-        CD_ALLOC(ctx->oz_ea, sizeof(int) * (size_t)(padded_rows(v, BM) * ib), false);
-        CD_ALLOC(ctx->oz_eb, sizeof(int) * (size_t)(padded_rows(N, BN) * ib), false);
         for (int64_t i0 = lo; i0 < hi; i0 += ib) {
             const int64_t nb = std::min(ib, hi - i0);
-            OzakiOperand A = ozaki_operand(v, M, BM, (int)nb), B = ozaki_operand(N, M, BN, (int)nb);
-            A.q = ctx->oz_a.as<int8_t>();  A.e = ctx->oz_ea.as<int>();
-            B.q = ctx->oz_b.as<int8_t>();  B.e = ctx->oz_eb.as<int>();
-            CD_CUDA(ozaki_slice(Gm + i0 * vp * Mp, Mp, vp * Mp, A, ctx->num_sms, ctx->stream));
-            CD_CUDA(ozaki_slice_t(Y + (i0 - lo) * M * N, N, M * N, B, ctx->stream));
-            CD_CUDA(ozaki_gemm(A, false, B, false, ctx->oz_p.as<double>(), N, v * N, 1.0, 0.0, err, ctx->num_sms,
-                               ctx->stream));
-            ctx->launches += 5;
+            OzakiOperand A = oz_operand<Cfg>(v, M, !sw, nb), B = oz_operand<Cfg>(N, M, sw, nb);
+            CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+            CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
+            CD_CUDA(ozaki_slice<Cfg>(Gm + i0 * vp * Mp, Mp, vp * Mp, A, ctx->num_sms, ctx->stream));
+            CD_CUDA(ozaki_slice_t<Cfg>(Y + (i0 - lo) * M * N, N, M * N, B, ctx->stream));
+            ctx->launches += 3;
+            CD_RC(oz_mul<Cfg>(ctx, A, false, B, false, sw, ctx->oz_p.as<double>(), N, v * N, 1.0, 0.0));
             CD_RC(sum_batches(ctx, ctx->oz_p.as<double>(), (int)nb, v * N, scale, i0 > lo, dC + o * N));
         }
     }
-    // W[i][Q][nu] into the Y buffer: A = Gamma_i^T (rows Q, K = a, strided by Mp),
-    // B = C_vir^T (rows nu, K = a, strided by N), shared
+    // W[i][Q][nu] into the Y buffer: Gamma_i^T (rows Q, K = a, strided by Mp)
+    // against C_vir^T (rows nu, K = a, strided by N), shared
     {
-        OzakiOperand B = ozaki_operand(N, v, BN, 1);
-        const size_t pa = operand_bytes(padded_rows(M, BM), padded_k(v));
+        const bool sw = oz_swap<Cfg>(M, N);
+        const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(M, v, !sw, 1));
         const int64_t ib = std::max<int64_t>(1, std::min<int64_t>(ni, (int64_t)(kSliceBytes / pa)));
-        CD_ALLOC(ctx->oz_a, pa * ib, false);
-        CD_ALLOC(ctx->oz_ea, sizeof(int) * (size_t)(padded_rows(M, BM) * ib), false);
-        CD_ALLOC(ctx->oz_b, operand_bytes(B.Rp, B.Kp), false);
-        CD_ALLOC(ctx->oz_eb, sizeof(int) * (size_t)B.Rp, false);
-        B.q = ctx->oz_b.as<int8_t>();  B.e = ctx->oz_eb.as<int>();
-        CD_CUDA(ozaki_slice_t(C + o * N, N, 0, B, ctx->stream));
-        ctx->launches += 3;
+        OzakiOperand B = oz_operand<Cfg>(N, v, sw, 1);
+        CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(B), B));
+        CD_CUDA(ozaki_slice_t<Cfg>(C + o * N, N, 0, B, ctx->stream));
+        ctx->launches += 2;
         for (int64_t i0 = lo; i0 < hi; i0 += ib) {
             const int64_t nb = std::min(ib, hi - i0);
-            OzakiOperand A = ozaki_operand(M, v, BM, (int)nb);
-            A.q = ctx->oz_a.as<int8_t>();  A.e = ctx->oz_ea.as<int>();
-            CD_CUDA(ozaki_slice_t(Gm + i0 * vp * Mp, Mp, vp * Mp, A, ctx->stream));
-            CD_CUDA(ozaki_gemm(A, false, B, true, Y + (i0 - lo) * M * N, N, M * N, 1.0, 0.0, err, ctx->num_sms,
-                               ctx->stream));
-            ctx->launches += 4;
+            OzakiOperand A = oz_operand<Cfg>(M, v, !sw, nb);
+            CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+            CD_CUDA(ozaki_slice_t<Cfg>(Gm + i0 * vp * Mp, Mp, vp * Mp, A, ctx->stream));
+            ctx->launches += 2;
+            CD_RC(oz_mul<Cfg>(ctx, A, false, B, true, sw, Y + (i0 - lo) * M * N, N, M * N, 1.0, 0.0));
         }
         ctx->Y_spin = -1;
     }
-    // dC[mu, i]: A = W_Q (rows i, K = nu), B = L_Q (rows mu, K = nu, strided by N)
+    // dC[mu, i]: W_Q (rows i, K = nu) against L_Q (rows mu, K = nu, strided by N)
     {
-        const size_t pa = operand_bytes(padded_rows(ni, BM), padded_k(N));
-        const size_t pb = operand_bytes(padded_rows(N, BN), padded_k(N));
+        const bool sw = oz_swap<Cfg>(ni, N);
+        const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(ni, N, !sw, 1));
+        const size_t pb = oz_bytes<Cfg>(oz_operand<Cfg>(N, N, sw, 1));
         const size_t pp = sizeof(double) * (size_t)(ni * N);
         const int64_t nq_max = std::max<int64_t>(1, (int64_t)(2 * kSliceBytes / (pa + pb + pp)));
         const int64_t qc = vectors_chunk_size(ctx);
         // (batches are the z dimension of the transposed-slicing grid)
         const int64_t nq = std::min<int64_t>(std::min(nq_max, qc), 65535);
-        CD_ALLOC(ctx->oz_a, pa * nq, false);
-        CD_ALLOC(ctx->oz_b, pb * nq, false);
         CD_ALLOC(ctx->oz_p, pp * nq, false);
-        CD_ALLOC(ctx->oz_ea, sizeof(int) * (size_t)(padded_rows(ni, BM) * nq), false);
-        CD_ALLOC(ctx->oz_eb, sizeof(int) * (size_t)(padded_rows(N, BN) * nq), false);
         for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
             const int64_t mc = std::min(qc, M - Q0);
             const double* Lc = nullptr;
             CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
             for (int64_t q0 = 0; q0 < mc; q0 += nq) {
                 const int64_t nb = std::min(nq, mc - q0);
-                OzakiOperand A = ozaki_operand(ni, N, BM, (int)nb), B = ozaki_operand(N, N, BN, (int)nb);
-                A.q = ctx->oz_a.as<int8_t>();  A.e = ctx->oz_ea.as<int>();
-                B.q = ctx->oz_b.as<int8_t>();  B.e = ctx->oz_eb.as<int>();
-                CD_CUDA(ozaki_slice(Y + (Q0 + q0) * N, M * N, N, A, ctx->num_sms, ctx->stream));
-                CD_CUDA(ozaki_slice_t(Lc + q0 * N * N, N, N * N, B, ctx->stream));
-                CD_CUDA(ozaki_gemm(A, false, B, false, ctx->oz_p.as<double>(), N, ni * N, 1.0, 0.0, err,
-                                   ctx->num_sms, ctx->stream));
-                ctx->launches += 5;
+                OzakiOperand A = oz_operand<Cfg>(ni, N, !sw, nb), B = oz_operand<Cfg>(N, N, sw, nb);
+                CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+                CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
+                CD_CUDA(ozaki_slice<Cfg>(Y + (Q0 + q0) * N, M * N, N, A, ctx->num_sms, ctx->stream));
+                CD_CUDA(ozaki_slice_t<Cfg>(Lc + q0 * N * N, N, N * N, B, ctx->stream));
+                ctx->launches += 3;
+                CD_RC(oz_mul<Cfg>(ctx, A, false, B, false, sw, ctx->oz_p.as<double>(), N, ni * N, 1.0, 0.0));
                 CD_RC(sum_batches(ctx, ctx->oz_p.as<double>(), (int)nb, ni * N, scale, Q0 + q0 > 0, dC + lo * N));
             }
         }
     }
-    int herr = 0;
-    CD_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (herr)
-        return set_error(MSHQC_CD_ERR_TIMEOUT, "int8 tensor-core transposed transform gave up waiting (site " +
-                                                   std::to_string(herr) + ")");
-    return MSHQC_CD_OK;
+    return oz_check(ctx, "int8 tensor-core transposed transform");
 }
 
 // dE/dC of one spin: the int8-slice transposed transforms for the mixed path
@@ -1166,8 +1337,8 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
 }
 
 // The FP64 counterpart of tc_backward_pass, over the same block pairs: S =
-// B_x[I] B_y[J]^T and the Gamma products as FP64 DMMA GEMMs around the
-// element-wise pass.  A diagonal block pair of the symmetric modes forms S
+// B_x[I] B_y[J]^T and the Gamma products around the element-wise pass, as int8
+// slices of full accuracy (larger block pairs) or FP64 DMMA GEMMs.  A diagonal block pair of the symmetric modes forms S
 // for j >= i only (GemmF64Args::tri), and the element-wise pass completes the
 // amplitude block with the transposes.
 template <int MODE>
@@ -1192,6 +1363,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
     double* prow = ctx->dsum.as<double>();
     double* pcol = prow + npairs * dx.vp;
     double* pocc = pcol + npairs * dy.vp;
+    CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
     double* S = ctx->W.as<double>();
     double* A = ctx->amp.as<double>();
     for (int64_t I0 = 0; I0 < dx.o; I0 += bI) {
@@ -1206,15 +1378,20 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             const int64_t ldS = (int64_t)nJ * dy.vp;
             const double* YJ = Y.B64.as<double>() + J0 * dy.vp * Mp;
             // S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q]
+            const bool sliced = sliced_pairs(ctx, nI * dx.vp, ldS);
             begin_stage(ctx, ST_AMPLITUDE);
-            GemmF64Args g{};
-            g.M = (int)(nI * dx.vp);  g.N = (int)ldS;  g.K = (int)Mp;  g.batch = 1;
-            g.A = XI;  g.lda = Mp;  g.sA = 0;
-            g.B = YJ;  g.ldb = Mp;  g.sB = 0;
-            g.C = S;  g.ldc = ldS;  g.sC = 0;
-            g.alpha = 1.0;  g.beta = 0.0;
-            g.tri = tri ? (int)dx.vp : 0;
-            CD_RC(gemm_run(ctx, g, true, true));
+            if (sliced) {
+                CD_RC(sliced_integrals(ctx, X, Y, I0, nI, J0, nJ, tri, S));
+            } else {
+                GemmF64Args g{};
+                g.M = (int)(nI * dx.vp);  g.N = (int)ldS;  g.K = (int)Mp;  g.batch = 1;
+                g.A = XI;  g.lda = Mp;  g.sA = 0;
+                g.B = YJ;  g.ldb = Mp;  g.sB = 0;
+                g.C = S;  g.ldc = ldS;  g.sC = 0;
+                g.alpha = 1.0;  g.beta = 0.0;
+                g.tri = tri ? (int)dx.vp : 0;
+                CD_RC(gemm_run(ctx, g, true, true));
+            }
             end_stage(ctx);
             AmpElemArgs e{};
             e.S = S;
@@ -1251,29 +1428,38 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             }
             end_stage(ctx);
             begin_stage(ctx, ST_GAMMA);
-            // Gamma_x[(i,a)][Q] += sum_{(j,b) in J} t[(i,a)][(j,b)] Y[(j,b)][Q]
-            GemmF64Args h{};
-            h.M = (int)(nI * dx.vp);  h.N = (int)Mp;  h.K = (int)ldS;  h.batch = 1;
-            h.A = A;  h.lda = ldS;  h.sA = 0;
-            h.B = YJ;  h.ldb = Mp;  h.sB = 0;
-            h.C = ctx->gam[sx].as<double>() + I0 * dx.vp * Mp;  h.ldc = Mp;  h.sC = 0;
-            h.alpha = 1.0;  h.beta = 1.0;
-            CD_RC(gemm_run(ctx, h, true, false));
-            if (mirror) {
-                // Gamma_y[(j,b)][Q] += sum_{(i,a) in I} t[(i,a)][(j,b)] X[(i,a)][Q]
-                GemmF64Args k{};
-                k.M = (int)ldS;  k.N = (int)Mp;  k.K = (int)(nI * dx.vp);  k.batch = 1;
-                k.A = A;  k.lda = ldS;  k.sA = 0;
-                k.B = XI;  k.ldb = Mp;  k.sB = 0;
-                k.C = ctx->gam[sy].as<double>() + J0 * dy.vp * Mp;  k.ldc = Mp;  k.sC = 0;
-                k.alpha = 1.0;  k.beta = 1.0;
-                CD_RC(gemm_run(ctx, k, false, false));
+            double* gx = ctx->gam[sx].as<double>() + I0 * dx.vp * Mp;
+            double* gy = ctx->gam[sy].as<double>() + J0 * dy.vp * Mp;
+            if (sliced) {
+                // the staged integrals are used up: their block takes the slices
+                CD_RC(sliced_gamma(ctx, A, ldS, false, nI * dx.vp, ldS, YJ, gx, ctx->W));
+                if (mirror) CD_RC(sliced_gamma(ctx, A, ldS, true, ldS, nI * dx.vp, XI, gy, ctx->W));
+                S = ctx->W.as<double>();
+            } else {
+                // Gamma_x[(i,a)][Q] += sum_{(j,b) in J} t[(i,a)][(j,b)] Y[(j,b)][Q]
+                GemmF64Args h{};
+                h.M = (int)(nI * dx.vp);  h.N = (int)Mp;  h.K = (int)ldS;  h.batch = 1;
+                h.A = A;  h.lda = ldS;  h.sA = 0;
+                h.B = YJ;  h.ldb = Mp;  h.sB = 0;
+                h.C = gx;  h.ldc = Mp;  h.sC = 0;
+                h.alpha = 1.0;  h.beta = 1.0;
+                CD_RC(gemm_run(ctx, h, true, false));
+                if (mirror) {
+                    // Gamma_y[(j,b)][Q] += sum_{(i,a) in I} t[(i,a)][(j,b)] X[(i,a)][Q]
+                    GemmF64Args k{};
+                    k.M = (int)ldS;  k.N = (int)Mp;  k.K = (int)(nI * dx.vp);  k.batch = 1;
+                    k.A = A;  k.lda = ldS;  k.sA = 0;
+                    k.B = XI;  k.ldb = Mp;  k.sB = 0;
+                    k.C = gy;  k.ldc = Mp;  k.sC = 0;
+                    k.alpha = 1.0;  k.beta = 1.0;
+                    CD_RC(gemm_run(ctx, k, false, false));
+                }
             }
             end_stage(ctx);
         }
     }
     CD_RC(reduce_deps(ctx, prow, pcol, pocc, dx.o, dy.o, dx.vp, dy.vp, dx.v, dy.v, deps_x, deps_y));
-    return MSHQC_CD_OK;
+    return oz_check(ctx, "int8 tensor-core FP64 backward");
 }
 
 // Restricted FP64 gradient: one FP64 block-pair pass, then the transposed

@@ -4,25 +4,34 @@
 // Yokota ("DGEMM on integer matrix multiplication unit", 2024).
 //
 // Every row r of an operand is scaled by its own power of two 2^e_r with
-// max_k |x_rk| < 2^e_r (frexp of the row maximum), rounded to the nearest
-// multiple of 2^{e_r - 7S} (an integer m with |m| <= 2^{7S} - 1, so the
-// representation error is at most 2^{e_r - 7S - 1} and unbiased) and the
-// magnitude of m is cut into S base-128 digits carrying the sign of m:
-//   x ~ 2^e_r sum_{s=0}^{S-1} d_s 2^{-7(s+1)},  d_s in [-127, 127].
-// A row x times a row y is then
-//   2^{e_x + e_y} sum_{w=0}^{S-1} 2^{-7(w+2)} sum_{s+t=w} (d^x_s . d^y_t),
-// keeping the S(S+1)/2 slice pairs with s + t < S.  Each slice product is an
-// exact 32-bit integer tensor-core accumulation (|sum| <= S 127^2 K < 2^31
-// for K <= 26624); the epilogue combines the S weighted sums exactly in 64-bit
-// integers and rounds once to FP64.
-// With S = 5 the error per term is below about 2^-32 (2^e_x 2^e_y): far
-// below the fixed-point splitting that follows on the mixed path, which is
-// the only path that uses these products (the FP64 path keeps FP64 FMAs).
+// max_k |x_rk| < 2^e_r, rounded to a multiple of a fixed fraction of 2^e_r and
+// cut into S signed 8-bit digits.  A row x times a row y is then a sum over
+// digit pairs (s, t) of exact 32-bit integer tensor-core products; the pairs of
+// equal s + t share an accumulator, and the epilogue combines the W
+// accumulators (s + t < W) in 64-bit integers and rounds to FP64.
 //
-// Operand storage (per batch, per slice): rows padded to the tile, K padded
-// to 32, the UMMA core-matrix K-major blocked layout in bytes
-//   (k / 32) * Rp * 32 + ((r / 8) * 2 + (k % 32) / 16) * 128 + (r % 8) * 16 + k % 16
-// so the 32-wide K chunk of a 128-row (96-row) tile is one 4 KB (3 KB) copy.
+//  * Mixed (S = 5, W = 5): 35-bit integers, base-128 digits with the sign of
+//    the number, the 15 pairs s + t < 5.  The error per term is below about
+//    2^-32 2^{e_x + e_y}: for the mixed path, whose fixed-point splitting keeps
+//    19 bits.  |sum| <= 5 127^2 K < 2^31 for K <= 26624.
+//  * Full (S = 7, W = 8): multiples of 2^{e-54} (elements within a binade of
+//    the row maximum are exact), base-256 digits in [-128, 127] (the bytes of
+//    (m + c) ^ c with c = 128 in every byte), the 34 pairs s + t < 8.  Dropped
+//    pairs are below 2^-59 2^{e_x + e_y} per term, the representation error
+//    below 2^-55 2^e per element, and nothing is rounded during the
+//    accumulation: against 80-bit sums of Gaussian rows the relative error is
+//    9e-17 at K = 60 and 1.3e-16 at K = 6000, where a chain of FP64 FMAs has
+//    2.5e-16 and 2.4e-15.  For the FP64 path.  K <= 21760 per accumulation;
+//    longer K runs in segments that are added in FP64.
+//
+// Operand storage: blocks of BR rows (128 for A, the tile's column count for
+// B), each holding its 32-wide K chunks one after the other, each chunk the S
+// digit slabs one after the other, each slab in the UMMA core-matrix K-major
+// layout:
+//   (rb * nkc + k / 32) * S * BR * 32 + s * BR * 32
+//     + ((r % BR / 8) * 2 + (k % 32) / 16) * 128 + (r % 8) * 16 + k % 16
+// so a K chunk of a tile is one bulk copy per operand (a bulk copy costs its
+// issuing thread about 70 cycles whatever its size).
 #pragma once
 
 #include <algorithm>
@@ -34,113 +43,224 @@
 namespace mshqc_cd {
 
 namespace ozaki {
-constexpr int S = 5;                       // slices per operand
-constexpr int BM = 128, BN = 96, KB = 32;  // tile rows (A), tile rows (B), K bytes per chunk
-constexpr int STAGES = 5;
-constexpr uint32_t SLAB_A = BM * KB;       // 4 KB
-constexpr uint32_t SLAB_B = BN * KB;       // 3 KB
-constexpr uint32_t OFF_B = S * SLAB_A;
-constexpr uint32_t STAGE_BYTES = S * (SLAB_A + SLAB_B);   // 35 KB
-constexpr uint32_t SMEM_DATA = STAGES * STAGE_BYTES;      // 175 KB
-constexpr int STG_LD = 17;                                // epilogue staging row (doubles)
-constexpr size_t SMEM_BYTES = SMEM_DATA + 1024 + 256 + 4 * 32 * STG_LD * sizeof(double);
-constexpr uint32_t TMEM_COLS = 512;        // S accumulators of BN columns
+constexpr int BM = 128, KB = 32;           // tile rows (A), K bytes per chunk
+constexpr uint32_t TMEM_COLS = 512;        // W accumulators of BN columns
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
-constexpr long long kMaxK = 26624;         // S * 127^2 * K < 2^31
-static_assert(S * BN <= (int)TMEM_COLS, "accumulators exceed TMEM");
-static_assert((long long)S * 127 * 127 * kMaxK < 2147483648LL, "int32 accumulation not exact");
+constexpr uint64_t kPaceLimitNs = 200000ull;
+constexpr int kBadExponent = 1 << 14;      // row with an infinity or NaN: its products are NaN
+constexpr int kTinyExponent = -890;        // rows below 2^-890 are sliced as zero
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
 
-// MMAs of A slice s: its N = (S - s) BN columns in mma_parts(s) equal parts
-// of mma_n(s) <= 256 columns (a multiple of 16, and of 8 rows of the B layout)
-__host__ __device__ constexpr int mma_parts(int s) { return ((S - s) * BN + 255) / 256; }
-__host__ __device__ constexpr int mma_n(int s) { return (S - s) * BN / mma_parts(s); }
-constexpr bool mma_split_ok() {
-    for (int s = 0; s < S; ++s)
-        if (mma_n(s) * mma_parts(s) != (S - s) * BN || mma_n(s) % 16 != 0 || mma_n(s) > 256) return false;
-    return true;
-}
-static_assert(mma_split_ok(), "MMA column split");
+struct Mixed {
+    static constexpr int S = 5, W = 5, BN = 96, STAGES = 6;
+    static constexpr int FIXED = 35;       // integer = x 2^{FIXED - e}
+    static constexpr int SHIFT = 42;       // product = T 2^{e_x + e_y - SHIFT}
+    static constexpr long long MAXK = 26624;
+};
+struct Full {
+    static constexpr int S = 7, W = 8, BN = 64, STAGES = 5;
+    static constexpr int FIXED = 54;
+    static constexpr int SHIFT = 68;
+    static constexpr long long MAXK = 21760;
+};
+static_assert(5LL * 127 * 127 * Mixed::MAXK < 2147483648LL, "int32 accumulation not exact");
+// Full: the leading digit is at most 65, so the largest accumulators are the
+// 7 pairs with two leading digits and the 6 pairs without
+static_assert((2LL * 65 * 128 + 5LL * 128 * 128) * Full::MAXK < 2147483648LL, "int32 accumulation not exact");
+static_assert(6LL * 128 * 128 * Full::MAXK < 2147483648LL, "int32 accumulation not exact");
+
+template <class C>
+struct Dims {
+    static constexpr uint32_t SLAB_A = BM * KB, SLAB_B = C::BN * KB;
+    static constexpr uint32_t OFF_B = C::S * SLAB_A;
+    static constexpr uint32_t STAGE_BYTES = C::S * (SLAB_A + SLAB_B);
+    static constexpr uint32_t SMEM_DATA = C::STAGES * STAGE_BYTES;
+    static constexpr size_t SMEM_BYTES = SMEM_DATA + 1024 + 256;
+    static_assert(C::W * C::BN <= (int)TMEM_COLS, "accumulators exceed TMEM");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+};
 
 inline long long padded_rows(long long rows, int tile) { return (rows + tile - 1) / tile * tile; }
 inline long long padded_k(long long k) { return (k + KB - 1) / KB * KB; }
 // bytes of one sliced operand (all slices, one batch)
-inline size_t operand_bytes(long long Rp, long long Kp) { return (size_t)S * (size_t)Rp * (size_t)Kp; }
+template <class C>
+inline size_t operand_bytes(long long Rp, long long Kp) { return (size_t)C::S * (size_t)Rp * (size_t)Kp; }
+
+// The S digits of x 2^{FIXED - e} as bytes: byte j of (lo, hi) is digit S - 1 - j.
+template <class C>
+__device__ __forceinline__ void digits(double xs, uint32_t& lo, uint32_t& hi) {
+    const long long m = __double2ll_rn(xs);
+    if constexpr (C::S == 7) {
+        constexpr long long c = 0x0080808080808080LL;
+        const unsigned long long u = (unsigned long long)((m + c) ^ c);
+        lo = (uint32_t)u;
+        hi = (uint32_t)(u >> 32);
+    } else {
+        const bool neg = m < 0;
+        const unsigned long long am = (unsigned long long)min(neg ? -m : m, (1LL << C::FIXED) - 1);
+        const uint32_t a = (uint32_t)am;
+        // 7-bit fields to bytes, then all bytes negated (each is at most 127)
+        uint32_t w = (a & 0x7Fu) | ((a & 0x3F80u) << 1) | ((a & 0x1FC000u) << 2) | ((a & 0xFE00000u) << 3);
+        uint32_t h = (uint32_t)(am >> 28);
+        if (neg) {
+            w = (0x80808080u - w) ^ 0x80808080u;
+            h = 0u - h;
+        }
+        lo = w;
+        hi = h & 0xFFu;
+    }
+}
+
+// bytes of four words gathered per byte position: out[j] = byte j of w0..w3
+__device__ __forceinline__ void transpose_bytes(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3,
+                                                uint32_t (&out)[4]) {
+    const uint32_t t0 = __byte_perm(w0, w1, 0x5140), t1 = __byte_perm(w2, w3, 0x5140);
+    const uint32_t t2 = __byte_perm(w0, w1, 0x7362), t3 = __byte_perm(w2, w3, 0x7362);
+    out[0] = __byte_perm(t0, t1, 0x5410);
+    out[1] = __byte_perm(t0, t1, 0x7632);
+    out[2] = __byte_perm(t2, t3, 0x5410);
+    out[3] = __byte_perm(t2, t3, 0x7632);
+}
+
+// four consecutive elements -> word[s] = their digits s
+template <class C>
+__device__ __forceinline__ void digit_words(const double (&xs)[4], uint32_t (&word)[C::S]) {
+    uint32_t lo[4], hi[4], t[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) digits<C>(xs[c], lo[c], hi[c]);
+    transpose_bytes(lo[0], lo[1], lo[2], lo[3], t);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) word[C::S - 1 - j] = t[j];
+    transpose_bytes(hi[0], hi[1], hi[2], hi[3], t);
+#pragma unroll
+    for (int j = 4; j < C::S; ++j) word[C::S - 1 - j] = t[j - 4];
+}
+
+// |x| as an ordered integer: infinities and NaN come out largest
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+// exponent e with |x| < 2^e of the largest |x| of a row
+__device__ __forceinline__ int row_exponent(unsigned long long mx) {
+    const int ef = (int)(mx >> 52);
+    return ef == 2047 ? kBadExponent : ef - 1022;
+}
+// the exponent used: 0 for zero or tiny rows
+__host__ __device__ inline int fixed_exponent(int e) { return e < kTinyExponent ? 0 : e; }
+// 2^{FIXED - e}, or 0 for rows whose digits are all zero
+template <class C>
+__device__ __forceinline__ double to_fixed(int e) {
+    return e == kBadExponent ? 0.0 : pow2d(C::FIXED - e);   // e >= kTinyExponent: in range
+}
 }  // namespace ozaki
 
 // Slices of the rows of row-major FP64 matrices (batch b: rows r < R at
-// src + b * src_batch + r * ld, K elements each).  One warp per group of 8
-// padded rows: lane = (chunk parity, half, row) so that each store of a
-// slice is 256 contiguous bytes per 16 lanes.  dst: [batch][slice][Kp x Rp
-// bytes]; e: [batch][Rp] row exponents (0 for zero or padding rows).
-static __global__ void ozaki_slice_kernel(const double* __restrict__ src, long long ld, long long src_batch,
-                                          long long R, long long K, long long Rp, long long Kp, int batch,
-                                          int8_t* __restrict__ dst, int* __restrict__ e) {
+// src + b * src_batch + r * ld, K elements each).  One CTA per group of 8
+// padded rows, a warp per 32-wide K chunk: lane = (row, 8 consecutive K), so
+// that the loads are 256 contiguous bytes per row and every store of a slice
+// is 256 contiguous bytes.  HELD: chunks a warp keeps in registers between
+// the row-maximum pass and the slicing pass (K <= 256 HELD); 0: the rows are
+// read twice.  HBM bound: 8 bytes read (16 for HELD = 0) and S written per
+// element.  N = 600 vectors (6.9 GB): 1 warp per 8 rows with 16-element lanes
+// took 18.4 ms per 30 calls, this form 5.5.
+// dst as in the header comment (blocks of BR rows); e: [batch][Rp].
+template <class C, int BR, int HELD, bool V2>
+static __global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* __restrict__ src, long long ld,
+                                                                 long long src_batch, int R, int K, int Rp, int Kp,
+                                                                 int8_t* __restrict__ dst, int* __restrict__ e) {
     using namespace ozaki;
-    const long long groups = Rp / 8 * batch;
-    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const int rr = lane & 7;
-    const long long nkc = Kp / KB;
-    for (long long gw = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); gw < groups;
-         gw += nwarps) {
-        const long long b = gw / (Rp / 8), r0 = gw % (Rp / 8) * 8, r = r0 + rr;
+    __shared__ unsigned long long smx[8][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rr = lane & 7, qd = lane >> 3;
+    const int nkc = Kp / KB;
+    const long long b = blockIdx.y;
+    auto load8 = [&](const double* row, bool live, int kc, double (&x)[8]) {
+        const int k = kc * KB + qd * 8;
+        if (V2 && live && k + 8 <= K) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double2 v = *reinterpret_cast<const double2*>(row + k + 2 * j);
+                x[2 * j] = v.x;
+                x[2 * j + 1] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = (live && k + j < K) ? row[k + j] : 0.0;
+        }
+    };
+    for (int g = blockIdx.x; g < Rp / 8; g += gridDim.x) {
+        const int r0 = g * 8, r = r0 + rr;
         const bool live = r < R;
         const double* row = src + b * src_batch + (live ? r : 0) * ld;
-        // row maxima: lanes with equal lane % 8 share a row
-        double mx = 0.0;
-        if (live)
-            for (long long k = lane >> 3; k < K; k += 4) mx = fmax(mx, fabs(row[k]));
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-        // |x| < 2^ex; rows below 2^-900 (none in practice) are sliced as zero
-        int ex = 0;
-        const bool keep = mx >= 0x1p-900;
-        if (keep) frexp(mx, &ex);
-        if (lane < 8) e[b * Rp + r] = ex;
-        const double to_fixed = pow2d(7 * S - ex);
-        constexpr long long kMaxFixed = (1LL << (7 * S)) - 1;
-        int8_t* out = dst + b * (long long)S * Kp * Rp + (r0 / 8) * 256 + (lane & 15) * 16;
-        const int half = (lane >> 3) & 1;
-        for (long long kc2 = 0; kc2 < nkc; kc2 += 2) {
-            const long long kc = kc2 + (lane >> 4);
-            if (kc >= nkc) continue;
-            const long long k0 = kc * KB + half * 16;
-            uint32_t word[S][4];
+        unsigned long long mx = 0;
+        double held[HELD > 0 ? HELD : 1][8];
+        if (HELD > 0) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-#pragma unroll
-                for (int s = 0; s < S; ++s) word[s][q] = 0u;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const long long k = k0 + q * 4 + c;
-                    // |x| 2^(7S - ex) < 2^(7S): exact scaling, one rounding
-                    const double xs = (live && keep && k < K) ? row[k] * to_fixed : 0.0;
-                    const long long m = __double2ll_rn(xs);
-                    const bool neg = m < 0;
-                    const unsigned long long am = (unsigned long long)min(neg ? -m : m, kMaxFixed);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        const uint32_t d = (uint32_t)(am >> (7 * (S - 1 - s))) & 127u;
-                        word[s][q] |= ((neg ? 0u - d : d) & 0xFFu) << (8 * c);
-                    }
-                }
+            for (int h = 0; h < HELD; ++h) {
+                if (warp + 8 * h < nkc) load8(row, live, warp + 8 * h, held[h]);
             }
 #pragma unroll
-            for (int s = 0; s < S; ++s)
-                *reinterpret_cast<uint4*>(out + (long long)s * Kp * Rp + kc * Rp * KB) =
-                    make_uint4(word[s][0], word[s][1], word[s][2], word[s][3]);
+            for (int h = 0; h < HELD; ++h)
+                if (warp + 8 * h < nkc)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) mx = max(mx, abs_bits(held[h][j]));
+        } else {
+            for (int kc = warp; kc < nkc; kc += 8) {
+                double x[8];
+                load8(row, live, kc, x);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) mx = max(mx, abs_bits(x[j]));
+            }
+        }
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        if (lane < 8) smx[warp][lane] = mx;
+        __syncthreads();
+        mx = smx[0][rr];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) mx = max(mx, smx[w][rr]);
+        __syncthreads();   // smx is rewritten by the next group
+        const int ex = fixed_exponent(row_exponent(mx));
+        if (threadIdx.x < 8) e[b * Rp + r] = ex;
+        const double f = to_fixed<C>(ex);
+        const bool zero = f == 0.0;   // 0 * infinity would not be 0
+        int8_t* out = dst + b * ((long long)C::S * Kp * Rp) + (long long)(r0 / BR) * nkc * (C::S * BR * KB) +
+                      (r0 % BR) / 8 * 256 + (qd >> 1) * 128 + rr * 16 + (qd & 1) * 8;
+        auto emit = [&](int kc, const double (&x)[8]) {
+            uint32_t w0[C::S], w1[C::S];
+            const double a[4] = {zero ? 0.0 : x[0] * f, zero ? 0.0 : x[1] * f, zero ? 0.0 : x[2] * f,
+                                 zero ? 0.0 : x[3] * f};
+            const double c[4] = {zero ? 0.0 : x[4] * f, zero ? 0.0 : x[5] * f, zero ? 0.0 : x[6] * f,
+                                 zero ? 0.0 : x[7] * f};
+            digit_words<C>(a, w0);
+            digit_words<C>(c, w1);
+            int8_t* o = out + (long long)kc * (C::S * BR * KB);
+#pragma unroll
+            for (int s = 0; s < C::S; ++s) *reinterpret_cast<uint2*>(o + s * BR * KB) = make_uint2(w0[s], w1[s]);
+        };
+        if (HELD > 0) {
+#pragma unroll
+            for (int h = 0; h < HELD; ++h)
+                if (warp + 8 * h < nkc) emit(warp + 8 * h, held[h]);
+        } else {
+            for (int kc = warp; kc < nkc; kc += 8) {
+                double x[8];
+                load8(row, live, kc, x);
+                emit(kc, x);
+            }
         }
     }
 }
 
 // Slices of the rows of matrices stored with the rows contiguous and K
 // strided (batch b: element (r, k) at src + b * src_batch + k * ld + r), in
-// three passes: row maxima over K splits (atomicMax of the frexp exponent
-// into e, which starts at kNoExponent), exponents of empty or tiny rows set
-// to 0, then one thread per (row, 16-wide K group) writing the S digits.
+// two passes: row maxima over K splits (atomicMax of the exponent into e,
+// which starts at kNoExponent), then one thread per (row, 16-wide K group)
+// writing the S digits; the second pass treats exponents below kTinyExponent
+// as 0 and leaves the fixed value for the product.
 namespace ozaki {
 constexpr int kNoExponent = (int)0x80808080;   // byte pattern 0x80 (memset)
-constexpr int kTinyExponent = -890;            // rows below 2^-890 are sliced as zero
 constexpr int kRowmaxSpan = 512;               // K elements per row-maximum thread
 }  // namespace ozaki
 
@@ -153,104 +273,133 @@ static __global__ void __launch_bounds__(256) ozaki_rowmax_t_kernel(const double
     if (r >= R) return;
     const long long k0 = (long long)blockIdx.y * kRowmaxSpan, k1 = std::min<long long>(K, k0 + kRowmaxSpan);
     const double* col = src + b * src_batch + r;
-    double mx = 0.0;
-    for (long long k = k0; k < k1; ++k) mx = fmax(mx, fabs(col[k * ld]));
-    if (mx > 0.0) {
-        int ex = 0;
-        frexp(mx, &ex);
-        atomicMax(e + b * Rp + r, ex);
+    unsigned long long mx = 0;
+    long long k = k0;
+    for (; k + 8 <= k1; k += 8) {
+        double x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = col[(k + j) * ld];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mx = max(mx, abs_bits(x[j]));
     }
-}
-
-static __global__ void ozaki_exp_fix_kernel(int* __restrict__ e, long long n) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n && e[i] < ozaki::kTinyExponent) e[i] = 0;
+    for (; k < k1; ++k) mx = max(mx, abs_bits(col[k * ld]));
+    if (mx > 0) atomicMax(e + b * Rp + r, row_exponent(mx));
 }
 
 // grid (Rp / 32, ceil(Kp / 128), batch), 256 threads: lane -> row, warp -> 16-wide K group
+template <class C, int BR>
 static __global__ void __launch_bounds__(256) ozaki_slice_t_kernel(const double* __restrict__ src, long long ld,
-                                                                   long long src_batch, long long R, long long K,
-                                                                   long long Rp, long long Kp,
+                                                                   long long src_batch, int R, int K, int Rp, int Kp,
                                                                    const int* __restrict__ e,
                                                                    int8_t* __restrict__ dst) {
     using namespace ozaki;
     const int lane = threadIdx.x & 31;
-    const long long r = blockIdx.x * 32LL + lane;
-    const long long k0 = ((long long)blockIdx.y * 8 + (threadIdx.x >> 5)) * 16;
+    const int r = blockIdx.x * 32 + lane;
+    const int k0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * 16;
     const long long b = blockIdx.z;
     if (k0 >= Kp) return;
     const bool live = r < R;
-    const int ex = e[b * Rp + r];
-    const double to_fixed = pow2d(7 * S - ex);
-    constexpr long long kMaxFixed = (1LL << (7 * S)) - 1;
-    const double* col = src + b * src_batch + r;
-    uint32_t word[S][4];
+    const int ex = fixed_exponent(e[b * Rp + r]);
+    const double f = to_fixed<C>(ex);
+    const double* col = src + b * src_batch + r + k0 * ld;
+    const int kv = live && f != 0.0 ? K - k0 : 0;   // valid K of this thread
+    double x[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = j < kv ? col[j * ld] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] *= f;
+    uint32_t word[4][C::S];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-#pragma unroll
-        for (int s = 0; s < S; ++s) word[s][q] = 0u;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const long long k = k0 + q * 4 + c;
-            const double xs = (live && k < K) ? col[k * ld] * to_fixed : 0.0;
-            const long long m = __double2ll_rn(xs);
-            const bool neg = m < 0;
-            const unsigned long long am = (unsigned long long)min(neg ? -m : m, kMaxFixed);
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                const uint32_t d = (uint32_t)(am >> (7 * (S - 1 - s))) & 127u;
-                word[s][q] |= ((neg ? 0u - d : d) & 0xFFu) << (8 * c);
-            }
-        }
+        const double a[4] = {x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]};
+        digit_words<C>(a, word[q]);
     }
-    int8_t* out = dst + b * (long long)S * Kp * Rp + (k0 >> 5) * Rp * KB +
-                  (((r >> 3) * 2 + ((k0 & 31) >> 4)) << 7) + ((r & 7) << 4);
+    int8_t* out = dst + b * ((long long)C::S * Kp * Rp) + ((long long)(r / BR) * (Kp / KB) + (k0 >> 5)) * (C::S * BR * KB) +
+                  (((r % BR >> 3) * 2 + ((k0 & 31) >> 4)) << 7) + ((r & 7) << 4);
 #pragma unroll
-    for (int s = 0; s < S; ++s)
-        *reinterpret_cast<uint4*>(out + (long long)s * Kp * Rp) =
-            make_uint4(word[s][0], word[s][1], word[s][2], word[s][3]);
+    for (int s = 0; s < C::S; ++s)
+        *reinterpret_cast<uint4*>(out + s * BR * KB) = make_uint4(word[0][s], word[1][s], word[2][s], word[3][s]);
 }
 
 struct OzakiArgs {
-    const int8_t* A; long long a_batch; long long RpA; const int* eA; long long ea_batch;
-    const int8_t* B; long long b_batch; long long RpB; const int* eB; long long eb_batch;
-    long long Kp;              // padded K (multiple of 32)
+    const int8_t* A; long long a_batch; const int* eA; long long ea_batch;
+    const int8_t* B; long long b_batch; const int* eB; long long eb_batch;
+    int nkc;                   // K chunks of the operands
+    int kc0, kc1;              // chunks of this product
     int M, N;                  // valid output rows and columns
-    int nmb, nnb, batch;       // row blocks (128), column blocks (96), batches
+    int nmb, nnb, batch;       // row blocks (128), column blocks (BN), batches
+    int group;                 // row blocks per tile group
+    int tri;                   // > 0: rows and columns in groups of tri; column groups before the row group skipped
     double* C; long long ldc, c_batch;
+    int trans;                 // 1: C(m, n) at C + n * ldc + m
     double alpha, beta;
+    int vec;                   // rows of C 32-byte aligned: 256-bit accesses
+    int* pace; int pace_every, pace_slack;
     int* err;
 };
 
+namespace ozaki {
+// Unit u -> (batch, row block, column block).  Tiles come in groups of `group`
+// row blocks with all column blocks, column-block-major inside a group: the
+// 148 tiles of one wave then read about 16 row blocks and 9 column blocks,
+// 0.6 MB per K chunk in place of 4 MB row-block-major, which HBM cannot feed.
+template <class Args>
+__device__ __forceinline__ void unit_tile(const Args& p, long long u, long long& b, int& mb, int& nb) {
+    const long long per = (long long)p.nmb * p.nnb;
+    b = u / per;
+    const int w = (int)(u - b * per);
+    const int pg = p.group * p.nnb, grp = w / pg;
+    const int g0 = grp * p.group, gsz = min(p.nmb - g0, p.group);
+    const int x = w - grp * pg;
+    nb = x / gsz;
+    mb = g0 + x - nb * gsz;
+}
+// 256-bit accesses of 4 doubles (32-byte aligned)
+__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ void ld4(const double* p, double (&x)[4]) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n"
+                 : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
+                 : "l"(p)
+                 : "memory");
+}
+}  // namespace ozaki
+
 // C = alpha * A B^T + beta * C per batch (A: M x K rows, B: N x K rows, both
-// sliced).  Warp 0 producer (bulk copies of the S slices of a 32-wide K chunk
-// of both tiles), warp 1 MMA issuer and TMEM owner (the S(S+1)/2 slice
-// products of a chunk as 8 MMAs into S accumulators), warps 2..5 epilogue
-// (exact 64-bit combination, one rounding to FP64, staged through shared
-// memory for row-contiguous stores).  Units run row block
-// fastest so that concurrent CTAs share the B tile.  Waits are bounded.
-static __global__ void __launch_bounds__(192, 1) ozaki_gemm_kernel(OzakiArgs p) {
+// sliced).  Warp 0 producer (one bulk copy per operand and 32-wide K chunk),
+// warp 1 MMA issuer and TMEM owner, warps 2..9 epilogue (exact 64-bit
+// combination, one or two roundings to FP64, 64 contiguous bytes of C per
+// thread or 256 per warp when transposed).
+//
+// The MMAs of a chunk: A slice s against the stacked B slices 0 .. min(S, W-s)-1,
+// in parts of at most 256 columns; B slice t lands in accumulator s + t.  An
+// MMA with 128 rows takes N / 2 cycles (at least about 48), so what counts is
+// the total of columns: 1440 per chunk of a 128 x 96 tile (Mixed), 2176 of a
+// 128 x 64 tile (Full).  Waits are bounded.
+template <class C>
+static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(OzakiArgs p) {
     using namespace ozaki;
     using namespace sm100;
+    using D = Dims<C>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + SMEM_DATA);
-    uint64_t* empty = full + STAGES;
-    uint64_t* tmem_full = empty + STAGES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + D::SMEM_DATA);
+    uint64_t* empty = full + C::STAGES;
+    uint64_t* tmem_full = empty + C::STAGES;
     uint64_t* tmem_empty = tmem_full + 1;
     uint64_t* drain = tmem_empty + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    double* stg_all = reinterpret_cast<double*>(smem + SMEM_DATA + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < C::STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         mbar_init(tmem_full, 1);
-        mbar_init(tmem_empty, 4);
+        mbar_init(tmem_empty, EPI_WARPS);
         mbar_init(drain, 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -264,57 +413,79 @@ static __global__ void __launch_bounds__(192, 1) ozaki_gemm_kernel(OzakiArgs p) 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    const long long per_batch = (long long)p.nmb * p.nnb;
-    const long long units = per_batch * p.batch;
+    const long long units = (long long)p.nmb * p.nnb * p.batch;
     const long long first = blockIdx.x, step = gridDim.x;
-    const long long nkc = p.Kp / KB;
-    const long long a_slice = p.Kp * p.RpA, b_slice = p.Kp * p.RpB;
+    const int nk = p.kc1 - p.kc0;
+    auto skipped = [&](int mb, int nb) { return p.tri > 0 && nb * C::BN / p.tri < mb * BM / p.tri; };
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t stage = 0, phase = 0, fill_phase = 0, filled = 0;
-            for (long long u = first; u < units && !*abort_flag; u += step) {
-                const long long b = u / per_batch, rem = u % per_batch;
-                const long long nb = rem / p.nmb, mb = rem % p.nmb;
-                const int8_t* a0 = p.A + b * p.a_batch + mb * BM * KB;
-                const int8_t* b0 = p.B + b * p.b_batch + nb * BN * KB;
-                for (long long kc = 0; kc < nkc; ++kc) {
-                    if (!mbar_wait_bounded(&empty[stage], phase ^ 1, kWaitLimitNs)) {
+        // producer: lane 0 issues the copies, the whole warp paces
+        WavePacer pacer;
+        pacer.init(p.pace, (int)gridDim.x, p.pace_every, p.pace_slack);
+        uint32_t stage = 0, phase = 0, fill_phase = 0, filled = 0;
+        bool stop = false;
+        for (long long u = first; u < units && !stop; u += step) {
+            long long b;
+            int mb, nb;
+            unit_tile(p, u, b, mb, nb);
+            if (skipped(mb, nb)) continue;
+            const int8_t* a0 = p.A + b * p.a_batch + ((long long)mb * p.nkc + p.kc0) * (C::S * (long long)D::SLAB_A);
+            const int8_t* b0 = p.B + b * p.b_batch + ((long long)nb * p.nkc + p.kc0) * (C::S * (long long)D::SLAB_B);
+            for (int kc = 0; kc < nk; ++kc) {
+                pacer.step(lane, kPaceLimitNs);
+                int ok = 1;
+                if (lane == 0) {
+                    if (*abort_flag) {
+                        ok = 0;
+                    } else if (!mbar_wait_bounded(&empty[stage], phase ^ 1, kWaitLimitNs)) {
                         atomicExch(p.err, 31);
                         *abort_flag = 1;
-                        break;
+                        ok = 0;
+                    } else {
+                        uint8_t* sb = smem + stage * D::STAGE_BYTES;
+                        mbar_arrive_expect_tx(&full[stage], D::STAGE_BYTES);
+                        bulk_g2s(sb, a0, C::S * D::SLAB_A, &full[stage]);
+                        bulk_g2s(sb + D::OFF_B, b0, C::S * D::SLAB_B, &full[stage]);
+                        a0 += C::S * D::SLAB_A;
+                        b0 += C::S * D::SLAB_B;
                     }
-                    uint8_t* sb = smem + stage * STAGE_BYTES;
-                    mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
-                    const long long ka = kc * p.RpA * KB, kb = kc * p.RpB * KB;
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        bulk_g2s(sb + s * SLAB_A, a0 + s * a_slice + ka, SLAB_A, &full[stage]);
-                        bulk_g2s(sb + OFF_B + s * SLAB_B, b0 + s * b_slice + kb, SLAB_B, &full[stage]);
-                    }
-                    fill_phase = (fill_phase & ~(1u << stage)) | (phase << stage);
-                    filled |= 1u << stage;
-                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
+                if (!__shfl_sync(0xffffffffu, ok, 0)) {
+                    stop = true;
+                    break;
+                }
+                fill_phase = (fill_phase & ~(1u << stage)) | (phase << stage);
+                filled |= 1u << stage;
+                if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
             }
+        }
+        pacer.finish(lane);
+        if (lane == 0) {
             if (!*abort_flag) {
-                for (int s = 0; s < STAGES; ++s) {
+                for (int s = 0; s < C::STAGES; ++s) {
                     if (!mbar_wait_bounded(&empty[stage], phase ^ 1, kWaitLimitNs)) {
                         atomicExch(p.err, 35);
                         break;
                     }
-                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                    if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             } else {
-                for (int s = 0; s < STAGES; ++s)
+                for (int s = 0; s < C::STAGES; ++s)
                     if ((filled >> s) & 1u) mbar_wait_bounded(&full[s], (fill_phase >> s) & 1u, kWaitLimitNs);
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             uint32_t stage = 0, phase = 0, acc_phase = 0;
-            const uint32_t sbase = smem_addr(smem);
+            // descriptors of the operands at stage 0; a byte offset adds to the
+            // low word in units of 16 bytes
+            const uint64_t da0 = smem_desc_kmajor(smem_addr(smem), 128, 256);
+            const uint64_t db0 = smem_desc_kmajor(smem_addr(smem) + D::OFF_B, 128, 256);
             for (long long u = first; u < units && !*abort_flag; u += step) {
+                long long b;
+                int mb, nb;
+                unit_tile(p, u, b, mb, nb);
+                if (skipped(mb, nb)) continue;
                 if (!mbar_wait_bounded(tmem_empty, acc_phase ^ 1, kWaitLimitNs)) {
                     atomicExch(p.err, 32);
                     *abort_flag = 1;
@@ -322,30 +493,53 @@ static __global__ void __launch_bounds__(192, 1) ozaki_gemm_kernel(OzakiArgs p) 
                 }
                 acc_phase ^= 1;
                 tc_fence_after();
-                for (long long kc = 0; kc < nkc; ++kc) {
+                for (int kc = 0; kc < nk; ++kc) {
                     if (!mbar_wait_bounded(&full[stage], phase, kWaitLimitNs)) {
                         atomicExch(p.err, 33);
                         *abort_flag = 1;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sb = sbase + stage * STAGE_BYTES;
-                    // A slice s against B slices 0 .. S-1-s in one N = (S - s) BN product
-                    // (split in parts of at most 256): B slice t lands in accumulator s + t.
-                    // The s = 0 product of the first chunk starts every accumulator.
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        const uint64_t ad = smem_desc_kmajor(sb + s * SLAB_A, 128, 256);
-#pragma unroll
-                        for (int h = 0; h < mma_parts(s); ++h) {
-                            const uint32_t r0 = (uint32_t)(h * mma_n(s));
-                            const uint64_t bd = smem_desc_kmajor(sb + OFF_B + r0 * KB, 128, 256);
-                            mma_i8(tmem + (uint32_t)(s * BN) + r0, ad, bd, idesc_s8_s32(BM, mma_n(s)),
-                                   (kc > 0 || s > 0) ? 1u : 0u);
-                        }
+                    const uint64_t so = (uint64_t)(stage * (D::STAGE_BYTES >> 4));
+                    const uint32_t more = kc > 0 ? 1u : 0u;
+                    // products of A slice s with B slices t0 .. t0 + n - 1 as one MMA
+                    auto mma = [&](int s, int t0, int cols, uint32_t acc) {
+                        mma_i8(tmem + (uint32_t)((s + t0) * C::BN), da0 + so + (uint64_t)(s * (D::SLAB_A >> 4)),
+                               db0 + so + (uint64_t)(t0 * (D::SLAB_B >> 4)), idesc_s8_s32(BM, cols), acc);
+                    };
+                    auto mma_half = [&](int s, int row0, int cols, uint32_t acc) {   // from stacked B row row0 on
+                        mma_i8(tmem + (uint32_t)(s * C::BN + row0), da0 + so + (uint64_t)(s * (D::SLAB_A >> 4)),
+                               db0 + so + (uint64_t)(row0 * (KB >> 4)), idesc_s8_s32(BM, cols), acc);
+                    };
+                    if constexpr (C::S == 5) {
+                        // 480, 384, 288, 192, 96 columns; the s = 0 products of the
+                        // first chunk start every accumulator
+                        mma_half(0, 0, 240, more);
+                        mma_half(0, 240, 240, more);
+                        mma_half(1, 0, 192, 1u);
+                        mma_half(1, 192, 192, 1u);
+                        mma_half(2, 0, 144, 1u);
+                        mma_half(2, 144, 144, 1u);
+                        mma(3, 0, 192, 1u);
+                        mma(4, 0, 96, 1u);
+                    } else {
+                        // 448, 448, 384, 320, 256, 192, 128 columns; accumulator 7 is
+                        // started by (s, t) = (1, 6)
+                        mma_half(0, 0, 224, more);
+                        mma_half(0, 224, 224, more);
+                        mma(1, 0, 192, 1u);
+                        mma(1, 3, 192, 1u);
+                        mma(1, 6, 64, more);
+                        mma(2, 0, 192, 1u);
+                        mma(2, 3, 192, 1u);
+                        mma_half(3, 0, 160, 1u);
+                        mma_half(3, 160, 160, 1u);
+                        mma(4, 0, 256, 1u);
+                        mma(5, 0, 192, 1u);
+                        mma(6, 0, 128, 1u);
                     }
                     mma_commit(&empty[stage]);
-                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                    if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
                 if (*abort_flag) break;
                 mma_commit(tmem_full);
@@ -354,15 +548,21 @@ static __global__ void __launch_bounds__(192, 1) ozaki_gemm_kernel(OzakiArgs p) 
             if (!mbar_wait_bounded(drain, 0, kWaitLimitNs)) atomicExch(p.err, 36);
         }
     } else {
-        const int q = warp & 3;
-        double* stg = stg_all + (warp - 2) * 32 * STG_LD;
+        const int q = warp & 3, half = (warp - 2) >> 2;   // TMEM lane quadrant, half of the columns
+        constexpr int HC = C::BN / 2;
         const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
-        const int col = lane & 15, rhalf = lane >> 4;
         uint32_t acc_phase = 0;
         for (long long u = first; u < units; u += step) {
             if (*abort_flag) break;
-            const long long b = u / per_batch, rem = u % per_batch;
-            const long long nb = rem / p.nmb, mb = rem % p.nmb;
+            long long b;
+            int mb, nb;
+            unit_tile(p, u, b, mb, nb);
+            if (skipped(mb, nb)) continue;
+            const int m = mb * BM + q * 32 + lane;   // this thread's TMEM row
+            const bool mrow = m < p.M;
+            const int ea = mrow ? fixed_exponent(p.eA[b * p.ea_batch + m]) : 0;
+            double* Cb = p.C + b * p.c_batch;
+            const int* eb = p.eB + b * p.eb_batch;
             if (!mbar_wait_bounded(tmem_full, acc_phase, kWaitLimitNs)) {
                 atomicExch(p.err, 34);
                 *abort_flag = 1;
@@ -370,42 +570,71 @@ static __global__ void __launch_bounds__(192, 1) ozaki_gemm_kernel(OzakiArgs p) 
             }
             acc_phase ^= 1;
             tc_fence_after();
-            const long long m_own = mb * BM + q * 32 + lane;   // this thread's TMEM row
-            // T 2^(-7(S+1)) is the scaled product; 2^eA of this row folded in
-            const double rs = m_own < p.M ? pow2d(p.eA[b * p.ea_batch + m_own] - 7 * (S + 1)) : 0.0;
-            double* Cb = p.C + b * p.c_batch;
-            const int* eb = p.eB + b * p.eb_batch;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 16) {
-                uint32_t acc[S][16];
+            for (int c0 = half * HC; c0 < half * HC + HC; c0 += 8) {
+                uint32_t acc[C::W][8];
 #pragma unroll
-                for (int w = 0; w < S; ++w) tmem_ld16(lane_base + (uint32_t)(w * BN + c0), acc[w]);
+                for (int w = 0; w < C::W; ++w) tmem_ld8(lane_base + (uint32_t)(w * C::BN + c0), acc[w]);
                 tmem_ld_wait();
+                const int n0 = nb * C::BN + c0;
+                double v[8];
 #pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    // sum_w acc_w 2^(7(S-1-w)) exactly in 64 bits (|T| < 2^60), one rounding
-                    long long T = (long long)(int)acc[0][k];
+                for (int k = 0; k < 8; ++k) {
+                    double t;
+                    if constexpr (C::S == 5) {
+                        // sum_w acc_w 2^(7(4-w)) exactly in 64 bits (|T| < 2^60), one rounding
+                        long long T = (long long)(int)acc[0][k];
 #pragma unroll
-                    for (int w = 1; w < S; ++w) T = T * 128 + (long long)(int)acc[w][k];
-                    stg[lane * STG_LD + k] = (double)T * rs;
+                        for (int w = 1; w < C::W; ++w) T = T * 128 + (long long)(int)acc[w][k];
+                        t = (double)T;
+                    } else {
+                        // sum_w acc_w 2^(8(7-w)) as two exact halves (|.| < 2^56)
+                        long long h = (long long)(int)acc[0][k], l = (long long)(int)acc[4][k];
+#pragma unroll
+                        for (int w = 1; w < 4; ++w) {
+                            h = h * 256 + (long long)(int)acc[w][k];
+                            l = l * 256 + (long long)(int)acc[w + 4][k];
+                        }
+                        t = fma((double)h, 0x1p32, (double)l);
+                    }
+                    const int n = n0 + k;
+                    const int en = n < p.N ? fixed_exponent(eb[n]) : 0;
+                    // the scale in two powers of two: no overflow or underflow on the way
+                    const int es = ea + en - C::SHIFT, e1 = es >> 1;
+                    v[k] = ea == kBadExponent || en == kBadExponent
+                               ? __longlong_as_double(0x7FF8000000000000LL)
+                               : p.alpha * (t * pow2d(e1) * pow2d(es - e1));
                 }
-                __syncwarp();
-                // two rows of 16 consecutive columns per store
-                const long long n = nb * BN + c0 + col;
-                const bool ncol = n < p.N;
-                const double cs = ncol ? pow2d(eb[n]) : 0.0;
-#pragma unroll 4
-                for (int r2 = 0; r2 < 32; r2 += 2) {
-                    const int r = r2 + rhalf;
-                    const long long m = mb * BM + q * 32 + r;
-                    if (ncol && m < p.M) {
-                        double* c = Cb + m * p.ldc + n;
-                        double out = p.alpha * (stg[r * STG_LD + col] * cs);
-                        if (p.beta != 0.0) out = fma(p.beta, *c, out);
-                        *c = out;
+                if (mrow) {
+                    if (p.trans) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            if (n0 + k < p.N) {
+                                double* c = Cb + (long long)(n0 + k) * p.ldc + m;
+                                *c = p.beta != 0.0 ? fma(p.beta, *c, v[k]) : v[k];
+                            }
+                    } else {
+                        double* c = Cb + (long long)m * p.ldc + n0;
+                        if (p.vec && n0 + 8 <= p.N) {
+                            if (p.beta != 0.0) {
+                                double x[4], y[4];
+                                ld4(c, x);
+                                ld4(c + 4, y);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    v[k] = fma(p.beta, x[k], v[k]);
+                                    v[4 + k] = fma(p.beta, y[k], v[4 + k]);
+                                }
+                            }
+                            st4(c, v[0], v[1], v[2], v[3]);
+                            st4(c + 4, v[4], v[5], v[6], v[7]);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                if (n0 + k < p.N) c[k] = p.beta != 0.0 ? fma(p.beta, c[k], v[k]) : v[k];
+                        }
                     }
                 }
-                __syncwarp();
             }
             tc_fence_before();
             __syncwarp();
@@ -422,17 +651,20 @@ static __global__ void __launch_bounds__(192, 1) ozaki_gemm_kernel(OzakiArgs p) 
 
 // ---- host side ---------------------------------------------------------------
 
-// One sliced operand: rows R (padded to Rp), K (padded to Kp), `batch` copies.
+// One sliced operand: rows R (padded to Rp, a multiple of the block BR), K
+// (padded to Kp), `batch` copies.
 struct OzakiOperand {
     int8_t* q = nullptr;
     int* e = nullptr;
     long long R = 0, Rp = 0, K = 0, Kp = 0;
+    int BR = 0;
     int batch = 1;
 };
 
 inline OzakiOperand ozaki_operand(long long R, long long K, int tile, int batch) {
     OzakiOperand op;
     op.R = R;
+    op.BR = tile;
     op.Rp = ozaki::padded_rows(R, tile);
     op.K = K;
     op.Kp = ozaki::padded_k(K);
@@ -440,16 +672,44 @@ inline OzakiOperand ozaki_operand(long long R, long long K, int tile, int batch)
     return op;
 }
 
+template <class C, int BR>
+inline cudaError_t ozaki_slice_br(const double* src, long long ld, long long src_batch, const OzakiOperand& op,
+                                  int num_sms, cudaStream_t st) {
+    const bool v2 = reinterpret_cast<uintptr_t>(src) % 16 == 0 && ld % 2 == 0 && src_batch % 2 == 0;
+    // enough CTAs for every SM; each walks its row groups
+    const long long want = std::max<long long>(1, 16LL * num_sms / op.batch);
+    const dim3 grid((unsigned)std::min<long long>(op.Rp / 8, want), (unsigned)op.batch);
+    const long long nkc = op.Kp / ozaki::KB;
+#define MSHQC_SLICE(H)                                                                                              \
+    do {                                                                                                            \
+        if (v2)                                                                                                     \
+            ozaki_slice_kernel<C, BR, H, true><<<grid, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K,      \
+                                                                     (int)op.Rp, (int)op.Kp, op.q, op.e);           \
+        else                                                                                                        \
+            ozaki_slice_kernel<C, BR, H, false><<<grid, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K,     \
+                                                                      (int)op.Rp, (int)op.Kp, op.q, op.e);          \
+    } while (0)
+    if (nkc <= 16)
+        MSHQC_SLICE(2);
+    else if (nkc <= 32)
+        MSHQC_SLICE(4);
+    else if (nkc <= 64)
+        MSHQC_SLICE(8);
+    else
+        MSHQC_SLICE(0);
+#undef MSHQC_SLICE
+    return cudaGetLastError();
+}
+template <class C>
 inline cudaError_t ozaki_slice(const double* src, long long ld, long long src_batch, const OzakiOperand& op,
                                int num_sms, cudaStream_t st) {
-    const long long groups = op.Rp / 8 * op.batch;
-    const long long blocks = std::min<long long>((groups + 7) / 8, (long long)num_sms * 16);
-    ozaki_slice_kernel<<<(unsigned)std::max<long long>(blocks, 1), 256, 0, st>>>(
-        src, ld, src_batch, op.R, op.K, op.Rp, op.Kp, op.batch, op.q, op.e);
-    return cudaGetLastError();
+    if (op.Rp <= 0 || op.batch <= 0) return cudaSuccess;
+    return op.BR == ozaki::BM ? ozaki_slice_br<C, ozaki::BM>(src, ld, src_batch, op, num_sms, st)
+                              : ozaki_slice_br<C, C::BN>(src, ld, src_batch, op, num_sms, st);
 }
 
 // Transposed source: element (r, k) of batch b at src + b * src_batch + k * ld + r.
+template <class C>
 inline cudaError_t ozaki_slice_t(const double* src, long long ld, long long src_batch, const OzakiOperand& op,
                                  cudaStream_t st) {
     using namespace ozaki;
@@ -462,50 +722,74 @@ inline cudaError_t ozaki_slice_t(const double* src, long long ld, long long src_
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }
-    const long long n = op.Rp * op.batch;
-    ozaki_exp_fix_kernel<<<(unsigned)std::max<long long>(1, (n + 255) / 256), 256, 0, st>>>(op.e, n);
-    err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
     dim3 g2((unsigned)(op.Rp / 32), (unsigned)((op.Kp + 127) / 128), (unsigned)op.batch);
-    ozaki_slice_t_kernel<<<g2, 256, 0, st>>>(src, ld, src_batch, op.R, op.K, op.Rp, op.Kp, op.e, op.q);
+    if (op.BR == BM)
+        ozaki_slice_t_kernel<C, BM><<<g2, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K, (int)op.Rp,
+                                                        (int)op.Kp, op.e, op.q);
+    else
+        ozaki_slice_t_kernel<C, C::BN><<<g2, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K, (int)op.Rp,
+                                                           (int)op.Kp, op.e, op.q);
     return cudaGetLastError();
 }
 
-// C[b] = alpha * A[b] B[b]^T + beta * C[b] over the batches; a shared operand
-// (a_shared / b_shared) is one matrix used by every batch.
-inline cudaError_t ozaki_gemm(const OzakiOperand& A, bool a_shared, const OzakiOperand& B, bool b_shared,
-                              double* C, long long ldc, long long c_batch, double alpha, double beta, int* err,
+// Options of a sliced product: a shared operand (a_shared / b_shared) is one
+// matrix used by every batch; trans and tri as in OzakiArgs; pace: progress
+// counters for CTAs with a long K (num_sms ints, zeroed here), or null.
+struct OzakiOpts {
+    bool a_shared = false, b_shared = false;
+    bool trans = false;
+    int tri = 0;
+    int* pace = nullptr;
+};
+
+// C[b] = alpha * A[b] B[b]^T + beta * C[b] over the batches.  K beyond what one
+// exact accumulation holds runs in segments that add up in C.
+template <class C>
+inline cudaError_t ozaki_gemm(const OzakiOperand& A, const OzakiOperand& B, double* Cp, long long ldc,
+                              long long c_batch, double alpha, double beta, const OzakiOpts& o, int* err,
                               int num_sms, cudaStream_t st) {
     using namespace ozaki;
-    static bool attr_set[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    cudaError_t e = cudaFuncSetAttribute(ozaki_gemm_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)Dims<C>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!attr_set[dev]) {
-        e = cudaFuncSetAttribute(ozaki_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e != cudaSuccess) return e;
-        attr_set[dev] = true;
-    }
-    const int batch = a_shared ? B.batch : A.batch;
-    if (A.Kp != B.Kp || A.Kp <= 0 || A.Rp % BM != 0 || B.Rp % BN != 0 || A.K > kMaxK ||
-        (!a_shared && !b_shared && A.batch != B.batch) || (a_shared && b_shared && batch != 1))
+    const int batch = o.a_shared ? B.batch : A.batch;
+    if (A.Kp != B.Kp || A.Kp <= 0 || A.BR != BM || B.BR != C::BN || A.Rp % BM != 0 || B.Rp % C::BN != 0 ||
+        (!o.a_shared && !o.b_shared && A.batch != B.batch) || (o.a_shared && o.b_shared && batch != 1))
         return cudaErrorInvalidValue;
     OzakiArgs p{};
-    p.A = A.q;  p.a_batch = a_shared ? 0 : (long long)operand_bytes(A.Rp, A.Kp);
-    p.RpA = A.Rp;  p.eA = A.e;  p.ea_batch = a_shared ? 0 : A.Rp;
-    p.B = B.q;  p.b_batch = b_shared ? 0 : (long long)operand_bytes(B.Rp, B.Kp);
-    p.RpB = B.Rp;  p.eB = B.e;  p.eb_batch = b_shared ? 0 : B.Rp;
-    p.Kp = A.Kp;
+    p.A = A.q;  p.a_batch = o.a_shared ? 0 : (long long)operand_bytes<C>(A.Rp, A.Kp);
+    p.eA = A.e;  p.ea_batch = o.a_shared ? 0 : A.Rp;
+    p.B = B.q;  p.b_batch = o.b_shared ? 0 : (long long)operand_bytes<C>(B.Rp, B.Kp);
+    p.eB = B.e;  p.eb_batch = o.b_shared ? 0 : B.Rp;
+    p.nkc = (int)(A.Kp / KB);
     p.M = (int)A.R;  p.N = (int)B.R;
-    p.nmb = (int)(A.Rp / BM);  p.nnb = (int)(B.Rp / BN);  p.batch = batch;
-    p.C = C;  p.ldc = ldc;  p.c_batch = c_batch;
-    p.alpha = alpha;  p.beta = beta;
+    p.nmb = (int)(A.Rp / BM);  p.nnb = (int)(B.Rp / C::BN);  p.batch = batch;
+    p.group = 16;
+    p.tri = o.tri;
+    p.C = Cp;  p.ldc = ldc;  p.c_batch = c_batch;
+    p.trans = o.trans ? 1 : 0;
+    p.alpha = alpha;
+    p.vec = reinterpret_cast<uintptr_t>(Cp) % 32 == 0 && ldc % 4 == 0 && c_batch % 4 == 0 ? 1 : 0;
     p.err = err;
     const long long units = (long long)p.nmb * p.nnb * p.batch;
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(units, num_sms));
-    ozaki_gemm_kernel<<<grid, 192, SMEM_BYTES, st>>>(p);
-    return cudaGetLastError();
+    const int max_chunks = (int)(C::MAXK / KB), segs = (p.nkc + max_chunks - 1) / max_chunks;
+    for (int s = 0; s < segs; ++s) {
+        p.kc0 = (int)((long long)p.nkc * s / segs);
+        p.kc1 = (int)((long long)p.nkc * (s + 1) / segs);
+        p.beta = s == 0 ? beta : 1.0;
+        if (o.pace) {
+            e = cudaMemsetAsync(o.pace, 0, sizeof(int) * (size_t)num_sms, st);
+            if (e != cudaSuccess) return e;
+            p.pace = o.pace;
+            p.pace_every = 16;
+            p.pace_slack = 2;
+        }
+        ozaki_gemm_kernel<C><<<grid, THREADS, Dims<C>::SMEM_BYTES, st>>>(p);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace mshqc_cd
