@@ -44,23 +44,24 @@ struct AmpElemArgs {
     const void* S;          // float (SPLIT) or double
     long long ldS;          // row length of S
     int rsx;                // rows per occupied i in S and in the output (multiple of 32)
-    int csy;                // columns per occupied j in S
-    int ksy;                // output K per occupied j (multiple of 32, <= csy)
+    int csy;                // columns per occupied j in S, rows of the transposed output (multiple of 32)
+    int ksy;                // output K per occupied j (multiple of 32, >= csy)
+    int ksx;                // K per occupied i of the transposed output (multiple of 32, >= rsx)
     int ox, oy, vx, vy, i0, nbi;   // oy: all column orbitals (pair index i * oy + j)
     int j0, nbj;            // the column orbitals of this block: j0 .. j0 + nbj - 1
     double wgt;             // weight of the pair sums (2 when the mirror block (J, I) is skipped)
     const double* eox; const double* evx;   // energies of the row spin
     const double* eoy; const double* evy;   // of the column spin
     uint16_t* Ahi; uint16_t* Alo; long long nkA;  // SPLIT: rows R = ii*rsx + a, K = jj*ksy + b (nkA = K / 16)
-    uint16_t* Thi; uint16_t* Tlo; long long nkT;  // SPLIT, optional transpose: rows jj*ksy + b, K = ii*rsx + a
+    uint16_t* Thi; uint16_t* Tlo; long long nkT;  // SPLIT, optional transpose: rows jj*csy + b, K = ii*ksx + a
     double* A64; long long ldA;                   // FP64: [R][K], K = jj*ksy + b
     double* partial;        // [ox * oy] energy of each pair (i, j), i over all row orbitals
     double* prow;           // [ox * oy][rsx] sum_b r per pair and row a (or null)
-    double* pcol;           // [ox * oy][ksy] sum_a r per pair and column b (or null)
+    double* pcol;           // [ox * oy][csy] sum_a r per pair and column b (or null)
     double* pocc;           // [ox * oy] sum_ab r per pair (or null)
     // nchunk > 1: each pair's row tiles are split over nchunk CTAs (CTA
     // lp * nchunk + c takes chunk c of local pair lp = ii * nbj + jj); their
-    // column sums, energies and totals go to cpcol [lp][c][ksy], cpart and
+    // column sums, energies and totals go to cpcol [lp][c][csy], cpart and
     // cpocc [lp][c], and amp_chunks_combine_kernel adds the chunks in order
     int nchunk;
     double* cpcol; double* cpart; double* cpocc;
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
     __shared__ double colpart[8][33];
     __shared__ double red_e[8], red_r[8];
     const TS* S = static_cast<const TS*>(p.S);
-    const int ta = p.rsx / 32, tb = p.ksy / 32;
+    const int ta = p.rsx / 32, tb = p.csy / 32;
     const int R = p.nchunk > 1 ? p.nchunk : 1;
     const int lp = (int)(blockIdx.x / R), ch = (int)(blockIdx.x % R);
     int ii, jj;
@@ -142,8 +143,8 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
     const double eij = p.eox[i] + p.eoy[j];
     double* prow = p.prow ? p.prow + pair * p.rsx : nullptr;
     double* pcol = !p.pcol ? nullptr
-                   : R == 1 ? p.pcol + pair * p.ksy
-                            : p.cpcol + ((long long)lp * R + ch) * p.ksy;
+                   : R == 1 ? p.pcol + pair * p.csy
+                            : p.cpcol + ((long long)lp * R + ch) * p.csy;
     const TS* Srow = S + (long long)ii * p.rsx * p.ldS + (long long)jj * p.csy;
     // this thread's four elements of tile (a0, b0): rows ty + 8k, column tx
     // (V); the transposed tile (b0, a0) for W
@@ -227,8 +228,8 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
                 } else if (write_t) {
                     const int w = threadIdx.x - 128;
                     const int r = w >> 2, g = w & 3;   // r: b offset, g: group of 8 a
-                    const long long R = (long long)jj * p.ksy + b0 + r;
-                    const long long kc = (long long)ii * p.rsx + a0 + g * 8;
+                    const long long R = (long long)jj * p.csy + b0 + r;
+                    const long long kc = (long long)ii * p.ksx + a0 + g * 8;
                     const long long off = amp_detail::blocked_offset(R, kc, p.nkT);
                     double col[8];
 #pragma unroll
@@ -292,16 +293,16 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
 // (local pair, column b); the b == 0 thread also does energy and total.
 static __global__ void amp_chunks_combine_kernel(AmpElemArgs p, int npl) {
     const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)npl * p.ksy) return;
-    const int lp = (int)(idx / p.ksy), b = (int)(idx % p.ksy);
+    if (idx >= (long long)npl * p.csy) return;
+    const int lp = (int)(idx / p.csy), b = (int)(idx % p.csy);
     const int R = p.nchunk;
     int ii, jj;
     amp_detail::local_pair(p, lp, ii, jj);
     const long long pair = (long long)(p.i0 + ii) * p.oy + p.j0 + jj;
     if (p.pcol) {
         double sc = 0.0;
-        for (int c = 0; c < R; ++c) sc += p.cpcol[((long long)lp * R + c) * p.ksy + b];
-        p.pcol[pair * p.ksy + b] = sc;
+        for (int c = 0; c < R; ++c) sc += p.cpcol[((long long)lp * R + c) * p.csy + b];
+        p.pcol[pair * p.csy + b] = sc;
     }
     if (b == 0) {
         double e = 0.0, r = 0.0;

@@ -41,7 +41,7 @@ struct SpinState {
     DevBuf Bhi, Blo;        // Blo unused in the pair layout (hi and lo interleaved in Bhi)
     DevBuf expo;            // per-row power-of-two exponents [o][rows]
     DevBuf diag;            // exact (ia|ia) [o][rows]
-    DevBuf norms;           // sum hi^2, sum lo^2 per row [2][o][rows]
+    DevBuf norms;           // largest sum hi^2 and sum lo^2 of a row (bit patterns)
     int64_t vp16 = 0, Mp16 = 0;
     double max_norm_hi = 0, max_norm_lo = 0;
     bool B16_valid = false;

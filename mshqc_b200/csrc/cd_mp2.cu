@@ -635,29 +635,28 @@ int64_t tc_rows(int64_t v) { return 128 * round_up(cdiv(v, 128), 2); }
 int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
     SpinState& s = ctx->spin[spin];
     const int64_t o = s.nocc, v = ctx->N - s.nocc, M = ctx->M, Mp = ctx->Mp;
-    const int64_t rows = tc_rows(v), nqc = Mp / 16;
-    const size_t n = (size_t)o * nqc * rows * 16;
     const bool pair_layout = layout == 1;
+    // rows per orbital; the integral-tile layout packs them across orbitals
+    const int64_t rows = pair_layout ? tc_rows(v) : round_up(v, 32), nqc = Mp / 16;
+    const size_t n = (size_t)nqc * (pair_layout ? o * rows : round_up(o * rows, 256)) * 16;
     CD_ALLOC(s.Bhi, (pair_layout ? 2 : 1) * n * sizeof(uint16_t), false);
     if (!pair_layout) CD_ALLOC(s.Blo, n * sizeof(uint16_t), false);
     CD_ALLOC(s.expo, sizeof(int) * o * rows, true);
     CD_ALLOC(s.diag, sizeof(double) * o * rows, true);
-    CD_ALLOC(s.norms, sizeof(double) * 2 * o * rows, true);
+    CD_ALLOC(s.norms, sizeof(unsigned long long) * 2, true);
     s.vp16 = rows;
     s.Mp16 = Mp;
-    double* nh = s.norms.as<double>();
-    double* nl = nh + o * rows;
     {
         const int64_t warps = o * rows;
         const int blocks = (int)std::min<int64_t>(cdiv(warps * 32, 256), (int64_t)ctx->num_sms * 32);
         row_scale_kernel<<<blocks, 256, 0, ctx->stream>>>(
             s.B64.as<double>(), s.vp, Mp, (int)v, (int)M, o, rows, s.expo.as<int>(),
-            s.diag.as<double>(), nh, nl, nullptr, 0, 0, 0, nullptr);
+            s.diag.as<double>(), nullptr, 0, 0, 0, nullptr, s.norms.as<unsigned long long>());
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
     }
     {
-        const int64_t threads = o * nqc * rows * 2;
+        const int64_t threads = (int64_t)(n / 8);
         const int blocks = (int)std::min<int64_t>(cdiv(threads, 256), (int64_t)ctx->num_sms * 16);
         split_fixed_blocked_kernel<<<blocks, 256, 0, ctx->stream>>>(
             s.B64.as<double>(), s.vp, Mp, (int)v, (int)M, o, nqc, rows, s.expo.as<int>(),
@@ -666,15 +665,11 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
         ctx->launches++;
     }
     // largest row norms: the Cauchy-Schwarz bound of the integer accumulators
-    std::vector<double> hn(2 * o * rows);
-    CD_CUDA(cudaMemcpyAsync(hn.data(), nh, sizeof(double) * 2 * o * rows, cudaMemcpyDeviceToHost,
-                            ctx->stream));
+    double hn[2];
+    CD_CUDA(cudaMemcpyAsync(hn, s.norms.p, sizeof(hn), cudaMemcpyDeviceToHost, ctx->stream));
     CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    s.max_norm_hi = s.max_norm_lo = 0.0;
-    for (int64_t r = 0; r < o * rows; ++r) {
-        s.max_norm_hi = std::max(s.max_norm_hi, hn[r]);
-        s.max_norm_lo = std::max(s.max_norm_lo, hn[o * rows + r]);
-    }
+    s.max_norm_hi = hn[0];
+    s.max_norm_lo = hn[1];
     s.B16_valid = true;
     s.B16_layout = layout;
     return MSHQC_CD_OK;
@@ -689,15 +684,14 @@ int opposite_spin_diag(mshqc_cd_ctx* ctx) {
     const int o2 = (int)std::min(A.nocc, B.nocc);
     const int v2 = (int)std::min(ctx->N - A.nocc, ctx->N - B.nocc);
     CD_ALLOC(ctx->diag_os, sizeof(double) * std::max<int64_t>(1, (int64_t)o2 * rows), true);
-    CD_ALLOC(ctx->scratch, sizeof(double) * (size_t)(oa * rows * 4), false);
+    CD_ALLOC(ctx->scratch, sizeof(double) * (size_t)(oa * rows * 2), false);
     double* tmp = ctx->scratch.as<double>();
-    int* etmp = reinterpret_cast<int*>(tmp + 3 * oa * rows);
+    int* etmp = reinterpret_cast<int*>(tmp + oa * rows);
     const int64_t warps = oa * rows;
     const int blocks = (int)std::min<int64_t>(cdiv(warps * 32, 256), (int64_t)ctx->num_sms * 32);
     row_scale_kernel<<<blocks, 256, 0, ctx->stream>>>(
-        A.B64.as<double>(), A.vp, ctx->Mp, (int)va, (int)ctx->M, oa, rows, etmp, tmp,
-        tmp + oa * rows, tmp + 2 * oa * rows, B.B64.as<double>(), B.vp, o2, v2,
-        ctx->diag_os.as<double>());
+        A.B64.as<double>(), A.vp, ctx->Mp, (int)va, (int)ctx->M, oa, rows, etmp, tmp, B.B64.as<double>(), B.vp, o2,
+        v2, ctx->diag_os.as<double>(), nullptr);
     CD_CUDA(cudaGetLastError());
     ctx->launches++;
     ctx->diag_os_valid = true;
@@ -1107,7 +1101,9 @@ int transposed_dispatch(mshqc_cd_ctx* ctx, int spin, double scale, double* dC, i
 // ---------------------------------------------------------------------------
 struct BwdDims {
     int64_t o, v, vp;       // occupied, virtual, FP64 padding (64)
-    int64_t VR, nby, VS;    // tensor-core staging: rows per i (128), column ranges (256) per j
+    int64_t RS;             // tensor-core staging and amplitude rows per orbital (32)
+    int64_t VR;             // amplitude K per orbital (128)
+    int64_t VS;             // columns per orbital the block sizes are reckoned with (256)
 };
 
 BwdDims bwd_dims(const mshqc_cd_ctx* ctx, int spin) {
@@ -1115,9 +1111,9 @@ BwdDims bwd_dims(const mshqc_cd_ctx* ctx, int spin) {
     d.o = ctx->spin[spin].nocc;
     d.v = ctx->N - d.o;
     d.vp = ctx->spin[spin].vp;
-    d.VR = cdiv(d.v, 128) * 128;
-    d.nby = cdiv(d.VR, 256);
-    d.VS = d.nby * 256;
+    d.RS = round_up(d.v, 32);
+    d.VR = round_up(d.v, 128);
+    d.VS = round_up(d.VR, 256);
     return d;
 }
 
@@ -1143,20 +1139,24 @@ int make_bt(mshqc_cd_ctx* ctx, int spin, DevBuf& buf, int64_t RQ, const uint16_t
     return MSHQC_CD_OK;
 }
 
-// gamma[(i0 + R / VR, R % VR)][Q] (+)= sum_K A[R][K] BT[Q][K] for R < rows;
-// a_rbs / b_rbs: K chunks per row block of A (128 rows) and of BT (256 rows),
-// bhi / blo pointing at the first K chunk used
+// gamma[(i0 + R / RS, R % RS)][Q] (+)= sum_K A[R][K] BT[Q][K] for R < rows;
+// K in orbital groups of VRk (vk of them valid); a_rbs / b_rbs: K chunks per row
+// block of A (128 rows) and of BT (256 rows), bhi / blo pointing at the first K
+// chunk used
 int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* ahi, const uint16_t* alo, int64_t a_rbs, const uint16_t* bhi,
-                 const uint16_t* blo, int64_t b_rbs, int64_t RQ, int64_t K, int64_t rows, int64_t VR, int64_t v,
-                 int64_t vp, int i0, double* gamma, int accumulate) {
+                 const uint16_t* blo, int64_t b_rbs, int64_t RQ, int64_t K, int64_t VRk, int64_t vk, int64_t rows,
+                 int64_t RS, int64_t v, int64_t vp, int i0, double* gamma, int accumulate) {
     GammaTcArgs g{};
     g.Ahi = ahi;  g.Alo = alo;  g.Bhi = bhi;  g.Blo = blo;
     g.a_rbs = a_rbs;  g.b_rbs = b_rbs;
     g.nk = (int)(K / 16);
     g.KP = 32;
-    g.nrb = (int)(rows / 128);
+    g.kg = (int)(VRk / 16);
+    g.kv = (int)cdiv(vk, 16);
+    g.nrb = (int)cdiv(rows, 128);
     g.nqb = (int)(RQ / 256);
-    g.VR = (int)VR;  g.v = (int)v;  g.vp = (int)vp;  g.Mp = (int)ctx->Mp;  g.i0 = i0;
+    g.rows = rows;
+    g.RS = (int)RS;  g.v = (int)v;  g.vp = (int)vp;  g.Mp = (int)ctx->Mp;  g.i0 = i0;
     g.gamma = gamma;
     g.err = ctx->flag.as<int>() + 2;
     g.accumulate = accumulate;
@@ -1180,11 +1180,11 @@ int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* ahi, const uint16_t* alo, in
 
 // dE/de of one backward pass from its per-pair sums (amp_elem.cuh)
 int reduce_deps(mshqc_cd_ctx* ctx, const double* prow, const double* pcol, const double* pocc, int64_t ox,
-                int64_t oy, int64_t rsx, int64_t ksy, int64_t vx, int64_t vy, double* deps_x, double* deps_y) {
+                int64_t oy, int64_t rsx, int64_t csy, int64_t vx, int64_t vy, double* deps_x, double* deps_y) {
     const int64_t npairs = ox * oy;
     deps_rows_kernel<<<(unsigned)cdiv(vx, 16), 1024, 0, ctx->stream>>>(prow, npairs, (int)rsx, (int)vx,
                                                                        deps_x + ox);
-    deps_rows_kernel<<<(unsigned)cdiv(vy, 16), 1024, 0, ctx->stream>>>(pcol, npairs, (int)ksy, (int)vy,
+    deps_rows_kernel<<<(unsigned)cdiv(vy, 16), 1024, 0, ctx->stream>>>(pcol, npairs, (int)csy, (int)vy,
                                                                        deps_y + oy);
     deps_occ_kernel<<<(unsigned)cdiv(std::max(ox, oy), 128), 128, 0, ctx->stream>>>(pocc, (int)ox, (int)oy,
                                                                                     deps_x, deps_y);
@@ -1228,13 +1228,13 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
     CD_ALLOC(ctx->amp2, n_amp, false);
     CD_ALLOC(ctx->ampT, n_amp, false);
     CD_ALLOC(ctx->ampT2, n_amp, false);
-    CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VS), false);
+    CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.RS) * (size_t)(bJ * dy.RS), false);
     const int64_t npairs = dx.o * dy.o;
-    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (dx.VR + dy.VR + 1)), true);
+    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (dx.RS + dy.RS + 1)), true);
     CD_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)npairs, ctx->stream));
     double* prow = ctx->dsum.as<double>();
-    double* pcol = prow + npairs * dx.VR;
-    double* pocc = pcol + npairs * dy.VR;
+    double* pcol = prow + npairs * dx.RS;
+    double* pocc = pcol + npairs * dy.RS;
     if (X.B16_layout != 0 || Y.B16_layout != 0)
         return set_error(MSHQC_CD_ERR_STATE, "fixed-point operands not in the integral-tile layout");
     const size_t vsm = vtile_tc::SMEM_BYTES;
@@ -1254,16 +1254,19 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             a.Yhi = Y.Bhi.as<uint16_t>();  a.Ylo = Y.Blo.as<uint16_t>();
             a.ex = X.expo.as<int>();  a.ey = Y.expo.as<int>();
             a.diag = sx == sy ? X.diag.as<double>() : nullptr;
-            a.rows_x = (int)X.vp16;  a.rows_y = (int)Y.vp16;
+            a.RSx = (int)dx.RS;  a.RSy = (int)dy.RS;
             a.nqc = (int)(Mp / 16);
-            a.j0 = (int)J0;  a.nbj = nJ;
             a.vx = (int)dx.v;  a.vy = (int)dy.v;
-            a.VR = (int)dx.VR;  a.i0 = (int)I0;  a.nbi = nI;
-            a.nbx = (int)(dx.VR / 128);  a.nby = (int)dy.nby;  a.VS = (int)dy.VS;
+            a.r0 = I0 * dx.RS;  a.r1 = (I0 + nI) * dx.RS;
+            a.c0 = J0 * dy.RS;  a.c1 = (J0 + nJ) * dy.RS;
+            a.ldS = nJ * dy.RS;
+            a.rb0 = (int)(a.r0 / 128);  a.nrb = (int)cdiv(a.r1, 128) - a.rb0;
+            a.cb0 = (int)(a.c0 / 256);  a.ncb = (int)cdiv(a.c1, 256) - a.cb0;
+            a.group = 12;
             a.S = ctx->W.as<float>();
             a.err = ctx->flag.as<int>();
             a.tri = tri ? 1 : 0;
-            const int64_t vunits = (int64_t)npl * a.nbx * a.nby;
+            const int64_t vunits = (int64_t)a.nrb * a.ncb;
             const int vgrid = (int)std::min<int64_t>(vunits, ctx->num_sms);
             pace_params(&a.pace_every, &a.pace_slack, "MSHQC_CD_PACE_TILES", false);
             if (a.pace_every > 0) {
@@ -1277,8 +1280,8 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             ctx->launches++;
             AmpElemArgs e{};
             e.S = ctx->W.as<float>();
-            e.ldS = (long long)nJ * dy.VS;
-            e.rsx = (int)dx.VR;  e.csy = (int)dy.VS;  e.ksy = (int)dy.VR;
+            e.ldS = (long long)nJ * dy.RS;
+            e.rsx = (int)dx.RS;  e.csy = (int)dy.RS;  e.ksy = (int)dy.VR;  e.ksx = (int)dx.VR;
             e.ox = (int)dx.o;  e.oy = (int)dy.o;  e.vx = (int)dx.v;  e.vy = (int)dy.v;
             e.i0 = (int)I0;  e.nbi = nI;  e.j0 = (int)J0;  e.nbj = nJ;
             e.wgt = (kSym && mirror) ? 2.0 : 1.0;
@@ -1297,15 +1300,15 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             e.prow = prow;  e.pcol = pcol;  e.pocc = pocc;
             // split each pair's row tiles over several CTAs when the block
             // pair alone does not fill the GPU several times over
-            const int ta = (int)(dx.VR / 32);
+            const int ta = (int)(dx.RS / 32);
             int nch = 1;
             while (nch < 16 && 2 * nch <= ta && (int64_t)npl * nch < 8LL * ctx->num_sms) nch *= 2;
             e.nchunk = nch;
             if (nch > 1) {
                 const size_t per = (size_t)npl * nch;
-                CD_ALLOC(ctx->amp_chunks, sizeof(double) * per * ((size_t)dy.VR + 2), false);
+                CD_ALLOC(ctx->amp_chunks, sizeof(double) * per * ((size_t)dy.RS + 2), false);
                 e.cpcol = ctx->amp_chunks.as<double>();
-                e.cpart = e.cpcol + per * dy.VR;
+                e.cpart = e.cpcol + per * dy.RS;
                 e.cpocc = e.cpart + per;
             }
             begin_stage(ctx, ST_AMP_ELEM);
@@ -1313,7 +1316,7 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             CD_CUDA(cudaGetLastError());
             ctx->launches++;
             if (nch > 1) {
-                amp_chunks_combine_kernel<<<(unsigned)cdiv((int64_t)npl * dy.VR, 256), 256, 0, ctx->stream>>>(e, npl);
+                amp_chunks_combine_kernel<<<(unsigned)cdiv((int64_t)npl * dy.RS, 256), 256, 0, ctx->stream>>>(e, npl);
                 CD_CUDA(cudaGetLastError());
                 ctx->launches++;
             }
@@ -1322,17 +1325,17 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             // first K chunk of block J (I) inside a 256-row block of BT
             const size_t kJ = (size_t)J0 * dy.VR / 16 * 4096, kI = (size_t)I0 * dx.VR / 16 * 4096;
             const int64_t nkBy = dy.o * dy.VR / 16, nkBx = dx.o * dx.VR / 16;
-            CD_RC(launch_gamma(ctx, e.Ahi, e.Alo, e.nkA, bty[0] + kJ, bty[1] + kJ, nkBy, RQ, (int64_t)nJ * dy.VR,
-                               (int64_t)nI * dx.VR, dx.VR, dx.v, dx.vp, (int)I0, ctx->gam[sx].as<double>(), 1));
+            CD_RC(launch_gamma(ctx, e.Ahi, e.Alo, e.nkA, bty[0] + kJ, bty[1] + kJ, nkBy, RQ, (int64_t)nJ * dy.VR, dy.VR,
+                               dy.v, (int64_t)nI * dx.RS, dx.RS, dx.v, dx.vp, (int)I0, ctx->gam[sx].as<double>(), 1));
             if (mirror) {
                 // Gamma_sy[J] += A^T x B_sx[I]
                 CD_RC(launch_gamma(ctx, e.Thi, e.Tlo, e.nkT, btx[0] + kI, btx[1] + kI, nkBx, RQ,
-                                   (int64_t)nI * dx.VR, (int64_t)nJ * dy.VR, dy.VR, dy.v, dy.vp, (int)J0,
+                                   (int64_t)nI * dx.VR, dx.VR, dx.v, (int64_t)nJ * dy.RS, dy.RS, dy.v, dy.vp, (int)J0,
                                    ctx->gam[sy].as<double>(), 1));
             }
         }
     }
-    CD_RC(reduce_deps(ctx, prow, pcol, pocc, dx.o, dy.o, dx.VR, dy.VR, dx.v, dy.v, deps_x, deps_y));
+    CD_RC(reduce_deps(ctx, prow, pcol, pocc, dx.o, dy.o, dx.RS, dy.RS, dx.v, dy.v, deps_x, deps_y));
     return MSHQC_CD_OK;
 }
 
@@ -1396,7 +1399,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             AmpElemArgs e{};
             e.S = S;
             e.ldS = ldS;
-            e.rsx = (int)dx.vp;  e.csy = (int)dy.vp;  e.ksy = (int)dy.vp;
+            e.rsx = (int)dx.vp;  e.csy = (int)dy.vp;  e.ksy = (int)dy.vp;  e.ksx = (int)dx.vp;
             e.ox = (int)dx.o;  e.oy = (int)dy.o;  e.vx = (int)dx.v;  e.vy = (int)dy.v;
             e.i0 = (int)I0;  e.nbi = nI;  e.j0 = (int)J0;  e.nbj = nJ;
             e.wgt = (kSym && mirror) ? 2.0 : 1.0;

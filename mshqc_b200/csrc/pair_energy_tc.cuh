@@ -199,7 +199,14 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
             constexpr uint32_t IDESC = idesc_f16_f32(BM, BN);          // N = 128
             constexpr uint32_t IDESC2 = idesc_f16_f32(BM, 2 * BN);     // N = 256: [hi; lo]
             uint32_t stage = 0, phase = 0, acc_phase = 0;
+            // descriptors of the four operands at stage 0; a byte offset adds to the
+            // low word in units of 16
             const uint32_t sbase = smem_addr(smem);
+            const uint64_t d0 = smem_desc_kmajor(sbase + 0 * PIECE, 128, 256);
+            const uint64_t d1 = smem_desc_kmajor(sbase + 1 * PIECE, 128, 256);
+            const uint64_t d2 = MODE == PAIR_OPPOSITE_SPIN ? d0 : smem_desc_kmajor(sbase + 2 * PIECE, 128, 256);
+            const uint64_t d3 = smem_desc_kmajor(sbase + 3 * PIECE, 128, 256);
+            constexpr uint64_t LO = SLAB >> 4;   // the lo slab after the hi slab
             for (long long u = first; u < p.units && !*abort_flag; u += step) {
                 // accumulators free? (epilogue of the previous unit done)
                 if (!mbar_wait_bounded(tmem_empty, acc_phase ^ 1, kWaitLimitNs)) {
@@ -216,21 +223,18 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sb = sbase + stage * STAGE_BYTES;
                     const int nks = min(KS, nk - kq);
-                    for (int c = 0; c < nks; ++c) {
-                        const uint32_t o0 = sb + 0 * PIECE + c * CHUNK, o1 = sb + 1 * PIECE + c * CHUNK;
-                        const uint32_t o2 = (MODE == PAIR_OPPOSITE_SPIN ? sb : sb + 2 * PIECE) + c * CHUNK;
-                        const uint32_t o3 = sb + 3 * PIECE + c * CHUNK;
-                        // hi at +0, lo at +SLAB; [hi; lo] is the 256-row operand at +0
-                        const uint64_t p0h = smem_desc_kmajor(o0, 128, 256), p0l = smem_desc_kmajor(o0 + SLAB, 128, 256);
-                        const uint64_t p2h = smem_desc_kmajor(o2, 128, 256), p2l = smem_desc_kmajor(o2 + SLAB, 128, 256);
-                        const uint64_t p1 = smem_desc_kmajor(o1, 128, 256), p3 = smem_desc_kmajor(o3, 128, 256);
-                        const uint32_t acc = (kq + c) > 0 ? 1u : 0u;
-                        mma_f16(tmem + 0, p0h, p1, IDESC2, acc);     // hh | hi*lo'
-                        mma_f16(tmem + 128, p0l, p1, IDESC, 1u);     // + lo*hi'
-                        mma_f16(tmem + 256, p2h, p3, IDESC2, acc);
-                        mma_f16(tmem + 384, p2l, p3, IDESC, 1u);
+#pragma unroll
+                    for (int c = 0; c < KS; ++c) {
+                        if (c < nks) {
+                            // [hi; lo] is the 256-row operand at the chunk's start
+                            const uint64_t so = (uint64_t)(stage * (STAGE_BYTES >> 4)) + c * (CHUNK >> 4);
+                            const uint32_t acc = c > 0 || kq > 0 ? 1u : 0u;
+                            mma_f16(tmem + 0, d0 + so, d1 + so, IDESC2, acc);          // hh | hi*lo'
+                            mma_f16(tmem + 128, d0 + so + LO, d1 + so, IDESC, 1u);     // + lo*hi'
+                            mma_f16(tmem + 256, d2 + so, d3 + so, IDESC2, acc);
+                            mma_f16(tmem + 384, d2 + so + LO, d3 + so, IDESC, 1u);
+                        }
                     }
                     mma_commit(&empty[stage]);       // frees the stage when these MMAs finish
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }

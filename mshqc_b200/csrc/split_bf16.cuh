@@ -28,17 +28,18 @@ namespace mshqc_cd {
 constexpr int kFixedHiBits = 10;   // |hi| <= 2^10
 constexpr double kFixedLoScale = 256.0;   // lo step = u / 256, |lo| <= 128
 
-// One warp per row: exponent, exact diagonal and the norms of hi and lo.
+// One warp per row: exponent, exact diagonal, and over all rows the largest
+// norms of hi and lo (max_norms[0], [1]: bit patterns, zeroed by the caller).
 // src: [o][vp][Mp] FP64.  rows (a) beyond v get e = 0 and zeros.
 // src2 (may be null): second spin's rows for the opposite-spin diagonal
 // sum_Q B_alpha[i][a][Q] * B_beta[i][a][Q] (i < o2, a < v2).
 static __global__ void row_scale_kernel(const double* __restrict__ src, int64_t vp, int64_t Mp,
                                         int v, int M, int64_t o, int64_t rows,
                                         int* __restrict__ expo, double* __restrict__ diag,
-                                        double* __restrict__ norm_hi, double* __restrict__ norm_lo,
                                         const double* __restrict__ src2, int64_t vp2, int o2, int v2,
-                                        double* __restrict__ diag_os) {
+                                        double* __restrict__ diag_os, unsigned long long* __restrict__ max_norms) {
     const int lane = threadIdx.x & 31;
+    double top_hi = 0.0, top_lo = 0.0;
     const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = wid; r < o * rows; r += nw) {
@@ -91,10 +92,15 @@ static __global__ void row_scale_kernel(const double* __restrict__ src, int64_t 
         if (lane == 0) {
             expo[r] = e;
             diag[r] = d;
-            norm_hi[r] = nh;
-            norm_lo[r] = nl;
+            top_hi = fmax(top_hi, nh);
+            top_lo = fmax(top_lo, nl);
             if (want_os) diag_os[i * rows + a] = dos;
         }
+    }
+    // (bit patterns of non-negative doubles order like unsigned integers)
+    if (lane == 0 && max_norms) {
+        atomicMax(max_norms, (unsigned long long)__double_as_longlong(top_hi));
+        atomicMax(max_norms + 1, (unsigned long long)__double_as_longlong(top_lo));
     }
 }
 
@@ -102,38 +108,37 @@ static __global__ void row_scale_kernel(const double* __restrict__ src, int64_t 
 // dst, two layouts of FP16 bits, blocked inside a 16-wide Q chunk as
 // (a/8, (Q%16)/8, a%8, Q%8) (the canonical K-major no-swizzle UMMA layout):
 //  * pair_layout = false (integral tiles of the backward): hi and lo in
-//    separate arrays of 256-row blocks, each holding its nqc chunks one after
-//    the other:
-//      element (i, a, Q) at ((i*rows/256 + a/256)*nqc + Q/16)*4096
-//                           + ((a%256)/8*16 + (Q%16)/8*8 + a%8)*8 + Q%8
+//    separate arrays over the composite rows g = i*rows + a (rows a multiple
+//    of 32), in 256-row blocks that run across orbitals, each holding its nqc
+//    chunks one after the other:
+//      element (g, Q) at ((g/256)*nqc + Q/16)*4096
+//                        + ((g%256)/8*16 + (Q%16)/8*8 + g%8)*8 + Q%8
 //    so a 128-row slab of one chunk is 4 KB and a 256-row slab of consecutive
 //    chunks is one contiguous run;
-//  * pair_layout = true (fused pair energies): one array of 128-row blocks
-//    whose chunks hold the hi slab and then the lo slab of the same rows:
+//  * pair_layout = true (fused pair energies; rows a multiple of 256): one
+//    array of 128-row blocks whose chunks hold the hi slab and then the lo
+//    slab of the same rows:
 //      hi of (i, a, Q) at ((i*rows/128 + a/128)*nqc + Q/16)*4096
 //                         + ((a%128)/8*16 + (Q%16)/8*8 + a%8)*8 + Q%8,
 //      lo at the same + 2048,
 //    so one contiguous copy brings both halves of a 128-row slab for several
 //    chunks, and each chunk's [hi; lo] is a 256-row operand.
-// rows is a multiple of 256.
 static __global__ void split_fixed_blocked_kernel(const double* __restrict__ src, int64_t vp,
                                                   int64_t Mp, int v, int M, int64_t o, int64_t nqc,
                                                   int64_t rows, const int* __restrict__ expo,
                                                   uint16_t* __restrict__ hi, uint16_t* __restrict__ lo,
                                                   bool pair_layout) {
-    // one thread = one core-matrix row: 8 consecutive Q of one a
-    const int64_t total = o * nqc * rows * 2;
+    // one thread = one core-matrix row: 8 consecutive Q of one composite row
+    const int64_t ngrp = pair_layout ? o * rows / 8 : (o * rows + 255) / 256 * 32;   // groups of 8 rows
+    const int64_t total = nqc * ngrp * 2 * 8;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
          t += (int64_t)gridDim.x * blockDim.x) {
-        // t enumerates (i, qc, g, kk, r) with r fastest
+        // t enumerates (qc, g, kk, r) with r fastest
         const int64_t r = t & 7;
         const int64_t kk = (t >> 3) & 1;
-        const int64_t rest = t >> 4;               // (i*nqc + qc)*ngrp + g
-        const int64_t ngrp = rows / 8;
-        const int64_t g = rest % ngrp;
-        const int64_t iq = rest / ngrp;             // i * nqc + qc
-        const int64_t qc = iq % nqc, i = iq / nqc;
-        const int64_t a = g * 8 + r;
+        const int64_t rest = t >> 4;               // qc * ngrp + g
+        const int64_t g = rest % ngrp, qc = rest / ngrp;
+        const int64_t row = g * 8 + r, i = row / rows, a = i < o ? row % rows : (int64_t)v;
         const int64_t q0 = qc * 16 + kk * 8;
         const int e = (a < v) ? expo[i * rows + a] : 0;
         const double inv_u = ldexp(1.0, kFixedHiBits - e), u = ldexp(1.0, e - kFixedHiBits);
@@ -147,9 +152,8 @@ static __global__ void split_fixed_blocked_kernel(const double* __restrict__ src
             h[k] = __half_as_ushort(__double2half(hv));   // exact: |hv| <= 1024
             l[k] = __half_as_ushort(__double2half(lv));   // exact: |lv| <= 128
         }
-        const int64_t off = pair_layout
-                                ? ((i * (rows / 128) + (g >> 4)) * nqc + qc) * 4096 + ((g & 15) * 16 + kk * 8 + r) * 8
-                                : ((i * (rows / 256) + (g >> 5)) * nqc + qc) * 4096 + ((g & 31) * 16 + kk * 8 + r) * 8;
+        const int64_t off = pair_layout ? ((g >> 4) * nqc + qc) * 4096 + ((g & 15) * 16 + kk * 8 + r) * 8
+                                        : ((g >> 5) * nqc + qc) * 4096 + ((g & 31) * 16 + kk * 8 + r) * 8;
         uint4 vh, vl;
         vh.x = h[0] | (uint32_t(h[1]) << 16); vh.y = h[2] | (uint32_t(h[3]) << 16);
         vh.z = h[4] | (uint32_t(h[5]) << 16); vh.w = h[6] | (uint32_t(h[7]) << 16);

@@ -7,7 +7,11 @@
 // X and Y are the MO vectors of one spin (restricted, same spin) or of the
 // two spins (opposite spin: X alpha, Y beta).
 // Operands are the exact fixed-point hi/lo of split_bf16.cuh in its 256-row
-// blocked layout; a stage holds KS = 2 Q steps: the A slab (128 rows) per
+// blocked layout over the composite rows (i, a) and (j, b), packed at v rounded
+// to 32 per orbital, so a tile runs across orbitals (padding every orbital's
+// rows to 128 and columns to 256 took 1.66 times the tiles at v = 540).  Tiles
+// lie on the grid of the composite rows; the edge tiles of a block store only
+// the block's rows and columns.  A stage holds KS = 2 Q steps: the A slab (128 rows) per
 // step, the B slab (256 rows) of both steps in one copy (one-step copies
 // left the kernel feed-bound: 7.7 ms for a launch whose MMAs take 5.8 ms;
 // 5.9 ms with the two-step B copies).  Per 16-wide Q step three 128x256x16 MMAs
@@ -32,36 +36,33 @@ namespace mshqc_cd {
 struct VtileArgs {
     const uint16_t* Xhi; const uint16_t* Xlo;   // blocked fixed-point operands (rows i, a)
     const uint16_t* Yhi; const uint16_t* Ylo;   // (columns j, b)
-    const int* ex; const int* ey;               // row exponents [o][rows]
-    const double* diag;                         // exact (ia|ia) [o][rows_x] when X = Y, else null
-    int rows_x, rows_y;     // allocated rows per occupied orbital (operand layouts)
+    const int* ex; const int* ey;               // row exponents of the composite rows
+    const double* diag;                         // exact (ia|ia) per composite row when X = Y, else null
+    int RSx, RSy;           // composite rows per orbital
     int nqc;                // 16-wide Q chunks
-    int j0, nbj;            // column orbitals j0 .. j0 + nbj - 1
-    int vx, vy, VR, i0, nbi;       // VR: staging rows per orbital i (nbx * 128)
-    int nbx, nby;           // row blocks (128) per orbital i, column ranges (256) per orbital j
-    int VS;                 // staging columns per orbital j (nby * 256)
-    float* S;               // staging [nbi * VR][nbj * VS]
+    int vx, vy;
+    long long r0, r1, c0, c1;   // the block's composite rows and columns
+    int rb0, nrb, cb0, ncb;     // its row blocks (128) and column blocks (256)
+    int group;              // row blocks per tile group, see vtile_unit
+    float* S;               // staging [r1 - r0][ldS]
+    long long ldS;
     int* err;
-    int tri;                // 1: only the pairs ii <= jj of a diagonal block (nbi == nbj)
+    int tri;                // 1: a diagonal block of X = Y: tiles with a pair i <= j only
     int* pace;              // gridDim.x zeroed progress counters (WavePacer), or null
     int pace_every, pace_slack;
 };
 
-// Local pair pr -> (ii, jj): row-major over nbi x nbj, or over the upper
-// triangle ii <= jj (rows of nbi - ii pairs) when p.tri.
-__device__ __forceinline__ void vtile_pair(const VtileArgs& p, long long pr, int& ii, int& jj) {
-    if (!p.tri) {
-        ii = (int)(pr / p.nbj);
-        jj = (int)(pr % p.nbj);
-        return;
-    }
-    int r = (int)pr, i = 0;
-    while (r >= p.nbi - i) {
-        r -= p.nbi - i;
-        ++i;
-    }
-    ii = i;
-    jj = i + r;
+// Unit u -> (row block, column block), in groups of `group` row blocks with all
+// column blocks, column-block-major inside a group: a wave of 148 tiles then
+// reads about 12 row blocks and 12 column blocks.  False: no pair i <= j in the
+// tile (tri).
+__device__ __forceinline__ bool vtile_unit(const VtileArgs& p, int u, int& rb, int& cb) {
+    const int pg = p.group * p.ncb, grp = u / pg, g0 = grp * p.group;
+    const int gsz = min(p.nrb - g0, p.group), x = u - grp * pg;
+    cb = x / gsz;
+    rb = p.rb0 + g0 + x - cb * gsz;
+    cb += p.cb0;
+    return !p.tri || (cb * 256 + 255) / p.RSy >= rb * 128 / p.RSx;
 }
 
 namespace vtile_tc {
@@ -112,11 +113,8 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // unit u -> (ii, j, x, y): pair-major so that concurrent CTAs share slabs
-    const long long per_pair = (long long)p.nbx * p.nby;
-    const long long npl = p.tri ? (long long)p.nbi * (p.nbi + 1) / 2 : (long long)p.nbi * p.nbj;
-    const long long units = npl * per_pair;
-    const long long first = blockIdx.x, step = gridDim.x;
+    const int units = p.nrb * p.ncb;
+    const int first = blockIdx.x, step = gridDim.x;
     const int nk = p.nqc;
 
     if (warp == 0) {
@@ -125,16 +123,13 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
         pacer.init(p.pace, (int)gridDim.x, p.pace_every, p.pace_slack);
         uint32_t stage = 0, phase = 0, fill_phase = 0, filled = 0;
         bool stop = false;
-        for (long long u = first; u < units && !stop; u += step) {
-            const long long pr = u / per_pair, bb = u % per_pair;
-            int ii, jj;
-            vtile_pair(p, pr, ii, jj);
-            const int i = p.i0 + ii, j = p.j0 + jj;
-            const int x = (int)(bb / p.nby), y = (int)(bb % p.nby);
+        for (int u = first; u < units && !stop; u += step) {
+            int rb, cb;
+            if (!vtile_unit(p, u, rb, cb)) continue;
             // slab bases at Q step 0 (256-row blocks of nqc steps, 4096 elements a step)
             const size_t nq = (size_t)p.nqc;
-            const size_t xa = (((size_t)i * (p.rows_x / 256) + x / 2) * nq) * 4096 + (size_t)(x % 2) * 2048;
-            const size_t yb = (((size_t)j * (p.rows_y / 256) + y) * nq) * 4096;
+            const size_t xa = (size_t)(rb / 2) * nq * 4096 + (size_t)(rb % 2) * 2048;
+            const size_t yb = (size_t)cb * nq * 4096;
             const uint16_t* ah = p.Xhi + xa;
             const uint16_t* al = p.Xlo + xa;
             const uint16_t* bh = p.Yhi + yb;
@@ -190,8 +185,15 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
         if (lane == 0) {
             constexpr uint32_t IDESC = idesc_f16_f32(BM, BN);
             uint32_t stage = 0, phase = 0, acc_phase = 0;
+            // descriptors at stage 0; a byte offset adds to the low word in units of 16
             const uint32_t sbase = smem_addr(smem);
-            for (long long u = first; u < units && !*abort_flag; u += step) {
+            const uint64_t dah = smem_desc_kmajor(sbase + OFF_AH, 128, 256);
+            const uint64_t dal = smem_desc_kmajor(sbase + OFF_AL, 128, 256);
+            const uint64_t dbh = smem_desc_kmajor(sbase + OFF_BH, 128, 256);
+            const uint64_t dbl = smem_desc_kmajor(sbase + OFF_BL, 128, 256);
+            for (int u = first; u < units && !*abort_flag; u += step) {
+                int rb, cb;
+                if (!vtile_unit(p, u, rb, cb)) continue;
                 if (!mbar_wait_bounded(tmem_empty, acc_phase ^ 1, kWaitLimitNs)) {
                     atomicExch(p.err, 22);
                     *abort_flag = 1;
@@ -206,17 +208,16 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sb = sbase + stage * STAGE_BYTES;
-                    const int nks = min(KS, nk - kq);
-                    for (int q2 = 0; q2 < nks; ++q2) {
-                        const uint64_t ah = smem_desc_kmajor(sb + OFF_AH + q2 * SLAB_A, 128, 256);
-                        const uint64_t al = smem_desc_kmajor(sb + OFF_AL + q2 * SLAB_A, 128, 256);
-                        const uint64_t bh = smem_desc_kmajor(sb + OFF_BH + q2 * SLAB_B, 128, 256);
-                        const uint64_t bl = smem_desc_kmajor(sb + OFF_BL + q2 * SLAB_B, 128, 256);
-                        const uint32_t acc = (kq + q2) > 0 ? 1u : 0u;
-                        mma_f16(tmem, ah, bh, IDESC, acc);
-                        mma_f16(tmem + BN, ah, bl, IDESC, acc);
-                        mma_f16(tmem + BN, al, bh, IDESC, 1u);
+                    const uint64_t so = (uint64_t)(stage * (STAGE_BYTES >> 4));
+                    const uint32_t more = kq > 0 ? 1u : 0u;
+                    mma_f16(tmem, dah + so, dbh + so, IDESC, more);
+                    mma_f16(tmem + BN, dah + so, dbl + so, IDESC, more);
+                    mma_f16(tmem + BN, dal + so, dbh + so, IDESC, 1u);
+                    if (kq + 1 < nk) {
+                        const uint64_t sa = so + (SLAB_A >> 4), sb = so + (SLAB_B >> 4);
+                        mma_f16(tmem, dah + sa, dbh + sb, IDESC, 1u);
+                        mma_f16(tmem + BN, dah + sa, dbl + sb, IDESC, 1u);
+                        mma_f16(tmem + BN, dal + sa, dbh + sb, IDESC, 1u);
                     }
                     mma_commit(&empty[stage]);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -231,18 +232,14 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
         const int q = warp & 3;
         const int row = q * 32 + lane;
         const int etid = threadIdx.x - 64;
-        const long long ldS = (long long)p.nbj * p.VS;
         uint32_t acc_phase = 0;
-        for (long long u = first; u < units; u += step) {
-            const long long pr = u / per_pair, bb = u % per_pair;
-            int ii, jj;
-            vtile_pair(p, pr, ii, jj);
-            const int i = p.i0 + ii, j = p.j0 + jj;
-            const int x = (int)(bb / p.nby), y = (int)(bb % p.nby);
-            const int a = x * BM + row, b0 = y * BN;
+        for (int u = first; u < units; u += step) {
+            int rb, cb;
+            if (!vtile_unit(p, u, rb, cb)) continue;
+            const long long r = (long long)rb * BM + row, h0 = (long long)cb * BN;   // composite row, first column
             for (int c = etid; c < BN; c += 128) {
-                const int b = b0 + c;
-                cs_s[c] = (b < p.vy) ? pow2d(p.ey[(size_t)j * p.rows_y + b] - kFixedHiBits) : 0.0;
+                const long long h = h0 + c;
+                cs_s[c] = h < p.c1 && h % p.RSy < p.vy ? pow2d(p.ey[h] - kFixedHiBits) : 0.0;
             }
             // the four epilogue warps leave together (a named barrier must
             // never wait for a warp that already left the loop)
@@ -255,11 +252,12 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
             }
             acc_phase ^= 1;
             tc_fence_after();
-            const bool arow = a < p.vx;
-            const double rs = arow ? pow2d(p.ex[(size_t)i * p.rows_x + a] - kFixedHiBits) : 0.0;
-            const int dcol = (p.diag && arow && i == j && a >= b0 && a < b0 + BN) ? a - b0 : -1;
-            const double dg = dcol >= 0 ? p.diag[(size_t)i * p.rows_x + a] : 0.0;
-            float* dst = p.S + ((long long)ii * p.VR + a) * ldS + (long long)jj * p.VS + b0;
+            const bool rin = r >= p.r0 && r < p.r1;   // a row of the block
+            const bool arow = rin && r % p.RSx < p.vx;
+            const double rs = arow ? pow2d(p.ex[r] - kFixedHiBits) : 0.0;
+            const int dcol = p.diag && arow && r >= h0 && r < h0 + BN ? (int)(r - h0) : -1;
+            const double dg = dcol >= 0 ? p.diag[r] : 0.0;
+            float* dst = p.S + (r - p.r0) * p.ldS + (h0 - p.c0);
             const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
             float amax = 0.0f;   // integer accumulators stay exact below 2^24
 #pragma unroll 1
@@ -277,7 +275,8 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
                     if (c0 + k == dcol) V = dg;
                     out[k] = arow ? (float)V : 0.0f;
                 }
-                if (a < p.VR) {
+                // (the block's ends are multiples of 32 columns)
+                if (rin && h0 + c0 >= p.c0 && h0 + c0 < p.c1) {
                     // streaming stores (evict first): the staging is read once
                     // by the element-wise pass, and must not push the
                     // operands that other CTAs still read out of L2
