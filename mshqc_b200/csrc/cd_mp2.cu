@@ -1228,7 +1228,8 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
     CD_ALLOC(ctx->amp2, n_amp, false);
     CD_ALLOC(ctx->ampT, n_amp, false);
     CD_ALLOC(ctx->ampT2, n_amp, false);
-    CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.RS) * (size_t)(bJ * dy.RS), false);
+    // (the size the block sizes are reckoned with; the packed rows take less of it)
+    CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VS), false);
     const int64_t npairs = dx.o * dy.o;
     CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (dx.RS + dy.RS + 1)), true);
     CD_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)npairs, ctx->stream));
