@@ -81,7 +81,15 @@ struct mshqc_cd_ctx {
 
     // workspaces
     mshqc_cd::DevBuf Y;             // half-transformed vectors
-    int Y_spin = -1;                // spin whose Y is in the buffer (-1: none)
+    // half-transformed vectors held in Y: per spin, the occupied orbitals
+    // [lo, hi) from row `row` on (rows of M * N), made by int8 slices or not
+    struct YRange {
+        bool ok = false, i8 = false;
+        int64_t row = 0, lo = 0, hi = 0;
+    } Yr[2];
+    mshqc_cd::DevBuf cpack;         // occupied orbitals of both spins, one after the other
+    mshqc_cd::DevBuf occ_parts;     // dE/dC_occ of both spins in one product
+    int L_sym = -1;                 // stored vectors symmetric to the bit (-1: not looked at yet)
     mshqc_cd::DevBuf scratch;       // uploads / unpacking
     mshqc_cd::DevBuf tables;        // pair and block tables
     mshqc_cd::DevBuf partial;       // per-unit energies
@@ -126,15 +134,14 @@ struct mshqc_cd_ctx {
     // of a partitioned gradient are shared over occupied orbitals too
     mshqc_cd_collectives coll{};
     bool coll_set = false;
-    int64_t Y_lo = 0, Y_hi = 0;     // occupied orbitals whose half-transformed vectors Y holds
-
     std::vector<double> pair_energy[3];  // host copies, row-major [i][j]
 
     void invalidate_all() {
         spin[0].invalidate();
         spin[1].invalidate();
         diag_os_valid = false;
-        Y_spin = -1;
+        Yr[0].ok = Yr[1].ok = false;
+        L_sym = -1;
         for (auto& p : pair_energy) p.clear();
     }
     size_t held_bytes() const {
@@ -161,6 +168,8 @@ struct mshqc_cd_ctx {
         totals.release();
         flag.release();
         gemm_ws.release();
+        cpack.release();
+        occ_parts.release();
         pace.release();
         amp.release();
         BT.release();
@@ -240,6 +249,7 @@ int check_finite_device(mshqc_cd_ctx* ctx, const double* x, int64_t n, const cha
 // layout: of the fixed-point operands of a mixed-precision request
 // (0: integral tiles of the backward, 1: fused pair energies)
 int ensure_transform(mshqc_cd_ctx* ctx, int spin, int precision, int layout = 0);
+int ensure_transforms(mshqc_cd_ctx* ctx, int precision, int layout = 0);   // alpha and beta
 int run_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* out);
 int run_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* e_out,
                  double* dC_a, double* dC_b, double* deps_a, double* deps_b, int where);
@@ -249,5 +259,6 @@ int invalidate_spin(mshqc_cd_ctx* ctx, int spin);   // orbitals of `spin` change
 // each, contiguous): the stored array, or a chunk generated into ctx->Lchunk
 // (valid until the next call); vectors_chunk_size is the chunk to ask for.
 int64_t vectors_chunk_size(const mshqc_cd_ctx* ctx);
+int vectors_symmetric(mshqc_cd_ctx* ctx, bool* yes);   // L[Q][mu][nu] == L[Q][nu][mu] for all
 int vectors_chunk(mshqc_cd_ctx* ctx, int64_t Q0, int64_t mc, const double** out);
 }  // namespace mshqc_cd

@@ -216,7 +216,12 @@ int oz_check(mshqc_cd_ctx* ctx, const char* what) {
     return MSHQC_CD_OK;
 }
 
-// Second half of the forward transform from Y [i - lo][Q][nu]:
+// the rows of Y that hold a spin's half-transformed vectors
+double* y_rows(mshqc_cd_ctx* ctx, int spin) {
+    return ctx->Y.as<double>() + ctx->Yr[spin].row * ctx->M * ctx->N;
+}
+
+// Second half of the forward transform from the spin's rows of Y [i - lo][Q][nu]:
 // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu], a batch of orbitals i at a time
 template <class C>
 int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
@@ -233,7 +238,7 @@ int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
         const int64_t nb = std::min(ib, hi - i0);
         OzakiOperand By = oz_operand<C>(M, N, sw, nb);
         CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, (size_t)(per_i * nb), By));
-        CD_CUDA(ozaki_slice<C>(ctx->Y.as<double>() + (i0 - lo) * M * N, N, M * N, By, ctx->num_sms, ctx->stream));
+        CD_CUDA(ozaki_slice<C>(y_rows(ctx, spin) + (i0 - lo) * M * N, N, M * N, By, ctx->num_sms, ctx->stream));
         ctx->launches++;
         CD_RC(oz_mul<C>(ctx, Av, true, By, false, sw, s.B64.as<double>() + i0 * vp * Mp, Mp, vp * Mp, 1.0, 0.0));
     }
@@ -256,61 +261,6 @@ bool fp64_slices(double flops, double min_flops, int64_t reuse) {
     return flops >= min_flops && reuse >= kSlicedMinReuse;
 }
 
-// FP64 half transform of one spin into the padded [i][a][Q] layout, for the
-// occupied orbitals [lo, hi) (Y holds rows i - lo; B rows outside stay zero).
-// The first half reads every vector once for few occupied orbitals and stays
-// on the DMMA pipe.
-int transform_f64(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
-    SpinState& s = ctx->spin[spin];
-    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, ni = hi - lo;
-    const int64_t vp = round_up(v, 64);
-    CD_ALLOC(ctx->Y, sizeof(double) * (size_t)std::max<int64_t>(1, ni) * M * N, false);
-    CD_ALLOC(s.B64, sizeof(double) * (size_t)b_rows(ctx, o) * vp * Mp, true);
-    s.vp = vp;
-    ctx->Y_spin = spin;
-    ctx->Y_lo = lo;
-    ctx->Y_hi = hi;
-    s.B64_valid = true;
-    s.B64_prec = MSHQC_CD_FP64;
-    if (ni <= 0) return MSHQC_CD_OK;
-    const double* C = s.C.as<double>();
-    // Y[i][(Q,nu)] = sum_mu C[mu,i] L[Q][nu*N + mu], one chunk of Q at a time
-    const int64_t qc = vectors_chunk_size(ctx);
-    for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
-        const int64_t mc = std::min(qc, M - Q0);
-        const double* Lc = nullptr;
-        CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
-        GemmF64Args g1{};
-        g1.M = (int)ni;
-        g1.N = (int)(mc * N);
-        g1.K = (int)N;
-        g1.batch = 1;
-        g1.A = C + lo * N;  g1.lda = N;  g1.sA = 0;
-        g1.B = Lc;  g1.ldb = N;  g1.sB = 0;
-        g1.C = ctx->Y.as<double>() + Q0 * N;  g1.ldc = M * N;  g1.sC = 0;
-        g1.alpha = 1.0;  g1.beta = 0.0;
-        CD_RC(gemm_run(ctx, g1, true, true));
-    }
-    const char* tenv = std::getenv("MSHQC_CD_TRANSFORM");   // f64: DMMA for both halves
-    if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
-        CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
-        CD_RC(second_half_sliced<ozaki::Full>(ctx, spin, lo, hi));
-        return oz_check(ctx, "int8 tensor-core transform");
-    }
-    // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu]
-    GemmF64Args g2{};
-    g2.M = (int)v;
-    g2.N = (int)M;
-    g2.K = (int)N;
-    g2.batch = (int)ni;
-    g2.A = C + o * N;  g2.lda = N;  g2.sA = 0;
-    g2.B = ctx->Y.as<double>();  g2.ldb = N;  g2.sB = M * N;
-    g2.C = s.B64.as<double>() + lo * vp * Mp;  g2.ldc = Mp;  g2.sC = vp * Mp;
-    g2.alpha = 1.0;  g2.beta = 0.0;
-    CD_RC(gemm_run(ctx, g2, true, true));
-    return MSHQC_CD_OK;
-}
-
 bool int8_transform_enabled(const mshqc_cd_ctx* ctx) {
     if (ctx->N > ozaki::Mixed::MAXK) return false;
     const char* env = std::getenv("MSHQC_CD_TRANSFORM");
@@ -331,35 +281,54 @@ bool int8_forward_enabled(const mshqc_cd_ctx* ctx) {
     return ctx->N >= kInt8ForwardMinN;
 }
 
-// The same half transform as transform_f64 with both products on the int8
-// tensor cores (ozaki::Mixed): Y = C_occ^T L per vectors chunk, then
-// B_i = C_vir^T Y_i^T in batches of occupied orbitals.  Accuracy of the
-// slices (about 2^-33 of the row maxima per term), not FP64 rounding: used by
-// the mixed-precision path only.
-int transform_i8(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
+// First half of the forward transform for the occupied orbitals [lo, hi) of the
+// given spins: Y[row of i][(Q,nu)] = sum_mu C[mu,i] L[Q][nu*N + mu], one chunk of
+// vectors at a time.  Two spins are one product over both spins' orbitals, so
+// the vectors are read (and sliced) once: unrestricted N = 600, 60 + 58
+// orbitals, 10.5 -> 6.3 ms with the second halves.  i8: int8 slices of the mixed
+// accuracy, else FP64 on the DMMA pipe (every vector element meets few
+// orbitals: full slices would cost more than the products).
+int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, const int64_t* hi, bool i8) {
+    const int64_t N = ctx->N, M = ctx->M;
+    int64_t rows = 0;
+    ctx->Yr[0].ok = ctx->Yr[1].ok = false;
+    for (int k = 0; k < nsp; ++k) rows += std::max<int64_t>(0, hi[k] - lo[k]);
+    CD_ALLOC(ctx->Y, sizeof(double) * (size_t)std::max<int64_t>(1, rows) * M * N, false);
+    int64_t r = 0;
+    for (int k = 0; k < nsp; ++k) {
+        auto& y = ctx->Yr[spins[k]];
+        y.ok = true;
+        y.i8 = i8;
+        y.row = r;
+        y.lo = lo[k];
+        y.hi = hi[k];
+        r += std::max<int64_t>(0, hi[k] - lo[k]);
+    }
+    if (rows == 0) return MSHQC_CD_OK;
+    // the orbitals as contiguous rows
+    const double* C = ctx->spin[spins[0]].C.as<double>() + lo[0] * N;
+    if (nsp == 2) {
+        CD_ALLOC(ctx->cpack, sizeof(double) * (size_t)(rows * N), false);
+        r = 0;
+        for (int k = 0; k < nsp; ++k) {
+            const int64_t ni = std::max<int64_t>(0, hi[k] - lo[k]);
+            CD_CUDA(cudaMemcpyAsync(ctx->cpack.as<double>() + r * N, ctx->spin[spins[k]].C.as<double>() + lo[k] * N,
+                                    sizeof(double) * (size_t)(ni * N), cudaMemcpyDeviceToDevice, ctx->stream));
+            r += ni;
+        }
+        C = ctx->cpack.as<double>();
+    }
     using Cfg = ozaki::Mixed;
-    SpinState& s = ctx->spin[spin];
-    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, ni = hi - lo;
-    const int64_t vp = round_up(v, 64);
-    CD_ALLOC(ctx->Y, sizeof(double) * (size_t)std::max<int64_t>(1, ni) * M * N, false);
-    CD_ALLOC(s.B64, sizeof(double) * (size_t)b_rows(ctx, o) * vp * Mp, true);
-    CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
-    s.vp = vp;
-    ctx->Y_spin = spin;
-    ctx->Y_lo = lo;
-    ctx->Y_hi = hi;
-    s.B64_valid = true;
-    s.B64_prec = MSHQC_CD_FP16X3;
-    if (ni <= 0) return MSHQC_CD_OK;
-    // Y[i][(Q,nu)] = sum_mu C[mu,i] L[Q][nu*N + mu]: rows of C^T (the occupied
-    // orbitals of the slice) against the vectors' rows
-    const bool sw = round_up(ni, Cfg::BN) < round_up(ni, ozaki::BM);
-    OzakiOperand Ao = oz_operand<Cfg>(ni, N, !sw, 1);
-    CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(Ao), Ao));
-    CD_CUDA(ozaki_slice<Cfg>(s.C.as<double>() + lo * N, N, 0, Ao, ctx->num_sms, ctx->stream));
-    ctx->launches++;
+    const bool sw = round_up(rows, Cfg::BN) < round_up(rows, ozaki::BM);
+    OzakiOperand Ao = oz_operand<Cfg>(rows, N, !sw, 1);
+    if (i8) {
+        CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
+        CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(Ao), Ao));
+        CD_CUDA(ozaki_slice<Cfg>(C, N, 0, Ao, ctx->num_sms, ctx->stream));
+        ctx->launches++;
+    }
     const int64_t per_q = (int64_t)ozaki::operand_bytes<Cfg>(round_up(N, ozaki::BM), ozaki::padded_k(N));
-    const int64_t qs = std::max<int64_t>(1, (int64_t)kSliceBytes / per_q);
+    const int64_t qs = i8 ? std::max<int64_t>(1, (int64_t)kSliceBytes / per_q) : M;
     const int64_t qc = vectors_chunk_size(ctx);
     for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
         const int64_t mc = std::min(qc, M - Q0);
@@ -367,15 +336,88 @@ int transform_i8(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
         CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
         for (int64_t q0 = 0; q0 < mc; q0 += qs) {
             const int64_t ms = std::min(qs, mc - q0);
-            OzakiOperand Bl = oz_operand<Cfg>(ms * N, N, sw, 1);
-            CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Bl), Bl));
-            CD_CUDA(ozaki_slice<Cfg>(Lc + q0 * N * N, N, 0, Bl, ctx->num_sms, ctx->stream));
-            ctx->launches++;
-            CD_RC(oz_mul<Cfg>(ctx, Ao, true, Bl, false, sw, ctx->Y.as<double>() + (Q0 + q0) * N, M * N, 0, 1.0, 0.0));
+            const double* L = Lc + q0 * N * N;
+            double* Y = ctx->Y.as<double>() + (Q0 + q0) * N;
+            if (i8) {
+                OzakiOperand Bl = oz_operand<Cfg>(ms * N, N, sw, 1);
+                CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Bl), Bl));
+                CD_CUDA(ozaki_slice<Cfg>(L, N, 0, Bl, ctx->num_sms, ctx->stream));
+                ctx->launches++;
+                CD_RC(oz_mul<Cfg>(ctx, Ao, true, Bl, false, sw, Y, M * N, 0, 1.0, 0.0));
+            } else {
+                GemmF64Args g{};
+                g.M = (int)rows;  g.N = (int)(ms * N);  g.K = (int)N;  g.batch = 1;
+                g.A = C;  g.lda = N;
+                g.B = L;  g.ldb = N;
+                g.C = Y;  g.ldc = M * N;
+                g.alpha = 1.0;  g.beta = 0.0;
+                CD_RC(gemm_run(ctx, g, true, true));
+            }
         }
     }
-    CD_RC(second_half_sliced<Cfg>(ctx, spin, lo, hi));
-    return oz_check(ctx, "int8 tensor-core transform");
+    return MSHQC_CD_OK;
+}
+
+// Forward half transforms of the given spins into the padded [i][a][Q] layout,
+// for this rank's occupied orbitals (B rows outside stay zero).  FP64, or with
+// i8 both products on the int8 tensor cores at the mixed accuracy (about 2^-33
+// of the row maxima per term), which only the mixed-precision path uses.
+int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
+    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp;
+    int64_t lo[2], hi[2];
+    for (int k = 0; k < nsp; ++k) {
+        SpinState& s = ctx->spin[spins[k]];
+        shard_range(ctx, s.nocc, &lo[k], &hi[k]);
+        s.vp = round_up(N - s.nocc, 64);
+        CD_ALLOC(s.B64, sizeof(double) * (size_t)b_rows(ctx, s.nocc) * s.vp * Mp, true);
+        s.B64_valid = true;
+        s.B64_prec = i8 ? MSHQC_CD_FP16X3 : MSHQC_CD_FP64;
+    }
+    CD_RC(first_half(ctx, nsp, spins, lo, hi, i8));
+    bool sliced = i8;
+    for (int k = 0; k < nsp; ++k) {
+        SpinState& s = ctx->spin[spins[k]];
+        const int64_t o = s.nocc, v = N - o, ni = hi[k] - lo[k];
+        if (ni <= 0) continue;
+        if (i8) {
+            CD_RC(second_half_sliced<ozaki::Mixed>(ctx, spins[k], lo[k], hi[k]));
+            continue;
+        }
+        const char* tenv = std::getenv("MSHQC_CD_TRANSFORM");   // f64: DMMA for both halves
+        if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
+            CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, !sliced);
+            sliced = true;
+            CD_RC(second_half_sliced<ozaki::Full>(ctx, spins[k], lo[k], hi[k]));
+            continue;
+        }
+        // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu]
+        GemmF64Args g{};
+        g.M = (int)v;  g.N = (int)M;  g.K = (int)N;  g.batch = (int)ni;
+        g.A = s.C.as<double>() + o * N;  g.lda = N;  g.sA = 0;
+        g.B = y_rows(ctx, spins[k]);  g.ldb = N;  g.sB = M * N;
+        g.C = s.B64.as<double>() + lo[k] * s.vp * Mp;  g.ldc = Mp;  g.sC = s.vp * Mp;
+        g.alpha = 1.0;  g.beta = 0.0;
+        CD_RC(gemm_run(ctx, g, true, true));
+    }
+    return sliced ? oz_check(ctx, "int8 tensor-core transform") : MSHQC_CD_OK;
+}
+
+// Whether the half-transformed vectors of both spins may be held at once: the
+// buffer already has the room, or it is at most a quarter of the free memory.
+int both_spins_fit(mshqc_cd_ctx* ctx, bool* yes) {
+    int64_t rows = 0;
+    for (int s = 0; s < 2; ++s) {
+        int64_t lo, hi;
+        shard_range(ctx, ctx->spin[s].nocc, &lo, &hi);
+        rows += hi - lo;
+    }
+    const size_t need = sizeof(double) * (size_t)(rows * ctx->M * ctx->N);
+    *yes = need <= ctx->Y.bytes;
+    if (*yes) return MSHQC_CD_OK;
+    size_t free_b = 0, total_b = 0;
+    CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    *yes = need <= (free_b + ctx->Y.bytes) / 4;
+    return MSHQC_CD_OK;
 }
 
 // Whether the FP64 integral and Gamma products of blocks of `rows` x `cols`
@@ -817,35 +859,60 @@ int pair_pass_tc(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
 int invalidate_spin(mshqc_cd_ctx* ctx, int spin) {
     ctx->spin[spin].invalidate();
     ctx->diag_os_valid = false;
-    if (ctx->Y_spin == spin) ctx->Y_spin = -1;
+    ctx->Yr[spin].ok = false;
     return MSHQC_CD_OK;
 }
+
+namespace {
+
+// an FP64 request never reuses int8-slice products; a mixed one reuses either
+bool transform_needed(const mshqc_cd_ctx* ctx, int spin, int precision) {
+    const SpinState& s = ctx->spin[spin];
+    return !s.B64_valid || (precision == MSHQC_CD_FP64 && s.B64_prec != MSHQC_CD_FP64);
+}
+
+int run_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, int precision) {
+    begin_stage(ctx, ST_TRANSFORM);
+    CD_RC(transform(ctx, nsp, spins, precision == MSHQC_CD_FP16X3 && int8_forward_enabled(ctx)));
+    for (int k = 0; k < nsp; ++k) {
+        SpinState& s = ctx->spin[spins[k]];
+        // shared over ranks: this rank's orbitals so far, now all of them
+        if (sharded(ctx))
+            CD_RC(run_collective(ctx, true, s.B64.as<double>(), shard_p(ctx, s.nocc) * s.vp * ctx->Mp));
+        s.B16_valid = false;
+    }
+    end_stage(ctx);
+    return MSHQC_CD_OK;
+}
+
+}  // namespace
 
 int ensure_transform(mshqc_cd_ctx* ctx, int spin, int precision, int layout) {
     CD_RC(require_inputs(ctx, spin));
     SpinState& s = ctx->spin[spin];
     if (precision != MSHQC_CD_FP64 && precision != MSHQC_CD_FP16X3)
         return set_error(MSHQC_CD_ERR_ARG, "unknown precision");
-    // an FP64 request never reuses int8-slice products; a mixed one reuses either
-    if (!s.B64_valid || (precision == MSHQC_CD_FP64 && s.B64_prec != MSHQC_CD_FP64)) {
-        begin_stage(ctx, ST_TRANSFORM);
-        // shared over ranks: this rank's orbitals, then the gather of all
-        int64_t lo = 0, hi = s.nocc;
-        shard_range(ctx, s.nocc, &lo, &hi);
-        if (precision == MSHQC_CD_FP16X3 && int8_forward_enabled(ctx))
-            CD_RC(transform_i8(ctx, spin, lo, hi));
-        else
-            CD_RC(transform_f64(ctx, spin, lo, hi));
-        if (sharded(ctx))
-            CD_RC(run_collective(ctx, true, s.B64.as<double>(), shard_p(ctx, s.nocc) * s.vp * ctx->Mp));
-        end_stage(ctx);
-        s.B16_valid = false;
-    }
+    if (transform_needed(ctx, spin, precision)) CD_RC(run_transforms(ctx, 1, &spin, precision));
     if (precision == MSHQC_CD_FP16X3 && (!s.B16_valid || s.B16_layout != layout)) {
         begin_stage(ctx, ST_SPLIT);
         CD_RC(split_fixed(ctx, spin, layout));
         end_stage(ctx);
     }
+    return MSHQC_CD_OK;
+}
+
+// Both spins: in one pass over the vectors where both need it and fit.
+int ensure_transforms(mshqc_cd_ctx* ctx, int precision, int layout) {
+    CD_RC(require_inputs(ctx, 0));
+    CD_RC(require_inputs(ctx, 1));
+    if ((precision == MSHQC_CD_FP64 || precision == MSHQC_CD_FP16X3) && transform_needed(ctx, 0, precision) &&
+        transform_needed(ctx, 1, precision)) {
+        bool fit = false;
+        CD_RC(both_spins_fit(ctx, &fit));
+        const int spins[2] = {0, 1};
+        if (fit) CD_RC(run_transforms(ctx, 2, spins, precision));
+    }
+    for (int s = 0; s < 2; ++s) CD_RC(ensure_transform(ctx, s, precision, layout));
     return MSHQC_CD_OK;
 }
 
@@ -862,8 +929,10 @@ int run_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* out)
     if (kind == MSHQC_CD_UNRESTRICTED) CD_RC(require_inputs(ctx, 1));
     cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2];
     CD_CUDA(cudaEventRecord(e0, ctx->stream));
-    CD_RC(ensure_transform(ctx, 0, precision, 1));
-    if (kind == MSHQC_CD_UNRESTRICTED) CD_RC(ensure_transform(ctx, 1, precision, 1));
+    if (kind == MSHQC_CD_UNRESTRICTED)
+        CD_RC(ensure_transforms(ctx, precision, 1));
+    else
+        CD_RC(ensure_transform(ctx, 0, precision, 1));
     CD_CUDA(cudaEventRecord(e1, ctx->stream));
     for (auto& p : ctx->pair_energy) p.clear();
     if (kind == MSHQC_CD_RESTRICTED) {
@@ -899,124 +968,73 @@ int run_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* out)
 // ---------------------------------------------------------------------------
 namespace {
 
-// dE/dC of one spin from Gamma (ctx->gam[spin], [o][vp][Mp] FP64) with
-// dE/dB = scale * Gamma (4 restricted, 2 unrestricted):
-// dC[nu, o+a] = sum_{i,Q} dE/dB[i][a][Q] Y[i][Q][nu],
-// dC[mu, i]   = sum_{Q,nu} L[Q][nu][mu] sum_a dE/dB[i][a][Q] C[nu, o+a].
-// The transforms shared over ranks: rank r's Gamma rows [lo, hi) are
-// completed by the reduce-scatter, and its transposed transforms cover those
-// orbitals only (dC's other occupied columns zero); unshared: [0, o).
-// Makes sure the buffer Y holds the half-transformed vectors of [lo, hi).
-int transposed_prepare(mshqc_cd_ctx* ctx, int spin, bool i8, int64_t* lo, int64_t* hi, double* dC) {
-    SpinState& s = ctx->spin[spin];
-    shard_range(ctx, s.nocc, lo, hi);
-    if (sharded(ctx))
-        CD_RC(run_collective(ctx, false, ctx->gam[spin].as<double>(), shard_p(ctx, s.nocc) * s.vp * ctx->Mp));
-    if (ctx->Y_spin != spin || ctx->Y_lo != *lo || ctx->Y_hi != *hi) {
-        // recomputing Y rewrites B as well; shared, only this rank's rows of it
-        if (i8)
-            CD_RC(transform_i8(ctx, spin, *lo, *hi));
-        else
-            CD_RC(transform_f64(ctx, spin, *lo, *hi));
-        if (sharded(ctx)) s.B64_valid = false;
-    }
-    if (*hi - *lo < s.nocc) CD_CUDA(cudaMemsetAsync(dC, 0, sizeof(double) * (size_t)(s.nocc * ctx->N), ctx->stream));
-    if (*hi <= *lo)
-        CD_CUDA(cudaMemsetAsync(dC + s.nocc * ctx->N, 0, sizeof(double) * (size_t)((ctx->N - s.nocc) * ctx->N),
-                                ctx->stream));
-    return MSHQC_CD_OK;
-}
-
-int transposed_transforms(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
-    SpinState& s = ctx->spin[spin];
-    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, vp = s.vp;
-    // Y[i][Q][nu] (half-transformed vectors of this spin) is needed
-    int64_t lo = 0, hi = o;
-    CD_RC(transposed_prepare(ctx, spin, false, &lo, &hi, dC));
-    const int64_t ni = hi - lo;
-    if (ni <= 0) return MSHQC_CD_OK;
-    const double* C = s.C.as<double>();
-    const double* Gm = ctx->gam[spin].as<double>();
-    // dC[nu, o+a] = scale sum_{i,Q} Gamma[i][a][Q] Y[i][Q][nu]   (row-major [a][nu] == column-major dC)
-    // one product over the composite K = (i, Q): v x N output tiles alone
-    // leave most SMs idle at small v
-    {
-        GemmF64Args g{};
-        g.M = (int)v;  g.N = (int)N;  g.K = (int)M;  g.batch = 1;
-        g.kb = (int)ni;
-        g.A = Gm + lo * vp * Mp;  g.lda = Mp;  g.skA = vp * Mp;
-        g.B = ctx->Y.as<double>();  g.ldb = N;  g.skB = M * N;
-        g.C = dC + o * N;  g.ldc = N;  g.sC = 0;
-        g.alpha = scale;  g.beta = 0.0;
-        CD_RC(gemm_run(ctx, g, true, false));
-    }
-    // W[i][Q][nu] = sum_a Gamma[i][a][Q] C[nu, o+a]   (into the Y buffer)
-    {
-        GemmF64Args g{};
-        g.M = (int)M;  g.N = (int)N;  g.K = (int)v;  g.batch = (int)ni;
-        g.A = Gm + lo * vp * Mp;  g.lda = Mp;  g.sA = vp * Mp;
-        g.B = C + o * N;  g.ldb = N;  g.sB = 0;
-        g.C = ctx->Y.as<double>();  g.ldc = N;  g.sC = M * N;
-        g.alpha = 1.0;  g.beta = 0.0;
-        CD_RC(gemm_run(ctx, g, false, false));
-        ctx->Y_spin = -1;
-    }
-    // dC[mu, i] = scale sum_{(Q,nu)} W[i][(Q,nu)] L[(Q,nu)][mu], one chunk of
-    // vectors at a time (only ni rows: K is what fills the GPU)
-    const int64_t qc = vectors_chunk_size(ctx);
-    for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
-        const int64_t mc = std::min(qc, M - Q0);
-        const double* Lc = nullptr;
-        CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
-        GemmF64Args g{};
-        g.M = (int)ni;  g.N = (int)N;  g.K = (int)(mc * N);  g.batch = 1;
-        g.A = ctx->Y.as<double>() + Q0 * N;  g.lda = M * N;  g.sA = 0;
-        g.B = Lc;  g.ldb = N;  g.sB = 0;
-        g.C = dC + lo * N;  g.ldc = N;  g.sC = 0;
-        g.alpha = scale;  g.beta = Q0 == 0 ? 0.0 : 1.0;
-        CD_RC(gemm_run(ctx, g, true, false));
-    }
-    return MSHQC_CD_OK;
-}
-
-// out[k] = (accumulate ? out[k] : 0) + alpha * sum_b parts[b * n + k], b in order
-__global__ void sum_batches_kernel(const double* __restrict__ parts, int nb, int64_t n, double alpha,
+// out[k] = (accumulate ? out[k] : 0) + alpha * sum_b parts[b * stride + k], b in order
+__global__ void sum_batches_kernel(const double* __restrict__ parts, int nb, int64_t stride, int64_t n, double alpha,
                                    int accumulate, double* __restrict__ out) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
     double acc = 0.0;
-    for (int b = 0; b < nb; ++b) acc += parts[(int64_t)b * n + k];
+#pragma unroll 8
+    for (int b = 0; b < nb; ++b) acc += parts[(int64_t)b * stride + k];
     out[k] = accumulate ? out[k] + alpha * acc : alpha * acc;
 }
 
-int sum_batches(mshqc_cd_ctx* ctx, const double* parts, int nb, int64_t n, double alpha, bool accumulate,
-                double* out) {
-    sum_batches_kernel<<<(unsigned)cdiv(n, 256), 256, 0, ctx->stream>>>(parts, nb, n, alpha, accumulate ? 1 : 0,
-                                                                         out);
+int sum_batches(mshqc_cd_ctx* ctx, const double* parts, int nb, int64_t stride, int64_t n, double alpha,
+                bool accumulate, double* out) {
+    if (n <= 0) return MSHQC_CD_OK;
+    sum_batches_kernel<<<(unsigned)cdiv(n, 256), 256, 0, ctx->stream>>>(parts, nb, stride, n, alpha,
+                                                                         accumulate ? 1 : 0, out);
     CD_CUDA(cudaGetLastError());
     ctx->launches++;
     return MSHQC_CD_OK;
 }
 
-// The transposed transforms of the mixed path on the int8 tensor cores
-// (ozaki_i8.cuh), batched so that every product has K = M, v or N:
-//   dC[nu, o+a] = scale sum_i (Gamma_i Y_i)[a][nu]        batches of i, partials summed in order
-//   W_i[Q][nu]  = sum_a Gamma_i[a][Q] C[nu, o+a]           batches of i, C_vir shared
-//   dC[mu, i]   = scale sum_Q (W_Q L_Q)[i][mu]             batches of Q per vectors chunk
-// with W_Q[i][nu] = W[i][Q][nu] and L_Q[mu][nu] = L[Q][nu][mu].
-int transposed_transforms_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
+// dE/dC from Gamma (ctx->gam[spin], [o][vp][Mp] FP64) with dE/dB = scale * Gamma
+// (4 restricted, 2 unrestricted):
+//   dC[nu, o+a] = sum_{i,Q} dE/dB[i][a][Q] Y[i][Q][nu],
+//   W[i][Q][nu] = sum_a dE/dB[i][a][Q] C[nu, o+a]      (into the rows of Y),
+//   dC[mu, i]   = sum_{Q,nu} L[Q][nu][mu] W[i][Q][nu].
+// The first two per spin here, the last for all spins at once in occupied_part.
+// The transforms shared over ranks: rank r's Gamma rows [lo, hi) are completed
+// by the reduce-scatter, and its transposed transforms cover those orbitals
+// only (dC's other occupied columns zero); unshared: [0, o).
+int virtual_part_f64(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
+    const SpinState& s = ctx->spin[spin];
+    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, vp = s.vp;
+    const int64_t lo = ctx->Yr[spin].lo, ni = ctx->Yr[spin].hi - lo;
+    const double* Gm = ctx->gam[spin].as<double>() + lo * vp * Mp;
+    double* Y = y_rows(ctx, spin);
+    // dC[nu, o+a] (row-major [a][nu] == column-major dC): one product over the
+    // composite K = (i, Q); v x N output tiles alone leave most SMs idle at
+    // small v
+    GemmF64Args g{};
+    g.M = (int)v;  g.N = (int)N;  g.K = (int)M;  g.batch = 1;
+    g.kb = (int)ni;
+    g.A = Gm;  g.lda = Mp;  g.skA = vp * Mp;
+    g.B = Y;  g.ldb = N;  g.skB = M * N;
+    g.C = dC + o * N;  g.ldc = N;  g.sC = 0;
+    g.alpha = scale;  g.beta = 0.0;
+    CD_RC(gemm_run(ctx, g, true, false));
+    GemmF64Args w{};
+    w.M = (int)M;  w.N = (int)N;  w.K = (int)v;  w.batch = (int)ni;
+    w.A = Gm;  w.lda = Mp;  w.sA = vp * Mp;
+    w.B = s.C.as<double>() + o * N;  w.ldb = N;  w.sB = 0;
+    w.C = Y;  w.ldc = N;  w.sC = M * N;
+    w.alpha = 1.0;  w.beta = 0.0;
+    return gemm_run(ctx, w, false, false);
+}
+
+// The same on the int8 tensor cores (ozaki::Mixed), batched over orbitals i so
+// that every product has K = M or v; the partial dC of the batches are summed
+// in order.
+int virtual_part_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
     using Cfg = ozaki::Mixed;
-    SpinState& s = ctx->spin[spin];
-    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o;
-    int64_t lo = 0, hi = o;
-    CD_RC(transposed_prepare(ctx, spin, true, &lo, &hi, dC));
-    const int64_t ni = hi - lo;
-    if (ni <= 0) return MSHQC_CD_OK;
-    const int64_t vp = s.vp;
+    const SpinState& s = ctx->spin[spin];
+    const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, vp = s.vp;
+    const int64_t lo = ctx->Yr[spin].lo, hi = ctx->Yr[spin].hi, ni = hi - lo;
     const double* C = s.C.as<double>();
     const double* Gm = ctx->gam[spin].as<double>();
-    double* Y = ctx->Y.as<double>();
-    CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
+    double* Y = y_rows(ctx, spin);
     // dC[nu, o+a]: Gamma_i (rows a, K = Q) against Y_i^T (rows nu, K = Q, strided by N)
     {
         const bool sw = oz_swap<Cfg>(v, N);
@@ -1034,11 +1052,11 @@ int transposed_transforms_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* 
             CD_CUDA(ozaki_slice_t<Cfg>(Y + (i0 - lo) * M * N, N, M * N, B, ctx->stream));
             ctx->launches += 3;
             CD_RC(oz_mul<Cfg>(ctx, A, false, B, false, sw, ctx->oz_p.as<double>(), N, v * N, 1.0, 0.0));
-            CD_RC(sum_batches(ctx, ctx->oz_p.as<double>(), (int)nb, v * N, scale, i0 > lo, dC + o * N));
+            CD_RC(sum_batches(ctx, ctx->oz_p.as<double>(), (int)nb, v * N, v * N, scale, i0 > lo, dC + o * N));
         }
     }
-    // W[i][Q][nu] into the Y buffer: Gamma_i^T (rows Q, K = a, strided by Mp)
-    // against C_vir^T (rows nu, K = a, strided by N), shared
+    // W[i][Q][nu] into Y: Gamma_i^T (rows Q, K = a, strided by Mp) against
+    // C_vir^T (rows nu, K = a, strided by N), shared
     {
         const bool sw = oz_swap<Cfg>(M, N);
         const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(M, v, !sw, 1));
@@ -1055,45 +1073,140 @@ int transposed_transforms_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* 
             ctx->launches += 2;
             CD_RC(oz_mul<Cfg>(ctx, A, false, B, true, sw, Y + (i0 - lo) * M * N, N, M * N, 1.0, 0.0));
         }
-        ctx->Y_spin = -1;
     }
-    // dC[mu, i]: W_Q (rows i, K = nu) against L_Q (rows mu, K = nu, strided by N)
-    {
-        const bool sw = oz_swap<Cfg>(ni, N);
-        const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(ni, N, !sw, 1));
-        const size_t pb = oz_bytes<Cfg>(oz_operand<Cfg>(N, N, sw, 1));
-        const size_t pp = sizeof(double) * (size_t)(ni * N);
-        const int64_t nq_max = std::max<int64_t>(1, (int64_t)(2 * kSliceBytes / (pa + pb + pp)));
-        const int64_t qc = vectors_chunk_size(ctx);
-        // (batches are the z dimension of the transposed-slicing grid)
-        const int64_t nq = std::min<int64_t>(std::min(nq_max, qc), 65535);
-        CD_ALLOC(ctx->oz_p, pp * nq, false);
+    return MSHQC_CD_OK;
+}
+
+// dC[mu, i] = scale sum_{Q,nu} W[i][Q][nu] L[Q][nu][mu] for the W rows of the
+// given spins (consecutive rows of Y, both spins in one product): over chunks of
+// vectors, FP64 with K = (Q, nu), or per vector on the int8 tensor cores
+// (W_Q rows i against L_Q rows mu, K = nu) with the partials summed in order.
+// The rows of L_Q are contiguous when the vectors are symmetric (the same
+// digits either way); otherwise they are sliced from the strided columns.
+int occupied_part(mshqc_cd_ctx* ctx, int nsp, const int* spins, double scale, double* const* dC, bool i8) {
+    using Cfg = ozaki::Mixed;
+    const int64_t N = ctx->N, M = ctx->M;
+    int64_t rows = 0, off[2] = {0, 0}, ni[2] = {0, 0};
+    for (int k = 0; k < nsp; ++k) {
+        const auto& y = ctx->Yr[spins[k]];
+        off[k] = rows;
+        ni[k] = y.hi - y.lo;
+        rows += ni[k];
+    }
+    if (rows <= 0) return MSHQC_CD_OK;
+    const double* W = y_rows(ctx, spins[0]);
+    const int64_t qc = vectors_chunk_size(ctx);
+    if (!i8) {
+        double* out = dC[0] + ctx->Yr[spins[0]].lo * N;
+        if (nsp == 2) {
+            CD_ALLOC(ctx->occ_parts, sizeof(double) * (size_t)(rows * N), false);
+            out = ctx->occ_parts.as<double>();
+        }
         for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
             const int64_t mc = std::min(qc, M - Q0);
             const double* Lc = nullptr;
             CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
-            for (int64_t q0 = 0; q0 < mc; q0 += nq) {
-                const int64_t nb = std::min(nq, mc - q0);
-                OzakiOperand A = oz_operand<Cfg>(ni, N, !sw, nb), B = oz_operand<Cfg>(N, N, sw, nb);
-                CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
-                CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
-                CD_CUDA(ozaki_slice<Cfg>(Y + (Q0 + q0) * N, M * N, N, A, ctx->num_sms, ctx->stream));
+            // only `rows` rows: K is what fills the GPU
+            GemmF64Args g{};
+            g.M = (int)rows;  g.N = (int)N;  g.K = (int)(mc * N);  g.batch = 1;
+            g.A = W + Q0 * N;  g.lda = M * N;  g.sA = 0;
+            g.B = Lc;  g.ldb = N;  g.sB = 0;
+            g.C = out;  g.ldc = N;  g.sC = 0;
+            g.alpha = scale;  g.beta = Q0 == 0 ? 0.0 : 1.0;
+            CD_RC(gemm_run(ctx, g, true, false));
+        }
+        for (int k = 0; k < nsp && nsp == 2; ++k)
+            if (ni[k] > 0)
+                CD_CUDA(cudaMemcpyAsync(dC[k] + ctx->Yr[spins[k]].lo * N, out + off[k] * N,
+                                        sizeof(double) * (size_t)(ni[k] * N), cudaMemcpyDeviceToDevice, ctx->stream));
+        return MSHQC_CD_OK;
+    }
+    bool sym = false;
+    CD_RC(vectors_symmetric(ctx, &sym));
+    const bool sw = oz_swap<Cfg>(rows, N);
+    const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(rows, N, !sw, 1));
+    const size_t pb = oz_bytes<Cfg>(oz_operand<Cfg>(N, N, sw, 1));
+    const size_t pp = sizeof(double) * (size_t)(rows * N);
+    const int64_t nq_max = std::max<int64_t>(1, (int64_t)(2 * kSliceBytes / (pa + pb + pp)));
+    // (batches are a grid dimension of the slicing kernels)
+    const int64_t nq = std::min<int64_t>(std::min(nq_max, qc), 65535);
+    CD_ALLOC(ctx->oz_p, pp * nq, false);
+    for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
+        const int64_t mc = std::min(qc, M - Q0);
+        const double* Lc = nullptr;
+        CD_RC(vectors_chunk(ctx, Q0, mc, &Lc));
+        for (int64_t q0 = 0; q0 < mc; q0 += nq) {
+            const int64_t nb = std::min(nq, mc - q0);
+            OzakiOperand A = oz_operand<Cfg>(rows, N, !sw, nb), B = oz_operand<Cfg>(N, N, sw, nb);
+            CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+            CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
+            CD_CUDA(ozaki_slice<Cfg>(W + (Q0 + q0) * N, M * N, N, A, ctx->num_sms, ctx->stream));
+            if (sym)
+                CD_CUDA(ozaki_slice<Cfg>(Lc + q0 * N * N, N, N * N, B, ctx->num_sms, ctx->stream));
+            else
                 CD_CUDA(ozaki_slice_t<Cfg>(Lc + q0 * N * N, N, N * N, B, ctx->stream));
-                ctx->launches += 3;
-                CD_RC(oz_mul<Cfg>(ctx, A, false, B, false, sw, ctx->oz_p.as<double>(), N, ni * N, 1.0, 0.0));
-                CD_RC(sum_batches(ctx, ctx->oz_p.as<double>(), (int)nb, ni * N, scale, Q0 + q0 > 0, dC + lo * N));
-            }
+            ctx->launches += sym ? 2 : 3;
+            CD_RC(oz_mul<Cfg>(ctx, A, false, B, false, sw, ctx->oz_p.as<double>(), N, rows * N, 1.0, 0.0));
+            for (int k = 0; k < nsp; ++k)
+                CD_RC(sum_batches(ctx, ctx->oz_p.as<double>() + off[k] * N, (int)nb, rows * N, ni[k] * N, scale,
+                                  Q0 + q0 > 0, dC[k] + ctx->Yr[spins[k]].lo * N));
         }
     }
-    return oz_check(ctx, "int8 tensor-core transposed transform");
+    return MSHQC_CD_OK;
 }
 
-// dE/dC of one spin: the int8-slice transposed transforms for the mixed path
-// (unless switched off), FP64 otherwise
-int transposed_dispatch(mshqc_cd_ctx* ctx, int spin, double scale, double* dC, int precision) {
-    if (precision == MSHQC_CD_FP16X3 && int8_transform_enabled(ctx))
-        return transposed_transforms_i8(ctx, spin, scale, dC);
-    return transposed_transforms(ctx, spin, scale, dC);
+// The transposed transforms of the given spins.  Y of the orbitals is reused
+// where the forward transforms left it; the open-shell int8 products take it
+// from int8 slices always (the sizes whose forward transform is FP64 form it
+// again).
+int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double scale, double* const* dC, bool i8) {
+    int64_t lo[2], hi[2];
+    bool have = true;
+    for (int k = 0; k < nsp; ++k) {
+        const SpinState& s = ctx->spin[spins[k]];
+        shard_range(ctx, s.nocc, &lo[k], &hi[k]);
+        if (sharded(ctx))
+            CD_RC(run_collective(ctx, false, ctx->gam[spins[k]].as<double>(),
+                                 shard_p(ctx, s.nocc) * s.vp * ctx->Mp));
+        if (hi[k] - lo[k] < s.nocc)
+            CD_CUDA(cudaMemsetAsync(dC[k], 0, sizeof(double) * (size_t)(s.nocc * ctx->N), ctx->stream));
+        if (hi[k] <= lo[k])
+            CD_CUDA(cudaMemsetAsync(dC[k] + s.nocc * ctx->N, 0,
+                                    sizeof(double) * (size_t)((ctx->N - s.nocc) * ctx->N), ctx->stream));
+        const auto& y = ctx->Yr[spins[k]];
+        have = have && y.ok && y.lo == lo[k] && y.hi == hi[k] && !(nsp == 2 && i8 && !y.i8);
+    }
+    if (!have) {
+        bool fit = nsp == 1;
+        if (nsp == 2) CD_RC(both_spins_fit(ctx, &fit));
+        if (!fit) {   // one spin after the other
+            for (int k = 0; k < nsp; ++k) {
+                CD_RC(first_half(ctx, 1, &spins[k], &lo[k], &hi[k], i8));
+                if (hi[k] <= lo[k]) continue;
+                CD_RC(i8 ? virtual_part_i8(ctx, spins[k], scale, dC[k])
+                         : virtual_part_f64(ctx, spins[k], scale, dC[k]));
+                CD_RC(occupied_part(ctx, 1, &spins[k], scale, &dC[k], i8));
+                ctx->Yr[spins[k]].ok = false;
+            }
+            return MSHQC_CD_OK;
+        }
+        CD_RC(first_half(ctx, nsp, spins, lo, hi, i8));
+    }
+    if (i8) CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, have);   // (the first half has zeroed it otherwise)
+    for (int k = 0; k < nsp; ++k) {
+        if (hi[k] <= lo[k]) continue;
+        CD_RC(i8 ? virtual_part_i8(ctx, spins[k], scale, dC[k]) : virtual_part_f64(ctx, spins[k], scale, dC[k]));
+    }
+    CD_RC(occupied_part(ctx, nsp, spins, scale, dC, i8));
+    for (int k = 0; k < nsp; ++k) ctx->Yr[spins[k]].ok = false;   // W is there now
+    return MSHQC_CD_OK;
+}
+
+// the int8 products for the mixed path (unless switched off), FP64 otherwise
+int transposed_dispatch(mshqc_cd_ctx* ctx, int nsp, const int* spins, double scale, double* const* dC, int precision) {
+    const bool i8 = precision == MSHQC_CD_FP16X3 && int8_transform_enabled(ctx);
+    CD_RC(transposed_transforms(ctx, nsp, spins, scale, dC, i8));
+    return i8 ? oz_check(ctx, "int8 tensor-core transposed transform") : MSHQC_CD_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1482,7 +1595,8 @@ int gradient_restricted_f64(mshqc_cd_ctx* ctx, double* dC, double* deps, double*
     CD_CUDA(cudaMemcpyAsync(energy, ctx->totals.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CD_CUDA(cudaStreamSynchronize(ctx->stream));
     begin_stage(ctx, ST_TRANSPOSED);
-    CD_RC(transposed_dispatch(ctx, 0, 4.0, dC, MSHQC_CD_FP64));
+    const int spins[1] = {0};
+    CD_RC(transposed_dispatch(ctx, 1, spins, 4.0, &dC, MSHQC_CD_FP64));
     end_stage(ctx);
     return MSHQC_CD_OK;
 }
@@ -1514,7 +1628,8 @@ int gradient_restricted_tc(mshqc_cd_ctx* ctx, double* dC, double* deps, double* 
                                                    std::to_string(herr[0] ? herr[0] : herr[2]) + ")");
     if (herr[1]) ctx->fixed_point_exact = 0;
     begin_stage(ctx, ST_TRANSPOSED);
-    CD_RC(transposed_dispatch(ctx, 0, 4.0, dC, MSHQC_CD_FP16X3));
+    const int spins[1] = {0};
+    CD_RC(transposed_dispatch(ctx, 1, spins, 4.0, &dC, MSHQC_CD_FP16X3));
     end_stage(ctx);
     return MSHQC_CD_OK;
 }
@@ -1566,8 +1681,8 @@ int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2],
                                                    std::to_string(herr[0] ? herr[0] : herr[2]) + ")");
     if (herr[1]) ctx->fixed_point_exact = 0;
     begin_stage(ctx, ST_TRANSPOSED);
-    CD_RC(transposed_dispatch(ctx, 0, 2.0, dC[0], precision));
-    CD_RC(transposed_dispatch(ctx, 1, 2.0, dC[1], precision));
+    const int spins[2] = {0, 1};
+    CD_RC(transposed_dispatch(ctx, 2, spins, 2.0, dC, precision));
     end_stage(ctx);
     return MSHQC_CD_OK;
 }
@@ -1660,8 +1775,10 @@ int run_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* e_
     cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2];
     reset_stages(ctx);
     CD_CUDA(cudaEventRecord(e0, ctx->stream));
-    CD_RC(ensure_transform(ctx, 0, precision));
-    if (unres) CD_RC(ensure_transform(ctx, 1, precision));
+    if (unres)
+        CD_RC(ensure_transforms(ctx, precision));
+    else
+        CD_RC(ensure_transform(ctx, 0, precision));
     CD_CUDA(cudaEventRecord(e1, ctx->stream));
     if (ctx->part_active) CD_RC(plan_partition(ctx, kind, precision));
     double* dC[2] = {nullptr, nullptr};

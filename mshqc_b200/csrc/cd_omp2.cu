@@ -259,7 +259,7 @@ int occupied_density(mshqc_cd_ctx* ctx, const double* C, int64_t o, double* P) {
 // *e_mp2 receives the OMP2 energy (same-spin + opposite-spin).
 int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffers& b, double* e_mp2) {
     const int64_t N = ctx->N, M = ctx->M, NN = N * N;
-    for (int s = 0; s < 2; ++s) CD_RC(ensure_transform(ctx, s, MSHQC_CD_FP64));
+    CD_RC(ensure_transforms(ctx, MSHQC_CD_FP64));
     CD_RC(omp2_buffers(ctx, b));
     const int64_t o0 = ctx->spin[0].nocc, o1 = ctx->spin[1].nocc;
     const int64_t vp0 = ctx->spin[0].vp, vp1 = ctx->spin[1].vp;

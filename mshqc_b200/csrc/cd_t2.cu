@@ -52,8 +52,10 @@ extern "C" MSHQC_CD_API int mshqc_cd_get_t2_block(mshqc_cd_ctx* ctx, int block, 
     const int64_t ox = ctx->spin[sx].nocc, oy = ctx->spin[sy].nocc;
     if (i0 < 0 || ni < 1 || i0 + ni > ox || j0 < 0 || nj < 1 || j0 + nj > oy)
         return set_error(MSHQC_CD_ERR_ARG, "pair block outside the occupied orbitals");
-    CD_RC(ensure_transform(ctx, sx, MSHQC_CD_FP64));
-    if (sy != sx) CD_RC(ensure_transform(ctx, sy, MSHQC_CD_FP64));
+    if (sy != sx)
+        CD_RC(ensure_transforms(ctx, MSHQC_CD_FP64));
+    else
+        CD_RC(ensure_transform(ctx, sx, MSHQC_CD_FP64));
     const SpinState& X = ctx->spin[sx];
     const SpinState& Y = ctx->spin[sy];
     const int64_t vx = ctx->N - ox, vy = ctx->N - oy, Mp = ctx->Mp;

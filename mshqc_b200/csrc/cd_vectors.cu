@@ -99,6 +99,34 @@ __global__ void __launch_bounds__(256) gen_vectors_kernel(uint64_t seed, const d
     }
 }
 
+// *diff != 0 when an element differs from its mirror image (grid: tile pairs of
+// 32 x 32, vectors); bits are compared, so a NaN or a signed zero counts as is
+__global__ void __launch_bounds__(256) symmetry_kernel(const double* __restrict__ L, int64_t N, int64_t M,
+                                                       int* __restrict__ diff) {
+    __shared__ long long tile[32][33];
+    const int nb = (int)((N + 31) / 32);
+    const int x = (int)(blockIdx.x / nb), y = (int)(blockIdx.x % nb);
+    if (y < x) return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    bool bad = false;
+    for (int64_t q = blockIdx.y; q < M; q += gridDim.y) {
+        const double* l = L + q * N * N;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t mu = (int64_t)x * 32 + ty + 8 * k, nu = (int64_t)y * 32 + tx;
+            tile[ty + 8 * k][tx] = mu < N && nu < N ? __double_as_longlong(l[mu * N + nu]) : 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t nu = (int64_t)y * 32 + ty + 8 * k, mu = (int64_t)x * 32 + tx;
+            if (mu < N && nu < N) bad |= __double_as_longlong(l[nu * N + mu]) != tile[tx][ty + 8 * k];
+        }
+        __syncthreads();
+    }
+    if (bad) *diff = 1;
+}
+
 constexpr size_t kChunkBytes = size_t(2) << 30;   // generated vectors per chunk: 2 GB
 
 }  // namespace
@@ -112,6 +140,30 @@ int64_t vectors_chunk_size(const mshqc_cd_ctx* ctx) {
     }
     const int64_t per_q = ctx->N * ctx->N * (int64_t)sizeof(double);
     return std::max<int64_t>(1, std::min<int64_t>(ctx->M, (int64_t)kChunkBytes / per_q));
+}
+
+// One pass over the stored vectors, once per set of vectors (generated ones are
+// symmetric as written).
+int vectors_symmetric(mshqc_cd_ctx* ctx, bool* yes) {
+    if (ctx->L_gen) {
+        *yes = true;
+        return MSHQC_CD_OK;
+    }
+    if (ctx->L_sym < 0) {
+        const int64_t nb = cdiv(ctx->N, 32);
+        CD_ALLOC(ctx->pace, sizeof(int) * 256, false);
+        CD_CUDA(cudaMemsetAsync(ctx->pace.p, 0, sizeof(int), ctx->stream));
+        dim3 grid((unsigned)(nb * nb), (unsigned)std::min<int64_t>(ctx->M, 65535));
+        symmetry_kernel<<<grid, 256, 0, ctx->stream>>>(ctx->L.as<double>(), ctx->N, ctx->M, ctx->pace.as<int>());
+        CD_CUDA(cudaGetLastError());
+        ctx->launches++;
+        int diff = 0;
+        CD_CUDA(cudaMemcpyAsync(&diff, ctx->pace.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CD_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->L_sym = diff ? 0 : 1;
+    }
+    *yes = ctx->L_sym == 1;
+    return MSHQC_CD_OK;
 }
 
 int vectors_chunk(mshqc_cd_ctx* ctx, int64_t Q0, int64_t mc, const double** out) {
