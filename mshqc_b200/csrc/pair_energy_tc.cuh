@@ -27,8 +27,11 @@
 // pair_energy_f64.cuh) into partial[unit].  (ia|jb) and the amplitudes are
 // never written to memory.
 //
-// Warp roles (192 threads): warp 0 producer (bulk copies), warp 1 MMA issuer
-// and TMEM owner, warps 2..5 epilogue (TMEM lane quadrant = warp % 4).
+// Warp roles (576 threads): warp 0 producer (bulk copies), warp 1 MMA issuer
+// and TMEM owner, warps 2..17 epilogue (TMEM lane quadrant warp % 4, 32 of the
+// 128 columns each).  The accumulators fill TMEM, so a unit's MMAs wait for the
+// epilogue before it; with four epilogue warps half of a unit's time at 100 Q
+// chunks was that wait.
 // Every wait is bounded (kWaitLimitNs); on a timeout the kernel records the
 // site in *err, drains its own copies and MMAs (again bounded), frees TMEM and
 // returns.
@@ -69,13 +72,14 @@ constexpr int BN = 128;
 constexpr int KC = 16;
 constexpr int KS = 2;                      // Q chunks per stage
 constexpr int STAGES = 3;
-constexpr int THREADS = 192;
+constexpr int EPI_WARPS = 16;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr uint32_t SLAB = 128 * KC * 2;    // 4096 bytes: 128 rows x one chunk, hi or lo
 constexpr uint32_t CHUNK = 2 * SLAB;       // hi and lo of one chunk
 constexpr uint32_t PIECE = KS * CHUNK;     // one operand of a stage (16 KB)
 constexpr uint32_t STAGE_BYTES = 4 * PIECE;                  // 65536: P0 P1 P2 P3
 constexpr uint32_t SMEM_DATA = STAGES * STAGE_BYTES;         // 196608
-// after the data: barriers (< 256 B), reduction scratch (64 B at +256),
+// after the data: barriers (< 256 B), reduction scratch (256 B at +256),
 // per-unit column tables at +512: eps (2 x 128 doubles), column scales
 // (2 x 128 doubles)
 constexpr uint32_t OFF_AUX = 512;
@@ -90,7 +94,7 @@ __device__ __forceinline__ double pow2d(int e) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
+__global__ void __launch_bounds__(pair_tc::THREADS, 1) pair_energy_tc_kernel(PairTcArgs p) {
     using namespace pair_tc;
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
@@ -102,7 +106,7 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
     uint64_t* drain = tmem_empty + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    double* red = reinterpret_cast<double*>(smem + SMEM_DATA + 256);           // 8 doubles
+    double* red = reinterpret_cast<double*>(smem + SMEM_DATA + 256);           // 32 doubles
     double* eb_s = reinterpret_cast<double*>(smem + SMEM_DATA + OFF_AUX);      // 256
     double* cs_s = eb_s + 256;                                                 // 256
 
@@ -114,7 +118,7 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
             mbar_init(&empty[s], 1);
         }
         mbar_init(tmem_full, 1);
-        mbar_init(tmem_empty, 4);
+        mbar_init(tmem_empty, EPI_WARPS);
         mbar_init(drain, 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -249,8 +253,9 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
     } else {
         // ------------------------------------------------------------ epilogue
         const int q = warp & 3;                       // TMEM lane quadrant of this warp
+        const int part = (warp - 2) >> 2;             // its quarter of the columns
         const int row = q * 32 + lane;                // a offset within the row block
-        const int etid = threadIdx.x - 64;            // 0..127
+        const int etid = threadIdx.x - 64;
         uint32_t acc_phase = 0;
         for (long long u = first; u < p.units; u += step) {
             const int2 ij = p.pairs[u / p.nblocks];
@@ -259,7 +264,7 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
             const int a = xy.x * BM + row;
             const int b0 = xy.y * BN;
             // per-unit column tables (eps and scales of T1 / T2 columns)
-            for (int c = etid; c < 2 * BN; c += 128) {
+            for (int c = etid; c < 2 * BN; c += 32 * EPI_WARPS) {
                 const int half = c / BN, cc = c % BN;
                 double eb = 0.0, cs = 0.0;
                 if (MODE == PAIR_OPPOSITE_SPIN) {
@@ -279,11 +284,11 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
                 eb_s[c] = eb;
                 cs_s[c] = cs;
             }
-            // the four epilogue warps leave together (a named barrier must
+            // the epilogue warps leave together (a named barrier must
             // never wait for a warp that already left the loop)
-            if (bar_any(1, 128, *abort_flag != 0)) break;
+            if (bar_any(1, 32 * EPI_WARPS, *abort_flag != 0)) break;
             const bool got = mbar_wait_bounded(tmem_full, acc_phase, kWaitLimitNs);
-            if (bar_any(1, 128, !got)) {
+            if (bar_any(1, 32 * EPI_WARPS, !got)) {
                 if (!got) atomicExch(p.err, 4);
                 *abort_flag = 1;
                 break;
@@ -316,9 +321,9 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
             double s_acc = 0.0, o_acc = 0.0;
             float amax = 0.0f;
             const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
-            constexpr int CW = 32;   // columns per TMEM read
+            constexpr int CW = 8;    // columns per TMEM read (18 warps: 96 registers a thread)
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += CW) {
+            for (int c0 = part * (BN / 4); c0 < (part + 1) * (BN / 4); c0 += CW) {
                 uint32_t h1[CW], x1[CW], h2[CW], x2[CW];
                 tmem_ld<CW>(lane_base + 0 + c0, h1);
                 tmem_ld<CW>(lane_base + 128 + c0, x1);
@@ -386,13 +391,18 @@ __global__ void __launch_bounds__(192, 1) pair_energy_tc_kernel(PairTcArgs p) {
                 tot2 += __shfl_xor_sync(0xffffffffu, tot2, off);
             }
             if (lane == 0) {
-                red[q] = tot1;
-                red[4 + q] = tot2;
+                red[warp - 2] = tot1;
+                red[EPI_WARPS + warp - 2] = tot2;
             }
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");
-            if (etid == 0) {
-                p.partial[u] = ((red[0] + red[1]) + (red[2] + red[3]));
-                if (MODE == PAIR_RESTRICTED) p.partial2[u] = ((red[4] + red[5]) + (red[6] + red[7]));
+            asm volatile("bar.sync 1, %0;\n" ::"n"(32 * EPI_WARPS) : "memory");
+            // the 16 warps' parts in a fixed tree; red is written again only after
+            // the next unit's first barrier
+            if (etid < 32) {
+                double t = red[etid];
+#pragma unroll
+                for (int off = EPI_WARPS / 2; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+                if (etid == 0) p.partial[u] = t;
+                if (MODE == PAIR_RESTRICTED && etid == EPI_WARPS) p.partial2[u] = t;
             }
         }
     }

@@ -22,8 +22,11 @@
 // stores it rounded to FP32 into the row-major staging matrix S (row length
 // nbj * VS).  amp_elem.cuh turns S into amplitudes.
 //
-// Warp roles (192 threads): warp 0 producer, warp 1 MMA issuer and TMEM
-// owner, warps 2..5 epilogue.  Waits are bounded as in pair_energy_tc.cuh.
+// Warp roles (576 threads): warp 0 producer, warp 1 MMA issuer and TMEM
+// owner, warps 2..17 epilogue (TMEM lane quadrant warp % 4, column quarter
+// (warp - 2) / 4): the two accumulators fill TMEM, so a tile's MMAs wait for
+// the epilogue of the one before it, and four warps took as long over it as the
+// MMAs of 100 Q steps.  Waits are bounded as in pair_energy_tc.cuh.
 #pragma once
 
 #include "cd_common.cuh"
@@ -66,7 +69,7 @@ __device__ __forceinline__ bool vtile_unit(const VtileArgs& p, int u, int& rb, i
 }
 
 namespace vtile_tc {
-constexpr int BM = 128, BN = 256, KC = 16, KS = 2, STAGES = 4, THREADS = 192;
+constexpr int BM = 128, BN = 256, KC = 16, KS = 2, STAGES = 4, EPI_WARPS = 16, THREADS = 64 + 32 * EPI_WARPS;
 constexpr uint32_t SLAB_A = BM * KC * 2;     // 4 KB per Q step
 constexpr uint32_t SLAB_B = BN * KC * 2;     // 8 KB per Q step
 constexpr uint32_t OFF_AH = 0, OFF_AL = KS * SLAB_A, OFF_BH = 2 * KS * SLAB_A, OFF_BL = 2 * KS * SLAB_A + KS * SLAB_B;
@@ -78,7 +81,7 @@ constexpr uint64_t kPaceLimitNs = 200000ull;   // a pacing wait longer than this
 constexpr uint32_t TMEM_COLS = 512;
 }  // namespace vtile_tc
 
-__global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
+__global__ void __launch_bounds__(vtile_tc::THREADS, 1) vtile_tc_kernel(VtileArgs p) {
     using namespace vtile_tc;
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
@@ -99,7 +102,7 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
             mbar_init(&empty[s], 1);
         }
         mbar_init(tmem_full, 1);
-        mbar_init(tmem_empty, 4);
+        mbar_init(tmem_empty, EPI_WARPS);
         mbar_init(drain, 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
             if (!mbar_wait_bounded(drain, 0, kWaitLimitNs)) atomicExch(p.err, 26);
         }
     } else {
-        const int q = warp & 3;
+        const int q = warp & 3, part = (warp - 2) >> 2;
         const int row = q * 32 + lane;
         const int etid = threadIdx.x - 64;
         uint32_t acc_phase = 0;
@@ -237,15 +240,15 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
             int rb, cb;
             if (!vtile_unit(p, u, rb, cb)) continue;
             const long long r = (long long)rb * BM + row, h0 = (long long)cb * BN;   // composite row, first column
-            for (int c = etid; c < BN; c += 128) {
+            for (int c = etid; c < BN; c += 32 * EPI_WARPS) {
                 const long long h = h0 + c;
                 cs_s[c] = h < p.c1 && h % p.RSy < p.vy ? pow2d(p.ey[h] - kFixedHiBits) : 0.0;
             }
-            // the four epilogue warps leave together (a named barrier must
+            // the epilogue warps leave together (a named barrier must
             // never wait for a warp that already left the loop)
-            if (bar_any(1, 128, *abort_flag != 0)) break;
+            if (bar_any(1, 32 * EPI_WARPS, *abort_flag != 0)) break;
             const bool got = mbar_wait_bounded(tmem_full, acc_phase, kWaitLimitNs);
-            if (bar_any(1, 128, !got)) {
+            if (bar_any(1, 32 * EPI_WARPS, !got)) {
                 if (!got) atomicExch(p.err, 24);
                 *abort_flag = 1;
                 break;
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
             const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
             float amax = 0.0f;   // integer accumulators stay exact below 2^24
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 16) {
+            for (int c0 = part * (BN / 4); c0 < (part + 1) * (BN / 4); c0 += 16) {
                 uint32_t h[16], xx[16];
                 tmem_ld16(lane_base + c0, h);
                 tmem_ld16(lane_base + BN + c0, xx);
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(192, 1) vtile_tc_kernel(VtileArgs p) {
             __syncwarp();
             if (lane == 0) mbar_arrive(tmem_empty);
             if (amax >= 16777216.0f) atomicOr(p.err + 1, 1);
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");   // cs_s reused by the next unit
+            asm volatile("bar.sync 1, %0;\n" ::"n"(32 * EPI_WARPS) : "memory");   // cs_s reused by the next unit
         }
     }
 
