@@ -52,8 +52,8 @@ struct AmpElemArgs {
     double wgt;             // weight of the pair sums (2 when the mirror block (J, I) is skipped)
     const double* eox; const double* evx;   // energies of the row spin
     const double* eoy; const double* evy;   // of the column spin
-    uint16_t* Ahi; uint16_t* Alo; long long nkA;  // SPLIT: rows R = ii*rsx + a, K = jj*ksy + b (nkA = K / 16)
-    uint16_t* Thi; uint16_t* Tlo; long long nkT;  // SPLIT, optional transpose: rows jj*csy + b, K = ii*ksx + a
+    uint16_t* A16; long long nkA;   // SPLIT: hi / lo operand, rows R = ii*rsx + a, K = jj*ksy + b (nkA = K / 16)
+    uint16_t* T16; long long nkT;   // SPLIT, optional transpose: rows jj*csy + b, K = ii*ksx + a
     double* A64; long long ldA;                   // FP64: [R][K], K = jj*ksy + b
     double* partial;        // [ox * oy] energy of each pair (i, j), i over all row orbitals
     double* prow;           // [ox * oy][rsx] sum_b r per pair and row a (or null)
@@ -68,7 +68,7 @@ struct AmpElemArgs {
     // tri: a diagonal block pair of the symmetric modes with only its pairs
     // ii <= jj (nbi == nbj, local pairs in the order of vtile_pair): an
     // off-diagonal pair stands for (i, j) and (j, i) -- weight 2 -- and its
-    // transposed amplitudes go into the same operand (Thi / Tlo = Ahi / Alo)
+    // transposed amplitudes go into the same operand (T16 = A16)
     int tri;
 };
 
@@ -91,12 +91,13 @@ __device__ __forceinline__ void local_pair(const AmpElemArgs& p, int lp, int& ii
 }  // namespace amp_detail
 
 namespace amp_detail {
-// blocked K-major element offset of (row R, column k) in the operand layout
-// of the Gamma kernel: 128-row blocks, each holding its nkc 16-wide K chunks
-// one after the other (so consecutive K chunks of a tile are one copy), 8 x 8
-// core matrices inside a 128 x 16 chunk
+// blocked K-major element offset of hi of (row R, column k) in the operand
+// layout of the Gamma kernel (lo: + 2048): 128-row blocks, each holding its nkc
+// 16-wide K chunks one after the other (so consecutive K chunks of a tile are
+// one copy), the hi slab and then the lo slab in a chunk, 8 x 8 core matrices
+// inside a slab
 __device__ __forceinline__ long long blocked_offset(long long R, long long k, long long nkc) {
-    return ((R >> 7) * nkc + (k >> 4)) * 2048 + (((R & 127) >> 3) * 16 + ((k & 15) >> 3) * 8 + (R & 7)) * 8 +
+    return ((R >> 7) * nkc + (k >> 4)) * 4096 + (((R & 127) >> 3) * 16 + ((k & 15) >> 3) * 8 + (R & 7)) * 8 +
            (k & 7);
 }
 
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
     int ii, jj;
     amp_detail::local_pair(p, lp, ii, jj);
     const double wgt = p.tri ? (ii < jj ? 2.0 : 1.0) : p.wgt;
-    const bool write_t = p.Thi != nullptr && !(p.tri && ii == jj);
+    const bool write_t = p.T16 != nullptr && !(p.tri && ii == jj);
     // FP64 operand of a diagonal block pair: the (j, i) amplitudes go into A64
     // as the transposes of the (i, j) ones
     const bool write_t64 = !SPLIT && p.tri && ii != jj;
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
                     const long long R = (long long)ii * p.rsx + a0 + r;
                     const long long kc = (long long)jj * p.ksy + b0 + g * 8;
                     const long long off = amp_detail::blocked_offset(R, kc, p.nkA);
-                    amp_detail::store_hilo8(&T[r][g * 8], p.Ahi + off, p.Alo + off);
+                    amp_detail::store_hilo8(&T[r][g * 8], p.A16 + off, p.A16 + off + 2048);
                 } else if (write_t) {
                     const int w = threadIdx.x - 128;
                     const int r = w >> 2, g = w & 3;   // r: b offset, g: group of 8 a
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
                     double col[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) col[e] = T[g * 8 + e][r];
-                    amp_detail::store_hilo8(col, p.Thi + off, p.Tlo + off);
+                    amp_detail::store_hilo8(col, p.T16 + off, p.T16 + off + 2048);
                 }
             }
             if (write_t64) {

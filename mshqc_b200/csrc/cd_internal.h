@@ -38,14 +38,14 @@ struct SpinState {
     bool B64_valid = false;
     int B64_prec = 0;       // MSHQC_CD_FP64: FP64 products; MSHQC_CD_FP16X3: int8-slice products
     // fixed-point hi/lo (BF16 carriers) of the MO vectors for the tensor-core path
-    DevBuf Bhi, Blo;        // Blo unused in the pair layout (hi and lo interleaved in Bhi)
+    DevBuf B16;             // hi and lo interleaved (split_bf16.cuh)
     DevBuf expo;            // per-row power-of-two exponents [o][rows]
     DevBuf diag;            // exact (ia|ia) [o][rows]
     DevBuf norms;           // largest sum hi^2 and sum lo^2 of a row (bit patterns)
     int64_t vp16 = 0, Mp16 = 0;
     double max_norm_hi = 0, max_norm_lo = 0;
     bool B16_valid = false;
-    int B16_layout = 0;     // 0: integral-tile layout, 1: pair layout (split_bf16.cuh)
+    int B16_layout = 0;     // rows per orbital: 0 packed (integral tiles), 1 multiples of 256 (pair energies)
     void invalidate() {
         B64_valid = false;
         B16_valid = false;
@@ -102,8 +102,7 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf gam[2];        // backward: Gamma per spin
     mshqc_cd::DevBuf BT;            // backward: transposed MO vectors (hi/lo BF16), alpha
     mshqc_cd::DevBuf BT_b;          // backward: the same for beta
-    mshqc_cd::DevBuf amp2;          // backward: second half of the staging (lo)
-    mshqc_cd::DevBuf ampT, ampT2;   // backward: transposed opposite-spin amplitudes (hi, lo)
+    mshqc_cd::DevBuf ampT;          // backward: transposed amplitudes
     mshqc_cd::DevBuf dsum;          // backward: per-pair row / column / total sums for dE/de
     mshqc_cd::DevBuf amp_chunks;    // backward: per-chunk column sums, energies, totals of split pairs
     mshqc_cd::DevBuf W;             // backward: integral staging / C_vir-contracted Gamma
@@ -146,9 +145,9 @@ struct mshqc_cd_ctx {
     }
     size_t held_bytes() const {
         size_t b = L.bytes + Y.bytes + scratch.bytes + tables.bytes + partial.bytes +
-                   pair_sum.bytes + totals.bytes + flag.bytes + amp.bytes + amp2.bytes + BT.bytes + W.bytes;
+                   pair_sum.bytes + totals.bytes + flag.bytes + amp.bytes + ampT.bytes + BT.bytes + W.bytes;
         for (const auto& s : spin)
-            b += s.C.bytes + s.eps.bytes + s.B64.bytes + s.Bhi.bytes + s.Blo.bytes + s.expo.bytes +
+            b += s.C.bytes + s.eps.bytes + s.B64.bytes + s.B16.bytes + s.expo.bytes +
                  s.diag.bytes + s.norms.bytes;
         b += gemm_ws.bytes + dens_x.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
         for (const auto& g : gam) b += g.bytes;
@@ -173,10 +172,8 @@ struct mshqc_cd_ctx {
         pace.release();
         amp.release();
         BT.release();
-        amp2.release();
         BT_b.release();
         ampT.release();
-        ampT2.release();
         dsum.release();
         amp_chunks.release();
         W.release();
@@ -184,8 +181,7 @@ struct mshqc_cd_ctx {
             s.C.release();
             s.eps.release();
             s.B64.release();
-            s.Bhi.release();
-            s.Blo.release();
+            s.B16.release();
             s.expo.release();
             s.diag.release();
             s.norms.release();

@@ -680,9 +680,9 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
     const bool pair_layout = layout == 1;
     // rows per orbital; the integral-tile layout packs them across orbitals
     const int64_t rows = pair_layout ? tc_rows(v) : round_up(v, 32), nqc = Mp / 16;
-    const size_t n = (size_t)nqc * (pair_layout ? o * rows : round_up(o * rows, 256)) * 16;
-    CD_ALLOC(s.Bhi, (pair_layout ? 2 : 1) * n * sizeof(uint16_t), false);
-    if (!pair_layout) CD_ALLOC(s.Blo, n * sizeof(uint16_t), false);
+    const int64_t total = round_up(o * rows, 256);
+    const size_t n = (size_t)(nqc * total * 16);   // elements of hi, as many of lo
+    CD_ALLOC(s.B16, 2 * n * sizeof(uint16_t), false);
     CD_ALLOC(s.expo, sizeof(int) * o * rows, true);
     CD_ALLOC(s.diag, sizeof(double) * o * rows, true);
     CD_ALLOC(s.norms, sizeof(unsigned long long) * 2, true);
@@ -701,8 +701,8 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
         const int64_t threads = (int64_t)(n / 8);
         const int blocks = (int)std::min<int64_t>(cdiv(threads, 256), (int64_t)ctx->num_sms * 16);
         split_fixed_blocked_kernel<<<blocks, 256, 0, ctx->stream>>>(
-            s.B64.as<double>(), s.vp, Mp, (int)v, (int)M, o, nqc, rows, s.expo.as<int>(),
-            s.Bhi.as<uint16_t>(), pair_layout ? nullptr : s.Blo.as<uint16_t>(), pair_layout);
+            s.B64.as<double>(), s.vp, Mp, (int)v, (int)M, o, nqc, rows, total / 8, s.expo.as<int>(),
+            s.B16.as<uint16_t>());
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
     }
@@ -811,8 +811,8 @@ int pair_pass_tc(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     if (X.B16_layout != 1 || Y.B16_layout != 1)
         return set_error(MSHQC_CD_ERR_STATE, "fixed-point operands not in the pair layout");
     PairTcArgs a{};
-    a.Xp = X.Bhi.as<uint16_t>();
-    a.Yp = Y.Bhi.as<uint16_t>();
+    a.Xp = X.B16.as<uint16_t>();
+    a.Yp = Y.B16.as<uint16_t>();
     a.ex = X.expo.as<int>();  a.ey = Y.expo.as<int>();
     if (mode == PAIR_OPPOSITE_SPIN) {
         a.diag = ctx->diag_os.as<double>();
@@ -1232,35 +1232,32 @@ BwdDims bwd_dims(const mshqc_cd_ctx* ctx, int spin) {
 
 // BF16 hi/lo copy of one spin's MO vectors transposed to rows Q (RQ rows),
 // K = (j, b) with b padded to VR: the B operand of the Gamma GEMM.
-int make_bt(mshqc_cd_ctx* ctx, int spin, DevBuf& buf, int64_t RQ, const uint16_t** hi, const uint16_t** lo) {
+int make_bt(mshqc_cd_ctx* ctx, int spin, DevBuf& buf, int64_t RQ, const uint16_t** bt) {
     SpinState& s = ctx->spin[spin];
     const BwdDims d = bwd_dims(ctx, spin);
     const size_t nbt = (size_t)RQ * d.o * d.VR;
     CD_ALLOC(buf, 2 * nbt * sizeof(uint16_t), false);
-    uint16_t* h = buf.as<uint16_t>();
-    uint16_t* l = h + nbt;
     const int64_t threads = (d.o * d.VR / 16) * RQ * 2;
     const int blocks = (int)std::min<int64_t>(cdiv(threads, 256), (int64_t)ctx->num_sms * 16);
     begin_stage(ctx, ST_SPLIT);
     bt_split_kernel<<<blocks, 256, 0, ctx->stream>>>(s.B64.as<double>(), s.vp, ctx->Mp, (int)d.v, (int)ctx->M,
-                                                     d.o, d.VR, RQ, h, l);
+                                                     d.o, d.VR, RQ, buf.as<uint16_t>());
     end_stage(ctx);
     CD_CUDA(cudaGetLastError());
     ctx->launches++;
-    *hi = h;
-    *lo = l;
+    *bt = buf.as<uint16_t>();
     return MSHQC_CD_OK;
 }
 
 // gamma[(i0 + R / RS, R % RS)][Q] (+)= sum_K A[R][K] BT[Q][K] for R < rows;
 // K in orbital groups of VRk (vk of them valid); a_rbs / b_rbs: K chunks per row
-// block of A (128 rows) and of BT (256 rows), bhi / blo pointing at the first K
-// chunk used
-int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* ahi, const uint16_t* alo, int64_t a_rbs, const uint16_t* bhi,
-                 const uint16_t* blo, int64_t b_rbs, int64_t RQ, int64_t K, int64_t VRk, int64_t vk, int64_t rows,
-                 int64_t RS, int64_t v, int64_t vp, int i0, double* gamma, int accumulate) {
+// block of A (128 rows) and of BT (256 rows), bt pointing at the first K chunk
+// used
+int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* amp, int64_t a_rbs, const uint16_t* bt, int64_t b_rbs, int64_t RQ,
+                 int64_t K, int64_t VRk, int64_t vk, int64_t rows, int64_t RS, int64_t v, int64_t vp, int i0,
+                 double* gamma, int accumulate) {
     GammaTcArgs g{};
-    g.Ahi = ahi;  g.Alo = alo;  g.Bhi = bhi;  g.Blo = blo;
+    g.A = amp;  g.B = bt;
     g.a_rbs = a_rbs;  g.b_rbs = b_rbs;
     g.nk = (int)(K / 16);
     g.KP = 32;
@@ -1319,9 +1316,8 @@ int reduce_deps(mshqc_cd_ctx* ctx, const double* prow, const double* pcol, const
 // Energies go to `partial` (ox * oy, one per ordered pair, zero where a
 // mirrored pair stands in), dE/de to deps_x / deps_y.
 template <int MODE>
-int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const btx[2],
-                     const uint16_t* const bty[2], int64_t RQ, double* deps_x, double* deps_y,
-                     double* partial) {
+int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, const uint16_t* bty, int64_t RQ,
+                     double* deps_x, double* deps_y, double* partial) {
     constexpr bool kSym = MODE != AMP_OPPOSITE_SPIN;
     SpinState& X = ctx->spin[sx];
     SpinState& Y = ctx->spin[sy];
@@ -1331,16 +1327,14 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
     CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
     // the staging this pass reuses counts as available, so that the block size
     // of a repeated call does not shrink because the previous call holds it
-    const size_t held = ctx->amp.bytes + ctx->amp2.bytes + ctx->ampT.bytes + ctx->ampT2.bytes + ctx->W.bytes;
+    const size_t held = ctx->amp.bytes + ctx->ampT.bytes + ctx->W.bytes;
     const size_t budget = std::min<size_t>((free_b + held) / 3, size_t(40) << 30);
     // block sizes: rows bI, columns bJ (all of them for the opposite spin)
     int64_t bI, bJ;
     tc_block_sizes(ctx, dx.o, dy.o, dx.VR, dy.VR, dy.VS, kSym, budget, &bI, &bJ);
     const size_t n_amp = sizeof(uint16_t) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VR);
-    CD_ALLOC(ctx->amp, n_amp, false);
-    CD_ALLOC(ctx->amp2, n_amp, false);
-    CD_ALLOC(ctx->ampT, n_amp, false);
-    CD_ALLOC(ctx->ampT2, n_amp, false);
+    CD_ALLOC(ctx->amp, 2 * n_amp, false);   // hi and lo
+    CD_ALLOC(ctx->ampT, 2 * n_amp, false);
     // (the size the block sizes are reckoned with; the packed rows take less of it)
     CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VS), false);
     const int64_t npairs = dx.o * dy.o;
@@ -1364,8 +1358,8 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             const bool tri = kSym && J0 == I0;
             const int npl = tri ? nI * (nI + 1) / 2 : nI * nJ;
             VtileArgs a{};
-            a.Xhi = X.Bhi.as<uint16_t>();  a.Xlo = X.Blo.as<uint16_t>();
-            a.Yhi = Y.Bhi.as<uint16_t>();  a.Ylo = Y.Blo.as<uint16_t>();
+            a.X = X.B16.as<uint16_t>();
+            a.Y = Y.B16.as<uint16_t>();
             a.ex = X.expo.as<int>();  a.ey = Y.expo.as<int>();
             a.diag = sx == sy ? X.diag.as<double>() : nullptr;
             a.RSx = (int)dx.RS;  a.RSy = (int)dy.RS;
@@ -1401,13 +1395,13 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             e.wgt = (kSym && mirror) ? 2.0 : 1.0;
             e.eox = X.eps.as<double>();  e.evx = e.eox + dx.o;
             e.eoy = Y.eps.as<double>();  e.evy = e.eoy + dy.o;
-            e.Ahi = ctx->amp.as<uint16_t>();  e.Alo = ctx->amp2.as<uint16_t>();
+            e.A16 = ctx->amp.as<uint16_t>();
             e.nkA = (long long)nJ * dy.VR / 16;
             if (mirror) {
-                e.Thi = ctx->ampT.as<uint16_t>();  e.Tlo = ctx->ampT2.as<uint16_t>();
+                e.T16 = ctx->ampT.as<uint16_t>();
                 e.nkT = (long long)nI * dx.VR / 16;
             } else if (tri) {
-                e.Thi = e.Ahi;  e.Tlo = e.Alo;  e.nkT = e.nkA;
+                e.T16 = e.A16;  e.nkT = e.nkA;
                 e.tri = 1;
             }
             e.partial = partial;
@@ -1437,13 +1431,13 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* const bt
             end_stage(ctx);
             // Gamma_sx[I] += A x B_sy[J]  (K range of J inside the transposed B of spin sy)
             // first K chunk of block J (I) inside a 256-row block of BT
-            const size_t kJ = (size_t)J0 * dy.VR / 16 * 4096, kI = (size_t)I0 * dx.VR / 16 * 4096;
+            const size_t kJ = (size_t)J0 * dy.VR / 16 * 8192, kI = (size_t)I0 * dx.VR / 16 * 8192;
             const int64_t nkBy = dy.o * dy.VR / 16, nkBx = dx.o * dx.VR / 16;
-            CD_RC(launch_gamma(ctx, e.Ahi, e.Alo, e.nkA, bty[0] + kJ, bty[1] + kJ, nkBy, RQ, (int64_t)nJ * dy.VR, dy.VR,
+            CD_RC(launch_gamma(ctx, e.A16, e.nkA, bty + kJ, nkBy, RQ, (int64_t)nJ * dy.VR, dy.VR,
                                dy.v, (int64_t)nI * dx.RS, dx.RS, dx.v, dx.vp, (int)I0, ctx->gam[sx].as<double>(), 1));
             if (mirror) {
                 // Gamma_sy[J] += A^T x B_sx[I]
-                CD_RC(launch_gamma(ctx, e.Thi, e.Tlo, e.nkT, btx[0] + kI, btx[1] + kI, nkBx, RQ,
+                CD_RC(launch_gamma(ctx, e.T16, e.nkT, btx + kI, nkBx, RQ,
                                    (int64_t)nI * dx.VR, dx.VR, dx.v, (int64_t)nJ * dy.RS, dy.RS, dy.v, dy.vp, (int)J0,
                                    ctx->gam[sy].as<double>(), 1));
             }
@@ -1607,8 +1601,8 @@ int gradient_restricted_tc(mshqc_cd_ctx* ctx, double* dC, double* deps, double* 
     SpinState& s = ctx->spin[0];
     const BwdDims d = bwd_dims(ctx, 0);
     const int64_t N = ctx->N, Mp = ctx->Mp, RQ = round_up(ctx->M, 256);
-    const uint16_t* bt[2] = {nullptr, nullptr};
-    CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bt[0], &bt[1]));
+    const uint16_t* bt = nullptr;
+    CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bt));
     CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, d.o) * s.vp * Mp, true);
     CD_CUDA(cudaMemsetAsync(deps, 0, sizeof(double) * N, ctx->stream));
     CD_ALLOC(ctx->flag, sizeof(int) * 4, true);
@@ -1643,11 +1637,10 @@ int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2],
     const BwdDims da = bwd_dims(ctx, 0), db = bwd_dims(ctx, 1);
     const int64_t N = ctx->N, Mp = ctx->Mp, RQ = round_up(ctx->M, 256);
     const bool tc = precision == MSHQC_CD_FP16X3;
-    const uint16_t* bta[2] = {nullptr, nullptr};
-    const uint16_t* btb[2] = {nullptr, nullptr};
+    const uint16_t *bta = nullptr, *btb = nullptr;
     if (tc) {
-        CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bta[0], &bta[1]));
-        CD_RC(make_bt(ctx, 1, ctx->BT_b, RQ, &btb[0], &btb[1]));
+        CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bta));
+        CD_RC(make_bt(ctx, 1, ctx->BT_b, RQ, &btb));
     }
     CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, da.o) * da.vp * Mp, true);
     CD_ALLOC(ctx->gam[1], sizeof(double) * (size_t)b_rows(ctx, db.o) * db.vp * Mp, true);

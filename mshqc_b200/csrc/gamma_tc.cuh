@@ -7,13 +7,15 @@
 // a multiple of 128); B operand: BT, the MO vectors transposed to rows Q, K = (j, b).
 // Both are BF16 hi/lo pairs in a row-block-major blocked K-major layout: the
 // matrix is cut into blocks of BR rows (128 for A, 256 for B), each block
-// stores its 16-wide K chunks one after the other (BR x 16 elements each,
-// 8 x 8 core matrices inside), so element (r, k) sits at
-//   ((r / BR) * nkc + k / 16) * BR * 16 + ((r % BR) / 8 * 16 + (k % 16) / 8 * 8 + r % 8) * 8 + k % 8
-// with nkc the K chunks per block (a_rbs, b_rbs).  Consecutive K steps of a
-// tile are contiguous, so one bulk copy moves KS = 2 steps: the copies of a
-// 128 x 256 tile are feed-bound at one step per copy (measured: 10.1 ms for a
-// launch whose MMAs alone take 7.3 ms; 7.7 ms with two steps per copy).
+// stores its 16-wide K chunks one after the other, a chunk its hi slab and then
+// its lo slab (BR x 16 elements each, 8 x 8 core matrices inside), so hi of
+// (r, k) sits at
+//   ((r / BR) * nkc + k / 16) * BR * 32 + ((r % BR) / 8 * 16 + (k % 16) / 8 * 8 + r % 8) * 8 + k % 8
+// with nkc the K chunks per block (a_rbs, b_rbs), lo BR * 16 elements further.
+// One bulk copy per operand moves KS = 2 K steps with both halves (16 and
+// 32 KB): a copy costs its issuing thread about 70 cycles besides its bytes, and
+// the six MMAs of a stage take 768.  The last Q block is as narrow as the
+// vectors left (a multiple of 16): M = 1600 needs 6.25 blocks, not 7.
 // K steps that lie in an orbital's padding (kv .. kg - 1) are neither copied
 // nor multiplied; the promotion chunks keep their place in the padded K, so a
 // sum has the same roundings as with the zeros added.  Packed rows and skipped
@@ -40,8 +42,8 @@
 namespace mshqc_cd {
 
 struct GammaTcArgs {
-    const uint16_t* Ahi; const uint16_t* Alo;   // staging (128-row blocks of a_rbs K chunks)
-    const uint16_t* Bhi; const uint16_t* Blo;   // BT from the first K chunk used (256-row blocks of b_rbs chunks)
+    const uint16_t* A;      // staging (128-row blocks of a_rbs K chunks)
+    const uint16_t* B;      // BT from the first K chunk used (256-row blocks of b_rbs chunks)
     long long a_rbs, b_rbs;
     int nk;                 // K steps of 16 (even), padding included
     int kg, kv;             // K steps per orbital (even, a multiple of 8), of them with data
@@ -61,7 +63,7 @@ namespace gamma_tc {
 constexpr int BM = 128, BN = 256, KC = 16, KS = 2, STAGES = 4, THREADS = 576, EPI_WARPS = 16;
 constexpr uint32_t SLAB_A = BM * KC * 2;        // 4 KB per K step
 constexpr uint32_t SLAB_B = BN * KC * 2;        // 8 KB per K step
-constexpr uint32_t OFF_AH = 0, OFF_AL = KS * SLAB_A, OFF_BH = 2 * KS * SLAB_A, OFF_BL = 2 * KS * SLAB_A + KS * SLAB_B;
+constexpr uint32_t OFF_B = 2 * KS * SLAB_A;     // A: KS x (hi, lo), then B: KS x (hi, lo)
 constexpr uint32_t STAGE_BYTES = KS * 2 * (SLAB_A + SLAB_B);   // 48 KB: KS steps
 constexpr uint32_t SMEM_DATA = STAGES * STAGE_BYTES;           // 192 KB
 constexpr size_t SMEM_BYTES = SMEM_DATA + 1024 + 256;
@@ -144,7 +146,7 @@ __global__ void __launch_bounds__(576, 1) gamma_tc_kernel(GammaTcArgs p) {
         for (long long u = first; u < units && !stop; u += step) {
             long long rb, qb;
             gamma_tile(p, u, rb, qb);
-            const size_t ra0 = (size_t)rb * p.a_rbs * (BM * 16), rq0 = (size_t)qb * p.b_rbs * (BN * 16);
+            const size_t ra0 = (size_t)rb * p.a_rbs * (BM * 32), rq0 = (size_t)qb * p.b_rbs * (BN * 32);
             for (int kq = 0, c = 0; kq < p.nk; next_step(p, kq, c)) {
                 pacer.step(lane, kPaceLimitNs);
                 int ok = 1;
@@ -158,12 +160,10 @@ __global__ void __launch_bounds__(576, 1) gamma_tc_kernel(GammaTcArgs p) {
                     } else {
                         uint8_t* sb = smem + stage * STAGE_BYTES;
                         const uint32_t nks = (uint32_t)min(KS, p.kv - c);
+                        const uint16_t* b0 = p.B + rq0 + (size_t)kq * (BN * 32);
                         mbar_arrive_expect_tx(&full[stage], nks * 2 * (SLAB_A + SLAB_B));
-                        const size_t ka = ra0 + (size_t)kq * (BM * 16), kb = rq0 + (size_t)kq * (BN * 16);
-                        bulk_g2s(sb + OFF_AH, p.Ahi + ka, nks * SLAB_A, &full[stage]);
-                        bulk_g2s(sb + OFF_AL, p.Alo + ka, nks * SLAB_A, &full[stage]);
-                        bulk_g2s(sb + OFF_BH, p.Bhi + kb, nks * SLAB_B, &full[stage]);
-                        bulk_g2s(sb + OFF_BL, p.Blo + kb, nks * SLAB_B, &full[stage]);
+                        bulk_g2s(sb, p.A + ra0 + (size_t)kq * (BM * 32), nks * 2 * SLAB_A, &full[stage]);
+                        bulk_g2s(sb + OFF_B, b0, nks * 2 * SLAB_B, &full[stage]);
                     }
                 }
                 if (!__shfl_sync(0xffffffffu, ok, 0)) {
@@ -197,10 +197,9 @@ __global__ void __launch_bounds__(576, 1) gamma_tc_kernel(GammaTcArgs p) {
             uint32_t chunk_ctr = 0;      // global chunk counter: buffer = ctr & 1
             // descriptors at stage 0; a byte offset adds to the low word in units of 16
             const uint32_t sbase = smem_addr(smem);
-            const uint64_t dah = smem_desc_kmajor(sbase + OFF_AH, 128, 256);
-            const uint64_t dal = smem_desc_kmajor(sbase + OFF_AL, 128, 256);
-            const uint64_t dbh = smem_desc_kmajor(sbase + OFF_BH, 128, 256);
-            const uint64_t dbl = smem_desc_kmajor(sbase + OFF_BL, 128, 256);
+            const uint64_t da = smem_desc_kmajor(sbase, 128, 256);
+            const uint64_t db = smem_desc_kmajor(sbase + OFF_B, 128, 256);
+            constexpr uint64_t LA = SLAB_A >> 4, LB = SLAB_B >> 4;   // from hi to lo, and on to the next step
             for (long long u = first; u < units && !*abort_flag; u += step) {
                 int kq = 0, kc = 0;
                 for (int c = 0; c < nchunks && !*abort_flag; ++c, ++chunk_ctr) {
@@ -222,14 +221,14 @@ __global__ void __launch_bounds__(576, 1) gamma_tc_kernel(GammaTcArgs p) {
                         }
                         tc_fence_after();
                         const uint64_t so = (uint64_t)(stage * (STAGE_BYTES >> 4));
-                        mma_f16(d, dah + so, dbh + so, IDESC, more);
-                        mma_f16(d, dah + so, dbl + so, IDESC, 1u);
-                        mma_f16(d, dal + so, dbh + so, IDESC, 1u);
+                        mma_f16(d, da + so, db + so, IDESC, more);
+                        mma_f16(d, da + so, db + so + LB, IDESC, 1u);
+                        mma_f16(d, da + so + LA, db + so, IDESC, 1u);
                         if (kc + 1 < p.kv) {
-                            const uint64_t sa = so + (SLAB_A >> 4), sb = so + (SLAB_B >> 4);
-                            mma_f16(d, dah + sa, dbh + sb, IDESC, 1u);
-                            mma_f16(d, dah + sa, dbl + sb, IDESC, 1u);
-                            mma_f16(d, dal + sa, dbh + sb, IDESC, 1u);
+                            const uint64_t sa = so + 2 * LA, sb = so + 2 * LB;
+                            mma_f16(d, da + sa, db + sb, IDESC, 1u);
+                            mma_f16(d, da + sa, db + sb + LB, IDESC, 1u);
+                            mma_f16(d, da + sa + LA, db + sb, IDESC, 1u);
                         }
                         more = 1u;
                         mma_commit(&empty[stage]);
@@ -302,8 +301,7 @@ __global__ void __launch_bounds__(576, 1) gamma_tc_kernel(GammaTcArgs p) {
 // b < v, Q < M.  Layout: 256-row blocks of o * VR / 16 K chunks (the B
 // operand layout of gamma_tc_kernel).
 static __global__ void bt_split_kernel(const double* __restrict__ B, int64_t vp, int64_t Mp, int v, int M,
-                                       int64_t o, int64_t VR, int64_t RQ, uint16_t* __restrict__ hi,
-                                       uint16_t* __restrict__ lo) {
+                                       int64_t o, int64_t VR, int64_t RQ, uint16_t* __restrict__ bt) {
     // one thread = one core-matrix row: 8 consecutive k of one Q
     const int64_t nkc = o * VR / 16;
     const int64_t total = nkc * RQ * 2;
@@ -326,14 +324,14 @@ static __global__ void bt_split_kernel(const double* __restrict__ B, int64_t vp,
             h[e] = __bfloat16_as_ushort(bh);
             l[e] = __bfloat16_as_ushort(bl);
         }
-        const int64_t off = ((g >> 5) * nkc + kc) * 4096 + ((g & 31) * 16 + kk * 8 + r) * 8;
+        const int64_t off = ((g >> 5) * nkc + kc) * 8192 + ((g & 31) * 16 + kk * 8 + r) * 8;
         uint4 vh, vl;
         vh.x = h[0] | (uint32_t(h[1]) << 16); vh.y = h[2] | (uint32_t(h[3]) << 16);
         vh.z = h[4] | (uint32_t(h[5]) << 16); vh.w = h[6] | (uint32_t(h[7]) << 16);
         vl.x = l[0] | (uint32_t(l[1]) << 16); vl.y = l[2] | (uint32_t(l[3]) << 16);
         vl.z = l[4] | (uint32_t(l[5]) << 16); vl.w = l[6] | (uint32_t(l[7]) << 16);
-        *reinterpret_cast<uint4*>(hi + off) = vh;
-        *reinterpret_cast<uint4*>(lo + off) = vl;
+        *reinterpret_cast<uint4*>(bt + off) = vh;
+        *reinterpret_cast<uint4*>(bt + off + 4096) = vl;
     }
 }
 

@@ -105,31 +105,23 @@ static __global__ void row_scale_kernel(const double* __restrict__ src, int64_t 
 }
 
 // src: [o][vp][Mp] FP64 (zeros outside v x M); expo from row_scale_kernel.
-// dst, two layouts of FP16 bits, blocked inside a 16-wide Q chunk as
-// (a/8, (Q%16)/8, a%8, Q%8) (the canonical K-major no-swizzle UMMA layout):
-//  * pair_layout = false (integral tiles of the backward): hi and lo in
-//    separate arrays over the composite rows g = i*rows + a (rows a multiple
-//    of 32), in 256-row blocks that run across orbitals, each holding its nqc
-//    chunks one after the other:
-//      element (g, Q) at ((g/256)*nqc + Q/16)*4096
-//                        + ((g%256)/8*16 + (Q%16)/8*8 + g%8)*8 + Q%8
-//    so a 128-row slab of one chunk is 4 KB and a 256-row slab of consecutive
-//    chunks is one contiguous run;
-//  * pair_layout = true (fused pair energies; rows a multiple of 256): one
-//    array of 128-row blocks whose chunks hold the hi slab and then the lo
-//    slab of the same rows:
-//      hi of (i, a, Q) at ((i*rows/128 + a/128)*nqc + Q/16)*4096
-//                         + ((a%128)/8*16 + (Q%16)/8*8 + a%8)*8 + Q%8,
-//      lo at the same + 2048,
-//    so one contiguous copy brings both halves of a 128-row slab for several
-//    chunks, and each chunk's [hi; lo] is a 256-row operand.
+// dst: FP16 bits over the composite rows g = i*rows + a, in 128-row blocks whose
+// 16-wide Q chunks hold the hi slab and then the lo slab of the same rows, each
+// blocked as (g/8, (Q%16)/8, g%8, Q%8) (the canonical K-major no-swizzle UMMA
+// layout):
+//   hi of (g, Q) at ((g/128)*nqc + Q/16)*4096
+//                   + ((g%128)/8*16 + (Q%16)/8*8 + g%8)*8 + Q%8,
+//   lo at the same + 2048,
+// so one contiguous copy brings both halves of a 128-row block for several
+// chunks, and each chunk's [hi; lo] is one 256-row operand.  rows: a multiple of
+// 256 for the fused pair energies (blocks inside one orbital), of 32 for the
+// integral tiles of the backward (blocks run across orbitals).  ngrp: groups of
+// 8 rows written, the rows beyond o*rows as zeros.
 static __global__ void split_fixed_blocked_kernel(const double* __restrict__ src, int64_t vp,
                                                   int64_t Mp, int v, int M, int64_t o, int64_t nqc,
-                                                  int64_t rows, const int* __restrict__ expo,
-                                                  uint16_t* __restrict__ hi, uint16_t* __restrict__ lo,
-                                                  bool pair_layout) {
+                                                  int64_t rows, int64_t ngrp, const int* __restrict__ expo,
+                                                  uint16_t* __restrict__ dst) {
     // one thread = one core-matrix row: 8 consecutive Q of one composite row
-    const int64_t ngrp = pair_layout ? o * rows / 8 : (o * rows + 255) / 256 * 32;   // groups of 8 rows
     const int64_t total = nqc * ngrp * 2 * 8;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
          t += (int64_t)gridDim.x * blockDim.x) {
@@ -152,15 +144,14 @@ static __global__ void split_fixed_blocked_kernel(const double* __restrict__ src
             h[k] = __half_as_ushort(__double2half(hv));   // exact: |hv| <= 1024
             l[k] = __half_as_ushort(__double2half(lv));   // exact: |lv| <= 128
         }
-        const int64_t off = pair_layout ? ((g >> 4) * nqc + qc) * 4096 + ((g & 15) * 16 + kk * 8 + r) * 8
-                                        : ((g >> 5) * nqc + qc) * 4096 + ((g & 31) * 16 + kk * 8 + r) * 8;
+        const int64_t off = ((g >> 4) * nqc + qc) * 4096 + ((g & 15) * 16 + kk * 8 + r) * 8;
         uint4 vh, vl;
         vh.x = h[0] | (uint32_t(h[1]) << 16); vh.y = h[2] | (uint32_t(h[3]) << 16);
         vh.z = h[4] | (uint32_t(h[5]) << 16); vh.w = h[6] | (uint32_t(h[7]) << 16);
         vl.x = l[0] | (uint32_t(l[1]) << 16); vl.y = l[2] | (uint32_t(l[3]) << 16);
         vl.z = l[4] | (uint32_t(l[5]) << 16); vl.w = l[6] | (uint32_t(l[7]) << 16);
-        *reinterpret_cast<uint4*>(hi + off) = vh;
-        *reinterpret_cast<uint4*>((pair_layout ? hi + 2048 : lo) + off) = vl;
+        *reinterpret_cast<uint4*>(dst + off) = vh;
+        *reinterpret_cast<uint4*>(dst + 2048 + off) = vl;
     }
 }
 

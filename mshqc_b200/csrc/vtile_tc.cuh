@@ -11,12 +11,15 @@
 // to 32 per orbital, so a tile runs across orbitals (padding every orbital's
 // rows to 128 and columns to 256 took 1.66 times the tiles at v = 540).  Tiles
 // lie on the grid of the composite rows; the edge tiles of a block store only
-// the block's rows and columns.  A stage holds KS = 2 Q steps: the A slab (128 rows) per
-// step, the B slab (256 rows) of both steps in one copy (one-step copies
-// left the kernel feed-bound: 7.7 ms for a launch whose MMAs take 5.8 ms;
-// 5.9 ms with the two-step B copies).  Per 16-wide Q step three 128x256x16 MMAs
-// accumulate the hi*hi' and the hi*lo' + lo*hi' integers exactly in two TMEM
-// accumulators (columns [0,256) and [256,512)), and the epilogue recovers
+// the block's rows and columns.  A stage holds KS = 2 Q steps of three 128-row
+// blocks with both halves, one 16 KB copy each: the tile's rows (A) and its two
+// column blocks (B0, B1); each step's [hi; lo] of a column block is one 256-row
+// operand.  Per 16-wide Q step
+//   A hi . [B0 hi; B0 lo] -> hh in columns [0,128), hi*lo' in [128,256)
+//   A lo . B0 hi          -> += [128,256)           and the same for B1 in [256,512)
+// (384 cycles as with three 128x256 products, but three copies a stage instead of
+// six, which took longer to issue than the MMAs).  The integers accumulate
+// exactly, and the epilogue recovers
 //   (ia|jb) = u_ia u_jb (hh + x / 256)
 // in FP64, substitutes the exact (ia|ia) for i = j, a = b when X = Y, and
 // stores it rounded to FP32 into the row-major staging matrix S (row length
@@ -37,8 +40,7 @@
 namespace mshqc_cd {
 
 struct VtileArgs {
-    const uint16_t* Xhi; const uint16_t* Xlo;   // blocked fixed-point operands (rows i, a)
-    const uint16_t* Yhi; const uint16_t* Ylo;   // (columns j, b)
+    const uint16_t* X; const uint16_t* Y;       // blocked fixed-point operands (rows i, a; columns j, b)
     const int* ex; const int* ey;               // row exponents of the composite rows
     const double* diag;                         // exact (ia|ia) per composite row when X = Y, else null
     int RSx, RSy;           // composite rows per orbital
@@ -70,10 +72,10 @@ __device__ __forceinline__ bool vtile_unit(const VtileArgs& p, int u, int& rb, i
 
 namespace vtile_tc {
 constexpr int BM = 128, BN = 256, KC = 16, KS = 2, STAGES = 4, EPI_WARPS = 16, THREADS = 64 + 32 * EPI_WARPS;
-constexpr uint32_t SLAB_A = BM * KC * 2;     // 4 KB per Q step
-constexpr uint32_t SLAB_B = BN * KC * 2;     // 8 KB per Q step
-constexpr uint32_t OFF_AH = 0, OFF_AL = KS * SLAB_A, OFF_BH = 2 * KS * SLAB_A, OFF_BL = 2 * KS * SLAB_A + KS * SLAB_B;
-constexpr uint32_t STAGE_BYTES = KS * 2 * (SLAB_A + SLAB_B);   // 48 KB
+constexpr uint32_t SLAB = 128 * KC * 2;      // 4 KB: 128 rows of a Q step, hi or lo
+constexpr uint32_t CHUNK = 2 * SLAB;         // hi and lo
+constexpr uint32_t PIECE = KS * CHUNK;       // a 128-row block's part of a stage (16 KB)
+constexpr uint32_t STAGE_BYTES = 3 * PIECE;  // A, B0, B1: 48 KB
 constexpr uint32_t SMEM_DATA = STAGES * STAGE_BYTES;           // 192 KB
 constexpr size_t SMEM_BYTES = SMEM_DATA + 1024 + 256 + BN * 8;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
@@ -129,14 +131,10 @@ __global__ void __launch_bounds__(vtile_tc::THREADS, 1) vtile_tc_kernel(VtileArg
         for (int u = first; u < units && !stop; u += step) {
             int rb, cb;
             if (!vtile_unit(p, u, rb, cb)) continue;
-            // slab bases at Q step 0 (256-row blocks of nqc steps, 4096 elements a step)
-            const size_t nq = (size_t)p.nqc;
-            const size_t xa = (size_t)(rb / 2) * nq * 4096 + (size_t)(rb % 2) * 2048;
-            const size_t yb = (size_t)cb * nq * 4096;
-            const uint16_t* ah = p.Xhi + xa;
-            const uint16_t* al = p.Xlo + xa;
-            const uint16_t* bh = p.Yhi + yb;
-            const uint16_t* bl = p.Ylo + yb;
+            // 128-row blocks at Q step 0 (nqc steps of 4096 elements each)
+            const size_t nq = (size_t)p.nqc * 4096;
+            const uint16_t* a0 = p.X + (size_t)rb * nq;
+            const uint16_t* b0 = p.Y + (size_t)(2 * cb) * nq;
             for (int kq = 0; kq < nk; kq += KS) {
                 pacer.step(lane, kPaceLimitNs);
                 int ok = 1;
@@ -148,16 +146,13 @@ __global__ void __launch_bounds__(vtile_tc::THREADS, 1) vtile_tc_kernel(VtileArg
                         *abort_flag = 1;
                         ok = 0;
                     } else {
-                        const int nks = min(KS, nk - kq);
+                        const uint32_t bytes = (uint32_t)min(KS, nk - kq) * CHUNK;
                         uint8_t* sb = smem + stage * STAGE_BYTES;
-                        mbar_arrive_expect_tx(&full[stage], (uint32_t)nks * 2 * (SLAB_A + SLAB_B));
+                        mbar_arrive_expect_tx(&full[stage], 3 * bytes);
                         const size_t kk = (size_t)kq * 4096;
-                        for (int q2 = 0; q2 < nks; ++q2) {
-                            bulk_g2s(sb + OFF_AH + q2 * SLAB_A, ah + kk + q2 * 4096, SLAB_A, &full[stage]);
-                            bulk_g2s(sb + OFF_AL + q2 * SLAB_A, al + kk + q2 * 4096, SLAB_A, &full[stage]);
-                        }
-                        bulk_g2s(sb + OFF_BH, bh + kk, nks * SLAB_B, &full[stage]);
-                        bulk_g2s(sb + OFF_BL, bl + kk, nks * SLAB_B, &full[stage]);
+                        bulk_g2s(sb, a0 + kk, bytes, &full[stage]);
+                        bulk_g2s(sb + PIECE, b0 + kk, bytes, &full[stage]);
+                        bulk_g2s(sb + 2 * PIECE, b0 + nq + kk, bytes, &full[stage]);
                     }
                 }
                 if (!__shfl_sync(0xffffffffu, ok, 0)) {
@@ -186,14 +181,14 @@ __global__ void __launch_bounds__(vtile_tc::THREADS, 1) vtile_tc_kernel(VtileArg
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t IDESC = idesc_f16_f32(BM, BN);
+            constexpr uint32_t IDESC = idesc_f16_f32(BM, 128), IDESC2 = idesc_f16_f32(BM, 256);
             uint32_t stage = 0, phase = 0, acc_phase = 0;
             // descriptors at stage 0; a byte offset adds to the low word in units of 16
             const uint32_t sbase = smem_addr(smem);
-            const uint64_t dah = smem_desc_kmajor(sbase + OFF_AH, 128, 256);
-            const uint64_t dal = smem_desc_kmajor(sbase + OFF_AL, 128, 256);
-            const uint64_t dbh = smem_desc_kmajor(sbase + OFF_BH, 128, 256);
-            const uint64_t dbl = smem_desc_kmajor(sbase + OFF_BL, 128, 256);
+            const uint64_t da = smem_desc_kmajor(sbase, 128, 256);
+            const uint64_t d0 = smem_desc_kmajor(sbase + PIECE, 128, 256);
+            const uint64_t d1 = smem_desc_kmajor(sbase + 2 * PIECE, 128, 256);
+            constexpr uint64_t LO = SLAB >> 4;   // the lo slab after the hi slab
             for (int u = first; u < units && !*abort_flag; u += step) {
                 int rb, cb;
                 if (!vtile_unit(p, u, rb, cb)) continue;
@@ -211,16 +206,16 @@ __global__ void __launch_bounds__(vtile_tc::THREADS, 1) vtile_tc_kernel(VtileArg
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t so = (uint64_t)(stage * (STAGE_BYTES >> 4));
-                    const uint32_t more = kq > 0 ? 1u : 0u;
-                    mma_f16(tmem, dah + so, dbh + so, IDESC, more);
-                    mma_f16(tmem + BN, dah + so, dbl + so, IDESC, more);
-                    mma_f16(tmem + BN, dal + so, dbh + so, IDESC, 1u);
-                    if (kq + 1 < nk) {
-                        const uint64_t sa = so + (SLAB_A >> 4), sb = so + (SLAB_B >> 4);
-                        mma_f16(tmem, dah + sa, dbh + sb, IDESC, 1u);
-                        mma_f16(tmem + BN, dah + sa, dbl + sb, IDESC, 1u);
-                        mma_f16(tmem + BN, dal + sa, dbh + sb, IDESC, 1u);
+#pragma unroll
+                    for (int c = 0; c < KS; ++c) {
+                        if (kq + c < nk) {
+                            const uint64_t so = (uint64_t)(stage * (STAGE_BYTES >> 4)) + c * (CHUNK >> 4);
+                            const uint32_t more = c > 0 || kq > 0 ? 1u : 0u;
+                            mma_f16(tmem, da + so, d0 + so, IDESC2, more);
+                            mma_f16(tmem + 128, da + so + LO, d0 + so, IDESC, 1u);
+                            mma_f16(tmem + 256, da + so, d1 + so, IDESC2, more);
+                            mma_f16(tmem + 384, da + so + LO, d1 + so, IDESC, 1u);
+                        }
                     }
                     mma_commit(&empty[stage]);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -266,8 +261,10 @@ __global__ void __launch_bounds__(vtile_tc::THREADS, 1) vtile_tc_kernel(VtileArg
 #pragma unroll 1
             for (int c0 = part * (BN / 4); c0 < (part + 1) * (BN / 4); c0 += 16) {
                 uint32_t h[16], xx[16];
-                tmem_ld16(lane_base + c0, h);
-                tmem_ld16(lane_base + BN + c0, xx);
+                // column c of block c / 128: hh at 256 (c / 128) + c % 128, x 128 further
+                const uint32_t col = (uint32_t)((c0 >> 7) * 256 + (c0 & 127));
+                tmem_ld16(lane_base + col, h);
+                tmem_ld16(lane_base + 128 + col, xx);
                 tmem_ld_wait();
                 float out[16];
 #pragma unroll
