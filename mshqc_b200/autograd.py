@@ -40,7 +40,8 @@ class CDMP2Energy(torch.autograd.Function):
         else:
             e = context.mp2_energy(kind, precision)["total"]
         fctx.kind = kind
-        return torch.tensor(e, dtype=torch.float64, device=C_a.device)
+        # (a fill, not a copy from the host that would wait for the device)
+        return torch.full((), e, dtype=torch.float64, device=C_a.device)
 
     @staticmethod
     def backward(fctx, grad_e):
@@ -68,6 +69,5 @@ def mp2_energy(context: capi.Context, C: torch.Tensor, eps: torch.Tensor, nocc: 
     kind = capi.UNRESTRICTED if C_b is not None else capi.RESTRICTED
     if kind == capi.UNRESTRICTED and (eps_b is None or nocc_b is None):
         raise ValueError("C_b needs eps_b and nocc_b")
-    torch.cuda.current_stream(C.device).synchronize()
     return CDMP2Energy.apply(context, kind, PRECISIONS[precision], int(nocc),
                              int(nocc_b) if nocc_b is not None else 0, C, eps, C_b, eps_b)

@@ -153,6 +153,22 @@ __global__ void count_nonfinite_kernel(const double* __restrict__ x, int64_t n,
     if (local) atomicAdd(bad, local);
 }
 
+// dst = src for two arrays, bad[k] set when array k holds a NaN or infinity
+__global__ void copy_check2_kernel(const double* __restrict__ a, double* __restrict__ da, int64_t na,
+                                   const double* __restrict__ b, double* __restrict__ db, int64_t nb,
+                                   int* __restrict__ bad) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < na + nb;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const bool second = t >= na;
+        const double x = second ? b[t - na] : a[t];
+        if (second)
+            db[t - na] = x;
+        else
+            da[t] = x;
+        if (!isfinite(x)) bad[second ? 1 : 0] = 1;
+    }
+}
+
 bool host_all_finite(const double* x, int64_t n) {
     for (int64_t k = 0; k < n; ++k)
         if (!std::isfinite(x[k])) return false;
@@ -182,7 +198,8 @@ bool is_pinned_host(const void* p) {
 namespace mshqc_cd {
 // Host -> device copy on the context stream.  Pinned sources go straight to
 // the copy engine; pageable ones are staged through two pinned bounce buffers
-// so the CPU memcpy of one chunk overlaps the DMA of the other.
+// so the CPU memcpy of one chunk overlaps the DMA of the other (4 MB: an upload
+// of a few chunks overlaps too, and pinning the buffers takes 2 ms, not 40).
 int upload(mshqc_cd_ctx* ctx, void* dst, const void* src, size_t nbytes) {
     if (nbytes == 0) return MSHQC_CD_OK;
     if (is_pinned_host(src) || nbytes <= (size_t(4) << 20)) {
@@ -190,7 +207,7 @@ int upload(mshqc_cd_ctx* ctx, void* dst, const void* src, size_t nbytes) {
         CD_CUDA(cudaStreamSynchronize(ctx->stream));
         return MSHQC_CD_OK;
     }
-    const size_t chunk = size_t(64) << 20;
+    const size_t chunk = size_t(4) << 20;
     if (!ctx->bounce[0]) {
         for (int b = 0; b < 2; ++b) {
             CD_CUDA(cudaMallocHost(&ctx->bounce[b], chunk));
@@ -221,6 +238,58 @@ int download(mshqc_cd_ctx* ctx, void* dst, const void* src, size_t nbytes, int w
                                                      : cudaMemcpyDeviceToHost,
                             ctx->stream));
     CD_CUDA(cudaStreamSynchronize(ctx->stream));
+    return MSHQC_CD_OK;
+}
+
+int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p) {
+    if (bytes > ctx->hpin_bytes) {
+        if (ctx->hpin) cudaFreeHost(ctx->hpin);
+        ctx->hpin = nullptr;
+        ctx->hpin_bytes = 0;
+        const size_t n = std::max<size_t>(bytes, 16384);
+        CD_CUDA(cudaMallocHost(&ctx->hpin, n));
+        ctx->hpin_bytes = n;
+    }
+    *p = ctx->hpin;
+    return MSHQC_CD_OK;
+}
+
+int begin_call(mshqc_cd_ctx* ctx) {
+    for (auto& s : ctx->spin)
+        if (s.norms_pending) {   // left by a call that failed
+            s.B16_valid = false;
+            s.norms_pending = false;
+        }
+    CD_ALLOC(ctx->status, sizeof(CallStatus), true);
+    return MSHQC_CD_OK;
+}
+
+int finish_call(mshqc_cd_ctx* ctx, CallStatus* out, const void* dev, size_t extra, const void** extra_host) {
+    void* h = nullptr;
+    CD_RC(pinned(ctx, sizeof(CallStatus) + extra, &h));
+    char* he = static_cast<char*>(h) + sizeof(CallStatus);
+    CD_CUDA(cudaMemcpyAsync(h, ctx->status.p, sizeof(CallStatus), cudaMemcpyDeviceToHost, ctx->stream));
+    if (extra) CD_CUDA(cudaMemcpyAsync(he, dev, extra, cudaMemcpyDeviceToHost, ctx->stream));
+    CD_CUDA(cudaStreamSynchronize(ctx->stream));
+    const CallStatus& st = *static_cast<const CallStatus*>(h);
+    for (int k = 0; k < 2; ++k)
+        if (ctx->spin[k].norms_pending) {
+            std::memcpy(&ctx->spin[k].max_norm_hi, &st.norms[k][0], sizeof(double));
+            std::memcpy(&ctx->spin[k].max_norm_lo, &st.norms[k][1], sizeof(double));
+            ctx->spin[k].norms_pending = false;
+        }
+    if (out) *out = st;
+    if (extra_host) *extra_host = he;
+    const char* what = st.tile_err[0]    ? "tensor-core pair kernel"
+                       : st.gamma_err[0] ? "tensor-core backward"
+                       : st.slice_err[0] ? "int8 tensor-core product"
+                                         : nullptr;
+    if (what)
+        return set_error(MSHQC_CD_ERR_TIMEOUT,
+                         std::string(what) + " gave up waiting (site " +
+                             std::to_string(st.tile_err[0] ? st.tile_err[0] : st.gamma_err[0] ? st.gamma_err[0]
+                                                                                               : st.slice_err[0]) +
+                             ")");
     return MSHQC_CD_OK;
 }
 
@@ -297,6 +366,7 @@ int mshqc_cd_ctx_destroy(mshqc_cd_ctx* ctx) {
         if (ctx->bounce[b]) cudaFreeHost(ctx->bounce[b]);
         if (ctx->bounce_ev[b]) cudaEventDestroy(ctx->bounce_ev[b]);
     }
+    if (ctx->hpin) cudaFreeHost(ctx->hpin);
     if (ctx->own) cudaStreamDestroy(ctx->own);
     delete ctx;
     return MSHQC_CD_OK;
@@ -439,20 +509,27 @@ int mshqc_cd_set_orbitals(mshqc_cd_ctx* ctx, int spin, const double* C, const do
         rc = upload(ctx, s.eps.p, eps, sizeof(double) * N);
         if (rc) return rc;
     } else {
-        CD_CUDA(cudaMemcpyAsync(s.C.p, C, sizeof(double) * N * N, cudaMemcpyDeviceToDevice, ctx->stream));
-        CD_CUDA(cudaMemcpyAsync(s.eps.p, eps, sizeof(double) * N, cudaMemcpyDeviceToDevice, ctx->stream));
-        int rc = check_finite_device(ctx, static_cast<double*>(s.C.p), N * N, "C");
-        if (rc) return rc;
-        rc = check_finite_device(ctx, static_cast<double*>(s.eps.p), N, "eps");
-        if (rc) return rc;
+        // copied and checked in one pass
+        CD_ALLOC(ctx->flag, 2 * sizeof(int), true);
+        const int blocks = (int)std::min<int64_t>(8LL * ctx->num_sms, cdiv(N * N + N, 256));
+        copy_check2_kernel<<<blocks, 256, 0, ctx->stream>>>(C, s.C.as<double>(), N * N, eps, s.eps.as<double>(), N,
+                                                            ctx->flag.as<int>());
+        CD_CUDA(cudaGetLastError());
+        ctx->launches++;
+        void* h = nullptr;
+        CD_RC(pinned(ctx, 2 * sizeof(int), &h));
+        CD_CUDA(cudaMemcpyAsync(h, ctx->flag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CD_CUDA(cudaStreamSynchronize(ctx->stream));
+        const int* bad = static_cast<const int*>(h);
+        if (bad[0] || bad[1])
+            return set_error(MSHQC_CD_ERR_NUMERIC, std::string(bad[0] ? "C" : "eps") + " contains NaN/Inf");
     }
     s.nocc = nocc;
     s.set = true;
     s.invalidate();
     ctx->diag_os_valid = false;
     ctx->Yr[spin].ok = false;
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    return MSHQC_CD_OK;
+    return MSHQC_CD_OK;   // (both branches have waited for their copies)
 }
 
 // ---------------------------------------------------------------------------
@@ -462,8 +539,9 @@ int mshqc_cd_transform(mshqc_cd_ctx* ctx, int spin, int precision, double* B_out
     CD_CHECK_CTX();
     if (spin != 0 && spin != 1) return set_error(MSHQC_CD_ERR_ARG, "bad spin");
     DeviceGuard g(ctx->device);
-    int rc = ensure_transform(ctx, spin, precision);
-    if (rc) return rc;
+    CD_RC(begin_call(ctx));
+    CD_RC(ensure_transform(ctx, spin, precision));
+    CD_RC(finish_call(ctx));
     if (B_out) {
         SpinState& s = ctx->spin[spin];
         const int64_t o = s.nocc, v = ctx->N - s.nocc, M = ctx->M;

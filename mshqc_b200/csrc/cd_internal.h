@@ -41,10 +41,10 @@ struct SpinState {
     DevBuf B16;             // hi and lo interleaved (split_bf16.cuh)
     DevBuf expo;            // per-row power-of-two exponents [o][rows]
     DevBuf diag;            // exact (ia|ia) [o][rows]
-    DevBuf norms;           // largest sum hi^2 and sum lo^2 of a row (bit patterns)
     int64_t vp16 = 0, Mp16 = 0;
     double max_norm_hi = 0, max_norm_lo = 0;
     bool B16_valid = false;
+    bool norms_pending = false;   // max_norm_* of the last split still on the device
     int B16_layout = 0;     // rows per orbital: 0 packed (integral tiles), 1 multiples of 256 (pair energies)
     void invalidate() {
         B64_valid = false;
@@ -61,6 +61,8 @@ struct mshqc_cd_ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[6] = {};
     void* bounce[2] = {nullptr, nullptr};
+    void* hpin = nullptr;           // pinned host memory that small results arrive in
+    size_t hpin_bytes = 0;
     cudaEvent_t bounce_ev[2] = {nullptr, nullptr};
 
     int64_t N = 0, M = 0, Mp = 0;
@@ -91,10 +93,9 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf occ_parts;     // dE/dC_occ of both spins in one product
     int L_sym = -1;                 // stored vectors symmetric to the bit (-1: not looked at yet)
     mshqc_cd::DevBuf scratch;       // uploads / unpacking
-    mshqc_cd::DevBuf tables;        // pair and block tables
     mshqc_cd::DevBuf partial;       // per-unit energies
     mshqc_cd::DevBuf pair_sum;      // per-pair energies
-    mshqc_cd::DevBuf totals;        // scalar results
+    mshqc_cd::DevBuf status;        // error flags and scalar results of a call, see CallStatus
     mshqc_cd::DevBuf flag;          // error / NaN flags
     mshqc_cd::DevBuf gemm_ws;       // split-K partials of the FP64 products
     mshqc_cd::DevBuf pace;          // wave-pacing progress counters of the persistent tile kernels
@@ -116,7 +117,6 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf dens_x;        // Fock builds: Cholesky factors of the densities
     mshqc_cd::DevBuf oz_a, oz_b;    // int8 slices of the transform operands (orbitals, vectors)
     mshqc_cd::DevBuf oz_ea, oz_eb;  // their row exponents
-    mshqc_cd::DevBuf oz_flag;       // int8-slice product error flag
     mshqc_cd::DevBuf oz_p;          // per-batch FP64 partial products (transposed transforms)
     bool diag_os_valid = false;
     int fixed_point_exact = 1;      // Cauchy-Schwarz bound of the last tensor-core pass held
@@ -144,11 +144,11 @@ struct mshqc_cd_ctx {
         for (auto& p : pair_energy) p.clear();
     }
     size_t held_bytes() const {
-        size_t b = L.bytes + Y.bytes + scratch.bytes + tables.bytes + partial.bytes +
-                   pair_sum.bytes + totals.bytes + flag.bytes + amp.bytes + ampT.bytes + BT.bytes + W.bytes;
+        size_t b = L.bytes + Y.bytes + scratch.bytes + partial.bytes +
+                   pair_sum.bytes + flag.bytes + amp.bytes + ampT.bytes + BT.bytes + W.bytes;
         for (const auto& s : spin)
             b += s.C.bytes + s.eps.bytes + s.B64.bytes + s.B16.bytes + s.expo.bytes +
-                 s.diag.bytes + s.norms.bytes;
+                 s.diag.bytes;
         b += gemm_ws.bytes + dens_x.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
         for (const auto& g : gam) b += g.bytes;
         for (const auto& g : grad) b += g.bytes;
@@ -161,10 +161,9 @@ struct mshqc_cd_ctx {
         L.release();
         Y.release();
         scratch.release();
-        tables.release();
         partial.release();
         pair_sum.release();
-        totals.release();
+        status.release();
         flag.release();
         gemm_ws.release();
         cpack.release();
@@ -184,7 +183,6 @@ struct mshqc_cd_ctx {
             s.B16.release();
             s.expo.release();
             s.diag.release();
-            s.norms.release();
         }
         diag_os.release();
         Hcore.release();
@@ -198,7 +196,6 @@ struct mshqc_cd_ctx {
         oz_b.release();
         oz_ea.release();
         oz_eb.release();
-        oz_flag.release();
         oz_p.release();
         for (auto& g : gam) g.release();
         for (auto& g : grad) g.release();
@@ -240,6 +237,24 @@ int check_finite_device(mshqc_cd_ctx* ctx, const double* x, int64_t n, const cha
         int _rc = (x);       \
         if (_rc) return _rc; \
     } while (0)
+
+// What a call's kernels report, in ctx->status: zeroed by begin_call, copied
+// back once by finish_call (one copy, one synchronization).
+struct CallStatus {
+    int tile_err[2];        // pair-energy / integral-tile kernel: wait given up, accumulator beyond 2^24
+    int gamma_err[2];
+    int slice_err[2];       // int8-slice products
+    int pad[2];
+    double totals[4];       // energies
+    unsigned long long norms[2][2];   // largest sum hi^2, sum lo^2 of a row per spin (bit patterns)
+};
+// pinned host memory of at least `bytes` (grow-only; contents not kept)
+int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p);
+int begin_call(mshqc_cd_ctx* ctx);
+// Waits for the call's work, reports kernels that gave up, and copies `extra`
+// bytes from dev to the pinned buffer behind the status (*extra_host).
+int finish_call(mshqc_cd_ctx* ctx, CallStatus* st = nullptr, const void* dev = nullptr, size_t extra = 0,
+                const void** extra_host = nullptr);
 
 // implemented in cd_mp2.cu
 // layout: of the fixed-point operands of a mixed-precision request

@@ -186,6 +186,7 @@ template <class C>
 size_t oz_bytes(const OzakiOperand& op) {
     return ozaki::operand_bytes<C>(op.Rp, op.Kp) * (size_t)op.batch;
 }
+int* slice_err(mshqc_cd_ctx* ctx) { return ctx->status.as<CallStatus>()->slice_err; }
 template <class C>
 int oz_mul(mshqc_cd_ctx* ctx, const OzakiOperand& X, bool x_shared, const OzakiOperand& Y, bool y_shared, bool sw,
            double* out, int64_t ldc, int64_t cb, double alpha, double beta) {
@@ -193,7 +194,7 @@ int oz_mul(mshqc_cd_ctx* ctx, const OzakiOperand& X, bool x_shared, const OzakiO
     o.a_shared = sw ? y_shared : x_shared;
     o.b_shared = sw ? x_shared : y_shared;
     o.trans = sw;
-    CD_CUDA(ozaki_gemm<C>(sw ? Y : X, sw ? X : Y, out, ldc, cb, alpha, beta, o, ctx->oz_flag.as<int>(), ctx->num_sms,
+    CD_CUDA(ozaki_gemm<C>(sw ? Y : X, sw ? X : Y, out, ldc, cb, alpha, beta, o, slice_err(ctx), ctx->num_sms,
                           ctx->stream));
     ctx->launches++;
     return MSHQC_CD_OK;
@@ -206,16 +207,6 @@ int oz_reserve(mshqc_cd_ctx* ctx, DevBuf& q, DevBuf& e, size_t bytes, OzakiOpera
     op.e = e.as<int>();
     return MSHQC_CD_OK;
 }
-int oz_check(mshqc_cd_ctx* ctx, const char* what) {
-    int herr = 0;
-    CD_CUDA(cudaMemcpyAsync(&herr, ctx->oz_flag.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (herr)
-        return set_error(MSHQC_CD_ERR_TIMEOUT,
-                         std::string(what) + " gave up waiting (site " + std::to_string(herr) + ")");
-    return MSHQC_CD_OK;
-}
-
 // the rows of Y that hold a spin's half-transformed vectors
 double* y_rows(mshqc_cd_ctx* ctx, int spin) {
     return ctx->Y.as<double>() + ctx->Yr[spin].row * ctx->M * ctx->N;
@@ -322,7 +313,6 @@ int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, 
     const bool sw = round_up(rows, Cfg::BN) < round_up(rows, ozaki::BM);
     OzakiOperand Ao = oz_operand<Cfg>(rows, N, !sw, 1);
     if (i8) {
-        CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
         CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(Ao), Ao));
         CD_CUDA(ozaki_slice<Cfg>(C, N, 0, Ao, ctx->num_sms, ctx->stream));
         ctx->launches++;
@@ -374,7 +364,6 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
         s.B64_prec = i8 ? MSHQC_CD_FP16X3 : MSHQC_CD_FP64;
     }
     CD_RC(first_half(ctx, nsp, spins, lo, hi, i8));
-    bool sliced = i8;
     for (int k = 0; k < nsp; ++k) {
         SpinState& s = ctx->spin[spins[k]];
         const int64_t o = s.nocc, v = N - o, ni = hi[k] - lo[k];
@@ -385,8 +374,6 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
         }
         const char* tenv = std::getenv("MSHQC_CD_TRANSFORM");   // f64: DMMA for both halves
         if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
-            CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, !sliced);
-            sliced = true;
             CD_RC(second_half_sliced<ozaki::Full>(ctx, spins[k], lo[k], hi[k]));
             continue;
         }
@@ -399,7 +386,7 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
         g.alpha = 1.0;  g.beta = 0.0;
         CD_RC(gemm_run(ctx, g, true, true));
     }
-    return sliced ? oz_check(ctx, "int8 tensor-core transform") : MSHQC_CD_OK;
+    return MSHQC_CD_OK;
 }
 
 // Whether the half-transformed vectors of both spins may be held at once: the
@@ -443,7 +430,7 @@ int sliced_integrals(mshqc_cd_ctx* ctx, const SpinState& X, const SpinState& Y, 
     CD_CUDA(ozaki_slice<Cfg>(Y.B64.as<double>() + J0 * Y.vp * Mp, Mp, 0, B, ctx->num_sms, ctx->stream));
     OzakiOpts o;
     o.tri = tri ? (int)X.vp : 0;
-    CD_CUDA(ozaki_gemm<Cfg>(A, B, S, nJ * Y.vp, 0, 1.0, 0.0, o, ctx->oz_flag.as<int>(), ctx->num_sms, ctx->stream));
+    CD_CUDA(ozaki_gemm<Cfg>(A, B, S, nJ * Y.vp, 0, 1.0, 0.0, o, slice_err(ctx), ctx->num_sms, ctx->stream));
     ctx->launches += 3;
     return MSHQC_CD_OK;
 }
@@ -468,112 +455,69 @@ int sliced_gamma(mshqc_cd_ctx* ctx, const double* A, int64_t lda, bool transpose
         CD_ALLOC(ctx->pace, sizeof(int) * (size_t)ctx->num_sms, false);
         o.pace = ctx->pace.as<int>();
     }
-    CD_CUDA(ozaki_gemm<Cfg>(Ta, Tb, gamma, Mp, 0, 1.0, 1.0, o, ctx->oz_flag.as<int>(), ctx->num_sms, ctx->stream));
+    CD_CUDA(ozaki_gemm<Cfg>(Ta, Tb, gamma, Mp, 0, 1.0, 1.0, o, slice_err(ctx), ctx->num_sms, ctx->stream));
     ctx->launches += transposed ? 5 : 4;
     return MSHQC_CD_OK;
 }
 
-struct UnitTables {
-    std::vector<int2> pairs, blocks;
+// One pair-energy pass: spins, where its pair sums go (ctx->pair_sum, doubles:
+// npairs sums, for the restricted mode npairs opposite-spin sums after them) and
+// its totals (CallStatus::totals).
+struct PairPass {
+    int mode, sx, sy;
+    int npairs, ox, oy;
+    int64_t off;
+    int total;
 };
 
-UnitTables make_tables(int mode, int ox, int oy, int nbx, int nby) {
-    UnitTables t;
-    if (mode == PAIR_OPPOSITE_SPIN) {
-        for (int i = 0; i < ox; ++i)
-            for (int j = 0; j < oy; ++j) t.pairs.push_back(make_int2(i, j));
-        for (int x = 0; x < nbx; ++x)
-            for (int y = 0; y < nby; y += 2) t.blocks.push_back(make_int2(x, y));
-    } else {
-        for (int i = 0; i < ox; ++i)
-            for (int j = (mode == PAIR_RESTRICTED ? i : i + 1); j < ox; ++j)
-                t.pairs.push_back(make_int2(i, j));
-        for (int x = 0; x < nbx; ++x)
-            for (int y = x; y < nbx; ++y) t.blocks.push_back(make_int2(x, y));
-    }
-    return t;
-}
-
-// Deterministic reductions of per-unit partials into pair energies and totals,
-// and the host copy of the ordered pair-energy matrix.
-int reduce_and_collect(mshqc_cd_ctx* ctx, int mode, const UnitTables& t, int64_t units, int npairs,
-                       int nblocks, int ox, int oy, double* total, std::vector<double>& pair_mat,
-                       double* total_os) {
+// Deterministic reductions of per-unit partials (ctx->partial, the opposite-spin
+// part of the restricted mode after them) into the pass's sums and totals.
+int reduce_units(mshqc_cd_ctx* ctx, const PairPass& p, int nblocks) {
+    const unsigned planes = p.mode == PAIR_RESTRICTED ? 2 : 1;
+    double* sums = ctx->pair_sum.as<double>() + p.off;
+    reduce_pairs_kernel<<<dim3((unsigned)cdiv(p.npairs, 128), planes), 128, 0, ctx->stream>>>(
+        ctx->partial.as<double>(), p.npairs, nblocks, sums);
+    CD_CUDA(cudaGetLastError());
+    reduce_total_kernel<<<planes, 256, 0, ctx->stream>>>(sums, p.npairs, ctx->status.as<CallStatus>()->totals + p.total);
+    CD_CUDA(cudaGetLastError());
     ctx->launches += 2;
-    reduce_pairs_kernel<<<(unsigned)cdiv(npairs, 128), 128, 0, ctx->stream>>>(
-        ctx->partial.as<double>(), npairs, nblocks, ctx->pair_sum.as<double>());
-    CD_CUDA(cudaGetLastError());
-    reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(ctx->pair_sum.as<double>(), npairs,
-                                                   ctx->totals.as<double>());
-    CD_CUDA(cudaGetLastError());
-    if (mode == PAIR_RESTRICTED && total_os) {
-        ctx->launches += 2;
-        reduce_pairs_kernel<<<(unsigned)cdiv(npairs, 128), 128, 0, ctx->stream>>>(
-            ctx->partial.as<double>() + units, npairs, nblocks, ctx->pair_sum.as<double>() + npairs);
-        CD_CUDA(cudaGetLastError());
-        reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(ctx->pair_sum.as<double>() + npairs, npairs,
-                                                       ctx->totals.as<double>() + 1);
-        CD_CUDA(cudaGetLastError());
-        CD_CUDA(cudaMemcpyAsync(total_os, ctx->totals.as<double>() + 1, sizeof(double),
-                                cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    std::vector<double> ps(npairs);
-    CD_CUDA(cudaMemcpyAsync(ps.data(), ctx->pair_sum.p, sizeof(double) * npairs,
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaMemcpyAsync(total, ctx->totals.p, sizeof(double), cudaMemcpyDeviceToHost,
-                            ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (int p = 0; p < npairs; ++p) {
-        const int i = t.pairs[p].x, j = t.pairs[p].y;
-        if (mode == PAIR_OPPOSITE_SPIN) {
-            pair_mat[(size_t)i * oy + j] = ps[p];
-        } else if (i == j) {
-            pair_mat[(size_t)i * ox + j] = ps[p];
-        } else {
-            pair_mat[(size_t)i * ox + j] = 0.5 * ps[p];
-            pair_mat[(size_t)j * ox + i] = 0.5 * ps[p];
-        }
-    }
     return MSHQC_CD_OK;
 }
 
-template <int MODE>
-int pair_pass_f64_staged(mshqc_cd_ctx* ctx, int sx, int sy, double* total, std::vector<double>& pair_mat,
-                         double* total_os);
+// The ordered pair-energy matrix (row-major ox * oy) from a pass's pair sums.
+void fill_pairs(const PairPass& p, const double* ps, std::vector<double>& m) {
+    const int ox = p.ox, oy = p.oy;
+    m.assign((size_t)ox * oy, 0.0);
+    if (p.mode == PAIR_OPPOSITE_SPIN) {
+        std::memcpy(m.data(), ps, sizeof(double) * m.size());
+        return;
+    }
+    for (int i = 0; i < ox; ++i)
+        for (int j = p.mode == PAIR_RESTRICTED ? i : i + 1; j < ox; ++j) {
+            const double e = *ps++;
+            m[(size_t)i * ox + j] = i == j ? e : 0.5 * e;
+            m[(size_t)j * ox + i] = i == j ? e : 0.5 * e;
+        }
+}
 
-// One FP64 pair-energy pass.  Returns the total in *total and fills the
-// ordered pair-energy matrix (row-major ox*oy) in pair_mat.
-int pair_pass_f64(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
-                  std::vector<double>& pair_mat, double* total_os = nullptr) {
-    const SpinState& X = ctx->spin[sx];
-    const SpinState& Y = ctx->spin[sy];
-    const int ox = (int)X.nocc, oy = (int)Y.nocc;
+template <int MODE>
+int pair_pass_f64_staged(mshqc_cd_ctx* ctx, const PairPass& pp);
+
+// One FP64 pair-energy pass.
+int pair_pass_f64(mshqc_cd_ctx* ctx, const PairPass& pp) {
+    const SpinState& X = ctx->spin[pp.sx];
+    const SpinState& Y = ctx->spin[pp.sy];
+    const int mode = pp.mode, ox = pp.ox, oy = pp.oy;
     const int vx = (int)(ctx->N - ox), vy = (int)(ctx->N - oy);
     const int nbx = (int)(X.vp / 64), nby = (int)(Y.vp / 64);
     if (sliced_pairs(ctx, ox * X.vp, oy * Y.vp)) {
-        if (mode == PAIR_RESTRICTED) return pair_pass_f64_staged<PAIR_RESTRICTED>(ctx, sx, sy, total, pair_mat, total_os);
-        if (mode == PAIR_SAME_SPIN) return pair_pass_f64_staged<PAIR_SAME_SPIN>(ctx, sx, sy, total, pair_mat, total_os);
-        return pair_pass_f64_staged<PAIR_OPPOSITE_SPIN>(ctx, sx, sy, total, pair_mat, total_os);
+        if (mode == PAIR_RESTRICTED) return pair_pass_f64_staged<PAIR_RESTRICTED>(ctx, pp);
+        if (mode == PAIR_SAME_SPIN) return pair_pass_f64_staged<PAIR_SAME_SPIN>(ctx, pp);
+        return pair_pass_f64_staged<PAIR_OPPOSITE_SPIN>(ctx, pp);
     }
-    UnitTables t = make_tables(mode, ox, oy, nbx, nby);
-    const int npairs = (int)t.pairs.size(), nblocks = (int)t.blocks.size();
-    pair_mat.assign((size_t)ox * oy, 0.0);
-    *total = 0.0;
-    if (npairs == 0 || nblocks == 0) return MSHQC_CD_OK;
-
-    const size_t tbytes = sizeof(int2) * (t.pairs.size() + t.blocks.size());
-    CD_ALLOC(ctx->tables, tbytes, false);
-    int2* dpairs = ctx->tables.as<int2>();
-    int2* dblocks = dpairs + npairs;
-    CD_CUDA(cudaMemcpyAsync(dpairs, t.pairs.data(), sizeof(int2) * npairs, cudaMemcpyHostToDevice,
-                            ctx->stream));
-    CD_CUDA(cudaMemcpyAsync(dblocks, t.blocks.data(), sizeof(int2) * nblocks,
-                            cudaMemcpyHostToDevice, ctx->stream));
+    const int npairs = pp.npairs, nblocks = (int)block_count(mode, nbx, nby);
     const int64_t units = (int64_t)npairs * nblocks;
     CD_ALLOC(ctx->partial, sizeof(double) * units * 2, false);
-    CD_ALLOC(ctx->pair_sum, sizeof(double) * npairs * 2, false);
-    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
-
     PairF64Args a{};
     a.X = X.B64.as<double>();
     a.Y = Y.B64.as<double>();
@@ -582,8 +526,7 @@ int pair_pass_f64(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     a.Mp = (int)ctx->Mp;
     a.eox = X.eps.as<double>();  a.evx = a.eox + ox;
     a.eoy = Y.eps.as<double>();  a.evy = a.eoy + oy;
-    a.pairs = dpairs;
-    a.blocks = dblocks;
+    a.ox = ox;  a.oy = oy;  a.nbx = nbx;  a.nby = nby;
     a.nblocks = nblocks;
     a.partial = ctx->partial.as<double>();
     a.partial2 = ctx->partial.as<double>() + units;
@@ -605,25 +548,19 @@ int pair_pass_f64(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     end_stage(ctx);
     CD_CUDA(cudaGetLastError());
     ctx->launches++;
-    CD_RC(reduce_and_collect(ctx, mode, t, units, npairs, nblocks, ox, oy, total, pair_mat, total_os));
-    return MSHQC_CD_OK;
+    return reduce_units(ctx, pp, nblocks);
 }
 
 
 // The FP64 pair-energy pass of larger systems: integrals of block pairs into a
 // staging block (int8 slices of full accuracy), energies from there.
 template <int MODE>
-int pair_pass_f64_staged(mshqc_cd_ctx* ctx, int sx, int sy, double* total, std::vector<double>& pair_mat,
-                         double* total_os) {
+int pair_pass_f64_staged(mshqc_cd_ctx* ctx, const PairPass& pp) {
     constexpr bool kSym = MODE != PAIR_OPPOSITE_SPIN;
-    const SpinState& X = ctx->spin[sx];
-    const SpinState& Y = ctx->spin[sy];
+    const SpinState& X = ctx->spin[pp.sx];
+    const SpinState& Y = ctx->spin[pp.sy];
     const int64_t ox = X.nocc, oy = Y.nocc;
-    UnitTables t = make_tables(MODE, (int)ox, (int)oy, 0, 0);
-    const int npairs = (int)t.pairs.size();
-    pair_mat.assign((size_t)(ox * oy), 0.0);
-    *total = 0.0;
-    if (npairs == 0) return MSHQC_CD_OK;
+    const int npairs = pp.npairs;
     size_t free_b = 0, total_b = 0;
     CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t budget = std::min<size_t>((free_b + ctx->W.bytes) / 3, size_t(40) << 30);
@@ -636,9 +573,6 @@ int pair_pass_f64_staged(mshqc_cd_ctx* ctx, int sx, int sy, double* total, std::
     const int64_t units = (int64_t)npairs * nch;
     CD_ALLOC(ctx->W, (size_t)(bI * bJ * per_row), false);
     CD_ALLOC(ctx->partial, sizeof(double) * (size_t)units * 2, false);
-    CD_ALLOC(ctx->pair_sum, sizeof(double) * (size_t)npairs * 2, false);
-    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
-    CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
     begin_stage(ctx, ST_PAIR);
     for (int64_t I0 = 0; I0 < ox; I0 += bI) {
         const int64_t nI = std::min(bI, ox - I0);
@@ -663,8 +597,7 @@ int pair_pass_f64_staged(mshqc_cd_ctx* ctx, int sx, int sy, double* total, std::
         }
     }
     end_stage(ctx);
-    CD_RC(reduce_and_collect(ctx, MODE, t, units, npairs, nch, (int)ox, (int)oy, total, pair_mat, total_os));
-    return oz_check(ctx, "int8 tensor-core pair integrals");
+    return reduce_units(ctx, pp, nch);
 }
 
 // ---------------------------------------------------------------------------
@@ -685,7 +618,8 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
     CD_ALLOC(s.B16, 2 * n * sizeof(uint16_t), false);
     CD_ALLOC(s.expo, sizeof(int) * o * rows, true);
     CD_ALLOC(s.diag, sizeof(double) * o * rows, true);
-    CD_ALLOC(s.norms, sizeof(unsigned long long) * 2, true);
+    // (a spin is split once per call: its slots in the status are zero)
+    unsigned long long* norms = ctx->status.as<CallStatus>()->norms[spin];
     s.vp16 = rows;
     s.Mp16 = Mp;
     {
@@ -693,7 +627,7 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
         const int blocks = (int)std::min<int64_t>(cdiv(warps * 32, 256), (int64_t)ctx->num_sms * 32);
         row_scale_kernel<<<blocks, 256, 0, ctx->stream>>>(
             s.B64.as<double>(), s.vp, Mp, (int)v, (int)M, o, rows, s.expo.as<int>(),
-            s.diag.as<double>(), nullptr, 0, 0, 0, nullptr, s.norms.as<unsigned long long>());
+            s.diag.as<double>(), nullptr, 0, 0, 0, nullptr, norms);
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
     }
@@ -706,12 +640,9 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
     }
-    // largest row norms: the Cauchy-Schwarz bound of the integer accumulators
-    double hn[2];
-    CD_CUDA(cudaMemcpyAsync(hn, s.norms.p, sizeof(hn), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    s.max_norm_hi = hn[0];
-    s.max_norm_lo = hn[1];
+    // largest row norms (the Cauchy-Schwarz bound of the integer accumulators):
+    // with the call's status
+    s.norms_pending = true;
     s.B16_valid = true;
     s.B16_layout = layout;
     return MSHQC_CD_OK;
@@ -740,23 +671,6 @@ int opposite_spin_diag(mshqc_cd_ctx* ctx) {
     return MSHQC_CD_OK;
 }
 
-UnitTables make_tables_tc(int mode, int ox, int oy, int nbx, int nby) {
-    UnitTables t;
-    if (mode == PAIR_OPPOSITE_SPIN) {
-        for (int i = 0; i < ox; ++i)
-            for (int j = 0; j < oy; ++j) t.pairs.push_back(make_int2(i, j));
-        for (int x = 0; x < nbx; ++x)
-            for (int y = 0; y < nby; y += 2) t.blocks.push_back(make_int2(x, y));
-    } else {
-        for (int i = 0; i < ox; ++i)
-            for (int j = (mode == PAIR_RESTRICTED ? i : i + 1); j < ox; ++j)
-                t.pairs.push_back(make_int2(i, j));
-        for (int x = 0; x < nbx; ++x)
-            for (int y = x; y < nbx; ++y) t.blocks.push_back(make_int2(x, y));
-    }
-    return t;
-}
-
 template <int MODE>
 cudaError_t launch_tc(const PairTcArgs& a, int grid, cudaStream_t st) {
     const size_t smem = pair_tc::SMEM_BYTES;
@@ -767,42 +681,27 @@ cudaError_t launch_tc(const PairTcArgs& a, int grid, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-int pair_pass_tc(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
-                 std::vector<double>& pair_mat, double* total_os = nullptr) {
-    const SpinState& X = ctx->spin[sx];
-    const SpinState& Y = ctx->spin[sy];
-    const int ox = (int)X.nocc, oy = (int)Y.nocc;
+// The integer accumulators of a pass are exact when every partial sum stays
+// below 2^24: |sum hi hi'| <= sqrt(max sum hi^2 * max sum hi'^2), likewise for
+// the cross terms (Cauchy-Schwarz over the Q index).
+bool pass_exact(const mshqc_cd_ctx* ctx, const PairPass& pp) {
+    const SpinState& X = ctx->spin[pp.sx];
+    const SpinState& Y = ctx->spin[pp.sy];
+    const double lim = 16777216.0;
+    const double bhh = std::sqrt(X.max_norm_hi * Y.max_norm_hi);
+    const double bx = std::sqrt(X.max_norm_hi * Y.max_norm_lo) + std::sqrt(X.max_norm_lo * Y.max_norm_hi);
+    return bhh < lim && bx < lim;
+}
+
+int pair_pass_tc(mshqc_cd_ctx* ctx, const PairPass& pp) {
+    const SpinState& X = ctx->spin[pp.sx];
+    const SpinState& Y = ctx->spin[pp.sy];
+    const int mode = pp.mode, ox = pp.ox, oy = pp.oy;
     const int vx = (int)(ctx->N - ox), vy = (int)(ctx->N - oy);
     const int nbx = (int)cdiv(vx, 128), nby = (int)cdiv(vy, 128);
-    UnitTables t = make_tables_tc(mode, ox, oy, nbx, nby);
-    const int npairs = (int)t.pairs.size(), nblocks = (int)t.blocks.size();
-    pair_mat.assign((size_t)ox * oy, 0.0);
-    *total = 0.0;
-    if (total_os) *total_os = 0.0;
-    if (npairs == 0 || nblocks == 0) return MSHQC_CD_OK;
-    const size_t tbytes = sizeof(int2) * (t.pairs.size() + t.blocks.size());
-    CD_ALLOC(ctx->tables, tbytes, false);
-    int2* dpairs = ctx->tables.as<int2>();
-    int2* dblocks = dpairs + npairs;
-    CD_CUDA(cudaMemcpyAsync(dpairs, t.pairs.data(), sizeof(int2) * npairs, cudaMemcpyHostToDevice,
-                            ctx->stream));
-    CD_CUDA(cudaMemcpyAsync(dblocks, t.blocks.data(), sizeof(int2) * nblocks,
-                            cudaMemcpyHostToDevice, ctx->stream));
+    const int npairs = pp.npairs, nblocks = (int)block_count(mode, nbx, nby);
     const int64_t units = (int64_t)npairs * nblocks;
     CD_ALLOC(ctx->partial, sizeof(double) * units * 2, false);
-    CD_ALLOC(ctx->pair_sum, sizeof(double) * npairs * 2, false);
-    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
-    CD_ALLOC(ctx->flag, sizeof(int) * 4, true);
-
-    // the integer accumulators are exact when every partial sum stays below
-    // 2^24: |sum hi hi'| <= sqrt(max sum hi^2 * max sum hi'^2), likewise for
-    // the cross terms (Cauchy-Schwarz over the Q index)
-    {
-        const double lim = 16777216.0;
-        const double bhh = std::sqrt(X.max_norm_hi * Y.max_norm_hi);
-        const double bx = std::sqrt(X.max_norm_hi * Y.max_norm_lo) + std::sqrt(X.max_norm_lo * Y.max_norm_hi);
-        if (!(bhh < lim && bx < lim)) ctx->fixed_point_exact = 0;
-    }
     if (mode == PAIR_OPPOSITE_SPIN) {
         begin_stage(ctx, ST_SPLIT);
         CD_RC(opposite_spin_diag(ctx));
@@ -828,11 +727,12 @@ int pair_pass_tc(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     a.vx = vx;  a.vy = vy;
     a.eox = X.eps.as<double>();  a.evx = a.eox + ox;
     a.eoy = Y.eps.as<double>();  a.evy = a.eoy + oy;
-    a.pairs = dpairs;  a.blocks = dblocks;  a.nblocks = nblocks;
+    a.ox = ox;  a.oy = oy;  a.nbx = nbx;  a.nby = nby;
+    a.nblocks = nblocks;
     a.units = units;
     a.partial = ctx->partial.as<double>();
     a.partial2 = ctx->partial.as<double>() + units;
-    a.err = ctx->flag.as<int>();
+    a.err = ctx->status.as<CallStatus>()->tile_err;
     const int grid = (int)std::min<int64_t>(units, ctx->num_sms);
     cudaError_t e;
     begin_stage(ctx, ST_PAIR);
@@ -845,13 +745,7 @@ int pair_pass_tc(mshqc_cd_ctx* ctx, int mode, int sx, int sy, double* total,
     end_stage(ctx);
     if (e != cudaSuccess) return cuda_error(e, "pair_energy_tc_kernel launch");
     ctx->launches++;
-    int herr = 0;
-    CD_CUDA(cudaMemcpyAsync(&herr, ctx->flag.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_RC(reduce_and_collect(ctx, mode, t, units, npairs, nblocks, ox, oy, total, pair_mat, total_os));
-    if (herr)
-        return set_error(MSHQC_CD_ERR_TIMEOUT,
-                         "tensor-core pair kernel gave up waiting (site " + std::to_string(herr) + ")");
-    return MSHQC_CD_OK;
+    return reduce_units(ctx, pp, nblocks);
 }
 
 }  // namespace
@@ -920,14 +814,10 @@ int run_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* out)
     std::memset(out, 0, sizeof(*out));
     ctx->fixed_point_exact = 1;
     reset_stages(ctx);
-    auto pass = [&](int mode, int sx, int sy, double* tot, std::vector<double>& pm,
-                    double* tot_os) {
-        return precision == MSHQC_CD_FP16X3 ? pair_pass_tc(ctx, mode, sx, sy, tot, pm, tot_os)
-                                            : pair_pass_f64(ctx, mode, sx, sy, tot, pm, tot_os);
-    };
     CD_RC(require_inputs(ctx, 0));
     if (kind == MSHQC_CD_UNRESTRICTED) CD_RC(require_inputs(ctx, 1));
     cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2];
+    CD_RC(begin_call(ctx));
     CD_CUDA(cudaEventRecord(e0, ctx->stream));
     if (kind == MSHQC_CD_UNRESTRICTED)
         CD_RC(ensure_transforms(ctx, precision, 1));
@@ -935,25 +825,53 @@ int run_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* out)
         CD_RC(ensure_transform(ctx, 0, precision, 1));
     CD_CUDA(cudaEventRecord(e1, ctx->stream));
     for (auto& p : ctx->pair_energy) p.clear();
+    // the passes, their sums one after the other: one copy back at the end
+    PairPass pass[3];
+    int np = 0;
+    int64_t copied = 0, sums = 0;
+    auto add = [&](int mode, int sx, int sy) {
+        PairPass& p = pass[np];
+        p.mode = mode;
+        p.sx = sx;
+        p.sy = sy;
+        p.ox = (int)ctx->spin[sx].nocc;
+        p.oy = (int)ctx->spin[sy].nocc;
+        p.npairs = (int)pair_count(mode, p.ox, p.oy);
+        p.off = copied;
+        p.total = np++;
+        copied += p.npairs;
+        sums = copied + (mode == PAIR_RESTRICTED ? p.npairs : 0);
+    };
     if (kind == MSHQC_CD_RESTRICTED) {
-        double e_os = 0.0, e_tot = 0.0;
-        CD_RC(pass(PAIR_RESTRICTED, 0, 0, &e_tot, ctx->pair_energy[0], &e_os));
-        out->total = e_tot;
-        out->os = e_os;
-        out->ss_aa = out->ss_bb = 0.5 * (e_tot - e_os);
+        add(PAIR_RESTRICTED, 0, 0);
     } else {
-        double ss_a = 0, ss_b = 0, os = 0;
-        CD_RC(pass(PAIR_SAME_SPIN, 0, 0, &ss_a, ctx->pair_energy[0], nullptr));
-        CD_RC(pass(PAIR_SAME_SPIN, 1, 1, &ss_b, ctx->pair_energy[1], nullptr));
-        CD_RC(pass(PAIR_OPPOSITE_SPIN, 0, 1, &os, ctx->pair_energy[2], nullptr));
-        out->ss_aa = ss_a;
-        out->ss_bb = ss_b;
-        out->os = os;
-        out->total = ss_a + ss_b + os;
+        add(PAIR_SAME_SPIN, 0, 0);
+        add(PAIR_SAME_SPIN, 1, 1);
+        add(PAIR_OPPOSITE_SPIN, 0, 1);
     }
+    CD_ALLOC(ctx->pair_sum, sizeof(double) * (size_t)std::max<int64_t>(1, sums), false);
+    for (int k = 0; k < np; ++k)
+        if (pass[k].npairs > 0)   // (no same-spin pair with one electron)
+            CD_RC(precision == MSHQC_CD_FP16X3 ? pair_pass_tc(ctx, pass[k]) : pair_pass_f64(ctx, pass[k]));
     CD_CUDA(cudaEventRecord(e2, ctx->stream));
-    CD_CUDA(cudaEventSynchronize(e2));
+    CallStatus st;
+    const void* hs = nullptr;
+    CD_RC(finish_call(ctx, &st, ctx->pair_sum.p, sizeof(double) * (size_t)copied, &hs));
     collect_stages(ctx);
+    for (int k = 0; k < np; ++k) {
+        fill_pairs(pass[k], static_cast<const double*>(hs) + pass[k].off, ctx->pair_energy[k]);
+        if (precision == MSHQC_CD_FP16X3 && pass[k].npairs > 0 && !pass_exact(ctx, pass[k])) ctx->fixed_point_exact = 0;
+    }
+    if (kind == MSHQC_CD_RESTRICTED) {
+        out->total = st.totals[0];
+        out->os = st.totals[1];
+        out->ss_aa = out->ss_bb = 0.5 * (out->total - out->os);
+    } else {
+        out->ss_aa = st.totals[0];
+        out->ss_bb = st.totals[1];
+        out->os = st.totals[2];
+        out->total = out->ss_aa + out->ss_bb + out->os;
+    }
     float t01 = 0, t12 = 0;
     CD_CUDA(cudaEventElapsedTime(&t01, e0, e1));
     CD_CUDA(cudaEventElapsedTime(&t12, e1, e2));
@@ -1192,7 +1110,6 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double s
         }
         CD_RC(first_half(ctx, nsp, spins, lo, hi, i8));
     }
-    if (i8) CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, have);   // (the first half has zeroed it otherwise)
     for (int k = 0; k < nsp; ++k) {
         if (hi[k] <= lo[k]) continue;
         CD_RC(i8 ? virtual_part_i8(ctx, spins[k], scale, dC[k]) : virtual_part_f64(ctx, spins[k], scale, dC[k]));
@@ -1205,8 +1122,7 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double s
 // the int8 products for the mixed path (unless switched off), FP64 otherwise
 int transposed_dispatch(mshqc_cd_ctx* ctx, int nsp, const int* spins, double scale, double* const* dC, int precision) {
     const bool i8 = precision == MSHQC_CD_FP16X3 && int8_transform_enabled(ctx);
-    CD_RC(transposed_transforms(ctx, nsp, spins, scale, dC, i8));
-    return i8 ? oz_check(ctx, "int8 tensor-core transposed transform") : MSHQC_CD_OK;
+    return transposed_transforms(ctx, nsp, spins, scale, dC, i8);
 }
 
 // ---------------------------------------------------------------------------
@@ -1228,6 +1144,18 @@ BwdDims bwd_dims(const mshqc_cd_ctx* ctx, int spin) {
     d.VR = round_up(d.v, 128);
     d.VS = round_up(d.VR, 256);
     return d;
+}
+
+// Bytes a backward pass may stage: a third of the free memory (the staging it
+// already holds included), at most 40 GB.  A pass of a small system whose
+// staging is held already does not ask the driver (20 us).
+int staging_budget(mshqc_cd_ctx* ctx, size_t held, double whole, size_t* budget) {
+    *budget = size_t(40) << 30;
+    if (whole <= (double)std::min<size_t>(held, size_t(256) << 20)) return MSHQC_CD_OK;
+    size_t free_b = 0, total_b = 0;
+    CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    *budget = std::min<size_t>((free_b + held) / 3, *budget);
+    return MSHQC_CD_OK;
 }
 
 // BF16 hi/lo copy of one spin's MO vectors transposed to rows Q (RQ rows),
@@ -1268,7 +1196,7 @@ int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* amp, int64_t a_rbs, const ui
     g.rows = rows;
     g.RS = (int)RS;  g.v = (int)v;  g.vp = (int)vp;  g.Mp = (int)ctx->Mp;  g.i0 = i0;
     g.gamma = gamma;
-    g.err = ctx->flag.as<int>() + 2;
+    g.err = ctx->status.as<CallStatus>()->gamma_err;
     g.accumulate = accumulate;
     const size_t gsm = gamma_tc::SMEM_BYTES;
     CD_CUDA(cudaFuncSetAttribute(gamma_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm));
@@ -1323,12 +1251,11 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
     SpinState& Y = ctx->spin[sy];
     const BwdDims dx = bwd_dims(ctx, sx), dy = bwd_dims(ctx, sy);
     const int64_t Mp = ctx->Mp;
-    size_t free_b = 0, total_b = 0;
-    CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
     // the staging this pass reuses counts as available, so that the block size
     // of a repeated call does not shrink because the previous call holds it
-    const size_t held = ctx->amp.bytes + ctx->ampT.bytes + ctx->W.bytes;
-    const size_t budget = std::min<size_t>((free_b + held) / 3, size_t(40) << 30);
+    size_t budget = 0;
+    CD_RC(staging_budget(ctx, ctx->amp.bytes + ctx->ampT.bytes + ctx->W.bytes,
+                         (double)(dx.o * dx.VR) * (double)dy.o * (4.0 * dy.VS + 8.0 * dy.VR), &budget));
     // block sizes: rows bI, columns bJ (all of them for the opposite spin)
     int64_t bI, bJ;
     tc_block_sizes(ctx, dx.o, dy.o, dx.VR, dy.VR, dy.VS, kSym, budget, &bI, &bJ);
@@ -1372,7 +1299,7 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
             a.cb0 = (int)(a.c0 / 256);  a.ncb = (int)cdiv(a.c1, 256) - a.cb0;
             a.group = 12;
             a.S = ctx->W.as<float>();
-            a.err = ctx->flag.as<int>();
+            a.err = ctx->status.as<CallStatus>()->tile_err;
             a.tri = tri ? 1 : 0;
             const int64_t vunits = (int64_t)a.nrb * a.ncb;
             const int vgrid = (int)std::min<int64_t>(vunits, ctx->num_sms);
@@ -1459,10 +1386,9 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
     SpinState& Y = ctx->spin[sy];
     const BwdDims dx = bwd_dims(ctx, sx), dy = bwd_dims(ctx, sy);
     const int64_t Mp = ctx->Mp;
-    size_t free_b = 0, total_b = 0;
-    CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const size_t held = ctx->amp.bytes + ctx->W.bytes;
-    const size_t budget = std::min<size_t>((free_b + held) / 3, size_t(40) << 30);
+    size_t budget = 0;
+    CD_RC(staging_budget(ctx, ctx->amp.bytes + ctx->W.bytes,
+                         2.0 * sizeof(double) * (double)(dx.o * dx.vp) * (double)(dy.o * dy.vp), &budget));
     int64_t bI, bJ;
     f64_block_sizes(ctx, dx.o, dy.o, dx.vp, dy.vp, kSym, budget, &bI, &bJ);
     const size_t n_stage = sizeof(double) * (size_t)(bI * dx.vp) * (size_t)(bJ * dy.vp);
@@ -1474,7 +1400,6 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
     double* prow = ctx->dsum.as<double>();
     double* pcol = prow + npairs * dx.vp;
     double* pocc = pcol + npairs * dy.vp;
-    CD_ALLOC(ctx->oz_flag, sizeof(int) * 2, true);
     double* S = ctx->W.as<double>();
     double* A = ctx->amp.as<double>();
     for (int64_t I0 = 0; I0 < dx.o; I0 += bI) {
@@ -1570,70 +1495,46 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
         }
     }
     CD_RC(reduce_deps(ctx, prow, pcol, pocc, dx.o, dy.o, dx.vp, dy.vp, dx.v, dy.v, deps_x, deps_y));
-    return oz_check(ctx, "int8 tensor-core FP64 backward");
-}
-
-// Restricted FP64 gradient: one FP64 block-pair pass, then the transposed
-// half transforms with dE/dB = 4 Gamma.
-int gradient_restricted_f64(mshqc_cd_ctx* ctx, double* dC, double* deps, double* energy) {
-    SpinState& s = ctx->spin[0];
-    const int64_t N = ctx->N, Mp = ctx->Mp, o = s.nocc;
-    CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, o) * s.vp * Mp, true);
-    CD_CUDA(cudaMemsetAsync(deps, 0, sizeof(double) * N, ctx->stream));
-    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
-    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(o * o), false);
-    CD_RC(f64_backward_pass<AMP_RESTRICTED>(ctx, 0, 0, deps, deps, ctx->partial.as<double>()));
-    reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(ctx->partial.as<double>(), (int)(o * o), ctx->totals.as<double>());
-    CD_CUDA(cudaGetLastError());
-    ctx->launches++;
-    CD_CUDA(cudaMemcpyAsync(energy, ctx->totals.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    begin_stage(ctx, ST_TRANSPOSED);
-    const int spins[1] = {0};
-    CD_RC(transposed_dispatch(ctx, 1, spins, 4.0, &dC, MSHQC_CD_FP64));
-    end_stage(ctx);
     return MSHQC_CD_OK;
 }
 
-// Restricted mixed-precision gradient: one tensor-core pass, then the FP64
-// transposed transforms with dE/dB = 4 Gamma.
-int gradient_restricted_tc(mshqc_cd_ctx* ctx, double* dC, double* deps, double* energy) {
-    SpinState& s = ctx->spin[0];
-    const BwdDims d = bwd_dims(ctx, 0);
-    const int64_t N = ctx->N, Mp = ctx->Mp, RQ = round_up(ctx->M, 256);
-    const uint16_t* bt = nullptr;
-    CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bt));
-    CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, d.o) * s.vp * Mp, true);
-    CD_CUDA(cudaMemsetAsync(deps, 0, sizeof(double) * N, ctx->stream));
-    CD_ALLOC(ctx->flag, sizeof(int) * 4, true);
-    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
-    const int64_t tiles = d.o * d.o;   // one energy per pair (i, j)
-    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)tiles, false);
-    CD_RC(tc_backward_pass<AMP_RESTRICTED>(ctx, 0, 0, bt, bt, RQ, deps, deps, ctx->partial.as<double>()));
-    reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(ctx->partial.as<double>(), (int)tiles, ctx->totals.as<double>());
+// The gradients below only queue work: energies and error flags come back with
+// the call's status.  One total per pass from its per-pair energies:
+int queue_total(mshqc_cd_ctx* ctx, const double* pairs, int64_t n, int k) {
+    reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(pairs, (int)n, ctx->status.as<CallStatus>()->totals + k);
     CD_CUDA(cudaGetLastError());
     ctx->launches++;
-    int herr[4] = {0, 0, 0, 0};
-    CD_CUDA(cudaMemcpyAsync(herr, ctx->flag.p, sizeof(herr), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaMemcpyAsync(energy, ctx->totals.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (herr[0] || herr[2])
-        return set_error(MSHQC_CD_ERR_TIMEOUT, "tensor-core backward gave up waiting (site " +
-                                                   std::to_string(herr[0] ? herr[0] : herr[2]) + ")");
-    if (herr[1]) ctx->fixed_point_exact = 0;
+    return MSHQC_CD_OK;
+}
+
+// Restricted gradient: one pass over block pairs (FP64 or tensor cores), then
+// the transposed half transforms with dE/dB = 4 Gamma.
+int gradient_restricted(mshqc_cd_ctx* ctx, int precision, double* dC, double* deps) {
+    SpinState& s = ctx->spin[0];
+    const int64_t N = ctx->N, Mp = ctx->Mp, RQ = round_up(ctx->M, 256), o = s.nocc;
+    const bool tc = precision == MSHQC_CD_FP16X3;
+    const uint16_t* bt = nullptr;
+    if (tc) CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bt));
+    CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, o) * s.vp * Mp, true);
+    CD_CUDA(cudaMemsetAsync(deps, 0, sizeof(double) * N, ctx->stream));
+    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(o * o), false);   // one energy per pair (i, j)
+    double* part = ctx->partial.as<double>();
+    if (tc)
+        CD_RC(tc_backward_pass<AMP_RESTRICTED>(ctx, 0, 0, bt, bt, RQ, deps, deps, part));
+    else
+        CD_RC(f64_backward_pass<AMP_RESTRICTED>(ctx, 0, 0, deps, deps, part));
+    CD_RC(queue_total(ctx, part, o * o, 0));
     begin_stage(ctx, ST_TRANSPOSED);
     const int spins[1] = {0};
-    CD_RC(transposed_dispatch(ctx, 1, spins, 4.0, &dC, MSHQC_CD_FP16X3));
+    CD_RC(transposed_dispatch(ctx, 1, spins, 4.0, &dC, precision));
     end_stage(ctx);
     return MSHQC_CD_OK;
 }
 
 // Unrestricted gradient (CD-UMP2 energy, the OMP2 step): same-spin passes for
 // alpha and beta and one opposite-spin pass, Gamma accumulated per spin, then
-// the transposed transforms of each spin with dE/dB = 2 Gamma.  e3 receives
-// ss_aa, ss_bb, os.
-int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2], double* const deps[2],
-                          double* e3) {
+// the transposed transforms with dE/dB = 2 Gamma.  Totals: ss_aa, ss_bb, os.
+int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2], double* const deps[2]) {
     const BwdDims da = bwd_dims(ctx, 0), db = bwd_dims(ctx, 1);
     const int64_t N = ctx->N, Mp = ctx->Mp, RQ = round_up(ctx->M, 256);
     const bool tc = precision == MSHQC_CD_FP16X3;
@@ -1645,8 +1546,6 @@ int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2],
     CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, da.o) * da.vp * Mp, true);
     CD_ALLOC(ctx->gam[1], sizeof(double) * (size_t)b_rows(ctx, db.o) * db.vp * Mp, true);
     for (int s = 0; s < 2; ++s) CD_CUDA(cudaMemsetAsync(deps[s], 0, sizeof(double) * N, ctx->stream));
-    CD_ALLOC(ctx->flag, sizeof(int) * 4, true);
-    CD_ALLOC(ctx->totals, sizeof(double) * 8, false);
     const int64_t n0 = da.o * da.o, n1 = db.o * db.o, n2 = da.o * db.o;   // one energy per pair
     CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(n0 + n1 + n2), false);
     double* part = ctx->partial.as<double>();
@@ -1659,20 +1558,9 @@ int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2],
         CD_RC(f64_backward_pass<AMP_SAME_SPIN>(ctx, 1, 1, deps[1], deps[1], part + n0));
         CD_RC(f64_backward_pass<AMP_OPPOSITE_SPIN>(ctx, 0, 1, deps[0], deps[1], part + n0 + n1));
     }
-    const int64_t offs[3] = {0, n0, n0 + n1}, cnt[3] = {n0, n1, n2};
-    for (int k = 0; k < 3; ++k) {
-        reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(part + offs[k], (int)cnt[k], ctx->totals.as<double>() + k);
-        CD_CUDA(cudaGetLastError());
-        ctx->launches++;
-    }
-    int herr[4] = {0, 0, 0, 0};
-    CD_CUDA(cudaMemcpyAsync(herr, ctx->flag.p, sizeof(herr), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaMemcpyAsync(e3, ctx->totals.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (herr[0] || herr[2])
-        return set_error(MSHQC_CD_ERR_TIMEOUT, "tensor-core backward gave up waiting (site " +
-                                                   std::to_string(herr[0] ? herr[0] : herr[2]) + ")");
-    if (herr[1]) ctx->fixed_point_exact = 0;
+    CD_RC(queue_total(ctx, part, n0, 0));
+    CD_RC(queue_total(ctx, part + n0, n1, 1));
+    CD_RC(queue_total(ctx, part + n0 + n1, n2, 2));
     begin_stage(ctx, ST_TRANSPOSED);
     const int spins[2] = {0, 1};
     CD_RC(transposed_dispatch(ctx, 2, spins, 2.0, dC, precision));
@@ -1767,6 +1655,7 @@ int run_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* e_
     } part_scope(ctx);
     cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1], e2 = ctx->ev[2];
     reset_stages(ctx);
+    CD_RC(begin_call(ctx));
     CD_CUDA(cudaEventRecord(e0, ctx->stream));
     if (unres)
         CD_RC(ensure_transforms(ctx, precision));
@@ -1781,30 +1670,30 @@ int run_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* e_
         dC[s] = ctx->grad[s].as<double>();
         de[s] = dC[s] + N * N;
     }
-    double e3[3] = {0.0, 0.0, 0.0};
-    double energy = 0.0;
     ctx->fixed_point_exact = 1;
-    if (unres) {
-        CD_RC(gradient_unrestricted(ctx, precision, dC, de, e3));
-        energy = e3[0] + e3[1] + e3[2];
-    } else if (precision == MSHQC_CD_FP64) {
-        CD_RC(gradient_restricted_f64(ctx, dC[0], de[0], &energy));
-    } else {
-        CD_RC(gradient_restricted_tc(ctx, dC[0], de[0], &energy));
-    }
+    CD_RC(unres ? gradient_unrestricted(ctx, precision, dC, de) : gradient_restricted(ctx, precision, dC[0], de[0]));
     if (ctx->part_active && ctx->part_next != (int64_t)ctx->part_owned.size())
         return set_error(MSHQC_CD_ERR_STATE, "partition plan covers " + std::to_string(ctx->part_owned.size()) +
                                                  " units, the backward visited " + std::to_string(ctx->part_next));
     CD_CUDA(cudaEventRecord(e2, ctx->stream));
-    CD_CUDA(cudaEventSynchronize(e2));
+    const cudaMemcpyKind dir = where == MSHQC_CD_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    double* out_c[2] = {dC_a, dC_b};
+    double* out_e[2] = {deps_a, deps_b};
+    for (int s = 0; s < (unres ? 2 : 1); ++s) {
+        if (out_c[s]) CD_CUDA(cudaMemcpyAsync(out_c[s], dC[s], sizeof(double) * N * N, dir, ctx->stream));
+        if (out_e[s]) CD_CUDA(cudaMemcpyAsync(out_e[s], de[s], sizeof(double) * N, dir, ctx->stream));
+    }
+    CallStatus st;
+    CD_RC(finish_call(ctx, &st));
     collect_stages(ctx);
+    if (st.tile_err[1]) ctx->fixed_point_exact = 0;
     if (e_out) {
         std::memset(e_out, 0, sizeof(*e_out));
-        e_out->total = energy;
+        e_out->total = unres ? st.totals[0] + st.totals[1] + st.totals[2] : st.totals[0];
         if (unres) {
-            e_out->ss_aa = e3[0];
-            e_out->ss_bb = e3[1];
-            e_out->os = e3[2];
+            e_out->ss_aa = st.totals[0];
+            e_out->ss_bb = st.totals[1];
+            e_out->os = st.totals[2];
         }
         float t01 = 0, t12 = 0;
         CD_CUDA(cudaEventElapsedTime(&t01, e0, e1));
@@ -1812,12 +1701,6 @@ int run_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* e_
         e_out->ms_transform = t01;
         e_out->ms_energy = t12;
         e_out->ms_total = t01 + t12;
-    }
-    CD_RC(download(ctx, dC_a, dC[0], sizeof(double) * N * N, where));
-    CD_RC(download(ctx, deps_a, de[0], sizeof(double) * N, where));
-    if (unres) {
-        CD_RC(download(ctx, dC_b, dC[1], sizeof(double) * N * N, where));
-        CD_RC(download(ctx, deps_b, de[1], sizeof(double) * N, where));
     }
     return MSHQC_CD_OK;
 }

@@ -169,11 +169,10 @@ extern "C" MSHQC_CD_API int mshqc_cd_rmp2_energy_noalloc(const double* B, const 
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "pair kernel launch");
     // deterministic reductions straight into the caller's two doubles
-    reduce_pairs_kernel<<<(unsigned)cdiv(npairs, 128), 128, 0, st>>>(partial, (int)npairs, (int)nblocks, pair_sum);
-    reduce_pairs_kernel<<<(unsigned)cdiv(npairs, 128), 128, 0, st>>>(partial2, (int)npairs, (int)nblocks,
-                                                                     pair_sum + npairs);
-    reduce_total_kernel<<<1, 256, 0, st>>>(pair_sum, (int)npairs, energy);
-    reduce_total_kernel<<<1, 256, 0, st>>>(pair_sum + npairs, (int)npairs, energy + 1);
+    // (partial2 follows partial, the opposite-spin sums the total ones)
+    reduce_pairs_kernel<<<dim3((unsigned)cdiv(npairs, 128), 2), 128, 0, st>>>(partial, (int)npairs, (int)nblocks,
+                                                                              pair_sum);
+    reduce_total_kernel<<<2, 256, 0, st>>>(pair_sum, (int)npairs, energy);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "reduction launch");
     return MSHQC_CD_OK;

@@ -259,6 +259,7 @@ int occupied_density(mshqc_cd_ctx* ctx, const double* C, int64_t o, double* P) {
 // *e_mp2 receives the OMP2 energy (same-spin + opposite-spin).
 int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffers& b, double* e_mp2) {
     const int64_t N = ctx->N, M = ctx->M, NN = N * N;
+    CD_RC(begin_call(ctx));
     CD_RC(ensure_transforms(ctx, MSHQC_CD_FP64));
     CD_RC(omp2_buffers(ctx, b));
     const int64_t o0 = ctx->spin[0].nocc, o1 = ctx->spin[1].nocc;
@@ -266,7 +267,6 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     // OPDM blocks start at zero
     CD_CUDA(cudaMemsetAsync(b.Goo[0], 0, sizeof(double) * (size_t)(round_up(o0 * o0 + o1 * o1, 2) + vp0 * vp0 + vp1 * vp1),
                             ctx->stream));
-    CD_ALLOC(ctx->totals, sizeof(double) * 16, false);
     const int64_t n0 = o0 * o0, n1 = o1 * o1, n2 = o0 * o1;   // one energy per pair
     CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(n0 + n1 + n2), false);
     double* part = ctx->partial.as<double>();
@@ -280,12 +280,11 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     end_stage(ctx);
     const int64_t offs[3] = {0, n0, n0 + n1}, cnt[3] = {n0, n1, n2};
     for (int k = 0; k < 3; ++k) {
-        reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(part + offs[k], (int)cnt[k], ctx->totals.as<double>() + k);
+        reduce_total_kernel<<<1, 256, 0, ctx->stream>>>(part + offs[k], (int)cnt[k],
+                                                        ctx->status.as<CallStatus>()->totals + k);
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
     }
-    double e3[3] = {0.0, 0.0, 0.0};
-    CD_CUDA(cudaMemcpyAsync(e3, ctx->totals.p, sizeof(e3), cudaMemcpyDeviceToHost, ctx->stream));
 
     begin_stage(ctx, ST_OTHER);
     // P_s = Pref_s + C_s blockdiag(Goo_s, Gvv_s) C_s^T
@@ -352,8 +351,9 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
         ctx->launches += 2;
     }
     end_stage(ctx);
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    *e_mp2 = e3[0] + e3[1] + e3[2];
+    CallStatus st;
+    CD_RC(finish_call(ctx, &st));
+    *e_mp2 = st.totals[0] + st.totals[1] + st.totals[2];
     return MSHQC_CD_OK;
 }
 

@@ -52,6 +52,7 @@ extern "C" MSHQC_CD_API int mshqc_cd_get_t2_block(mshqc_cd_ctx* ctx, int block, 
     const int64_t ox = ctx->spin[sx].nocc, oy = ctx->spin[sy].nocc;
     if (i0 < 0 || ni < 1 || i0 + ni > ox || j0 < 0 || nj < 1 || j0 + nj > oy)
         return set_error(MSHQC_CD_ERR_ARG, "pair block outside the occupied orbitals");
+    CD_RC(begin_call(ctx));
     if (sy != sx)
         CD_RC(ensure_transforms(ctx, MSHQC_CD_FP64));
     else
@@ -84,6 +85,5 @@ extern "C" MSHQC_CD_API int mshqc_cd_get_t2_block(mshqc_cd_ctx* ctx, int block, 
     ctx->launches++;
     if (where != MSHQC_CD_DEVICE)
         CD_CUDA(cudaMemcpyAsync(out, dst, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CD_CUDA(cudaStreamSynchronize(ctx->stream));
-    return MSHQC_CD_OK;
+    return finish_call(ctx);
 }

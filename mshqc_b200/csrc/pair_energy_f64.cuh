@@ -38,12 +38,46 @@ struct PairF64Args {
     int Mp;            // padded Q extent (multiple of 16; padding is zero)
     const double* eox; const double* evx;   // occupied / virtual energies of X
     const double* eoy; const double* evy;
-    const int2* pairs;  // (i, j) per pair
-    const int2* blocks; // (row block, column block) per unit of a pair, 64-blocks
+    const int2* pairs;  // (i, j) per pair, or null: pair_at
+    const int2* blocks; // (row block, column block) per unit of a pair, 64-blocks, or null: block_at
+    int ox, oy, nbx, nby;   // occupied orbitals and blocks (without tables)
     int nblocks;
     double* partial;    // [npairs * nblocks]
     double* partial2;   // RESTRICTED: opposite-spin part per unit
 };
+
+// Entry p of the rows of n, n - 1, ... 1 entries of an upper triangle: (row,
+// column - row).
+__device__ __forceinline__ int2 triangle_at(int p, int n) {
+    const double h = n + 0.5;
+    int r = (int)(h - sqrt(fmax(0.0, h * h - 2.0 * p)));
+    while (r > 0 && (long long)r * n - (long long)r * (r - 1) / 2 > p) --r;
+    while ((long long)(r + 1) * n - (long long)(r + 1) * r / 2 <= p) ++r;
+    return make_int2(r, p - (int)((long long)r * n - (long long)r * (r - 1) / 2));
+}
+// pair p of a mode: i <= j, i < j, or all (i, j)
+template <int MODE>
+__device__ __forceinline__ int2 pair_at(int p, int ox, int oy) {
+    if (MODE == PAIR_OPPOSITE_SPIN) return make_int2(p / oy, p % oy);
+    const int2 t = triangle_at(p, MODE == PAIR_RESTRICTED ? ox : ox - 1);
+    return make_int2(t.x, t.x + t.y + (MODE == PAIR_RESTRICTED ? 0 : 1));
+}
+// virtual block pair b of a mode: x <= y, or row blocks x column blocks in steps of two
+template <int MODE>
+__device__ __forceinline__ int2 block_at(int b, int nbx, int nby) {
+    if (MODE == PAIR_OPPOSITE_SPIN) {
+        const int h = (nby + 1) / 2;
+        return make_int2(b / h, 2 * (b % h));
+    }
+    const int2 t = triangle_at(b, nbx);
+    return make_int2(t.x, t.x + t.y);
+}
+inline long long pair_count(int mode, long long ox, long long oy) {
+    return mode == PAIR_OPPOSITE_SPIN ? ox * oy : mode == PAIR_RESTRICTED ? ox * (ox + 1) / 2 : ox * (ox - 1) / 2;
+}
+inline long long block_count(int mode, long long nbx, long long nby) {
+    return mode == PAIR_OPPOSITE_SPIN ? nbx * ((nby + 1) / 2) : nbx * (nbx + 1) / 2;
+}
 
 namespace pair_f64_detail {
 constexpr int BT = 64;          // tile edge
@@ -64,8 +98,8 @@ __global__ void __launch_bounds__(256, 2) pair_energy_f64_kernel(PairF64Args p) 
     const int64_t unit = blockIdx.x;
     const int pidx = (int)(unit / p.nblocks);
     const int bidx = (int)(unit % p.nblocks);
-    const int2 ij = p.pairs[pidx];
-    const int2 ab = p.blocks[bidx];
+    const int2 ij = p.pairs ? p.pairs[pidx] : pair_at<MODE>(pidx, p.ox, p.oy);
+    const int2 ab = p.blocks ? p.blocks[bidx] : block_at<MODE>(bidx, p.nbx, p.nby);
     const int i = ij.x, j = ij.y;
     const int a0 = ab.x * BT, b0 = ab.y * BT;
     const int64_t Mp = p.Mp;
@@ -243,24 +277,27 @@ __global__ void __launch_bounds__(256, 2) pair_energy_f64_kernel(PairF64Args p) 
 }
 
 // Deterministic compensated reduction of unit partials into per-pair sums
-// (one thread per pair, units in order) ...
+// (one thread per pair, units in order); blockIdx.y: planes of npairs * nblocks
+// partials and npairs sums ...
 static __global__ void reduce_pairs_kernel(const double* __restrict__ partial, int npairs, int nblocks,
                                     double* __restrict__ pair_sum) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npairs) return;
     KSum s;
     s.init();
-    const double* src = partial + (int64_t)p * nblocks;
+    const double* src = partial + ((int64_t)blockIdx.y * npairs + p) * nblocks;
     for (int b = 0; b < nblocks; ++b) s.add(src[b]);
-    pair_sum[p] = s.value();
+    pair_sum[(int64_t)blockIdx.y * npairs + p] = s.value();
 }
 
-// ... and of per-pair sums into one total (single CTA of 256 threads, fixed
-// order: strided per-thread sums, a tree in each warp, the 8 warps in order).
+// ... and of per-pair sums into one total per plane (blockIdx.x: x + plane * n
+// into out[plane]; one CTA of 256 threads, fixed order: strided per-thread sums,
+// a tree in each warp, the 8 warps in order).
 static __global__ void reduce_total_kernel(const double* __restrict__ x, int n, double* __restrict__ out) {
     __shared__ double ss[8], sc[8];
     KSum s;
     s.init();
+    x += (int64_t)blockIdx.x * n;
     for (int k = threadIdx.x; k < n; k += 256) s.add(x[k]);
     warp_reduce_ksum(s);
     if ((threadIdx.x & 31) == 0) {
@@ -275,7 +312,7 @@ static __global__ void reduce_total_kernel(const double* __restrict__ x, int n, 
             t.add(ss[k]);
             t.c += sc[k];
         }
-        *out = t.value();
+        out[blockIdx.x] = t.value();
     }
 }
 

@@ -57,8 +57,7 @@ struct PairTcArgs {
     int diag_o, diag_v;     // extent of the opposite-spin diagonal table
     const double* eox; const double* evx;
     const double* eoy; const double* evy;
-    const int2* pairs;      // (i, j)
-    const int2* blocks;     // (x, y) in 128-blocks
+    int ox, oy, nbx, nby;   // occupied orbitals, 128-blocks of virtuals (pair_at, block_at)
     int nblocks;
     long long units;        // npairs * nblocks
     double* partial;        // [units]
@@ -142,8 +141,8 @@ __global__ void __launch_bounds__(pair_tc::THREADS, 1) pair_energy_tc_kernel(Pai
             uint32_t fill_phase = 0, filled = 0;   // bit s: parity / presence of stage s's last fill
 #pragma unroll
             for (long long u = first; u < p.units && !*abort_flag; u += step) {
-                const int2 ij = p.pairs[u / p.nblocks];
-                const int2 xy = p.blocks[u % p.nblocks];
+                const int2 ij = pair_at<MODE>((int)(u / p.nblocks), p.ox, p.oy);
+                const int2 xy = block_at<MODE>((int)(u % p.nblocks), p.nbx, p.nby);
                 const size_t a0 = (size_t)xy.x * BM, b0 = (size_t)xy.y * BN;
                 // operand bases at Q chunk 0 (the 128 rows from r0 of orbital
                 // o); chunk kq adds kq * 4096 elements (hi and lo)
@@ -258,8 +257,8 @@ __global__ void __launch_bounds__(pair_tc::THREADS, 1) pair_energy_tc_kernel(Pai
         const int etid = threadIdx.x - 64;
         uint32_t acc_phase = 0;
         for (long long u = first; u < p.units; u += step) {
-            const int2 ij = p.pairs[u / p.nblocks];
-            const int2 xy = p.blocks[u % p.nblocks];
+            const int2 ij = pair_at<MODE>((int)(u / p.nblocks), p.ox, p.oy);
+            const int2 xy = block_at<MODE>((int)(u % p.nblocks), p.nbx, p.nby);
             const int i = ij.x, j = ij.y;
             const int a = xy.x * BM + row;
             const int b0 = xy.y * BN;
