@@ -21,12 +21,24 @@
 // transposed operand [(j, b)][(i - i0, a)]: Gamma_beta of the opposite-spin
 // pass, or, for the symmetric modes (t^{ji}_{ba} = t^{ij}_{ab}), the rows j of
 // a block pair (I, J) whose mirror (J, I) is not computed.
-// One CTA of 256 threads takes one pair (i, j) and walks its 32 x 32 tiles of
-// (a, b), row block outer, loading the next tile while it works on the
-// current one; the pair's energy, its row sums
-// sum_b r (per a), column sums sum_a r (per b) and total sum r go to per-pair
-// buffers, each written by one thread, and deps_*_kernel turn them into
-// dE/de (+r on a and b, -r on i and j) in a fixed order.
+// Symmetric modes (amp_sym_kernel): the tiles (A, B) and (B, A) of a pair go
+// together, so an integral is read once (it is V of one element and W of the
+// other), and the two elements share D and 1/D.  Row and column sums land in the
+// same place (dE/de of one spin), so one vector per pair holds both.
+// Opposite spin (amp_os_kernel): one tile at a time, row sums per a and column
+// sums per b.  A CTA of 256 threads takes a pair, or a share of its tiles, and
+// loads the next tile while it works on the current one; per-pair sums are
+// written by one thread each, and deps_*_kernel turn them into dE/de (+r on a
+// and b, -r on i and j) in a fixed order.
+// Bound by HBM traffic and, next to it, by FP64 arithmetic and conversions: the
+// mixed path reads 4 bytes of S and writes 4 of hi/lo per amplitude and operand.
+// An amplitude is split into hi and lo once, in registers, and the operands'
+// 16-byte rows are gathered from the packed words; with mirrored tiles apart
+// (every integral read twice, every 1/D taken twice) and one split per operand
+// the pass took 32.3 ms of the N = 1000, o = 100 restricted mixed backward and
+// 12.9 ms of the N = 600 unrestricted one, now 20.0 and 9.6 (4.1 TB/s at
+// N = 1000); FP64, N = 600, o = 60: 4.8 -> 3.7 ms.  5 CTAs per SM (mixed)
+// measured best of 3, 4, 5, 6 (20.7, 21.3, 19.9, 21.9 ms).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -56,8 +68,9 @@ struct AmpElemArgs {
     uint16_t* T16; long long nkT;   // SPLIT, optional transpose: rows jj*csy + b, K = ii*ksx + a
     double* A64; long long ldA;                   // FP64: [R][K], K = jj*ksy + b
     double* partial;        // [ox * oy] energy of each pair (i, j), i over all row orbitals
-    double* prow;           // [ox * oy][rsx] sum_b r per pair and row a (or null)
-    double* pcol;           // [ox * oy][csy] sum_a r per pair and column b (or null)
+    double* prow;           // opposite spin: [ox * oy][rsx] sum_b r per pair and row a (or null)
+    double* pcol;           // [ox * oy][csy] sum_a r per pair and column b; symmetric modes: row and
+                            // column sums of a pair together (or null)
     double* pocc;           // [ox * oy] sum_ab r per pair (or null)
     // nchunk > 1: each pair's row tiles are split over nchunk CTAs (CTA
     // lp * nchunk + c takes chunk c of local pair lp = ii * nbj + jj); their
@@ -101,42 +114,47 @@ __device__ __forceinline__ long long blocked_offset(long long R, long long k, lo
            (k & 7);
 }
 
-// eight consecutive-k values -> one 16-byte hi row and one 16-byte lo row
-__device__ __forceinline__ void store_hilo8(const double* t, uint16_t* hi, uint16_t* lo) {
-    uint32_t wh[4], wl[4];
+// amplitude -> BF16 hi (low half word) and lo (high half word)
+__device__ __forceinline__ uint32_t split_amp(double t) {
+    const __nv_bfloat16 h = __double2bfloat16(t);
+    const __nv_bfloat16 l = __double2bfloat16(t - (double)__bfloat162float(h));
+    return (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
+}
+
+// 32 x 32 amplitude tile T (rows R0.., columns k0..; transposed: the tile's
+// transpose) -> hi/lo operand: job = 0 .. 127 writes 8 consecutive k of one row,
+// 16 bytes of hi and 16 of lo; a warp fills four 128-byte lines of each
+__device__ __forceinline__ void store_tile(const uint32_t (*T)[33], bool transposed, int job, long long R0,
+                                           long long k0, long long nk, uint16_t* dst) {
+    const int r = job >> 2, g = job & 3;
+    const uint32_t* t = transposed ? &T[g * 8][r] : &T[r][g * 8];
+    const int step = transposed ? 33 : 1;
+    uint32_t w[8];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const __nv_bfloat16 h0 = __double2bfloat16(t[2 * e]), h1 = __double2bfloat16(t[2 * e + 1]);
-        const __nv_bfloat16 l0 = __double2bfloat16(t[2 * e] - (double)__bfloat162float(h0));
-        const __nv_bfloat16 l1 = __double2bfloat16(t[2 * e + 1] - (double)__bfloat162float(h1));
-        wh[e] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-        wl[e] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-    }
-    *reinterpret_cast<uint4*>(hi) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-    *reinterpret_cast<uint4*>(lo) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+    for (int e = 0; e < 8; ++e) w[e] = t[e * step];
+    uint16_t* d = dst + blocked_offset(R0 + r, k0 + g * 8, nk);
+    *reinterpret_cast<uint4*>(d) = make_uint4(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410),
+                                              __byte_perm(w[4], w[5], 0x5410), __byte_perm(w[6], w[7], 0x5410));
+    *reinterpret_cast<uint4*>(d + 2048) =
+        make_uint4(__byte_perm(w[0], w[1], 0x7632), __byte_perm(w[2], w[3], 0x7632),
+                   __byte_perm(w[4], w[5], 0x7632), __byte_perm(w[6], w[7], 0x7632));
 }
 }  // namespace amp_detail
 
-template <int MODE, bool SPLIT>
-__global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
+template <bool SPLIT>
+__global__ void __launch_bounds__(256, SPLIT ? 5 : 4) amp_os_kernel(AmpElemArgs p) {
     using TS = typename std::conditional<SPLIT, float, double>::type;
-    constexpr bool kW = MODE != AMP_OPPOSITE_SPIN;   // (ib|ja) needed
     __shared__ TS Vt[32][33];
-    __shared__ TS Wt[kW ? 32 : 1][33];
-    __shared__ double T[32][33];
+    __shared__ uint32_t T[SPLIT ? 32 : 1][33];   // amplitudes as BF16 hi and lo
     __shared__ double colpart[8][33];
     __shared__ double red_e[8], red_r[8];
     const TS* S = static_cast<const TS*>(p.S);
     const int ta = p.rsx / 32, tb = p.csy / 32;
     const int R = p.nchunk > 1 ? p.nchunk : 1;
     const int lp = (int)(blockIdx.x / R), ch = (int)(blockIdx.x % R);
-    int ii, jj;
-    amp_detail::local_pair(p, lp, ii, jj);
-    const double wgt = p.tri ? (ii < jj ? 2.0 : 1.0) : p.wgt;
-    const bool write_t = p.T16 != nullptr && !(p.tri && ii == jj);
-    // FP64 operand of a diagonal block pair: the (j, i) amplitudes go into A64
-    // as the transposes of the (i, j) ones
-    const bool write_t64 = !SPLIT && p.tri && ii != jj;
+    const int ii = lp / p.nbj, jj = lp % p.nbj;
+    const double wgt = p.wgt;
+    const bool write_t = p.T16 != nullptr;
     const int xb0 = ch * ta / R, xb1 = (ch + 1) * ta / R;   // this CTA's row tiles
     const int i = p.i0 + ii, j = p.j0 + jj;
     const long long pair = (long long)i * p.oy + j;          // over all occupied rows
@@ -148,18 +166,16 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
                             : p.cpcol + ((long long)lp * R + ch) * p.csy;
     const TS* Srow = S + (long long)ii * p.rsx * p.ldS + (long long)jj * p.csy;
     // this thread's four elements of tile (a0, b0): rows ty + 8k, column tx
-    // (V); the transposed tile (b0, a0) for W
-    auto load_tile = [&](int a0, int b0, TS (&v)[4], TS (&w)[4]) {
+    auto load_tile = [&](int a0, int b0, TS (&v)[4]) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int r = ty + 8 * k;
             // streaming loads: the staging is read here and never again
             v[k] = __ldcs(Srow + (long long)(a0 + r) * p.ldS + b0 + tx);
-            if (kW) w[k] = __ldcs(Srow + (long long)(b0 + r) * p.ldS + a0 + tx);
         }
     };
-    TS vn[4], wn[4];
-    if (xb0 < xb1) load_tile(xb0 * 32, 0, vn, wn);
+    TS vn[4];
+    if (xb0 < xb1) load_tile(xb0 * 32, 0, vn);
     double esum = 0.0, rtot = 0.0;
     // row blocks outer, column blocks inner: a thread's rows stay fixed over
     // the inner loop, so their sums over b stay in registers; the column sums
@@ -172,13 +188,12 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 Vt[ty + 8 * k][tx] = vn[k];
-                if (kW) Wt[ty + 8 * k][tx] = wn[k];
             }
             // the next tile's loads overlap this tile's arithmetic and stores
             if (yb + 1 < tb)
-                load_tile(a0, b0 + 32, vn, wn);
+                load_tile(a0, b0 + 32, vn);
             else if (xb + 1 < xb1)
-                load_tile(a0 + 32, 0, vn, wn);
+                load_tile(a0 + 32, 0, vn);
             __syncthreads();
             double cp = 0.0;
 #pragma unroll
@@ -191,59 +206,28 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
                     if (fabs(D) >= kDenomSkip) {
                         const double V = (double)Vt[r][tx];
                         const double rD = SPLIT ? sm100::recip_nr(D) : 1.0 / D;
-                        if (MODE == AMP_RESTRICTED) {
-                            const double W = (double)Wt[tx][r];
-                            const double t = V * rD;
-                            amp = (2.0 * V - W) * rD;
-                            rr = t * amp;
-                            esum = fma(V, amp, esum);
-                        } else if (MODE == AMP_SAME_SPIN) {
-                            const double W = (double)Wt[tx][r];
-                            const double g = V - W;
-                            amp = g * rD;
-                            rr = 0.25 * amp * amp;
-                            esum = fma(0.25 * g, amp, esum);
-                        } else {
-                            amp = V * rD;
-                            rr = amp * amp;
-                            esum = fma(V, amp, esum);
-                        }
+                        amp = V * rD;
+                        rr = amp * amp;
+                        esum = fma(V, amp, esum);
                     }
                 }
-                T[r][tx] = amp;
                 rsum[k] += rr;
                 cp += rr;
-                if (!SPLIT) p.A64[((long long)ii * p.rsx + a) * p.ldA + (long long)jj * p.ksy + b] = amp;
+                if (SPLIT)
+                    T[r][tx] = amp_detail::split_amp(amp);
+                else
+                    p.A64[((long long)ii * p.rsx + a) * p.ldA + (long long)jj * p.ksy + b] = amp;
             }
             rtot += cp;
             colpart[ty][tx] = cp;
             __syncthreads();
             if (SPLIT) {
-                // 32 rows x 4 groups of 8 K = 128 core-matrix rows per operand
-                if (threadIdx.x < 128) {
-                    const int r = threadIdx.x >> 2, g = threadIdx.x & 3;
-                    const long long R = (long long)ii * p.rsx + a0 + r;
-                    const long long kc = (long long)jj * p.ksy + b0 + g * 8;
-                    const long long off = amp_detail::blocked_offset(R, kc, p.nkA);
-                    amp_detail::store_hilo8(&T[r][g * 8], p.A16 + off, p.A16 + off + 2048);
-                } else if (write_t) {
-                    const int w = threadIdx.x - 128;
-                    const int r = w >> 2, g = w & 3;   // r: b offset, g: group of 8 a
-                    const long long R = (long long)jj * p.csy + b0 + r;
-                    const long long kc = (long long)ii * p.ksx + a0 + g * 8;
-                    const long long off = amp_detail::blocked_offset(R, kc, p.nkT);
-                    double col[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) col[e] = T[g * 8 + e][r];
-                    amp_detail::store_hilo8(col, p.T16 + off, p.T16 + off + 2048);
-                }
-            }
-            if (write_t64) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int rb = ty + 8 * k;   // b offset: row (j, b) of the operand
-                    p.A64[((long long)jj * p.ksy + b0 + rb) * p.ldA + (long long)ii * p.rsx + a0 + tx] = T[tx][rb];
-                }
+                if (threadIdx.x < 128)
+                    amp_detail::store_tile(T, false, threadIdx.x, (long long)ii * p.rsx + a0,
+                                           (long long)jj * p.ksy + b0, p.nkA, p.A16);
+                else if (write_t)
+                    amp_detail::store_tile(T, true, threadIdx.x - 128, (long long)jj * p.csy + b0,
+                                           (long long)ii * p.ksx + a0, p.nkT, p.T16);
             }
             if (pcol && ty == 0) {
                 double c = 0.0;
@@ -251,7 +235,7 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
                 for (int w = 0; w < 8; ++w) c += colpart[w][tx];
                 pcol[b0 + tx] = (xb == xb0 ? 0.0 : pcol[b0 + tx]) + wgt * c;
             }
-            __syncthreads();   // Vt, Wt, T, colpart are refilled by the next tile
+            __syncthreads();   // Vt, T, colpart are refilled by the next tile
         }
         if (prow) {
 #pragma unroll
@@ -289,7 +273,202 @@ __global__ void __launch_bounds__(256, 4) amp_elem_kernel(AmpElemArgs p) {
     }
 }
 
-// The chunk partials of amp_elem_kernel (nchunk > 1) of the nbi x nbj local
+template <int MODE, bool SPLIT>
+__global__ void __launch_bounds__(256, SPLIT ? 5 : 3) amp_sym_kernel(AmpElemArgs p) {
+    static_assert(MODE != AMP_OPPOSITE_SPIN, "symmetric modes");
+    using TS = typename std::conditional<SPLIT, float, double>::type;
+    __shared__ TS Vs[32][33], Ws[32][33];
+    // amplitudes (a, b) and (b, a), with SPLIT as BF16 hi and lo: split once, however
+    // many operands take them
+    using TA = typename std::conditional<SPLIT, uint32_t, double>::type;
+    __shared__ TA T1[32][33], T2[32][33];
+    __shared__ double colpart[8][33];
+    __shared__ double rowbuf[32];
+    __shared__ double red_e[8], red_r[8];
+    const TS* S = static_cast<const TS*>(p.S);
+    const int nt = p.rsx / 32, ntp = nt * (nt + 1) / 2;   // tiles a side, tile pairs A <= B
+    const int R = p.nchunk > 1 ? p.nchunk : 1;
+    const int lp = (int)(blockIdx.x / R), ch = (int)(blockIdx.x % R);
+    int ii, jj;
+    amp_detail::local_pair(p, lp, ii, jj);
+    const double wgt = p.tri ? (ii < jj ? 2.0 : 1.0) : p.wgt;
+    const bool write_t = p.T16 != nullptr && !(p.tri && ii == jj);
+    // FP64 operand of a diagonal block pair: the (j, i) amplitudes go into A64
+    // as the transposes of the (i, j) ones
+    const bool write_t64 = !SPLIT && p.tri && ii != jj;
+    const int i = p.i0 + ii, j = p.j0 + jj;
+    const long long pair = (long long)i * p.oy + j;          // over all occupied rows
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
+    const double eij = p.eox[i] + p.eoy[j];
+    double* psum = !p.pcol ? nullptr
+                   : R == 1 ? p.pcol + pair * p.csy
+                            : p.cpcol + ((long long)lp * R + ch) * p.csy;
+    // lane tx of warp 0 alone touches the elements of psum that are tx mod 32
+    if (psum && ty == 0)
+        for (int b = tx; b < p.csy; b += 32) psum[b] = 0.0;
+    const TS* Srow = S + (long long)ii * p.rsx * p.ldS + (long long)jj * p.csy;
+    const int t0 = (int)((long long)ch * ntp / R), t1 = (int)((long long)(ch + 1) * ntp / R);
+    int A = 0, B = t0;
+    while (B >= nt - A) {
+        B -= nt - A;
+        ++A;
+    }
+    B += A;
+    TS vn[4], wn[4];
+    auto load = [&](int a0, int b0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = ty + 8 * k;
+            // streaming loads: the staging is read here and never again
+            vn[k] = __ldcs(Srow + (long long)(a0 + r) * p.ldS + b0 + tx);
+            if (a0 != b0) wn[k] = __ldcs(Srow + (long long)(b0 + r) * p.ldS + a0 + tx);
+        }
+    };
+    if (t0 < t1) load(A * 32, B * 32);
+    double esum = 0.0, rtot = 0.0;
+    double rsum[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int t = t0; t < t1; ++t) {
+        const int a0 = A * 32, b0 = B * 32;
+        const bool diag = a0 == b0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            Vs[ty + 8 * k][tx] = vn[k];
+            Ws[ty + 8 * k][tx] = diag ? vn[k] : wn[k];
+        }
+        const bool row_end = B + 1 == nt || t + 1 == t1;   // last tile of this row block here
+        if (++B == nt) {
+            ++A;
+            B = A;
+        }
+        // the next tile's loads overlap this tile's arithmetic and stores
+        if (t + 1 < t1) load(A * 32, B * 32);
+        __syncthreads();
+        double cp = 0.0;
+        const int b = b0 + tx;
+        const double eb = b < p.vy ? eij - p.evy[b] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = ty * 4 + k, a = a0 + r;
+            double amp1 = 0.0, amp2 = 0.0, rr = 0.0;
+            if (a < p.vx && b < p.vy) {
+                const double D = eb - p.evx[a];
+                if (fabs(D) >= kDenomSkip) {
+                    const double V = (double)Vs[r][tx], W = (double)Ws[tx][r];
+                    const double rD = SPLIT ? sm100::recip_nr(D) : 1.0 / D;
+                    if (MODE == AMP_RESTRICTED) {
+                        amp1 = (2.0 * V - W) * rD;
+                        rr = V * rD * amp1;
+                        esum = fma(V, amp1, esum);
+                        if (!diag) {
+                            amp2 = (2.0 * W - V) * rD;
+                            rr = fma(W * rD, amp2, rr);
+                            esum = fma(W, amp2, esum);
+                        }
+                    } else {
+                        const double g = V - W;
+                        amp1 = g * rD;
+                        rr = 0.25 * amp1 * amp1;
+                        double e = 0.25 * g * amp1;
+                        if (!diag) {
+                            amp2 = -amp1;
+                            rr += rr;
+                            e += e;
+                        }
+                        esum += e;
+                    }
+                }
+            }
+            rsum[k] += rr;
+            cp += rr;
+            if constexpr (SPLIT) {
+                T1[r][tx] = amp_detail::split_amp(amp1);
+                if (!diag) T2[tx][r] = amp_detail::split_amp(amp2);
+            } else {
+                T1[r][tx] = amp1;
+                if (!diag) T2[tx][r] = amp2;
+                p.A64[((long long)ii * p.rsx + a) * p.ldA + (long long)jj * p.ksy + b] = amp1;
+            }
+        }
+        rtot += cp;
+        if (psum) {
+            colpart[ty][tx] = cp;
+            if (row_end) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    double rs = rsum[k];
+#pragma unroll
+                    for (int off = 16; off; off >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, off);
+                    if (tx == 0) rowbuf[ty * 4 + k] = rs;
+                    rsum[k] = 0.0;
+                }
+            }
+        }
+        __syncthreads();
+        if constexpr (SPLIT) {
+            // up to four operand tiles of 128 jobs: A (a, b), T of it, and their mirrors
+            const int ntile = (diag ? 1 : 2) * (write_t ? 2 : 1);
+            for (int job = threadIdx.x; job < 128 * ntile; job += 256) {
+                const int which = job >> 7;
+                const bool second = diag ? false : (which & 1) != 0;      // the tile (b, a)
+                const bool trans = diag ? which == 1 : which >= 2;
+                const uint32_t(*T)[33] = second ? T2 : T1;
+                const int ra = second ? b0 : a0, rb = second ? a0 : b0;   // its row and column virtuals
+                if (!trans)
+                    amp_detail::store_tile(T, false, job & 127, (long long)ii * p.rsx + ra,
+                                           (long long)jj * p.ksy + rb, p.nkA, p.A16);
+                else
+                    amp_detail::store_tile(T, true, job & 127, (long long)jj * p.csy + rb,
+                                           (long long)ii * p.ksx + ra, p.nkT, p.T16);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = ty + 8 * k;
+                if (!diag)
+                    p.A64[((long long)ii * p.rsx + b0 + r) * p.ldA + (long long)jj * p.ksy + a0 + tx] = T2[r][tx];
+                if (write_t64) {   // rows (j, b) of the operand, columns (i, a), and the mirror
+                    p.A64[((long long)jj * p.ksy + b0 + r) * p.ldA + (long long)ii * p.rsx + a0 + tx] = T1[tx][r];
+                    if (!diag)
+                        p.A64[((long long)jj * p.ksy + a0 + r) * p.ldA + (long long)ii * p.rsx + b0 + tx] = T2[tx][r];
+                }
+            }
+        }
+        if (psum && ty == 0) {
+            double c = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) c += colpart[w][tx];
+            psum[b0 + tx] += wgt * c;
+            if (row_end) psum[a0 + tx] += wgt * rowbuf[tx];
+        }
+        __syncthreads();   // the shared tiles are refilled by the next tile pair
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) {
+        esum += __shfl_xor_sync(0xffffffffu, esum, off);
+        rtot += __shfl_xor_sync(0xffffffffu, rtot, off);
+    }
+    if (tx == 0) {
+        red_e[ty] = esum;
+        red_r[ty] = rtot;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double e = 0.0, r = 0.0;
+        for (int w = 0; w < 8; ++w) {
+            e += red_e[w];
+            r += red_r[w];
+        }
+        if (R == 1) {
+            p.partial[pair] = wgt * e;
+            if (p.pocc) p.pocc[pair] = wgt * r;
+        } else {
+            p.cpart[(long long)lp * R + ch] = wgt * e;
+            if (p.pocc) p.cpocc[(long long)lp * R + ch] = wgt * r;
+        }
+    }
+}
+
+// The chunk partials of the kernels above (nchunk > 1) of the nbi x nbj local
 // pairs added in chunk order into the per-pair outputs: one thread per
 // (local pair, column b); the b == 0 thread also does energy and total.
 static __global__ void amp_chunks_combine_kernel(AmpElemArgs p, int npl) {
@@ -314,6 +493,14 @@ static __global__ void amp_chunks_combine_kernel(AmpElemArgs p, int npl) {
         p.partial[pair] = e;
         if (p.pocc) p.pocc[pair] = r;
     }
+}
+
+template <int MODE, bool SPLIT>
+inline void launch_amp(const AmpElemArgs& e, int64_t ctas, cudaStream_t st) {
+    if constexpr (MODE == AMP_OPPOSITE_SPIN)
+        amp_os_kernel<SPLIT><<<(unsigned)ctas, 256, 0, st>>>(e);
+    else
+        amp_sym_kernel<MODE, SPLIT><<<(unsigned)ctas, 256, 0, st>>>(e);
 }
 
 // dE/de from the per-pair sums, in a fixed order (no atomics):

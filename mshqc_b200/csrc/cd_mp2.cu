@@ -1220,14 +1220,17 @@ int launch_gamma(mshqc_cd_ctx* ctx, const uint16_t* amp, int64_t a_rbs, const ui
 int reduce_deps(mshqc_cd_ctx* ctx, const double* prow, const double* pcol, const double* pocc, int64_t ox,
                 int64_t oy, int64_t rsx, int64_t csy, int64_t vx, int64_t vy, double* deps_x, double* deps_y) {
     const int64_t npairs = ox * oy;
-    deps_rows_kernel<<<(unsigned)cdiv(vx, 16), 1024, 0, ctx->stream>>>(prow, npairs, (int)rsx, (int)vx,
-                                                                       deps_x + ox);
+    if (prow) {   // (the symmetric modes keep row and column sums together)
+        deps_rows_kernel<<<(unsigned)cdiv(vx, 16), 1024, 0, ctx->stream>>>(prow, npairs, (int)rsx, (int)vx,
+                                                                           deps_x + ox);
+        ctx->launches++;
+    }
     deps_rows_kernel<<<(unsigned)cdiv(vy, 16), 1024, 0, ctx->stream>>>(pcol, npairs, (int)csy, (int)vy,
                                                                        deps_y + oy);
     deps_occ_kernel<<<(unsigned)cdiv(std::max(ox, oy), 128), 128, 0, ctx->stream>>>(pocc, (int)ox, (int)oy,
                                                                                     deps_x, deps_y);
     CD_CUDA(cudaGetLastError());
-    ctx->launches += 3;
+    ctx->launches += 2;
     return MSHQC_CD_OK;
 }
 
@@ -1265,11 +1268,13 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
     // (the size the block sizes are reckoned with; the packed rows take less of it)
     CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VS), false);
     const int64_t npairs = dx.o * dy.o;
-    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (dx.RS + dy.RS + 1)), true);
+    // (zero where a mirrored pair stands in)
+    const int64_t nrow = kSym ? 0 : dx.RS;
+    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (nrow + dy.RS + 1)), true);
     CD_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)npairs, ctx->stream));
-    double* prow = ctx->dsum.as<double>();
-    double* pcol = prow + npairs * dx.RS;
+    double* pcol = ctx->dsum.as<double>();
     double* pocc = pcol + npairs * dy.RS;
+    double* prow = kSym ? nullptr : pocc + npairs;
     if (X.B16_layout != 0 || Y.B16_layout != 0)
         return set_error(MSHQC_CD_ERR_STATE, "fixed-point operands not in the integral-tile layout");
     const size_t vsm = vtile_tc::SMEM_BYTES;
@@ -1335,7 +1340,7 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
             e.prow = prow;  e.pcol = pcol;  e.pocc = pocc;
             // split each pair's row tiles over several CTAs when the block
             // pair alone does not fill the GPU several times over
-            const int ta = (int)(dx.RS / 32);
+            const int ta = (int)(dx.RS / 32) * (kSym ? (int)(dx.RS / 32) + 1 : 2) / 2;   // tile pairs, or tile rows
             int nch = 1;
             while (nch < 16 && 2 * nch <= ta && (int64_t)npl * nch < 8LL * ctx->num_sms) nch *= 2;
             e.nchunk = nch;
@@ -1347,7 +1352,7 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
                 e.cpocc = e.cpart + per;
             }
             begin_stage(ctx, ST_AMP_ELEM);
-            amp_elem_kernel<MODE, true><<<(unsigned)(npl * nch), 256, 0, ctx->stream>>>(e);
+            launch_amp<MODE, true>(e, npl * nch, ctx->stream);
             CD_CUDA(cudaGetLastError());
             ctx->launches++;
             if (nch > 1) {
@@ -1395,11 +1400,13 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
     CD_ALLOC(ctx->W, n_stage, false);
     CD_ALLOC(ctx->amp, n_stage, false);
     const int64_t npairs = dx.o * dy.o;
-    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (dx.vp + dy.vp + 1)), true);
+    // (zero where a mirrored pair stands in)
+    const int64_t nrow = kSym ? 0 : dx.vp;
+    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (nrow + dy.vp + 1)), true);
     CD_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)npairs, ctx->stream));
-    double* prow = ctx->dsum.as<double>();
-    double* pcol = prow + npairs * dx.vp;
+    double* pcol = ctx->dsum.as<double>();
     double* pocc = pcol + npairs * dy.vp;
+    double* prow = kSym ? nullptr : pocc + npairs;
     double* S = ctx->W.as<double>();
     double* A = ctx->amp.as<double>();
     for (int64_t I0 = 0; I0 < dx.o; I0 += bI) {
@@ -1442,7 +1449,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             e.A64 = A;  e.ldA = ldS;
             e.partial = partial;
             e.prow = prow;  e.pcol = pcol;  e.pocc = pocc;
-            const int ta = (int)(dx.vp / 32);
+            const int ta = (int)(dx.vp / 32) * (kSym ? (int)(dx.vp / 32) + 1 : 2) / 2;   // tile pairs, or tile rows
             int nch = 1;
             while (nch < 16 && 2 * nch <= ta && (int64_t)npl * nch < 8LL * ctx->num_sms) nch *= 2;
             e.nchunk = nch;
@@ -1454,7 +1461,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
                 e.cpocc = e.cpart + per;
             }
             begin_stage(ctx, ST_AMP_ELEM);
-            amp_elem_kernel<MODE, false><<<(unsigned)(npl * nch), 256, 0, ctx->stream>>>(e);
+            launch_amp<MODE, false>(e, npl * nch, ctx->stream);
             CD_CUDA(cudaGetLastError());
             ctx->launches++;
             if (nch > 1) {

@@ -186,7 +186,7 @@ int opdm_pass(mshqc_cd_ctx* ctx, int sx, int sy, double col_coef, double row_coe
         e.eoy = Y.eps.as<double>();  e.evy = e.eoy + oy;
         e.A64 = ctx->amp.as<double>();  e.ldA = ldS;
         e.partial = partial;   // no dE/de here: prow, pcol, pocc stay null
-        amp_elem_kernel<MODE, false><<<(unsigned)(nbi * oy), 256, 0, ctx->stream>>>(e);
+        launch_amp<MODE, false>(e, nbi * oy, ctx->stream);
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
         // column Gram: K batches i, K = (j, c)
