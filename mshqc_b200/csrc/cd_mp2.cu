@@ -252,6 +252,15 @@ bool fp64_slices(double flops, double min_flops, int64_t reuse) {
     return flops >= min_flops && reuse >= kSlicedMinReuse;
 }
 
+// The sliced FP64 products hold their slices next to the operands.  Each of the
+// functions below reserves them before it writes a result, so where the memory
+// does not hold them the FP64 products run instead.
+bool no_room(mshqc_cd_ctx* ctx, int rc) {
+    if (rc != MSHQC_CD_ERR_ALLOC) return false;
+    for (DevBuf* b : {&ctx->oz_a, &ctx->oz_b, &ctx->oz_p, &ctx->oz_ea, &ctx->oz_eb}) b->release();
+    return true;
+}
+
 bool int8_transform_enabled(const mshqc_cd_ctx* ctx) {
     if (ctx->N > ozaki::Mixed::MAXK) return false;
     const char* env = std::getenv("MSHQC_CD_TRANSFORM");
@@ -374,8 +383,11 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
         }
         const char* tenv = std::getenv("MSHQC_CD_TRANSFORM");   // f64: DMMA for both halves
         if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
-            CD_RC(second_half_sliced<ozaki::Full>(ctx, spins[k], lo[k], hi[k]));
-            continue;
+            const int rc = second_half_sliced<ozaki::Full>(ctx, spins[k], lo[k], hi[k]);
+            if (!no_room(ctx, rc)) {
+                CD_RC(rc);
+                continue;
+            }
         }
         // B[i][a][Q] = sum_nu C[nu, o+a] Y[i][Q][nu]
         GemmF64Args g{};
@@ -511,9 +523,11 @@ int pair_pass_f64(mshqc_cd_ctx* ctx, const PairPass& pp) {
     const int vx = (int)(ctx->N - ox), vy = (int)(ctx->N - oy);
     const int nbx = (int)(X.vp / 64), nby = (int)(Y.vp / 64);
     if (sliced_pairs(ctx, ox * X.vp, oy * Y.vp)) {
-        if (mode == PAIR_RESTRICTED) return pair_pass_f64_staged<PAIR_RESTRICTED>(ctx, pp);
-        if (mode == PAIR_SAME_SPIN) return pair_pass_f64_staged<PAIR_SAME_SPIN>(ctx, pp);
-        return pair_pass_f64_staged<PAIR_OPPOSITE_SPIN>(ctx, pp);
+        const int rc = mode == PAIR_RESTRICTED  ? pair_pass_f64_staged<PAIR_RESTRICTED>(ctx, pp)
+                       : mode == PAIR_SAME_SPIN ? pair_pass_f64_staged<PAIR_SAME_SPIN>(ctx, pp)
+                                                : pair_pass_f64_staged<PAIR_OPPOSITE_SPIN>(ctx, pp);
+        if (!no_room(ctx, rc)) return rc;
+        ctx->W.release();
     }
     const int npairs = pp.npairs, nblocks = (int)block_count(mode, nbx, nby);
     const int64_t units = (int64_t)npairs * nblocks;
@@ -578,7 +592,11 @@ int pair_pass_f64_staged(mshqc_cd_ctx* ctx, const PairPass& pp) {
         const int64_t nI = std::min(bI, ox - I0);
         for (int64_t J0 = kSym ? I0 : 0; J0 < oy; J0 += bJ) {
             const int64_t nJ = std::min(bJ, oy - J0);
-            CD_RC(sliced_integrals(ctx, X, Y, I0, nI, J0, nJ, kSym && I0 == J0, ctx->W.as<double>()));
+            const int rc = sliced_integrals(ctx, X, Y, I0, nI, J0, nJ, kSym && I0 == J0, ctx->W.as<double>());
+            if (rc != MSHQC_CD_OK) {
+                end_stage(ctx);
+                return rc;
+            }
             PairStagedArgs p{};
             p.S = ctx->W.as<double>();
             p.ldS = nJ * Y.vp;
@@ -942,11 +960,10 @@ int virtual_part_f64(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
     return gemm_run(ctx, w, false, false);
 }
 
-// The same on the int8 tensor cores (ozaki::Mixed), batched over orbitals i so
-// that every product has K = M or v; the partial dC of the batches are summed
-// in order.
+// The same on the int8 tensor cores, batched over orbitals i so that every
+// product has K = M or v; the partial dC of the batches are summed in order.
+template <class Cfg>
 int virtual_part_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
-    using Cfg = ozaki::Mixed;
     const SpinState& s = ctx->spin[spin];
     const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, vp = s.vp;
     const int64_t lo = ctx->Yr[spin].lo, hi = ctx->Yr[spin].hi, ni = hi - lo;
@@ -993,6 +1010,19 @@ int virtual_part_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
         }
     }
     return MSHQC_CD_OK;
+}
+
+int virtual_part(mshqc_cd_ctx* ctx, int spin, double scale, double* dC, bool i8) {
+    if (i8) return virtual_part_i8<ozaki::Mixed>(ctx, spin, scale, dC);
+    const auto& y = ctx->Yr[spin];
+    const int64_t v = ctx->N - ctx->spin[spin].nocc;
+    const bool full = int8_transform_enabled(ctx) &&
+                      fp64_slices(2.0 * v * ctx->M * ctx->N * (y.hi - y.lo), kSlicedMinFlops, v);
+    if (full) {   // N = 600, o = 60: the transposed transforms 12.8 -> 8.8 ms; N = 400, o = 40: 2.3 -> 1.9
+        const int rc = virtual_part_i8<ozaki::Full>(ctx, spin, scale, dC);
+        if (!no_room(ctx, rc)) return rc;
+    }
+    return virtual_part_f64(ctx, spin, scale, dC);
 }
 
 // dC[mu, i] = scale sum_{Q,nu} W[i][Q][nu] L[Q][nu][mu] for the W rows of the
@@ -1101,8 +1131,7 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double s
             for (int k = 0; k < nsp; ++k) {
                 CD_RC(first_half(ctx, 1, &spins[k], &lo[k], &hi[k], i8));
                 if (hi[k] <= lo[k]) continue;
-                CD_RC(i8 ? virtual_part_i8(ctx, spins[k], scale, dC[k])
-                         : virtual_part_f64(ctx, spins[k], scale, dC[k]));
+                CD_RC(virtual_part(ctx, spins[k], scale, dC[k], i8));
                 CD_RC(occupied_part(ctx, 1, &spins[k], scale, &dC[k], i8));
                 ctx->Yr[spins[k]].ok = false;
             }
@@ -1112,7 +1141,7 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double s
     }
     for (int k = 0; k < nsp; ++k) {
         if (hi[k] <= lo[k]) continue;
-        CD_RC(i8 ? virtual_part_i8(ctx, spins[k], scale, dC[k]) : virtual_part_f64(ctx, spins[k], scale, dC[k]));
+        CD_RC(virtual_part(ctx, spins[k], scale, dC[k], i8));
     }
     CD_RC(occupied_part(ctx, nsp, spins, scale, dC, i8));
     for (int k = 0; k < nsp; ++k) ctx->Yr[spins[k]].ok = false;   // W is there now
@@ -1421,11 +1450,14 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             const int64_t ldS = (int64_t)nJ * dy.vp;
             const double* YJ = Y.B64.as<double>() + J0 * dy.vp * Mp;
             // S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q]
-            const bool sliced = sliced_pairs(ctx, nI * dx.vp, ldS);
+            bool sliced = sliced_pairs(ctx, nI * dx.vp, ldS);
             begin_stage(ctx, ST_AMPLITUDE);
             if (sliced) {
-                CD_RC(sliced_integrals(ctx, X, Y, I0, nI, J0, nJ, tri, S));
-            } else {
+                const int rc = sliced_integrals(ctx, X, Y, I0, nI, J0, nJ, tri, S);
+                sliced = !no_room(ctx, rc);
+                if (sliced) CD_RC(rc);
+            }
+            if (!sliced) {
                 GemmF64Args g{};
                 g.M = (int)(nI * dx.vp);  g.N = (int)ldS;  g.K = (int)Mp;  g.batch = 1;
                 g.A = XI;  g.lda = Mp;  g.sA = 0;
@@ -1473,12 +1505,21 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             begin_stage(ctx, ST_GAMMA);
             double* gx = ctx->gam[sx].as<double>() + I0 * dx.vp * Mp;
             double* gy = ctx->gam[sy].as<double>() + J0 * dy.vp * Mp;
+            // the staged integrals are used up: their block takes the slices
+            bool todo_x = true, todo_y = mirror;
             if (sliced) {
-                // the staged integrals are used up: their block takes the slices
-                CD_RC(sliced_gamma(ctx, A, ldS, false, nI * dx.vp, ldS, YJ, gx, ctx->W));
-                if (mirror) CD_RC(sliced_gamma(ctx, A, ldS, true, ldS, nI * dx.vp, XI, gy, ctx->W));
+                int rc = sliced_gamma(ctx, A, ldS, false, nI * dx.vp, ldS, YJ, gx, ctx->W);
+                todo_x = no_room(ctx, rc);
+                if (!todo_x) CD_RC(rc);
+                if (mirror && !todo_x) {
+                    rc = sliced_gamma(ctx, A, ldS, true, ldS, nI * dx.vp, XI, gy, ctx->W);
+                    todo_y = no_room(ctx, rc);
+                    if (!todo_y) CD_RC(rc);
+                }
+                CD_ALLOC(ctx->W, n_stage, false);
                 S = ctx->W.as<double>();
-            } else {
+            }
+            if (todo_x) {
                 // Gamma_x[(i,a)][Q] += sum_{(j,b) in J} t[(i,a)][(j,b)] Y[(j,b)][Q]
                 GemmF64Args h{};
                 h.M = (int)(nI * dx.vp);  h.N = (int)Mp;  h.K = (int)ldS;  h.batch = 1;
@@ -1487,16 +1528,16 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
                 h.C = gx;  h.ldc = Mp;  h.sC = 0;
                 h.alpha = 1.0;  h.beta = 1.0;
                 CD_RC(gemm_run(ctx, h, true, false));
-                if (mirror) {
-                    // Gamma_y[(j,b)][Q] += sum_{(i,a) in I} t[(i,a)][(j,b)] X[(i,a)][Q]
-                    GemmF64Args k{};
-                    k.M = (int)ldS;  k.N = (int)Mp;  k.K = (int)(nI * dx.vp);  k.batch = 1;
-                    k.A = A;  k.lda = ldS;  k.sA = 0;
-                    k.B = XI;  k.ldb = Mp;  k.sB = 0;
-                    k.C = gy;  k.ldc = Mp;  k.sC = 0;
-                    k.alpha = 1.0;  k.beta = 1.0;
-                    CD_RC(gemm_run(ctx, k, false, false));
-                }
+            }
+            if (todo_y) {
+                // Gamma_y[(j,b)][Q] += sum_{(i,a) in I} t[(i,a)][(j,b)] X[(i,a)][Q]
+                GemmF64Args k{};
+                k.M = (int)ldS;  k.N = (int)Mp;  k.K = (int)(nI * dx.vp);  k.batch = 1;
+                k.A = A;  k.lda = ldS;  k.sA = 0;
+                k.B = XI;  k.ldb = Mp;  k.sB = 0;
+                k.C = gy;  k.ldc = Mp;  k.sC = 0;
+                k.alpha = 1.0;  k.beta = 1.0;
+                CD_RC(gemm_run(ctx, k, false, false));
             }
             end_stage(ctx);
         }
