@@ -904,21 +904,33 @@ int run_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* out)
 // ---------------------------------------------------------------------------
 namespace {
 
-// out[k] = (accumulate ? out[k] : 0) + alpha * sum_b parts[b * stride + k], b in order
-__global__ void sum_batches_kernel(const double* __restrict__ parts, int nb, int64_t stride, int64_t n, double alpha,
-                                   int accumulate, double* __restrict__ out) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n) return;
+// out[k] = (accumulate ? out[k] : 0) + alpha * sum_b parts[b * stride + k].
+// HBM bound: 32 elements x 8 lanes of batches per CTA (lane g takes b = g, g + 8,
+// ...; the lanes are added in order).  One thread per element walking all 1600
+// batches of a 40 x 400 product left most SMs idle (190 us, now 20; N = 400, o = 40
+// mixed transposed transforms 2.51 -> 2.34 ms).
+__global__ void __launch_bounds__(256) sum_batches_kernel(const double* __restrict__ parts, int nb, int64_t stride,
+                                                          int64_t n, double alpha, int accumulate,
+                                                          double* __restrict__ out) {
+    __shared__ double red[8][32];
+    const int c = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int64_t k = blockIdx.x * (int64_t)32 + c;
     double acc = 0.0;
+    if (k < n) {
 #pragma unroll 8
-    for (int b = 0; b < nb; ++b) acc += parts[(int64_t)b * stride + k];
+        for (int b = g; b < nb; b += 8) acc += parts[(int64_t)b * stride + k];
+    }
+    red[g][c] = acc;
+    __syncthreads();
+    if (g || k >= n) return;
+    for (int h = 1; h < 8; ++h) acc += red[h][c];
     out[k] = accumulate ? out[k] + alpha * acc : alpha * acc;
 }
 
 int sum_batches(mshqc_cd_ctx* ctx, const double* parts, int nb, int64_t stride, int64_t n, double alpha,
                 bool accumulate, double* out) {
     if (n <= 0) return MSHQC_CD_OK;
-    sum_batches_kernel<<<(unsigned)cdiv(n, 256), 256, 0, ctx->stream>>>(parts, nb, stride, n, alpha,
+    sum_batches_kernel<<<(unsigned)cdiv(n, 32), 256, 0, ctx->stream>>>(parts, nb, stride, n, alpha,
                                                                          accumulate ? 1 : 0, out);
     CD_CUDA(cudaGetLastError());
     ctx->launches++;
