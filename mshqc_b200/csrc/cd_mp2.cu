@@ -267,11 +267,12 @@ bool int8_transform_enabled(const mshqc_cd_ctx* ctx) {
     return !(env && std::strcmp(env, "f64") == 0);
 }
 
-// The forward half transform of a mixed request runs on the int8 tensor
-// cores from N = 512 on; below, the FP64 products are faster (forward
-// transform of the gradient step, one box: N=400 1.8 ms FP64 vs 2.6 ms int8,
-// N=600 8.8 vs 7.6 ms) and their B is exact.  The transposed transforms keep
-// the int8 products at every size (N=400: 3.4 vs 6.8 ms).
+// The forward half transform of a mixed request runs on the int8 tensor cores
+// from N = 512 on; below, the FP64 products (DMMA, full slices) take the same
+// time and their B is exact (forward transform of the gradient step: N = 400
+// 1.34 ms FP64, 1.38 int8; N = 520 4.3 DMMA, 3.2 int8; N = 600 7.1 and 4.7).
+// The transposed transforms keep the int8 products at every size (N = 400 2.3 ms
+// either way, N = 600 10.6 DMMA, 6.7 int8, open shell 23.2 and 10.9).
 // MSHQC_CD_TRANSFORM=i8 forces the int8 products, =f64 the FP64 ones.
 constexpr int64_t kInt8ForwardMinN = 512;
 bool int8_forward_enabled(const mshqc_cd_ctx* ctx) {
@@ -285,7 +286,7 @@ bool int8_forward_enabled(const mshqc_cd_ctx* ctx) {
 // given spins: Y[row of i][(Q,nu)] = sum_mu C[mu,i] L[Q][nu*N + mu], one chunk of
 // vectors at a time.  Two spins are one product over both spins' orbitals, so
 // the vectors are read (and sliced) once: unrestricted N = 600, 60 + 58
-// orbitals, 10.5 -> 6.3 ms with the second halves.  i8: int8 slices of the mixed
+// orbitals, 10.5 -> 7.1 ms with the second halves.  i8: int8 slices of the mixed
 // accuracy, else FP64 on the DMMA pipe (every vector element meets few
 // orbitals: full slices would cost more than the products).
 int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, const int64_t* hi, bool i8) {
