@@ -298,14 +298,18 @@ int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, 
     int64_t r = 0;
     for (int k = 0; k < nsp; ++k) {
         auto& y = ctx->Yr[spins[k]];
-        y.ok = true;
         y.i8 = i8;
         y.row = r;
         y.lo = lo[k];
         y.hi = hi[k];
         r += std::max<int64_t>(0, hi[k] - lo[k]);
     }
-    if (rows == 0) return MSHQC_CD_OK;
+    // the rows are valid once every product that fills them is queued
+    auto filled = [&]() {
+        for (int k = 0; k < nsp; ++k) ctx->Yr[spins[k]].ok = true;
+        return MSHQC_CD_OK;
+    };
+    if (rows == 0) return filled();
     // the orbitals as contiguous rows
     const double* C = ctx->spin[spins[0]].C.as<double>() + lo[0] * N;
     if (nsp == 2) {
@@ -355,7 +359,7 @@ int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, 
             }
         }
     }
-    return MSHQC_CD_OK;
+    return filled();
 }
 
 // Forward half transforms of the given spins into the padded [i][a][Q] layout,
@@ -369,8 +373,8 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
         SpinState& s = ctx->spin[spins[k]];
         shard_range(ctx, s.nocc, &lo[k], &hi[k]);
         s.vp = round_up(N - s.nocc, 64);
+        s.invalidate();   // run_transforms marks B valid, with its last launch queued
         CD_ALLOC(s.B64, sizeof(double) * (size_t)b_rows(ctx, s.nocc) * s.vp * Mp, true);
-        s.B64_valid = true;
         s.B64_prec = i8 ? MSHQC_CD_FP16X3 : MSHQC_CD_FP64;
     }
     CD_RC(first_half(ctx, nsp, spins, lo, hi, i8));
@@ -792,7 +796,7 @@ int run_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, int precision) 
         // shared over ranks: this rank's orbitals so far, now all of them
         if (sharded(ctx))
             CD_RC(run_collective(ctx, true, s.B64.as<double>(), shard_p(ctx, s.nocc) * s.vp * ctx->Mp));
-        s.B16_valid = false;
+        s.B64_valid = true;
     }
     end_stage(ctx);
     return MSHQC_CD_OK;
