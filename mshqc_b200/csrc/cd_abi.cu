@@ -255,11 +255,8 @@ int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p) {
 }
 
 int begin_call(mshqc_cd_ctx* ctx) {
-    for (auto& s : ctx->spin)
-        if (s.norms_pending) {   // left by a call that failed
-            s.B16_valid = false;
-            s.norms_pending = false;
-        }
+    if (ctx->call_open) ctx->invalidate_derived();
+    ctx->call_open = true;
     CD_ALLOC(ctx->status, sizeof(CallStatus), true);
     return MSHQC_CD_OK;
 }
@@ -290,6 +287,7 @@ int finish_call(mshqc_cd_ctx* ctx, CallStatus* out, const void* dev, size_t extr
                              std::to_string(st.tile_err[0] ? st.tile_err[0] : st.gamma_err[0] ? st.gamma_err[0]
                                                                                                : st.slice_err[0]) +
                              ")");
+    ctx->call_open = false;
     return MSHQC_CD_OK;
 }
 

@@ -91,6 +91,7 @@ struct mshqc_cd_ctx {
     } Yr[2];
     mshqc_cd::DevBuf cpack;         // occupied orbitals of both spins, one after the other
     mshqc_cd::DevBuf occ_parts;     // dE/dC_occ of both spins in one product
+    bool call_open = false;         // a call that began has not finished (see begin_call)
     int L_sym = -1;                 // stored vectors symmetric to the bit (-1: not looked at yet)
     mshqc_cd::DevBuf scratch;       // uploads / unpacking
     mshqc_cd::DevBuf partial;       // per-unit energies
@@ -135,11 +136,17 @@ struct mshqc_cd_ctx {
     bool coll_set = false;
     std::vector<double> pair_energy[3];  // host copies, row-major [i][j]
 
-    void invalidate_all() {
-        spin[0].invalidate();
-        spin[1].invalidate();
+    // what calls derive from the vectors and orbitals
+    void invalidate_derived() {
+        for (auto& s : spin) {
+            s.invalidate();
+            s.norms_pending = false;
+        }
         diag_os_valid = false;
         Yr[0].ok = Yr[1].ok = false;
+    }
+    void invalidate_all() {
+        invalidate_derived();
         L_sym = -1;
         for (auto& p : pair_energy) p.clear();
     }
@@ -250,6 +257,9 @@ struct CallStatus {
 };
 // pinned host memory of at least `bytes` (grow-only; contents not kept)
 int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p);
+// Zeroes the status.  A call that stopped in between (an allocation that failed,
+// a kernel that gave up) may have left a buffer half written, or W where Y was:
+// what it had derived is then formed again.
 int begin_call(mshqc_cd_ctx* ctx);
 // Waits for the call's work, reports kernels that gave up, and copies `extra`
 // bytes from dev to the pinned buffer behind the status (*extra_host).

@@ -957,6 +957,7 @@ int virtual_part_f64(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
     const int64_t lo = ctx->Yr[spin].lo, ni = ctx->Yr[spin].hi - lo;
     const double* Gm = ctx->gam[spin].as<double>() + lo * vp * Mp;
     double* Y = y_rows(ctx, spin);
+    ctx->Yr[spin].ok = false;   // W goes there
     // dC[nu, o+a] (row-major [a][nu] == column-major dC): one product over the
     // composite K = (i, Q); v x N output tiles alone leave most SMs idle at
     // small v
@@ -987,6 +988,7 @@ int virtual_part_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
     const double* C = s.C.as<double>();
     const double* Gm = ctx->gam[spin].as<double>();
     double* Y = y_rows(ctx, spin);
+    ctx->Yr[spin].ok = false;   // W goes there
     // dC[nu, o+a]: Gamma_i (rows a, K = Q) against Y_i^T (rows nu, K = Q, strided by N)
     {
         const bool sw = oz_swap<Cfg>(v, N);
@@ -1150,7 +1152,6 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double s
                 if (hi[k] <= lo[k]) continue;
                 CD_RC(virtual_part(ctx, spins[k], scale, dC[k], i8));
                 CD_RC(occupied_part(ctx, 1, &spins[k], scale, &dC[k], i8));
-                ctx->Yr[spins[k]].ok = false;
             }
             return MSHQC_CD_OK;
         }
@@ -1160,9 +1161,7 @@ int transposed_transforms(mshqc_cd_ctx* ctx, int nsp, const int* spins, double s
         if (hi[k] <= lo[k]) continue;
         CD_RC(virtual_part(ctx, spins[k], scale, dC[k], i8));
     }
-    CD_RC(occupied_part(ctx, nsp, spins, scale, dC, i8));
-    for (int k = 0; k < nsp; ++k) ctx->Yr[spins[k]].ok = false;   // W is there now
-    return MSHQC_CD_OK;
+    return occupied_part(ctx, nsp, spins, scale, dC, i8);
 }
 
 // the int8 products for the mixed path (unless switched off), FP64 otherwise

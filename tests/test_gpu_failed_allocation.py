@@ -71,3 +71,10 @@ def check_gradient(e_tol, d_tol):
 @pytest.mark.parametrize("kind", [capi.RESTRICTED, capi.UNRESTRICTED])
 def test_energy_after_failed_allocation(inp, kind):
     retry(inp, lambda ctx: ctx.mp2_energy(kind, capi.FP64), check_energy)
+
+
+@pytest.mark.parametrize("kind", [capi.RESTRICTED, capi.UNRESTRICTED])
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP16X3])
+def test_gradient_after_failed_allocation(inp, kind, precision):
+    tol = (1e-12, 1e-10) if precision == capi.FP64 else (1e-9, 1e-9)
+    retry(inp, lambda ctx: ctx.mp2_gradient(kind, precision), check_gradient(*tol))
