@@ -153,19 +153,13 @@ __global__ void count_nonfinite_kernel(const double* __restrict__ x, int64_t n,
     if (local) atomicAdd(bad, local);
 }
 
-// dst = src for two arrays, bad[k] set when array k holds a NaN or infinity
-__global__ void copy_check2_kernel(const double* __restrict__ a, double* __restrict__ da, int64_t na,
-                                   const double* __restrict__ b, double* __restrict__ db, int64_t nb,
-                                   int* __restrict__ bad) {
+// bad[k] set when array k (a, b) holds a NaN or infinity
+__global__ void check2_kernel(const double* __restrict__ a, int64_t na, const double* __restrict__ b, int64_t nb,
+                              int* __restrict__ bad) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < na + nb;
          t += (int64_t)gridDim.x * blockDim.x) {
         const bool second = t >= na;
-        const double x = second ? b[t - na] : a[t];
-        if (second)
-            db[t - na] = x;
-        else
-            da[t] = x;
-        if (!isfinite(x)) bad[second ? 1 : 0] = 1;
+        if (!isfinite(second ? b[t - na] : a[t])) bad[second ? 1 : 0] = 1;
     }
 }
 
@@ -182,6 +176,16 @@ bool is_device_pointer(const void* p) {
         return false;
     }
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+}
+
+// memory that CUDA does not know: a copy between devices may not be given it
+bool is_unregistered(const void* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
 }
 
 bool is_pinned_host(const void* p) {
@@ -495,6 +499,8 @@ int mshqc_cd_set_orbitals(mshqc_cd_ctx* ctx, int spin, const double* C, const do
     const int64_t N = ctx->N;
     if (nocc < 1 || nocc >= N)
         return set_error(MSHQC_CD_ERR_ARG, "nocc must satisfy 1 <= nocc < nbf");
+    if (where != MSHQC_CD_HOST && (is_unregistered(C) || is_unregistered(eps)))
+        return set_error(MSHQC_CD_ERR_ARG, "C and eps must be device pointers");
     DeviceGuard g(ctx->device);
     SpinState& s = ctx->spin[spin];
     CD_ALLOC(s.C, sizeof(double) * N * N, false);
@@ -507,20 +513,25 @@ int mshqc_cd_set_orbitals(mshqc_cd_ctx* ctx, int spin, const double* C, const do
         rc = upload(ctx, s.eps.p, eps, sizeof(double) * N);
         if (rc) return rc;
     } else {
-        // copied and checked in one pass
-        CD_ALLOC(ctx->flag, 2 * sizeof(int), true);
+        // Copies, which check the caller's ranges and reach another device's memory
+        // too; only the context's own copies are read by a kernel.
+        CD_CUDA(cudaMemcpyAsync(s.C.p, C, sizeof(double) * N * N, cudaMemcpyDeviceToDevice, ctx->stream));
+        CD_CUDA(cudaMemcpyAsync(s.eps.p, eps, sizeof(double) * N, cudaMemcpyDeviceToDevice, ctx->stream));
+        if (!ctx->orb_bad.p) CD_ALLOC(ctx->orb_bad, 2 * sizeof(int), true);   // zero but for a refused input
         const int blocks = (int)std::min<int64_t>(8LL * ctx->num_sms, cdiv(N * N + N, 256));
-        copy_check2_kernel<<<blocks, 256, 0, ctx->stream>>>(C, s.C.as<double>(), N * N, eps, s.eps.as<double>(), N,
-                                                            ctx->flag.as<int>());
+        check2_kernel<<<blocks, 256, 0, ctx->stream>>>(s.C.as<double>(), N * N, s.eps.as<double>(), N,
+                                                       ctx->orb_bad.as<int>());
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
         void* h = nullptr;
         CD_RC(pinned(ctx, 2 * sizeof(int), &h));
-        CD_CUDA(cudaMemcpyAsync(h, ctx->flag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CD_CUDA(cudaMemcpyAsync(h, ctx->orb_bad.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CD_CUDA(cudaStreamSynchronize(ctx->stream));
         const int* bad = static_cast<const int*>(h);
-        if (bad[0] || bad[1])
+        if (bad[0] || bad[1]) {
+            ctx->orb_bad.release();
             return set_error(MSHQC_CD_ERR_NUMERIC, std::string(bad[0] ? "C" : "eps") + " contains NaN/Inf");
+        }
     }
     s.nocc = nocc;
     s.set = true;

@@ -98,6 +98,7 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf pair_sum;      // per-pair energies
     mshqc_cd::DevBuf status;        // error flags and scalar results of a call, see CallStatus
     mshqc_cd::DevBuf flag;          // error / NaN flags
+    mshqc_cd::DevBuf orb_bad;       // NaN flags of set_orbitals, zero between calls
     mshqc_cd::DevBuf gemm_ws;       // split-K partials of the FP64 products
     mshqc_cd::DevBuf pace;          // wave-pacing progress counters of the persistent tile kernels
     mshqc_cd::DevBuf amp;           // backward: staged amplitudes
@@ -172,6 +173,7 @@ struct mshqc_cd_ctx {
         pair_sum.release();
         status.release();
         flag.release();
+        orb_bad.release();
         gemm_ws.release();
         cpack.release();
         occ_parts.release();
