@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(CHOL_THREADS) chol_decompose_kernel(CholArgs a
                 idx = e0 + x;
             }
         block_best(v, idx);
-        if (ne > 0) {
+        if (sidx < n2) {   // (none: no elements, or nothing but NaN, which is never a pivot)
             const int x = (int)(sidx - e0);
             double* row = a.rows + ((int64_t)buf * G + blockIdx.x) * n2;
             for (int64_t k = tid; k < m; k += CHOL_THREADS)
