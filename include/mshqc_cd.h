@@ -55,27 +55,31 @@ enum mshqc_cd_status {
 };
 
 enum mshqc_cd_precision {
-    MSHQC_CD_FP64 = 0,    /* FP64 contractions: FP64 tensor pipe (DMMA), or
-                             for larger products int8 slices with all 53 bits
-                             of each element within a binade of its row's
-                             maximum (7 x 8 bits, exact integer sums, error
-                             per term below 2^-54 of the row maxima; smaller
-                             than that of a chain of FP64 FMAs).
-                             MSHQC_CD_FP64_SLICES=off in the environment:
-                             DMMA only, =on: slices at every size           */
+    MSHQC_CD_FP64 = 0,    /* FP64 contractions on the FP64 tensor pipe
+                             (DMMA).  Larger integral and Gamma products,
+                             second half transforms and the virtual products
+                             of the transposed ones run as int8 slices (7 x 8
+                             bits, exact integer sums; elements held to
+                             2^-55 of the power of two above their row's
+                             maximum) where that is at least as accurate as a
+                             chain of FP64 FMAs; tiles of a result whose rows
+                             are large in different places are computed by
+                             DMMA.  MSHQC_CD_FP64_SLICES=off in the
+                             environment: DMMA only, =on: these products as
+                             slices at every size                           */
     MSHQC_CD_FP16X3 = 1   /* scaled FP16 x3: every MO row in fixed point with
                              one power-of-two scale, integer hi/lo carried in
                              FP16, three products per pair, exact FP32
                              accumulation on the tensor cores; FP64
                              denominators, diagonal integrals and energies;
                              the half transforms (from nbf = 512 on;
-                             below, FP64 DMMA) and the backward's
+                             below, those of MSHQC_CD_FP64) and the backward's
                              transposed transforms as FP64 products of
                              int8 slices (5 x 7 bits per operand row) on
                              the tensor cores, about 2^-32 of the row
                              maxima per term (MSHQC_CD_TRANSFORM=f64 in the
-                             environment: FP64 DMMA for both, =i8: int8
-                             slices for both at every size)              */
+                             environment: those of MSHQC_CD_FP64 for both,
+                             =i8: int8 slices for both at every size)    */
 };
 
 enum mshqc_cd_kind {
@@ -228,8 +232,8 @@ MSHQC_CD_API int mshqc_cd_set_orbitals(mshqc_cd_ctx* ctx, int spin, const double
  * CholeskyUMP2::transform_cholesky_vectors (src/mp2/cholesky_ump2.cc:244-293)
  * and CholeskyOMP2::transform_vectors (src/mp2/cholesky_omp2.cc:71-92).
  * B_out (o*v*M, see header) may be NULL to keep the result on the device
- * only.  MSHQC_CD_FP64 returns FP64 DMMA products; MSHQC_CD_FP16X3 may
- * return the int8-slice products (or reuse FP64 ones already computed). */
+ * only.  MSHQC_CD_FP64 returns products of FP64 accuracy; MSHQC_CD_FP16X3
+ * may return those of 35-bit int8 slices (or reuse FP64 ones). */
 MSHQC_CD_API int mshqc_cd_transform(mshqc_cd_ctx* ctx, int spin, int precision,
                        double* B_out, int where);
 /* MP2 correlation energy.  Replaces the pair loop of CholeskyRMP2::compute

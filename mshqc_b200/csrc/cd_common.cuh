@@ -12,6 +12,24 @@ constexpr double kDenomSkip = 1e-12;  // |D| < 1e-12 terms are skipped
 __host__ __device__ inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __host__ __device__ inline int64_t round_up(int64_t a, int64_t b) { return cdiv(a, b) * b; }
 
+// Unit u of a batched product in nmb x nnb tiles -> (batch, row block, column
+// block).  Tiles come in groups of `group` row blocks with all column blocks,
+// column-block-major inside a group: with 128 x 64 or 128 x 96 tiles of int8
+// slices (ozaki_i8.cuh) the 148 tiles of one wave then read about 16 row blocks
+// and 9 column blocks, 0.6 MB per K chunk in place of 4 MB row-block-major,
+// which HBM cannot feed.
+__device__ __forceinline__ void tile_of_unit(long long u, int nmb, int nnb, int group, long long& b, int& mb,
+                                             int& nb) {
+    const long long per = (long long)nmb * nnb;
+    b = u / per;
+    const int w = (int)(u - b * per);
+    const int pg = group * nnb, grp = w / pg;
+    const int g0 = grp * group, gsz = min(nmb - g0, group);
+    const int x = w - grp * pg;
+    nb = x / gsz;
+    mb = g0 + x - nb * gsz;
+}
+
 // ---------------------------------------------------------------------------
 // Neumaier-compensated FP64 accumulation
 // ---------------------------------------------------------------------------

@@ -118,7 +118,8 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf Zt;            // Fock builds: P L^Q (or the factored density's L^Q X) of a chunk of vectors
     mshqc_cd::DevBuf dens_x;        // Fock builds: Cholesky factors of the densities
     mshqc_cd::DevBuf oz_a, oz_b;    // int8 slices of the transform operands (orbitals, vectors)
-    mshqc_cd::DevBuf oz_ea, oz_eb;  // their row exponents
+    mshqc_cd::DevBuf oz_ea, oz_eb;  // their row exponents and digit squares
+    mshqc_cd::DevBuf oz_tiles;      // tiles of a sliced FP64 product that the FP64 product computes
     mshqc_cd::DevBuf oz_p;          // per-batch FP64 partial products (transposed transforms)
     bool diag_os_valid = false;
     int fixed_point_exact = 1;      // Cauchy-Schwarz bound of the last tensor-core pass held
@@ -157,7 +158,7 @@ struct mshqc_cd_ctx {
         for (const auto& s : spin)
             b += s.C.bytes + s.eps.bytes + s.B64.bytes + s.B16.bytes + s.expo.bytes +
                  s.diag.bytes;
-        b += gemm_ws.bytes + dens_x.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes;
+        b += gemm_ws.bytes + dens_x.bytes + Zt.bytes + diag_os.bytes + oz_a.bytes + oz_b.bytes + oz_ea.bytes + oz_eb.bytes + oz_p.bytes + oz_tiles.bytes;
         for (const auto& g : gam) b += g.bytes;
         for (const auto& g : grad) b += g.bytes;
         return b;
@@ -205,6 +206,7 @@ struct mshqc_cd_ctx {
         oz_b.release();
         oz_ea.release();
         oz_eb.release();
+        oz_tiles.release();
         oz_p.release();
         for (auto& g : gam) g.release();
         for (auto& g : grad) g.release();

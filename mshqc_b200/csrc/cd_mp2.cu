@@ -21,6 +21,7 @@
 #include "vtile_tc.cuh"
 #include "amp_elem.cuh"
 #include "ozaki_i8.cuh"
+#include "slice_guard.cuh"
 
 namespace mshqc_cd {
 
@@ -187,6 +188,47 @@ size_t oz_bytes(const OzakiOperand& op) {
     return ozaki::operand_bytes<C>(op.Rp, op.Kp) * (size_t)op.batch;
 }
 int* slice_err(mshqc_cd_ctx* ctx) { return ctx->status.as<CallStatus>()->slice_err; }
+// One sliced product; A has the 128-row blocks.  With C::GUARD its accuracy is
+// that of an FP64 chain or better: tiles whose rows say otherwise (slice_guard.cuh)
+// are left out and computed by the FP64 product from the operands' sources.
+// N = 400, o = 40, vectors of two fragments with couplings of 10^-6: FP64 energy
+// 15.7 ms without slices, 11.7 with, gradient 37.8 and 40.3 (nearly every tile
+// left out); rows of one kind 15.8 and 5.9, 37.8 and 17.6, the guards 0.2 and
+// 0.5 of them.  Reserves what it needs before it writes a result.
+template <class C>
+int oz_gemm(mshqc_cd_ctx* ctx, const OzakiOperand& A, const OzakiOperand& B, double* out, int64_t ldc, int64_t cb,
+            double alpha, double beta, OzakiOpts o) {
+    const int64_t nmb = A.Rp / ozaki::BM, nnb = B.Rp / C::BN;
+    GemmListed l{};
+    if (C::GUARD) {
+        const int64_t units = nmb * nnb * (o.a_shared ? B.batch : A.batch);
+        CD_ALLOC(ctx->oz_tiles, (size_t)(sizeof(int) * (units + 1) + units), false);
+        int* count = ctx->oz_tiles.as<int>();
+        uint8_t* left_out = reinterpret_cast<uint8_t*>(count + 1 + units);
+        CD_CUDA(guard_slices(A, B, o, left_out, count, count + 1, ctx->stream));
+        o.left_out = left_out;
+        l.count = count;
+        l.list = count + 1;
+        l.nmb = (int)nmb;  l.nnb = (int)nnb;  l.group = ozaki::GROUP;
+        l.trans = o.trans ? 1 : 0;
+    }
+    CD_CUDA(ozaki_gemm<C>(A, B, out, ldc, cb, alpha, beta, o, slice_err(ctx), ctx->num_sms, ctx->stream));
+    ctx->launches++;
+    if (C::GUARD) {
+        const OzakiOperand& X = o.trans ? B : A;   // rows of the result, and its columns
+        const OzakiOperand& Y = o.trans ? A : B;
+        const bool xs = o.trans ? o.b_shared : o.a_shared, ys = o.trans ? o.a_shared : o.b_shared;
+        GemmF64Args g{};
+        g.M = (int)X.R;  g.N = (int)Y.R;  g.K = (int)X.K;  g.batch = X.batch;
+        g.A = X.src;  g.lda = X.ld;  g.sA = xs ? 0 : X.sb;
+        g.B = Y.src;  g.ldb = Y.ld;  g.sB = ys ? 0 : Y.sb;
+        g.C = out;  g.ldc = ldc;  g.sC = cb;
+        g.alpha = alpha;  g.beta = beta;
+        CD_CUDA(gemm_f64_listed(g, !X.t, !Y.t, l, ctx->num_sms, ctx->stream));
+        ctx->launches += 2;
+    }
+    return MSHQC_CD_OK;
+}
 template <class C>
 int oz_mul(mshqc_cd_ctx* ctx, const OzakiOperand& X, bool x_shared, const OzakiOperand& Y, bool y_shared, bool sw,
            double* out, int64_t ldc, int64_t cb, double alpha, double beta) {
@@ -194,15 +236,13 @@ int oz_mul(mshqc_cd_ctx* ctx, const OzakiOperand& X, bool x_shared, const OzakiO
     o.a_shared = sw ? y_shared : x_shared;
     o.b_shared = sw ? x_shared : y_shared;
     o.trans = sw;
-    CD_CUDA(ozaki_gemm<C>(sw ? Y : X, sw ? X : Y, out, ldc, cb, alpha, beta, o, slice_err(ctx), ctx->num_sms,
-                          ctx->stream));
-    ctx->launches++;
-    return MSHQC_CD_OK;
+    return oz_gemm<C>(ctx, sw ? Y : X, sw ? X : Y, out, ldc, cb, alpha, beta, o);
 }
-// reserves an operand's digits and exponents
+// reserves an operand's digits and what goes with its rows
+template <class C>
 int oz_reserve(mshqc_cd_ctx* ctx, DevBuf& q, DevBuf& e, size_t bytes, OzakiOperand& op) {
     CD_ALLOC(q, bytes, false);
-    CD_ALLOC(e, sizeof(int) * (size_t)(op.Rp * op.batch), false);
+    CD_ALLOC(e, op.row_bytes(C::GUARD), false);
     op.q = q.as<int8_t>();
     op.e = e.as<int>();
     return MSHQC_CD_OK;
@@ -220,7 +260,7 @@ int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
     const int64_t N = ctx->N, M = ctx->M, Mp = ctx->Mp, o = s.nocc, v = N - o, ni = hi - lo, vp = s.vp;
     const bool sw = oz_swap<C>(v, M);
     OzakiOperand Av = oz_operand<C>(v, N, !sw, 1);
-    CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<C>(Av), Av));
+    CD_RC(oz_reserve<C>(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<C>(Av), Av));
     CD_CUDA(ozaki_slice<C>(s.C.as<double>() + o * N, N, 0, Av, ctx->num_sms, ctx->stream));
     ctx->launches++;
     const int64_t per_i = (int64_t)oz_bytes<C>(oz_operand<C>(M, N, sw, 1));
@@ -228,7 +268,7 @@ int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
     for (int64_t i0 = lo; i0 < hi; i0 += ib) {
         const int64_t nb = std::min(ib, hi - i0);
         OzakiOperand By = oz_operand<C>(M, N, sw, nb);
-        CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, (size_t)(per_i * nb), By));
+        CD_RC(oz_reserve<C>(ctx, ctx->oz_b, ctx->oz_eb, (size_t)(per_i * nb), By));
         CD_CUDA(ozaki_slice<C>(y_rows(ctx, spin) + (i0 - lo) * M * N, N, M * N, By, ctx->num_sms, ctx->stream));
         ctx->launches++;
         CD_RC(oz_mul<C>(ctx, Av, true, By, false, sw, s.B64.as<double>() + i0 * vp * Mp, Mp, vp * Mp, 1.0, 0.0));
@@ -257,7 +297,7 @@ bool fp64_slices(double flops, double min_flops, int64_t reuse) {
 // does not hold them the FP64 products run instead.
 bool no_room(mshqc_cd_ctx* ctx, int rc) {
     if (rc != MSHQC_CD_ERR_ALLOC) return false;
-    for (DevBuf* b : {&ctx->oz_a, &ctx->oz_b, &ctx->oz_p, &ctx->oz_ea, &ctx->oz_eb}) b->release();
+    for (DevBuf* b : {&ctx->oz_a, &ctx->oz_b, &ctx->oz_p, &ctx->oz_ea, &ctx->oz_eb, &ctx->oz_tiles}) b->release();
     return true;
 }
 
@@ -327,7 +367,7 @@ int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, 
     const bool sw = round_up(rows, Cfg::BN) < round_up(rows, ozaki::BM);
     OzakiOperand Ao = oz_operand<Cfg>(rows, N, !sw, 1);
     if (i8) {
-        CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(Ao), Ao));
+        CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(Ao), Ao));
         CD_CUDA(ozaki_slice<Cfg>(C, N, 0, Ao, ctx->num_sms, ctx->stream));
         ctx->launches++;
     }
@@ -344,7 +384,7 @@ int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, 
             double* Y = ctx->Y.as<double>() + (Q0 + q0) * N;
             if (i8) {
                 OzakiOperand Bl = oz_operand<Cfg>(ms * N, N, sw, 1);
-                CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Bl), Bl));
+                CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Bl), Bl));
                 CD_CUDA(ozaki_slice<Cfg>(L, N, 0, Bl, ctx->num_sms, ctx->stream));
                 ctx->launches++;
                 CD_RC(oz_mul<Cfg>(ctx, Ao, true, Bl, false, sw, Y, M * N, 0, 1.0, 0.0));
@@ -441,15 +481,14 @@ int sliced_integrals(mshqc_cd_ctx* ctx, const SpinState& X, const SpinState& Y, 
     using Cfg = ozaki::Full;
     const int64_t Mp = ctx->Mp;
     OzakiOperand A = oz_operand<Cfg>(nI * X.vp, Mp, true, 1), B = oz_operand<Cfg>(nJ * Y.vp, Mp, false, 1);
-    CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(A), A));
-    CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(B), B));
+    CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_a, ctx->oz_ea, oz_bytes<Cfg>(A), A));
+    CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(B), B));
     CD_CUDA(ozaki_slice<Cfg>(X.B64.as<double>() + I0 * X.vp * Mp, Mp, 0, A, ctx->num_sms, ctx->stream));
     CD_CUDA(ozaki_slice<Cfg>(Y.B64.as<double>() + J0 * Y.vp * Mp, Mp, 0, B, ctx->num_sms, ctx->stream));
     OzakiOpts o;
     o.tri = tri ? (int)X.vp : 0;
-    CD_CUDA(ozaki_gemm<Cfg>(A, B, S, nJ * Y.vp, 0, 1.0, 0.0, o, slice_err(ctx), ctx->num_sms, ctx->stream));
-    ctx->launches += 3;
-    return MSHQC_CD_OK;
+    ctx->launches += 2;
+    return oz_gemm<Cfg>(ctx, A, B, S, nJ * Y.vp, 0, 1.0, 0.0, o);
 }
 
 // gamma[r][Q] += sum_k A(r, k) B[k][Q] over `rows` amplitude rows and K columns
@@ -459,8 +498,8 @@ int sliced_gamma(mshqc_cd_ctx* ctx, const double* A, int64_t lda, bool transpose
     using Cfg = ozaki::Full;
     const int64_t Mp = ctx->Mp;
     OzakiOperand Ta = oz_operand<Cfg>(rows, K, true, 1), Tb = oz_operand<Cfg>(Mp, K, false, 1);
-    CD_RC(oz_reserve(ctx, work, ctx->oz_ea, oz_bytes<Cfg>(Ta), Ta));
-    CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Tb), Tb));
+    CD_RC(oz_reserve<Cfg>(ctx, work, ctx->oz_ea, oz_bytes<Cfg>(Ta), Ta));
+    CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(Tb), Tb));
     if (transposed)
         CD_CUDA(ozaki_slice_t<Cfg>(A, lda, 0, Ta, ctx->stream));
     else
@@ -472,9 +511,8 @@ int sliced_gamma(mshqc_cd_ctx* ctx, const double* A, int64_t lda, bool transpose
         CD_ALLOC(ctx->pace, sizeof(int) * (size_t)ctx->num_sms, false);
         o.pace = ctx->pace.as<int>();
     }
-    CD_CUDA(ozaki_gemm<Cfg>(Ta, Tb, gamma, Mp, 0, 1.0, 1.0, o, slice_err(ctx), ctx->num_sms, ctx->stream));
-    ctx->launches += transposed ? 5 : 4;
-    return MSHQC_CD_OK;
+    ctx->launches += transposed ? 4 : 3;
+    return oz_gemm<Cfg>(ctx, Ta, Tb, gamma, Mp, 0, 1.0, 1.0, o);
 }
 
 // One pair-energy pass: spins, where its pair sums go (ctx->pair_sum, doubles:
@@ -1000,8 +1038,8 @@ int virtual_part_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
         for (int64_t i0 = lo; i0 < hi; i0 += ib) {
             const int64_t nb = std::min(ib, hi - i0);
             OzakiOperand A = oz_operand<Cfg>(v, M, !sw, nb), B = oz_operand<Cfg>(N, M, sw, nb);
-            CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
-            CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
+            CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+            CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
             CD_CUDA(ozaki_slice<Cfg>(Gm + i0 * vp * Mp, Mp, vp * Mp, A, ctx->num_sms, ctx->stream));
             CD_CUDA(ozaki_slice_t<Cfg>(Y + (i0 - lo) * M * N, N, M * N, B, ctx->stream));
             ctx->launches += 3;
@@ -1016,13 +1054,13 @@ int virtual_part_i8(mshqc_cd_ctx* ctx, int spin, double scale, double* dC) {
         const size_t pa = oz_bytes<Cfg>(oz_operand<Cfg>(M, v, !sw, 1));
         const int64_t ib = std::max<int64_t>(1, std::min<int64_t>(ni, (int64_t)(kSliceBytes / pa)));
         OzakiOperand B = oz_operand<Cfg>(N, v, sw, 1);
-        CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(B), B));
+        CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_b, ctx->oz_eb, oz_bytes<Cfg>(B), B));
         CD_CUDA(ozaki_slice_t<Cfg>(C + o * N, N, 0, B, ctx->stream));
         ctx->launches += 2;
         for (int64_t i0 = lo; i0 < hi; i0 += ib) {
             const int64_t nb = std::min(ib, hi - i0);
             OzakiOperand A = oz_operand<Cfg>(M, v, !sw, nb);
-            CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+            CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
             CD_CUDA(ozaki_slice_t<Cfg>(Gm + i0 * vp * Mp, Mp, vp * Mp, A, ctx->stream));
             ctx->launches += 2;
             CD_RC(oz_mul<Cfg>(ctx, A, false, B, true, sw, Y + (i0 - lo) * M * N, N, M * N, 1.0, 0.0));
@@ -1105,8 +1143,8 @@ int occupied_part(mshqc_cd_ctx* ctx, int nsp, const int* spins, double scale, do
         for (int64_t q0 = 0; q0 < mc; q0 += nq) {
             const int64_t nb = std::min(nq, mc - q0);
             OzakiOperand A = oz_operand<Cfg>(rows, N, !sw, nb), B = oz_operand<Cfg>(N, N, sw, nb);
-            CD_RC(oz_reserve(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
-            CD_RC(oz_reserve(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
+            CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_a, ctx->oz_ea, pa * nb, A));
+            CD_RC(oz_reserve<Cfg>(ctx, ctx->oz_b, ctx->oz_eb, pb * nb, B));
             CD_CUDA(ozaki_slice<Cfg>(W + (Q0 + q0) * N, M * N, N, A, ctx->num_sms, ctx->stream));
             if (sym)
                 CD_CUDA(ozaki_slice<Cfg>(Lc + q0 * N * N, N, N * N, B, ctx->num_sms, ctx->stream));

@@ -138,8 +138,10 @@ __device__ __forceinline__ double frag(const double* sm, int r, int k) {
 }
 }  // namespace gemm_detail
 
+// One T x T tile of the product: rows m0.., columns n0.., batch b, K split `split`;
+// swap: the warp rows change places
 template <bool A_K, bool B_K, int VEC, int T>
-__global__ void __launch_bounds__(128, T == 64 ? 3 : 6) gemm_f64_kernel(GemmF64Args p) {
+__device__ __forceinline__ void gemm_tile(const GemmF64Args& p, int m0, int n0, int64_t b, int split, int swap) {
     using namespace gemm_detail;
     constexpr int TD = tile_doubles<T>();
     constexpr int WT = T / 2, NF = WT / 8;   // rows / columns per warp, 8-wide fragments
@@ -148,12 +150,7 @@ __global__ void __launch_bounds__(128, T == 64 ? 3 : 6) gemm_f64_kernel(GemmF64A
     double* smB = gemm_smem + STAGES * TD;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
-    if (p.tri > 0 && n0 / p.tri < m0 / p.tri) return;
-    if (p.sym && n0 < m0) return;
-    const int wm = (warp >> 1) ^ (int)(blockIdx.x & 1), wn = warp & 1;
-    const int64_t b = blockIdx.z / p.S;
-    const int split = (int)(blockIdx.z % p.S);
+    const int wm = (warp >> 1) ^ swap, wn = warp & 1;
     const double* A = p.A + b * p.sA;
     const double* B = p.B + b * p.sB;
 
@@ -272,6 +269,38 @@ __global__ void __launch_bounds__(128, T == 64 ? 3 : 6) gemm_f64_kernel(GemmF64A
     }
 }
 
+template <bool A_K, bool B_K, int VEC, int T>
+__global__ void __launch_bounds__(128, T == 64 ? 3 : 6) gemm_f64_kernel(GemmF64Args p) {
+    const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
+    if (p.tri > 0 && n0 / p.tri < m0 / p.tri) return;
+    if (p.sym && n0 < m0) return;
+    gemm_tile<A_K, B_K, VEC, T>(p, m0, n0, blockIdx.z / p.S, (int)(blockIdx.z % p.S), (int)(blockIdx.x & 1));
+}
+
+// Tiles of a product that are done here after all: unit u of `list` (count of
+// them) is batch b, row block mb (128) and column block nb (64) of the sliced
+// product (ozaki_i8.cuh); trans: its rows are the columns here.
+struct GemmListed {
+    const int* count;
+    const int* list;
+    int nmb, nnb, group;
+    int trans;
+};
+template <bool A_K, bool B_K, int VEC>
+__global__ void __launch_bounds__(128, 3) gemm_f64_listed_kernel(GemmF64Args p, GemmListed l) {
+    const int halves = 2 * *l.count;
+    for (int t = blockIdx.x; t < halves; t += gridDim.x) {
+        long long b;
+        int mb, nb;
+        tile_of_unit(l.list[t >> 1], l.nmb, l.nnb, l.group, b, mb, nb);
+        const int r0 = mb * 128 + (t & 1) * 64, c0 = nb * 64;
+        const int m0 = l.trans ? c0 : r0, n0 = l.trans ? r0 : c0;
+        if (m0 >= p.M || n0 >= p.N) continue;
+        gemm_tile<A_K, B_K, VEC, 64>(p, m0, n0, b, 0, t & 1);
+        __syncthreads();   // the next tile loads into the stages read here
+    }
+}
+
 // C = alpha * (sum of S partials, in a fixed order) + beta * C; partial s of
 // batch b is the M x N matrix at ws + (b * S + s) * M * N.  64 elements x 4
 // partial lanes per CTA.  symT > 0: only the tiles on and above the diagonal
@@ -319,18 +348,53 @@ inline cudaError_t gemm_f64_launch(const GemmF64Args& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// every operand row is 16-byte aligned
+inline bool gemm_aligned16(const GemmF64Args& a) {
+    auto al16 = [](const void* ptr, int64_t ld, int64_t s, int64_t sk) {
+        return (reinterpret_cast<uintptr_t>(ptr) % 16 == 0) && (ld % 2 == 0) && (s % 2 == 0) && (sk % 2 == 0);
+    };
+    return al16(a.A, a.lda, a.sA, a.skA) && al16(a.B, a.ldb, a.sB, a.skB);
+}
+
 // One kernel with the tile T and the K splits a.S x a.per already chosen;
 // picks 16-byte copies when every operand row is 16-byte aligned.
 template <int T>
 inline cudaError_t gemm_f64_tiled(const GemmF64Args& a, bool a_k, bool b_k, cudaStream_t st) {
-    auto al16 = [](const void* ptr, int64_t ld, int64_t s, int64_t sk) {
-        return (reinterpret_cast<uintptr_t>(ptr) % 16 == 0) && (ld % 2 == 0) && (s % 2 == 0) && (sk % 2 == 0);
-    };
-    const bool v16 = al16(a.A, a.lda, a.sA, a.skA) && al16(a.B, a.ldb, a.sB, a.skB);
+    const bool v16 = gemm_aligned16(a);
     if (a_k && b_k) return v16 ? gemm_f64_launch<true, true, 2, T>(a, st) : gemm_f64_launch<true, true, 1, T>(a, st);
     if (a_k) return v16 ? gemm_f64_launch<true, false, 2, T>(a, st) : gemm_f64_launch<true, false, 1, T>(a, st);
     if (b_k) return v16 ? gemm_f64_launch<false, true, 2, T>(a, st) : gemm_f64_launch<false, true, 1, T>(a, st);
     return v16 ? gemm_f64_launch<false, false, 2, T>(a, st) : gemm_f64_launch<false, false, 1, T>(a, st);
+}
+
+// The listed tiles of a product (a.S = 1, a.per = all K steps): as many CTAs as
+// fit, which leave at once when the list is empty (about 3 us).
+template <bool A_K, bool B_K, int VEC>
+inline cudaError_t gemm_f64_listed_launch(const GemmF64Args& a, const GemmListed& l, int num_sms, cudaStream_t st) {
+    constexpr size_t smem = gemm_detail::smem_bytes<64>();
+    cudaError_t e = cudaFuncSetAttribute(gemm_f64_listed_kernel<A_K, B_K, VEC>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    gemm_f64_listed_kernel<A_K, B_K, VEC><<<3 * num_sms, 128, smem, st>>>(a, l);
+    return cudaGetLastError();
+}
+inline cudaError_t gemm_f64_listed(GemmF64Args a, bool a_k, bool b_k, const GemmListed& l, int num_sms,
+                                   cudaStream_t st) {
+    a.kb = 1;
+    a.S = 1;
+    a.per = (int)cdiv(a.K, gemm_detail::BK);
+    const bool v16 = gemm_aligned16(a);
+    if (a_k && b_k)
+        return v16 ? gemm_f64_listed_launch<true, true, 2>(a, l, num_sms, st)
+                   : gemm_f64_listed_launch<true, true, 1>(a, l, num_sms, st);
+    if (a_k)
+        return v16 ? gemm_f64_listed_launch<true, false, 2>(a, l, num_sms, st)
+                   : gemm_f64_listed_launch<true, false, 1>(a, l, num_sms, st);
+    if (b_k)
+        return v16 ? gemm_f64_listed_launch<false, true, 2>(a, l, num_sms, st)
+                   : gemm_f64_listed_launch<false, true, 1>(a, l, num_sms, st);
+    return v16 ? gemm_f64_listed_launch<false, false, 2>(a, l, num_sms, st)
+               : gemm_f64_listed_launch<false, false, 1>(a, l, num_sms, st);
 }
 
 // The product with the tile and the K split chosen by shape, on the context's

@@ -21,8 +21,11 @@
 //    below 2^-55 2^e per element, and nothing is rounded during the
 //    accumulation: against 80-bit sums of Gaussian rows the relative error is
 //    9e-17 at K = 60 and 1.3e-16 at K = 6000, where a chain of FP64 FMAs has
-//    2.5e-16 and 2.4e-15.  For the FP64 path.  K <= 21760 per accumulation;
-//    longer K runs in segments that are added in FP64.
+//    2.5e-16 and 2.4e-15.  For the FP64 path, where both rows of a product are
+//    large in the same places: the errors are relative to the row maxima, not
+//    to the terms, and slice_guard.cuh leaves the other tiles to the FP64
+//    product.  K <= 21760 per accumulation; longer K runs in segments that are
+//    added in FP64.
 //
 // Operand storage: blocks of BR rows (128 for A, the tile's column count for
 // B), each holding its 32-wide K chunks one after the other, each chunk the S
@@ -33,6 +36,8 @@
 // so a K chunk of a tile is one bulk copy per operand (a bulk copy costs its
 // issuing thread about 70 cycles whatever its size).
 #pragma once
+
+#include <cuda_bf16.h>
 
 #include <algorithm>
 
@@ -48,7 +53,9 @@ constexpr uint32_t TMEM_COLS = 512;        // W accumulators of BN columns
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 constexpr uint64_t kPaceLimitNs = 200000ull;
 constexpr int kBadExponent = 1 << 14;      // row with an infinity or NaN: its products are NaN
+constexpr int kNoExponent = (int)0x80808080;   // row of zeros (byte pattern 0x80: memset)
 constexpr int kTinyExponent = -890;        // rows below 2^-890 are sliced as zero
+constexpr int GROUP = 16;                  // row blocks per tile group (tile_of_unit)
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 
@@ -57,12 +64,14 @@ struct Mixed {
     static constexpr int FIXED = 35;       // integer = x 2^{FIXED - e}
     static constexpr int SHIFT = 42;       // product = T 2^{e_x + e_y - SHIFT}
     static constexpr long long MAXK = 26624;
+    static constexpr bool GUARD = false;   // (the caller chose this accuracy)
 };
 struct Full {
     static constexpr int S = 7, W = 8, BN = 64, STAGES = 5;
     static constexpr int FIXED = 54;
     static constexpr int SHIFT = 68;
     static constexpr long long MAXK = 21760;
+    static constexpr bool GUARD = true;    // tiles below FP64 accuracy go to the FP64 product
 };
 static_assert(5LL * 127 * 127 * Mixed::MAXK < 2147483648LL, "int32 accumulation not exact");
 // Full: the leading digit is at most 65, so the largest accumulators are the
@@ -148,6 +157,24 @@ __device__ __forceinline__ int row_exponent(unsigned long long mx) {
 }
 // the exponent used: 0 for zero or tiny rows
 __host__ __device__ inline int fixed_exponent(int e) { return e < kTinyExponent ? 0 : e; }
+// Squares of x / 2^e for the guard (slice_guard.cuh), from the high word of x;
+// square_base is what brings the row's exponents to FP32 (rows of zeros, NaN or
+// infinity: all squares 0).
+__device__ __forceinline__ int square_base(int e) {
+    return e == kNoExponent || e == kBadExponent ? 0x7fffffff : (e + 896) << 20;
+}
+__device__ __forceinline__ float square(int xhi, int base) {
+    const float f = __int_as_float(max((xhi & 0x7fffffff) - base, 0) << 3);
+    return f * f;
+}
+__device__ __forceinline__ uint32_t square_pair(int x0hi, int x1hi, int base) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(square(x0hi, base), square(x1hi, base));
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// The two 32-wide K chunks whose squares are kept with the slices: the first one
+// (graded rows are largest there) and the middle one.  Words per row.
+constexpr int SAMPLE_WORDS = 32;
+__host__ __device__ inline int sample_chunk(int nkc) { return nkc / 2; }
 // 2^{FIXED - e}, or 0 for rows whose digits are all zero
 template <class C>
 __device__ __forceinline__ double to_fixed(int e) {
@@ -164,13 +191,18 @@ __device__ __forceinline__ double to_fixed(int e) {
 // read twice.  HBM bound: 8 bytes read (16 for HELD = 0) and S written per
 // element.  N = 600 vectors (6.9 GB): 1 warp per 8 rows with 16-element lanes
 // took 18.4 ms per 30 calls, this form 5.5.
-// dst as in the header comment (blocks of BR rows); e: [batch][Rp].
+// dst as in the header comment (blocks of BR rows); [batch][Rp] each: e the raw
+// exponents (kNoExponent: a row of zeros) and, with C::GUARD, sq the sums of the
+// leading digits' squares, sample the squares of two K chunks.
 template <class C, int BR, int HELD, bool V2>
 static __global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* __restrict__ src, long long ld,
                                                                  long long src_batch, int R, int K, int Rp, int Kp,
-                                                                 int8_t* __restrict__ dst, int* __restrict__ e) {
+                                                                 int8_t* __restrict__ dst, int* __restrict__ e,
+                                                                 unsigned* __restrict__ sq,
+                                                                 uint32_t* __restrict__ sample) {
     using namespace ozaki;
     __shared__ unsigned long long smx[8][8];
+    __shared__ int ssq[8][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rr = lane & 7, qd = lane >> 3;
     const int nkc = Kp / KB;
@@ -221,9 +253,10 @@ static __global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* _
 #pragma unroll
         for (int w = 1; w < 8; ++w) mx = max(mx, smx[w][rr]);
         __syncthreads();   // smx is rewritten by the next group
-        const int ex = fixed_exponent(row_exponent(mx));
-        if (threadIdx.x < 8) e[b * Rp + r] = ex;
-        const double f = to_fixed<C>(ex);
+        const int er = mx == 0 ? kNoExponent : row_exponent(mx);
+        if (threadIdx.x < 8) e[b * Rp + r] = er;
+        const double f = to_fixed<C>(fixed_exponent(er));
+        int squares = 0;   // of the leading digits
         const bool zero = f == 0.0;   // 0 * infinity would not be 0
         int8_t* out = dst + b * ((long long)C::S * Kp * Rp) + (long long)(r0 / BR) * nkc * (C::S * BR * KB) +
                       (r0 % BR) / 8 * 256 + (qd >> 1) * 128 + rr * 16 + (qd & 1) * 8;
@@ -235,6 +268,18 @@ static __global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* _
                                  zero ? 0.0 : x[7] * f};
             digit_words<C>(a, w0);
             digit_words<C>(c, w1);
+            if (C::GUARD) {
+                squares = __dp4a((int)w1[0], (int)w1[0], __dp4a((int)w0[0], (int)w0[0], squares));
+                if (kc == 0 || kc == sample_chunk(nkc)) {
+                    const int base = square_base(er);
+                    uint32_t w[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        w[j] = square_pair(__double2hiint(x[2 * j]), __double2hiint(x[2 * j + 1]), base);
+                    *reinterpret_cast<uint4*>(sample + (b * Rp + r) * SAMPLE_WORDS + (kc ? 16 : 0) + qd * 4) =
+                        make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
             int8_t* o = out + (long long)kc * (C::S * BR * KB);
 #pragma unroll
             for (int s = 0; s < C::S; ++s) *reinterpret_cast<uint2*>(o + s * BR * KB) = make_uint2(w0[s], w1[s]);
@@ -250,6 +295,18 @@ static __global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* _
                 emit(kc, x);
             }
         }
+        if (C::GUARD) {
+            squares += __shfl_xor_sync(0xffffffffu, squares, 8);
+            squares += __shfl_xor_sync(0xffffffffu, squares, 16);
+            if (lane < 8) ssq[warp][lane] = squares;
+            __syncthreads();
+            if (threadIdx.x < 8) {
+                unsigned n = 0;
+                for (int w = 0; w < 8; ++w) n += (unsigned)ssq[w][lane];
+                sq[b * Rp + r] = n;
+            }
+            // (ssq is written again after the next group's barriers)
+        }
     }
 }
 
@@ -257,10 +314,9 @@ static __global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* _
 // strided (batch b: element (r, k) at src + b * src_batch + k * ld + r), in
 // two passes: row maxima over K splits (atomicMax of the exponent into e,
 // which starts at kNoExponent), then one thread per (row, 16-wide K group)
-// writing the S digits; the second pass treats exponents below kTinyExponent
-// as 0 and leaves the fixed value for the product.
+// writing the S digits (and, with C::GUARD, the squares as above; sq starts at
+// 0).
 namespace ozaki {
-constexpr int kNoExponent = (int)0x80808080;   // byte pattern 0x80 (memset)
 constexpr int kRowmaxSpan = 512;               // K elements per row-maximum thread
 }  // namespace ozaki
 
@@ -291,7 +347,9 @@ template <class C, int BR>
 static __global__ void __launch_bounds__(256) ozaki_slice_t_kernel(const double* __restrict__ src, long long ld,
                                                                    long long src_batch, int R, int K, int Rp, int Kp,
                                                                    const int* __restrict__ e,
-                                                                   int8_t* __restrict__ dst) {
+                                                                   int8_t* __restrict__ dst,
+                                                                   unsigned* __restrict__ sq,
+                                                                   uint32_t* __restrict__ sample) {
     using namespace ozaki;
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * 32 + lane;
@@ -299,13 +357,24 @@ static __global__ void __launch_bounds__(256) ozaki_slice_t_kernel(const double*
     const long long b = blockIdx.z;
     if (k0 >= Kp) return;
     const bool live = r < R;
-    const int ex = fixed_exponent(e[b * Rp + r]);
-    const double f = to_fixed<C>(ex);
+    const int er = e[b * Rp + r];
+    const double f = to_fixed<C>(fixed_exponent(er));
     const double* col = src + b * src_batch + r + k0 * ld;
     const int kv = live && f != 0.0 ? K - k0 : 0;   // valid K of this thread
     double x[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) x[j] = j < kv ? col[j * ld] : 0.0;
+    if (C::GUARD && (k0 < KB || (k0 >> 5) == sample_chunk(Kp / KB))) {
+        const int base = square_base(er);
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            w[j] = square_pair(__double2hiint(x[2 * j]), __double2hiint(x[2 * j + 1]), base);
+        uint4* d = reinterpret_cast<uint4*>(sample + (b * Rp + r) * SAMPLE_WORDS + (k0 < KB ? 0 : 16) +
+                                            ((k0 & 31) >> 1));
+        d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
 #pragma unroll
     for (int j = 0; j < 16; ++j) x[j] *= f;
     uint32_t word[4][C::S];
@@ -313,6 +382,12 @@ static __global__ void __launch_bounds__(256) ozaki_slice_t_kernel(const double*
     for (int q = 0; q < 4; ++q) {
         const double a[4] = {x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]};
         digit_words<C>(a, word[q]);
+    }
+    if (C::GUARD) {
+        int squares = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) squares = __dp4a((int)word[q][0], (int)word[q][0], squares);
+        if (squares > 0) atomicAdd(sq + b * Rp + r, (unsigned)squares);
     }
     int8_t* out = dst + b * ((long long)C::S * Kp * Rp) + ((long long)(r / BR) * (Kp / KB) + (k0 >> 5)) * (C::S * BR * KB) +
                   (((r % BR >> 3) * 2 + ((k0 & 31) >> 4)) << 7) + ((r & 7) << 4);
@@ -328,32 +403,18 @@ struct OzakiArgs {
     int kc0, kc1;              // chunks of this product
     int M, N;                  // valid output rows and columns
     int nmb, nnb, batch;       // row blocks (128), column blocks (BN), batches
-    int group;                 // row blocks per tile group
+    int group;                 // row blocks per tile group (tile_of_unit)
     int tri;                   // > 0: rows and columns in groups of tri; column groups before the row group skipped
     double* C; long long ldc, c_batch;
     int trans;                 // 1: C(m, n) at C + n * ldc + m
     double alpha, beta;
     int vec;                   // rows of C 32-byte aligned: 256-bit accesses
     int* pace; int pace_every, pace_slack;
+    const uint8_t* left_out;   // per unit: 1 if the FP64 product computes the tile (C::GUARD)
     int* err;
 };
 
 namespace ozaki {
-// Unit u -> (batch, row block, column block).  Tiles come in groups of `group`
-// row blocks with all column blocks, column-block-major inside a group: the
-// 148 tiles of one wave then read about 16 row blocks and 9 column blocks,
-// 0.6 MB per K chunk in place of 4 MB row-block-major, which HBM cannot feed.
-template <class Args>
-__device__ __forceinline__ void unit_tile(const Args& p, long long u, long long& b, int& mb, int& nb) {
-    const long long per = (long long)p.nmb * p.nnb;
-    b = u / per;
-    const int w = (int)(u - b * per);
-    const int pg = p.group * p.nnb, grp = w / pg;
-    const int g0 = grp * p.group, gsz = min(p.nmb - g0, p.group);
-    const int x = w - grp * pg;
-    nb = x / gsz;
-    mb = g0 + x - nb * gsz;
-}
 // 256-bit accesses of 4 doubles (32-byte aligned)
 __device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
@@ -416,7 +477,9 @@ static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(Oz
     const long long units = (long long)p.nmb * p.nnb * p.batch;
     const long long first = blockIdx.x, step = gridDim.x;
     const int nk = p.kc1 - p.kc0;
-    auto skipped = [&](int mb, int nb) { return p.tri > 0 && nb * C::BN / p.tri < mb * BM / p.tri; };
+    auto skipped = [&](long long u, int mb, int nb) {
+        return (p.tri > 0 && nb * C::BN / p.tri < mb * BM / p.tri) || (C::GUARD && p.left_out[u]);
+    };
 
     if (warp == 0) {
         // producer: lane 0 issues the copies, the whole warp paces
@@ -427,8 +490,8 @@ static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(Oz
         for (long long u = first; u < units && !stop; u += step) {
             long long b;
             int mb, nb;
-            unit_tile(p, u, b, mb, nb);
-            if (skipped(mb, nb)) continue;
+            tile_of_unit(u, p.nmb, p.nnb, p.group, b, mb, nb);
+            if (skipped(u, mb, nb)) continue;
             const int8_t* a0 = p.A + b * p.a_batch + ((long long)mb * p.nkc + p.kc0) * (C::S * (long long)D::SLAB_A);
             const int8_t* b0 = p.B + b * p.b_batch + ((long long)nb * p.nkc + p.kc0) * (C::S * (long long)D::SLAB_B);
             for (int kc = 0; kc < nk; ++kc) {
@@ -484,8 +547,8 @@ static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(Oz
             for (long long u = first; u < units && !*abort_flag; u += step) {
                 long long b;
                 int mb, nb;
-                unit_tile(p, u, b, mb, nb);
-                if (skipped(mb, nb)) continue;
+                tile_of_unit(u, p.nmb, p.nnb, p.group, b, mb, nb);
+                if (skipped(u, mb, nb)) continue;
                 if (!mbar_wait_bounded(tmem_empty, acc_phase ^ 1, kWaitLimitNs)) {
                     atomicExch(p.err, 32);
                     *abort_flag = 1;
@@ -556,8 +619,8 @@ static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(Oz
             if (*abort_flag) break;
             long long b;
             int mb, nb;
-            unit_tile(p, u, b, mb, nb);
-            if (skipped(mb, nb)) continue;
+            tile_of_unit(u, p.nmb, p.nnb, p.group, b, mb, nb);
+            if (skipped(u, mb, nb)) continue;
             const int m = mb * BM + q * 32 + lane;   // this thread's TMEM row
             const bool mrow = m < p.M;
             const int ea = mrow ? fixed_exponent(p.eA[b * p.ea_batch + m]) : 0;
@@ -655,10 +718,20 @@ static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(Oz
 // (padded to Kp), `batch` copies.
 struct OzakiOperand {
     int8_t* q = nullptr;
-    int* e = nullptr;
+    int* e = nullptr;           // row exponents and, behind them, what the guard needs (row_bytes)
     long long R = 0, Rp = 0, K = 0, Kp = 0;
     int BR = 0;
     int batch = 1;
+    // the matrices it was sliced from: element (r, k) of batch b at
+    // src + b * sb + r * ld + k, or (t) src + b * sb + k * ld + r
+    const double* src = nullptr;
+    long long ld = 0, sb = 0;
+    bool t = false;
+    unsigned* sq() const { return reinterpret_cast<unsigned*>(e + Rp * batch); }
+    uint32_t* sample() const { return reinterpret_cast<uint32_t*>(e + 2 * Rp * batch); }
+    size_t row_bytes(bool guard) const {
+        return sizeof(int) * (size_t)(Rp * batch) * (guard ? 2 + ozaki::SAMPLE_WORDS : 1);
+    }
 };
 
 inline OzakiOperand ozaki_operand(long long R, long long K, int tile, int batch) {
@@ -684,10 +757,12 @@ inline cudaError_t ozaki_slice_br(const double* src, long long ld, long long src
     do {                                                                                                            \
         if (v2)                                                                                                     \
             ozaki_slice_kernel<C, BR, H, true><<<grid, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K,      \
-                                                                     (int)op.Rp, (int)op.Kp, op.q, op.e);           \
+                                                                     (int)op.Rp, (int)op.Kp, op.q, op.e, op.sq(),   \
+                                                                     op.sample());                                  \
         else                                                                                                        \
             ozaki_slice_kernel<C, BR, H, false><<<grid, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K,     \
-                                                                      (int)op.Rp, (int)op.Kp, op.q, op.e);          \
+                                                                      (int)op.Rp, (int)op.Kp, op.q, op.e, op.sq(),  \
+                                                                      op.sample());                                 \
     } while (0)
     if (nkc <= 16)
         MSHQC_SLICE(2);
@@ -701,8 +776,9 @@ inline cudaError_t ozaki_slice_br(const double* src, long long ld, long long src
     return cudaGetLastError();
 }
 template <class C>
-inline cudaError_t ozaki_slice(const double* src, long long ld, long long src_batch, const OzakiOperand& op,
-                               int num_sms, cudaStream_t st) {
+inline cudaError_t ozaki_slice(const double* src, long long ld, long long src_batch, OzakiOperand& op, int num_sms,
+                               cudaStream_t st) {
+    op.src = src;  op.ld = ld;  op.sb = src_batch;  op.t = false;
     if (op.Rp <= 0 || op.batch <= 0) return cudaSuccess;
     return op.BR == ozaki::BM ? ozaki_slice_br<C, ozaki::BM>(src, ld, src_batch, op, num_sms, st)
                               : ozaki_slice_br<C, C::BN>(src, ld, src_batch, op, num_sms, st);
@@ -710,11 +786,16 @@ inline cudaError_t ozaki_slice(const double* src, long long ld, long long src_ba
 
 // Transposed source: element (r, k) of batch b at src + b * src_batch + k * ld + r.
 template <class C>
-inline cudaError_t ozaki_slice_t(const double* src, long long ld, long long src_batch, const OzakiOperand& op,
+inline cudaError_t ozaki_slice_t(const double* src, long long ld, long long src_batch, OzakiOperand& op,
                                  cudaStream_t st) {
     using namespace ozaki;
+    op.src = src;  op.ld = ld;  op.sb = src_batch;  op.t = true;
     cudaError_t err = cudaMemsetAsync(op.e, 0x80, sizeof(int) * (size_t)(op.Rp * op.batch), st);
     if (err != cudaSuccess) return err;
+    if (C::GUARD) {
+        err = cudaMemsetAsync(op.sq(), 0, sizeof(unsigned) * (size_t)(op.Rp * op.batch), st);
+        if (err != cudaSuccess) return err;
+    }
     if (op.R > 0 && op.K > 0) {
         dim3 g1((unsigned)((op.R + 255) / 256), (unsigned)((op.K + kRowmaxSpan - 1) / kRowmaxSpan),
                 (unsigned)op.batch);
@@ -725,10 +806,10 @@ inline cudaError_t ozaki_slice_t(const double* src, long long ld, long long src_
     dim3 g2((unsigned)(op.Rp / 32), (unsigned)((op.Kp + 127) / 128), (unsigned)op.batch);
     if (op.BR == BM)
         ozaki_slice_t_kernel<C, BM><<<g2, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K, (int)op.Rp,
-                                                        (int)op.Kp, op.e, op.q);
+                                                        (int)op.Kp, op.e, op.q, op.sq(), op.sample());
     else
         ozaki_slice_t_kernel<C, C::BN><<<g2, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K, (int)op.Rp,
-                                                           (int)op.Kp, op.e, op.q);
+                                                           (int)op.Kp, op.e, op.q, op.sq(), op.sample());
     return cudaGetLastError();
 }
 
@@ -740,6 +821,7 @@ struct OzakiOpts {
     bool trans = false;
     int tri = 0;
     int* pace = nullptr;
+    const uint8_t* left_out = nullptr;
 };
 
 // C[b] = alpha * A[b] B[b]^T + beta * C[b] over the batches.  K beyond what one
@@ -754,7 +836,7 @@ inline cudaError_t ozaki_gemm(const OzakiOperand& A, const OzakiOperand& B, doub
     if (e != cudaSuccess) return e;
     const int batch = o.a_shared ? B.batch : A.batch;
     if (A.Kp != B.Kp || A.Kp <= 0 || A.BR != BM || B.BR != C::BN || A.Rp % BM != 0 || B.Rp % C::BN != 0 ||
-        (!o.a_shared && !o.b_shared && A.batch != B.batch) || (o.a_shared && o.b_shared && batch != 1))
+        (C::GUARD && !o.left_out) || (!o.a_shared && !o.b_shared && A.batch != B.batch) || (o.a_shared && o.b_shared && batch != 1))
         return cudaErrorInvalidValue;
     OzakiArgs p{};
     p.A = A.q;  p.a_batch = o.a_shared ? 0 : (long long)operand_bytes<C>(A.Rp, A.Kp);
@@ -764,7 +846,8 @@ inline cudaError_t ozaki_gemm(const OzakiOperand& A, const OzakiOperand& B, doub
     p.nkc = (int)(A.Kp / KB);
     p.M = (int)A.R;  p.N = (int)B.R;
     p.nmb = (int)(A.Rp / BM);  p.nnb = (int)(B.Rp / C::BN);  p.batch = batch;
-    p.group = 16;
+    p.group = GROUP;
+    p.left_out = o.left_out;
     p.tri = o.tri;
     p.C = Cp;  p.ldc = ldc;  p.c_batch = c_batch;
     p.trans = o.trans ? 1 : 0;
