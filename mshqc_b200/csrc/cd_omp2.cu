@@ -585,38 +585,74 @@ __global__ void __launch_bounds__(1024) density_factor_kernel(const double* __re
     if (tid == 0) *rank = k;
 }
 
-// bits[0] = max |P|, bits[1] = max |P - sum_k X[k] X[k]^T| (bit patterns of
-// non-negative doubles order like unsigned integers; NaN ends up largest)
+// *bad = 1 when the factor misses P: in some 32 x 32 tile of it,
+//   max |P - sum_k X[k] X[k]^T| > (8 + r / 4) 2^-52 max sum_k |X[k]| |X[k]^T|.
+// Tiles are held to their own size, so parts of P far below the rest keep their
+// relative accuracy (against the largest element of P alone, a block 10^-16 of
+// it was left out); the allowance is below the N 2^-53 of the chains of P L^Q
+// for r <= N / 4, and twice what densities formed in FP64 need (0.4 ... 0.8 of
+// (4 + r / 8) 2^-52, N = 96 ... 500).  Grid: tiles.  A NaN compares as a miss.
 __global__ void __launch_bounds__(256) density_residual_kernel(const double* __restrict__ P, int64_t N,
                                                                const double* __restrict__ X,
                                                                const int* __restrict__ rank,
-                                                               unsigned long long* __restrict__ bits) {
-    const int r = *rank;
-    unsigned long long mp = 0, mr = 0;
-    for (int64_t t = blockIdx.x * 256LL + threadIdx.x; t < N * N; t += (int64_t)gridDim.x * 256) {
-        const int64_t i = t / N, j = t % N;
-        double d = P[t];
-        mp = max(mp, (unsigned long long)__double_as_longlong(fabs(d)));
-        for (int k = 0; k < r; ++k) d = fma(-X[(int64_t)k * N + i], X[(int64_t)k * N + j], d);
-        mr = max(mr, (unsigned long long)__double_as_longlong(fabs(d)));
+                                                               unsigned long long* __restrict__ bad) {
+    __shared__ double sr[8], ss[8];
+    const int r = *rank, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    // columns and rows beyond N repeat the last ones
+    const int64_t j = min((int64_t)blockIdx.x * 32 + tx, N - 1);
+    int64_t i[4];
+    double d[4], sum[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        i[c] = min((int64_t)blockIdx.y * 32 + ty + 8 * c, N - 1);
+        d[c] = P[i[c] * N + j];
+        sum[c] = 0.0;
+    }
+    for (int k = 0; k < r; ++k) {
+        const double* x = X + (int64_t)k * N;
+        const double y = x[j];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double z = x[i[c]];
+            d[c] = fma(-z, y, d[c]);
+            sum[c] = fma(fabs(z), fabs(y), sum[c]);
+        }
+    }
+    double mr = 0.0, ms = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (!(mr >= fabs(d[c]))) mr = mr != mr ? mr : fabs(d[c]);   // (a NaN is taken and kept)
+        ms = fmax(ms, sum[c]);
     }
 #pragma unroll
     for (int off = 16; off; off >>= 1) {
-        mp = max(mp, __shfl_xor_sync(0xffffffffu, mp, off));
-        mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, off));
+        const double o = __shfl_xor_sync(0xffffffffu, mr, off);
+        if (!(mr >= o)) mr = mr != mr ? mr : o;
+        ms = fmax(ms, __shfl_xor_sync(0xffffffffu, ms, off));
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(bits, mp);
-        atomicMax(bits + 1, mr);
+    if (tx == 0) {
+        sr[ty] = mr;
+        ss[ty] = ms;
     }
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int w = 1; w < 8; ++w) {
+        if (!(mr >= sr[w])) mr = mr != mr ? mr : sr[w];
+        ms = fmax(ms, ss[w]);
+    }
+    if (!(mr <= (8.0 + r / 4.0) * 0x1p-52 * ms)) *bad = 1;
 }
 
 // Factors of the densities of an exchange build in ctx->dens_x (X[s] there,
 // rank[s] vectors each, the two spins' one after the other), or rank[s] = 0
-// where P[s] is not represented by at most N / 4 vectors to rounding: max |P - X^T X| <= (4 + r / 8) 2^-52 max |P|,
-// checked on every element (so an indefinite or unsymmetric P is refused too).
-// The exchange then takes 4 M N^2 r operations instead of 4 M N^3.
-constexpr int64_t kDensityFactorMinN = 96;   // below, the full products are as fast as finding the factors
+// where P[s] is not represented by at most N / 4 vectors to rounding
+// (density_residual_kernel looks at every element, so an indefinite or
+// unsymmetric P is refused too).  The exchange then takes 4 M N^2 r operations
+// instead of 4 M N^3.
+// UHF builds of N / 10 electrons, whole calls: N = 96 0.38 ms with factors, 0.55
+// without, N = 64 0.32 without, nearly all of it the host's copies.  A density of
+// full rank pays for N / 4 steps in vain: 1.1 of 34.7 ms at N = 400.
+constexpr int64_t kDensityFactorMinN = 96;
 int density_factors(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], const double* X[2], int rank[2]) {
     const int64_t N = ctx->N;
     const int rmax = (int)(N / 4);
@@ -625,15 +661,15 @@ int density_factors(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], cons
     if (N < kDensityFactorMinN) return MSHQC_CD_OK;
     CD_ALLOC(ctx->dens_x, sizeof(double) * (size_t)((2 * (rmax + 1) + rmax) * N + 8), false);
     double* base = ctx->dens_x.as<double>();
-    unsigned long long* tail = reinterpret_cast<unsigned long long*>(base + 2 * (rmax + 1) * N);   // [spin][P, R, rank]
+    unsigned long long* tail = reinterpret_cast<unsigned long long*>(base + 2 * (rmax + 1) * N);   // [spin][bad, unused, rank]
     CD_CUDA(cudaMemsetAsync(tail, 0, 6 * sizeof(unsigned long long), ctx->stream));
     for (int s = 0; s < nspin; ++s) {
         double* x = base + (int64_t)s * (rmax + 1) * N;
         int* rk = reinterpret_cast<int*>(tail + 3 * s + 2);
         density_factor_kernel<<<1, 1024, 0, ctx->stream>>>(P[s], N, rmax, x, x + (int64_t)rmax * N, rk);
         CD_CUDA(cudaGetLastError());
-        density_residual_kernel<<<(unsigned)std::min<int64_t>(cdiv(N * N, 256), 8LL * ctx->num_sms), 256, 0,
-                                  ctx->stream>>>(P[s], N, x, rk, tail + 3 * s);
+        const unsigned nt = (unsigned)cdiv(N, 32);
+        density_residual_kernel<<<dim3(nt, nt), 256, 0, ctx->stream>>>(P[s], N, x, rk, tail + 3 * s);
         CD_CUDA(cudaGetLastError());
         ctx->launches += 2;
         X[s] = x;
@@ -642,11 +678,7 @@ int density_factors(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], cons
     CD_CUDA(cudaMemcpyAsync(h, tail, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     CD_CUDA(cudaStreamSynchronize(ctx->stream));
     for (int s = 0; s < nspin; ++s) {
-        double mp, mr;
-        std::memcpy(&mp, &h[3 * s], sizeof(double));
-        std::memcpy(&mr, &h[3 * s + 1], sizeof(double));
-        const int r = (int)(h[3 * s + 2] & 0xffffffffull);
-        if (r > 0 && mr <= (4.0 + r / 8.0) * 0x1p-52 * mp) rank[s] = r;
+        if (h[3 * s] == 0) rank[s] = (int)(h[3 * s + 2] & 0xffffffffull);
     }
     if (rank[0] > 0 && rank[1] > 0) {
         // the second spin's rows right after the first's (never overlapping: rank <= N / 4)
