@@ -576,7 +576,7 @@ int mshqc_cd_mp2_energy(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_ene
     if (precision != MSHQC_CD_FP64 && precision != MSHQC_CD_FP16X3)
         return set_error(MSHQC_CD_ERR_ARG, "unknown precision");
     DeviceGuard g(ctx->device);
-    return run_energy(ctx, kind, precision, out);
+    return one_spin_retry(ctx, [&] { return run_energy(ctx, kind, precision, out); });
 }
 
 int mshqc_cd_pair_energies(mshqc_cd_ctx* ctx, int block, double* out, int where) {
@@ -602,7 +602,8 @@ int mshqc_cd_mp2_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_e
     if (precision != MSHQC_CD_FP64 && precision != MSHQC_CD_FP16X3)
         return set_error(MSHQC_CD_ERR_ARG, "unknown precision");
     DeviceGuard g(ctx->device);
-    return run_gradient(ctx, kind, precision, e_out, dC_a, dC_b, deps_a, deps_b, where);
+    return one_spin_retry(
+        ctx, [&] { return run_gradient(ctx, kind, precision, e_out, dC_a, dC_b, deps_a, deps_b, where); });
 }
 
 }  // extern "C"

@@ -91,6 +91,11 @@ struct mshqc_cd_ctx {
     } Yr[2];
     mshqc_cd::DevBuf cpack;         // occupied orbitals of both spins, one after the other
     mshqc_cd::DevBuf occ_parts;     // dE/dC_occ of both spins in one product
+    // Both spins' half-transformed vectors are held at once where they fit
+    // (both_spins_fit; both_used: they were); a call that then runs out of memory is
+    // done again with one spin's at a time (one_spin_retry, one_spin), and the
+    // calls after it ask for twice the free memory (cautious).
+    bool both_used = false, one_spin = false, cautious = false;
     bool call_open = false;         // a call that began has not finished (see begin_call)
     int L_sym = -1;                 // stored vectors symmetric to the bit (-1: not looked at yet)
     mshqc_cd::DevBuf scratch;       // uploads / unpacking
@@ -150,6 +155,7 @@ struct mshqc_cd_ctx {
     void invalidate_all() {
         invalidate_derived();
         L_sym = -1;
+        both_used = cautious = false;
         for (auto& p : pair_energy) p.clear();
     }
     size_t held_bytes() const {
@@ -162,6 +168,26 @@ struct mshqc_cd_ctx {
         for (const auto& g : gam) b += g.bytes;
         for (const auto& g : grad) b += g.bytes;
         return b;
+    }
+    // what only products use, between them (int8 slices, split-K partials);
+    // false: nothing held
+    bool release_slices() {
+        bool any = false;
+        for (mshqc_cd::DevBuf* b : {&oz_a, &oz_b, &oz_p, &oz_ea, &oz_eb, &oz_tiles, &gemm_ws}) {
+            any = any || b->p;
+            b->release();
+        }
+        return any;
+    }
+    // what a call forms again when it needs it (scratch holds OMP2's densities)
+    void release_workspaces() {
+        for (mshqc_cd::DevBuf* b : {&Y, &cpack, &occ_parts, &partial, &gemm_ws, &amp, &ampT, &BT, &BT_b,
+                                    &dsum, &amp_chunks, &W, &diag_os, &Zt, &oz_a, &oz_b, &oz_ea, &oz_eb, &oz_tiles,
+                                    &oz_p, &gam[0], &gam[1]})
+            b->release();
+        for (auto& s : spin)
+            for (mshqc_cd::DevBuf* b : {&s.B64, &s.B16, &s.expo, &s.diag}) b->release();
+        invalidate_derived();
     }
     void release_all() {
         for (auto& e : ev_pool)
@@ -243,6 +269,18 @@ int check_finite_device(mshqc_cd_ctx* ctx, const double* x, int64_t n, const cha
                                                      " bytes failed");                     \
         if (_e != cudaSuccess) return cuda_error(_e, "workspace");                         \
     } while (0)
+// the same where no operand is waiting for its product: where the memory is
+// short, what earlier products left goes first
+#define CD_ALLOC_FIRST(buf, nbytes, zero)                                                     \
+    do {                                                                                      \
+        const cudaError_t _f = (buf).reserve((nbytes), (zero), ctx->stream);                  \
+        if (_f == cudaErrorMemoryAllocation) {                                                \
+            ctx->release_slices();                                                            \
+            CD_ALLOC(buf, nbytes, zero);                                                      \
+        } else if (_f != cudaSuccess) {                                                       \
+            return cuda_error(_f, "workspace");                                               \
+        }                                                                                     \
+    } while (0)
 #define CD_RC(x)             \
     do {                     \
         int _rc = (x);       \
@@ -269,6 +307,22 @@ int begin_call(mshqc_cd_ctx* ctx);
 // bytes from dev to the pinned buffer behind the status (*extra_host).
 int finish_call(mshqc_cd_ctx* ctx, CallStatus* st = nullptr, const void* dev = nullptr, size_t extra = 0,
                 const void** extra_host = nullptr);
+
+// Runs a call (begin_call ... finish_call), and once more with one spin's
+// half-transformed vectors at a time if both were held and it ran out of memory.
+template <class F>
+int one_spin_retry(mshqc_cd_ctx* ctx, F call) {
+    const int rc = call();
+    // (ranks that share the transforms make the same collective calls: no second run)
+    if (rc != MSHQC_CD_ERR_ALLOC || !ctx->both_used || (ctx->coll_set && ctx->part_size > 1)) return rc;
+    cudaStreamSynchronize(ctx->stream);
+    ctx->release_workspaces();
+    ctx->both_used = false;
+    ctx->one_spin = ctx->cautious = true;
+    const int again = call();
+    ctx->one_spin = false;
+    return again;
+}
 
 // implemented in cd_mp2.cu
 // layout: of the fixed-point operands of a mixed-precision request

@@ -297,7 +297,7 @@ bool fp64_slices(double flops, double min_flops, int64_t reuse) {
 // does not hold them the FP64 products run instead.
 bool no_room(mshqc_cd_ctx* ctx, int rc) {
     if (rc != MSHQC_CD_ERR_ALLOC) return false;
-    for (DevBuf* b : {&ctx->oz_a, &ctx->oz_b, &ctx->oz_p, &ctx->oz_ea, &ctx->oz_eb, &ctx->oz_tiles}) b->release();
+    ctx->release_slices();
     return true;
 }
 
@@ -333,8 +333,9 @@ int first_half(mshqc_cd_ctx* ctx, int nsp, const int* spins, const int64_t* lo, 
     const int64_t N = ctx->N, M = ctx->M;
     int64_t rows = 0;
     ctx->Yr[0].ok = ctx->Yr[1].ok = false;
+    ctx->both_used |= nsp == 2;
     for (int k = 0; k < nsp; ++k) rows += std::max<int64_t>(0, hi[k] - lo[k]);
-    CD_ALLOC(ctx->Y, sizeof(double) * (size_t)std::max<int64_t>(1, rows) * M * N, false);
+    CD_ALLOC_FIRST(ctx->Y, sizeof(double) * (size_t)std::max<int64_t>(1, rows) * M * N, false);
     int64_t r = 0;
     for (int k = 0; k < nsp; ++k) {
         auto& y = ctx->Yr[spins[k]];
@@ -414,7 +415,7 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
         shard_range(ctx, s.nocc, &lo[k], &hi[k]);
         s.vp = round_up(N - s.nocc, 64);
         s.invalidate();   // run_transforms marks B valid, with its last launch queued
-        CD_ALLOC(s.B64, sizeof(double) * (size_t)b_rows(ctx, s.nocc) * s.vp * Mp, true);
+        CD_ALLOC_FIRST(s.B64, sizeof(double) * (size_t)b_rows(ctx, s.nocc) * s.vp * Mp, true);
         s.B64_prec = i8 ? MSHQC_CD_FP16X3 : MSHQC_CD_FP64;
     }
     CD_RC(first_half(ctx, nsp, spins, lo, hi, i8));
@@ -447,8 +448,13 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
 }
 
 // Whether the half-transformed vectors of both spins may be held at once: the
-// buffer already has the room, or it is at most a quarter of the free memory.
+// buffer already has the room, or it is at most a quarter of the free memory (an
+// eighth where an earlier call ran out of memory or this one cannot be done again,
+// one_spin_retry: the buffers formed after it are about three times its size, and
+// the staging needs its part).
 int both_spins_fit(mshqc_cd_ctx* ctx, bool* yes) {
+    *yes = false;
+    if (ctx->one_spin) return MSHQC_CD_OK;
     int64_t rows = 0;
     for (int s = 0; s < 2; ++s) {
         int64_t lo, hi;
@@ -460,7 +466,7 @@ int both_spins_fit(mshqc_cd_ctx* ctx, bool* yes) {
     if (*yes) return MSHQC_CD_OK;
     size_t free_b = 0, total_b = 0;
     CD_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    *yes = need <= (free_b + ctx->Y.bytes) / 4;
+    *yes = need <= (free_b + ctx->Y.bytes) / (sharded(ctx) || ctx->cautious ? 8 : 4);
     return MSHQC_CD_OK;
 }
 
@@ -574,7 +580,7 @@ int pair_pass_f64(mshqc_cd_ctx* ctx, const PairPass& pp) {
     }
     const int npairs = pp.npairs, nblocks = (int)block_count(mode, nbx, nby);
     const int64_t units = (int64_t)npairs * nblocks;
-    CD_ALLOC(ctx->partial, sizeof(double) * units * 2, false);
+    CD_ALLOC_FIRST(ctx->partial, sizeof(double) * units * 2, false);
     PairF64Args a{};
     a.X = X.B64.as<double>();
     a.Y = Y.B64.as<double>();
@@ -628,8 +634,8 @@ int pair_pass_f64_staged(mshqc_cd_ctx* ctx, const PairPass& pp) {
     // 4 CTAs a pair where the pairs alone do not fill the GPU several times
     const int nch = npairs < 32 * ctx->num_sms ? 4 : 1;
     const int64_t units = (int64_t)npairs * nch;
-    CD_ALLOC(ctx->W, (size_t)(bI * bJ * per_row), false);
-    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)units * 2, false);
+    CD_ALLOC_FIRST(ctx->W, (size_t)(bI * bJ * per_row), false);
+    CD_ALLOC_FIRST(ctx->partial, sizeof(double) * (size_t)units * 2, false);
     begin_stage(ctx, ST_PAIR);
     for (int64_t I0 = 0; I0 < ox; I0 += bI) {
         const int64_t nI = std::min(bI, ox - I0);
@@ -676,9 +682,9 @@ int split_fixed(mshqc_cd_ctx* ctx, int spin, int layout) {
     const int64_t rows = pair_layout ? tc_rows(v) : round_up(v, 32), nqc = Mp / 16;
     const int64_t total = round_up(o * rows, 256);
     const size_t n = (size_t)(nqc * total * 16);   // elements of hi, as many of lo
-    CD_ALLOC(s.B16, 2 * n * sizeof(uint16_t), false);
-    CD_ALLOC(s.expo, sizeof(int) * o * rows, true);
-    CD_ALLOC(s.diag, sizeof(double) * o * rows, true);
+    CD_ALLOC_FIRST(s.B16, 2 * n * sizeof(uint16_t), false);
+    CD_ALLOC_FIRST(s.expo, sizeof(int) * o * rows, true);
+    CD_ALLOC_FIRST(s.diag, sizeof(double) * o * rows, true);
     // (a spin is split once per call: its slots in the status are zero)
     unsigned long long* norms = ctx->status.as<CallStatus>()->norms[spin];
     s.vp16 = rows;
@@ -717,8 +723,8 @@ int opposite_spin_diag(mshqc_cd_ctx* ctx) {
     const int64_t oa = A.nocc, va = ctx->N - A.nocc, rows = A.vp16;
     const int o2 = (int)std::min(A.nocc, B.nocc);
     const int v2 = (int)std::min(ctx->N - A.nocc, ctx->N - B.nocc);
-    CD_ALLOC(ctx->diag_os, sizeof(double) * std::max<int64_t>(1, (int64_t)o2 * rows), true);
-    CD_ALLOC(ctx->scratch, sizeof(double) * (size_t)(oa * rows * 2), false);
+    CD_ALLOC_FIRST(ctx->diag_os, sizeof(double) * std::max<int64_t>(1, (int64_t)o2 * rows), true);
+    CD_ALLOC_FIRST(ctx->scratch, sizeof(double) * (size_t)(oa * rows * 2), false);
     double* tmp = ctx->scratch.as<double>();
     int* etmp = reinterpret_cast<int*>(tmp + oa * rows);
     const int64_t warps = oa * rows;
@@ -762,7 +768,7 @@ int pair_pass_tc(mshqc_cd_ctx* ctx, const PairPass& pp) {
     const int nbx = (int)cdiv(vx, 128), nby = (int)cdiv(vy, 128);
     const int npairs = pp.npairs, nblocks = (int)block_count(mode, nbx, nby);
     const int64_t units = (int64_t)npairs * nblocks;
-    CD_ALLOC(ctx->partial, sizeof(double) * units * 2, false);
+    CD_ALLOC_FIRST(ctx->partial, sizeof(double) * units * 2, false);
     if (mode == PAIR_OPPOSITE_SPIN) {
         begin_stage(ctx, ST_SPLIT);
         CD_RC(opposite_spin_diag(ctx));
@@ -1104,7 +1110,7 @@ int occupied_part(mshqc_cd_ctx* ctx, int nsp, const int* spins, double scale, do
     if (!i8) {
         double* out = dC[0] + ctx->Yr[spins[0]].lo * N;
         if (nsp == 2) {
-            CD_ALLOC(ctx->occ_parts, sizeof(double) * (size_t)(rows * N), false);
+            CD_ALLOC_FIRST(ctx->occ_parts, sizeof(double) * (size_t)(rows * N), false);
             out = ctx->occ_parts.as<double>();
         }
         for (int64_t Q0 = 0; Q0 < M; Q0 += qc) {
@@ -1247,7 +1253,7 @@ int make_bt(mshqc_cd_ctx* ctx, int spin, DevBuf& buf, int64_t RQ, const uint16_t
     SpinState& s = ctx->spin[spin];
     const BwdDims d = bwd_dims(ctx, spin);
     const size_t nbt = (size_t)RQ * d.o * d.VR;
-    CD_ALLOC(buf, 2 * nbt * sizeof(uint16_t), false);
+    CD_ALLOC_FIRST(buf, 2 * nbt * sizeof(uint16_t), false);
     const int64_t threads = (d.o * d.VR / 16) * RQ * 2;
     const int blocks = (int)std::min<int64_t>(cdiv(threads, 256), (int64_t)ctx->num_sms * 16);
     begin_stage(ctx, ST_SPLIT);
@@ -1346,14 +1352,14 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
     int64_t bI, bJ;
     tc_block_sizes(ctx, dx.o, dy.o, dx.VR, dy.VR, dy.VS, kSym, budget, &bI, &bJ);
     const size_t n_amp = sizeof(uint16_t) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VR);
-    CD_ALLOC(ctx->amp, 2 * n_amp, false);   // hi and lo
-    CD_ALLOC(ctx->ampT, 2 * n_amp, false);
+    CD_ALLOC_FIRST(ctx->amp, 2 * n_amp, false);   // hi and lo
+    CD_ALLOC_FIRST(ctx->ampT, 2 * n_amp, false);
     // (the size the block sizes are reckoned with; the packed rows take less of it)
-    CD_ALLOC(ctx->W, sizeof(float) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VS), false);
+    CD_ALLOC_FIRST(ctx->W, sizeof(float) * (size_t)(bI * dx.VR) * (size_t)(bJ * dy.VS), false);
     const int64_t npairs = dx.o * dy.o;
     // (zero where a mirrored pair stands in)
     const int64_t nrow = kSym ? 0 : dx.RS;
-    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (nrow + dy.RS + 1)), true);
+    CD_ALLOC_FIRST(ctx->dsum, sizeof(double) * (size_t)(npairs * (nrow + dy.RS + 1)), true);
     CD_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)npairs, ctx->stream));
     double* pcol = ctx->dsum.as<double>();
     double* pocc = pcol + npairs * dy.RS;
@@ -1429,7 +1435,7 @@ int tc_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, const uint16_t* btx, con
             e.nchunk = nch;
             if (nch > 1) {
                 const size_t per = (size_t)npl * nch;
-                CD_ALLOC(ctx->amp_chunks, sizeof(double) * per * ((size_t)dy.RS + 2), false);
+                CD_ALLOC_FIRST(ctx->amp_chunks, sizeof(double) * per * ((size_t)dy.RS + 2), false);
                 e.cpcol = ctx->amp_chunks.as<double>();
                 e.cpart = e.cpcol + per * dy.RS;
                 e.cpocc = e.cpart + per;
@@ -1480,12 +1486,12 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
     int64_t bI, bJ;
     f64_block_sizes(ctx, dx.o, dy.o, dx.vp, dy.vp, kSym, budget, &bI, &bJ);
     const size_t n_stage = sizeof(double) * (size_t)(bI * dx.vp) * (size_t)(bJ * dy.vp);
-    CD_ALLOC(ctx->W, n_stage, false);
-    CD_ALLOC(ctx->amp, n_stage, false);
+    CD_ALLOC_FIRST(ctx->W, n_stage, false);
+    CD_ALLOC_FIRST(ctx->amp, n_stage, false);
     const int64_t npairs = dx.o * dy.o;
     // (zero where a mirrored pair stands in)
     const int64_t nrow = kSym ? 0 : dx.vp;
-    CD_ALLOC(ctx->dsum, sizeof(double) * (size_t)(npairs * (nrow + dy.vp + 1)), true);
+    CD_ALLOC_FIRST(ctx->dsum, sizeof(double) * (size_t)(npairs * (nrow + dy.vp + 1)), true);
     CD_CUDA(cudaMemsetAsync(partial, 0, sizeof(double) * (size_t)npairs, ctx->stream));
     double* pcol = ctx->dsum.as<double>();
     double* pocc = pcol + npairs * dy.vp;
@@ -1541,7 +1547,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
             e.nchunk = nch;
             if (nch > 1) {
                 const size_t per = (size_t)npl * nch;
-                CD_ALLOC(ctx->amp_chunks, sizeof(double) * per * ((size_t)dy.vp + 2), false);
+                CD_ALLOC_FIRST(ctx->amp_chunks, sizeof(double) * per * ((size_t)dy.vp + 2), false);
                 e.cpcol = ctx->amp_chunks.as<double>();
                 e.cpart = e.cpcol + per * dy.vp;
                 e.cpocc = e.cpart + per;
@@ -1570,7 +1576,7 @@ int f64_backward_pass(mshqc_cd_ctx* ctx, int sx, int sy, double* deps_x, double*
                     todo_y = no_room(ctx, rc);
                     if (!todo_y) CD_RC(rc);
                 }
-                CD_ALLOC(ctx->W, n_stage, false);
+                CD_ALLOC_FIRST(ctx->W, n_stage, false);
                 S = ctx->W.as<double>();
             }
             if (todo_x) {
@@ -1617,9 +1623,9 @@ int gradient_restricted(mshqc_cd_ctx* ctx, int precision, double* dC, double* de
     const bool tc = precision == MSHQC_CD_FP16X3;
     const uint16_t* bt = nullptr;
     if (tc) CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bt));
-    CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, o) * s.vp * Mp, true);
+    CD_ALLOC_FIRST(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, o) * s.vp * Mp, true);
     CD_CUDA(cudaMemsetAsync(deps, 0, sizeof(double) * N, ctx->stream));
-    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(o * o), false);   // one energy per pair (i, j)
+    CD_ALLOC_FIRST(ctx->partial, sizeof(double) * (size_t)(o * o), false);   // one energy per pair (i, j)
     double* part = ctx->partial.as<double>();
     if (tc)
         CD_RC(tc_backward_pass<AMP_RESTRICTED>(ctx, 0, 0, bt, bt, RQ, deps, deps, part));
@@ -1645,11 +1651,11 @@ int gradient_unrestricted(mshqc_cd_ctx* ctx, int precision, double* const dC[2],
         CD_RC(make_bt(ctx, 0, ctx->BT, RQ, &bta));
         CD_RC(make_bt(ctx, 1, ctx->BT_b, RQ, &btb));
     }
-    CD_ALLOC(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, da.o) * da.vp * Mp, true);
-    CD_ALLOC(ctx->gam[1], sizeof(double) * (size_t)b_rows(ctx, db.o) * db.vp * Mp, true);
+    CD_ALLOC_FIRST(ctx->gam[0], sizeof(double) * (size_t)b_rows(ctx, da.o) * da.vp * Mp, true);
+    CD_ALLOC_FIRST(ctx->gam[1], sizeof(double) * (size_t)b_rows(ctx, db.o) * db.vp * Mp, true);
     for (int s = 0; s < 2; ++s) CD_CUDA(cudaMemsetAsync(deps[s], 0, sizeof(double) * N, ctx->stream));
     const int64_t n0 = da.o * da.o, n1 = db.o * db.o, n2 = da.o * db.o;   // one energy per pair
-    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(n0 + n1 + n2), false);
+    CD_ALLOC_FIRST(ctx->partial, sizeof(double) * (size_t)(n0 + n1 + n2), false);
     double* part = ctx->partial.as<double>();
     if (tc) {
         CD_RC(tc_backward_pass<AMP_SAME_SPIN>(ctx, 0, 0, bta, bta, RQ, deps[0], deps[0], part));
@@ -1768,7 +1774,7 @@ int run_gradient(mshqc_cd_ctx* ctx, int kind, int precision, mshqc_cd_energy* e_
     double* dC[2] = {nullptr, nullptr};
     double* de[2] = {nullptr, nullptr};
     for (int s = 0; s < (unres ? 2 : 1); ++s) {
-        CD_ALLOC(ctx->grad[s], sizeof(double) * (size_t)(N * N + N), false);
+        CD_ALLOC_FIRST(ctx->grad[s], sizeof(double) * (size_t)(N * N + N), false);
         dC[s] = ctx->grad[s].as<double>();
         de[s] = dC[s] + N * N;
     }

@@ -107,7 +107,7 @@ int coulomb(mshqc_cd_ctx* ctx, const double* L, int64_t n, int64_t mc, const dou
     const int64_t want = std::max<int64_t>(1, 8LL * ctx->num_sms / cdiv(n, 256));
     const int per = (int)std::max<int64_t>(4, cdiv(mc, want));
     const int S = (int)cdiv(mc, per);
-    CD_ALLOC(ctx->gemm_ws, sizeof(double) * (size_t)(S * n), false);
+    CD_ALLOC_FIRST(ctx->gemm_ws, sizeof(double) * (size_t)(S * n), false);
     coulomb_kernel<<<dim3(blocks_for(n), (unsigned)S), 256, 0, ctx->stream>>>(L, n, (int)mc, per, coef,
                                                                               ctx->gemm_ws.as<double>());
     CD_CUDA(cudaGetLastError());
@@ -155,8 +155,8 @@ int opdm_pass(mshqc_cd_ctx* ctx, int sx, int sy, double col_coef, double row_coe
     const size_t held = ctx->W.bytes + ctx->amp.bytes;
     const size_t budget = std::max<size_t>(per_i, std::min<size_t>((free_b + held) / 4, size_t(24) << 30));
     const int bi = (int)std::max<int64_t>(1, std::min<int64_t>(ox, (int64_t)(budget / per_i)));
-    CD_ALLOC(ctx->W, per_i / 2 * bi, false);
-    CD_ALLOC(ctx->amp, per_i / 2 * bi, false);
+    CD_ALLOC_FIRST(ctx->W, per_i / 2 * bi, false);
+    CD_ALLOC_FIRST(ctx->amp, per_i / 2 * bi, false);
     if (!partial) {
         // energies of this pass are not needed: throw-away slots, one per pair
         CD_ALLOC(ctx->pair_sum, sizeof(double) * (size_t)(ox * oy), false);
@@ -221,7 +221,7 @@ int omp2_buffers(mshqc_cd_ctx* ctx, Omp2Buffers& b) {
     // the blocks before the matrices padded to an even count: 16-byte rows for even N
     const int64_t noo = round_up(o0 * o0 + o1 * o1, 2);
     const int64_t n = noo + vp0 * vp0 + vp1 * vp1 + 9 * N * N + M + 2 * N;
-    CD_ALLOC(ctx->opdm, sizeof(double) * (size_t)n, false);
+    CD_ALLOC_FIRST(ctx->opdm, sizeof(double) * (size_t)n, false);
     double* p = ctx->opdm.as<double>();
     b.Goo[0] = p;  p += o0 * o0;
     b.Goo[1] = p;  p += noo - o0 * o0;
@@ -268,7 +268,7 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     CD_CUDA(cudaMemsetAsync(b.Goo[0], 0, sizeof(double) * (size_t)(round_up(o0 * o0 + o1 * o1, 2) + vp0 * vp0 + vp1 * vp1),
                             ctx->stream));
     const int64_t n0 = o0 * o0, n1 = o1 * o1, n2 = o0 * o1;   // one energy per pair
-    CD_ALLOC(ctx->partial, sizeof(double) * (size_t)(n0 + n1 + n2), false);
+    CD_ALLOC_FIRST(ctx->partial, sizeof(double) * (size_t)(n0 + n1 + n2), false);
     double* part = ctx->partial.as<double>();
     OpdmOut out{{b.Goo[0], b.Goo[1]}, {b.Gvv[0], b.Gvv[1]}};
     begin_stage(ctx, ST_AMPLITUDE);
@@ -314,7 +314,7 @@ int omp2_pieces_device(mshqc_cd_ctx* ctx, const double* const Pref[2], Omp2Buffe
     CD_CUDA(cudaGetLastError());
     ctx->launches += 2;
     CD_RC(coulomb(ctx, ctx->L.as<double>(), NN, M, b.coef, 0.0, b.J));
-    CD_ALLOC(ctx->Zt, sizeof(double) * (size_t)(M * NN), false);
+    CD_ALLOC_FIRST(ctx->Zt, sizeof(double) * (size_t)(M * NN), false);
     for (int s = 0; s < 2; ++s) {
         const double* C = ctx->spin[s].C.as<double>();
         // Z^Q = P_s L^Q for every Q (batched)
@@ -435,7 +435,7 @@ int rotate_spin(mshqc_cd_ctx* ctx, int spin, const std::vector<double>& F_host) 
         for (int64_t r = 0; r < N; ++r) col += std::abs(A[r * N + c]);
         norm1 = std::max(norm1, col);
     }
-    CD_ALLOC(ctx->omp2_ws, sizeof(double) * (size_t)(7 * NN), false);
+    CD_ALLOC_FIRST(ctx->omp2_ws, sizeof(double) * (size_t)(7 * NN), false);
     double* dA = ctx->omp2_ws.as<double>();
     double* E0 = dA + NN;
     double* E1 = E0 + NN;
@@ -659,7 +659,7 @@ int density_factors(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], cons
     rank[0] = rank[1] = 0;
     X[0] = X[1] = nullptr;
     if (N < kDensityFactorMinN) return MSHQC_CD_OK;
-    CD_ALLOC(ctx->dens_x, sizeof(double) * (size_t)((2 * (rmax + 1) + rmax) * N + 8), false);
+    CD_ALLOC_FIRST(ctx->dens_x, sizeof(double) * (size_t)((2 * (rmax + 1) + rmax) * N + 8), false);
     double* base = ctx->dens_x.as<double>();
     unsigned long long* tail = reinterpret_cast<unsigned long long*>(base + 2 * (rmax + 1) * N);   // [spin][bad, unused, rank]
     CD_CUDA(cudaMemsetAsync(tail, 0, 6 * sizeof(unsigned long long), ctx->stream));
@@ -729,8 +729,8 @@ int cholesky_jk_device(mshqc_cd_ctx* ctx, int nspin, const double* const P[2], b
     const int64_t mc_max = std::max<int64_t>(
         1, std::min<int64_t>({vectors_chunk_size(ctx), (int64_t)((size_t(2) << 30) / (sizeof(double) * per_q)),
                               (int64_t)65535}));
-    CD_ALLOC(ctx->Zt, sizeof(double) * (size_t)(mc_max * per_q), false);
-    CD_ALLOC(ctx->omp2_ws, sizeof(double) * (size_t)(2 * mc_max), false);
+    CD_ALLOC_FIRST(ctx->Zt, sizeof(double) * (size_t)(mc_max * per_q), false);
+    CD_ALLOC_FIRST(ctx->omp2_ws, sizeof(double) * (size_t)(2 * mc_max), false);
     double* coef = ctx->omp2_ws.as<double>();
     double* norm2 = coef + mc_max;
     double* Z = ctx->Zt.as<double>();
@@ -845,7 +845,7 @@ MSHQC_CD_API int mshqc_cd_omp2_pieces(mshqc_cd_ctx* ctx, const double* P_a, cons
     Omp2Buffers b{};
     double e = 0.0;
     const double* prc[2] = {pr[0], pr[1]};
-    CD_RC(omp2_pieces_device(ctx, prc, b, &e));
+    CD_RC(one_spin_retry(ctx, [&] { return omp2_pieces_device(ctx, prc, b, &e); }));
     collect_stages(ctx);
     if (e_mp2) *e_mp2 = e;
     // OPDM blocks out without the padding
@@ -896,7 +896,7 @@ MSHQC_CD_API int mshqc_cd_omp2(mshqc_cd_ctx* ctx, const mshqc_cd_omp2_config* cf
     while (iter < cfg->max_iterations) {
         ++iter;
         Omp2Buffers b{};
-        CD_RC(omp2_pieces_device(ctx, prc, b, &e_corr));
+        CD_RC(one_spin_retry(ctx, [&] { return omp2_pieces_device(ctx, prc, b, &e_corr); }));
         CD_CUDA(cudaMemcpyAsync(Fa.data(), b.F[0], sizeof(double) * NN, cudaMemcpyDeviceToHost, ctx->stream));
         CD_CUDA(cudaMemcpyAsync(Fb.data(), b.F[1], sizeof(double) * NN, cudaMemcpyDeviceToHost, ctx->stream));
         CD_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -958,7 +958,7 @@ MSHQC_CD_API int mshqc_cd_cholesky_fock(mshqc_cd_ctx* ctx, int nspin, const doub
     reset_stages(ctx);
     const int64_t NN = ctx->N * ctx->N;
     // P_a P_b H | J K_a K_b | F work
-    CD_ALLOC(ctx->opdm, sizeof(double) * (size_t)(8 * NN), false);
+    CD_ALLOC_FIRST(ctx->opdm, sizeof(double) * (size_t)(8 * NN), false);
     double* base = ctx->opdm.as<double>();
     double* P[2] = {base, base + NN};
     double* Hd = base + 2 * NN;

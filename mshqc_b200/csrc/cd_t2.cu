@@ -52,38 +52,40 @@ extern "C" MSHQC_CD_API int mshqc_cd_get_t2_block(mshqc_cd_ctx* ctx, int block, 
     const int64_t ox = ctx->spin[sx].nocc, oy = ctx->spin[sy].nocc;
     if (i0 < 0 || ni < 1 || i0 + ni > ox || j0 < 0 || nj < 1 || j0 + nj > oy)
         return set_error(MSHQC_CD_ERR_ARG, "pair block outside the occupied orbitals");
-    CD_RC(begin_call(ctx));
-    if (sy != sx)
-        CD_RC(ensure_transforms(ctx, MSHQC_CD_FP64));
-    else
-        CD_RC(ensure_transform(ctx, sx, MSHQC_CD_FP64));
-    const SpinState& X = ctx->spin[sx];
-    const SpinState& Y = ctx->spin[sy];
-    const int64_t vx = ctx->N - ox, vy = ctx->N - oy, Mp = ctx->Mp;
-    const size_t n = (size_t)(ni * nj * vx * vy);
-    double* dst = out;
-    if (where != MSHQC_CD_DEVICE) {
-        CD_ALLOC(ctx->scratch, n * sizeof(double), false);
-        dst = ctx->scratch.as<double>();
-    }
-    // (ia|jb) for j in the block, one batched GEMM per i: C_jj = B_i B_j^T
-    for (int64_t ii = 0; ii < ni; ++ii) {
-        GemmF64Args a{};
-        a.M = (int)vx;  a.N = (int)vy;  a.K = (int)Mp;  a.batch = (int)nj;
-        a.A = X.B64.as<double>() + (i0 + ii) * X.vp * Mp;  a.lda = Mp;  a.sA = 0;
-        a.B = Y.B64.as<double>() + j0 * Y.vp * Mp;  a.ldb = Mp;  a.sB = Y.vp * Mp;
-        a.C = dst + ii * nj * vx * vy;  a.ldc = vy;  a.sC = vx * vy;
-        a.alpha = 1.0;  a.beta = 0.0;
-        CD_RC(gemm_run(ctx, a, true, true));
-    }
-    const double* ex = X.eps.as<double>();
-    const double* ey = Y.eps.as<double>();
-    const int blocks = (int)std::min<int64_t>(cdiv((int64_t)n, 256), (int64_t)ctx->num_sms * 8);
-    t2_divide_kernel<<<blocks, 256, 0, ctx->stream>>>(dst, (int)ni, (int)nj, (int)vx, (int)vy, (int)i0, (int)j0, ex,
-                                                     ex + ox, ey, ey + oy);
-    CD_CUDA(cudaGetLastError());
-    ctx->launches++;
-    if (where != MSHQC_CD_DEVICE)
-        CD_CUDA(cudaMemcpyAsync(out, dst, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    return finish_call(ctx);
+    return one_spin_retry(ctx, [&]() -> int {
+        CD_RC(begin_call(ctx));
+        if (sy != sx)
+            CD_RC(ensure_transforms(ctx, MSHQC_CD_FP64));
+        else
+            CD_RC(ensure_transform(ctx, sx, MSHQC_CD_FP64));
+        const SpinState& X = ctx->spin[sx];
+        const SpinState& Y = ctx->spin[sy];
+        const int64_t vx = ctx->N - ox, vy = ctx->N - oy, Mp = ctx->Mp;
+        const size_t n = (size_t)(ni * nj * vx * vy);
+        double* dst = out;
+        if (where != MSHQC_CD_DEVICE) {
+            CD_ALLOC(ctx->scratch, n * sizeof(double), false);
+            dst = ctx->scratch.as<double>();
+        }
+        // (ia|jb) for j in the block, one batched GEMM per i: C_jj = B_i B_j^T
+        for (int64_t ii = 0; ii < ni; ++ii) {
+            GemmF64Args a{};
+            a.M = (int)vx;  a.N = (int)vy;  a.K = (int)Mp;  a.batch = (int)nj;
+            a.A = X.B64.as<double>() + (i0 + ii) * X.vp * Mp;  a.lda = Mp;  a.sA = 0;
+            a.B = Y.B64.as<double>() + j0 * Y.vp * Mp;  a.ldb = Mp;  a.sB = Y.vp * Mp;
+            a.C = dst + ii * nj * vx * vy;  a.ldc = vy;  a.sC = vx * vy;
+            a.alpha = 1.0;  a.beta = 0.0;
+            CD_RC(gemm_run(ctx, a, true, true));
+        }
+        const double* ex = X.eps.as<double>();
+        const double* ey = Y.eps.as<double>();
+        const int blocks = (int)std::min<int64_t>(cdiv((int64_t)n, 256), (int64_t)ctx->num_sms * 8);
+        t2_divide_kernel<<<blocks, 256, 0, ctx->stream>>>(dst, (int)ni, (int)nj, (int)vx, (int)vy, (int)i0, (int)j0, ex,
+                                                         ex + ox, ey, ey + oy);
+        CD_CUDA(cudaGetLastError());
+        ctx->launches++;
+        if (where != MSHQC_CD_DEVICE)
+            CD_CUDA(cudaMemcpyAsync(out, dst, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        return finish_call(ctx);
+    });
 }

@@ -428,13 +428,23 @@ inline int gemm_run(mshqc_cd_ctx* ctx, GemmF64Args a, bool a_k, bool b_k) {
     S = std::max<int64_t>(1, std::min<int64_t>(S, 65535 / a.batch));
     a.per = (int)std::max<int64_t>(1, cdiv(steps, S));
     a.S = (int)std::max<int64_t>(1, cdiv(steps, a.per));
+    if (a.S > 1) {
+        const size_t bytes = sizeof(double) * (size_t)(MN * a.S * a.batch);
+        cudaError_t e = ctx->gemm_ws.reserve(bytes, false, ctx->stream);
+        if (e == cudaErrorMemoryAllocation && ctx->release_slices()) e = ctx->gemm_ws.reserve(bytes, false, ctx->stream);
+        if (e == cudaErrorMemoryAllocation) {   // no room for the partials: no split
+            a.S = 1;
+            a.per = (int)steps;
+        } else {
+            CD_CUDA(e);
+        }
+    }
     if (a.S == 1) {
         if (a.sym) a.sym = 2;
         CD_CUDA(T == 32 ? gemm_f64_tiled<32>(a, a_k, b_k, ctx->stream) : gemm_f64_tiled<64>(a, a_k, b_k, ctx->stream));
         ctx->launches++;
         return MSHQC_CD_OK;
     }
-    CD_ALLOC(ctx->gemm_ws, sizeof(double) * (size_t)(MN * a.S * a.batch), false);
     GemmF64Args w = a;
     w.C = ctx->gemm_ws.as<double>();
     w.ldc = a.N;
