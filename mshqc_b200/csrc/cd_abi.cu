@@ -8,6 +8,7 @@
 //   B_s    [i][a][Q]   FP64, a padded to vp (multiple of 64) and Q to Mp
 //          (multiple of 16) with zeros, so the pair kernels need no bounds
 //          checks in their main loops.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -153,13 +154,17 @@ __global__ void count_nonfinite_kernel(const double* __restrict__ x, int64_t n,
     if (local) atomicAdd(bad, local);
 }
 
-// bad[k] set when array k (a, b) holds a NaN or infinity
-__global__ void check2_kernel(const double* __restrict__ a, int64_t na, const double* __restrict__ b, int64_t nb,
-                              int* __restrict__ bad) {
+// bad[k] set when array k (a, b) holds a NaN or infinity; copied to da and db
+// where these are not null
+__global__ void copy_check2_kernel(const double* __restrict__ a, double* __restrict__ da, int64_t na,
+                                   const double* __restrict__ b, double* __restrict__ db, int64_t nb,
+                                   int* __restrict__ bad) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < na + nb;
          t += (int64_t)gridDim.x * blockDim.x) {
         const bool second = t >= na;
-        if (!isfinite(second ? b[t - na] : a[t])) bad[second ? 1 : 0] = 1;
+        const double x = second ? b[t - na] : a[t];
+        if (da) (second ? db + (t - na) : da + t)[0] = x;
+        if (!isfinite(x)) bad[second ? 1 : 0] = 1;
     }
 }
 
@@ -186,6 +191,33 @@ bool is_unregistered(const void* p) {
         return true;
     }
     return at.type == cudaMemoryTypeUnregistered;
+}
+
+// whether a kernel on `device` may read n doubles at p: memory of this device, all
+// of it inside one allocation (asked of the driver, about 1 us)
+bool readable_here(const void* p, int64_t n, int device) {
+    cudaPointerAttributes at;
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(double) != 0) return false;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+    using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const Range range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &found) != cudaSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Range>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+    if (!range || range(&base, &size, q) != CUDA_SUCCESS) return false;
+    return q >= base && sizeof(double) * (size_t)n <= size - (size_t)(q - base);
 }
 
 bool is_pinned_host(const void* p) {
@@ -513,14 +545,19 @@ int mshqc_cd_set_orbitals(mshqc_cd_ctx* ctx, int spin, const double* C, const do
         rc = upload(ctx, s.eps.p, eps, sizeof(double) * N);
         if (rc) return rc;
     } else {
-        // Copies, which check the caller's ranges and reach another device's memory
-        // too; only the context's own copies are read by a kernel.
-        CD_CUDA(cudaMemcpyAsync(s.C.p, C, sizeof(double) * N * N, cudaMemcpyDeviceToDevice, ctx->stream));
-        CD_CUDA(cudaMemcpyAsync(s.eps.p, eps, sizeof(double) * N, cudaMemcpyDeviceToDevice, ctx->stream));
+        // Arrays that lie in this device's memory are copied and checked by one
+        // kernel; others (another device's, managed, page-locked) by copies, which
+        // reach them and check their ranges, and the kernel looks at the copies.
+        const bool here = readable_here(C, N * N, ctx->device) && readable_here(eps, N, ctx->device);
+        if (!here) {
+            CD_CUDA(cudaMemcpyAsync(s.C.p, C, sizeof(double) * N * N, cudaMemcpyDeviceToDevice, ctx->stream));
+            CD_CUDA(cudaMemcpyAsync(s.eps.p, eps, sizeof(double) * N, cudaMemcpyDeviceToDevice, ctx->stream));
+        }
         if (!ctx->orb_bad.p) CD_ALLOC(ctx->orb_bad, 2 * sizeof(int), true);   // zero but for a refused input
         const int blocks = (int)std::min<int64_t>(8LL * ctx->num_sms, cdiv(N * N + N, 256));
-        check2_kernel<<<blocks, 256, 0, ctx->stream>>>(s.C.as<double>(), N * N, s.eps.as<double>(), N,
-                                                       ctx->orb_bad.as<int>());
+        double *dC = s.C.as<double>(), *de = s.eps.as<double>();
+        copy_check2_kernel<<<blocks, 256, 0, ctx->stream>>>(here ? C : dC, here ? dC : nullptr, N * N, here ? eps : de,
+                                                            here ? de : nullptr, N, ctx->orb_bad.as<int>());
         CD_CUDA(cudaGetLastError());
         ctx->launches++;
         void* h = nullptr;
