@@ -293,6 +293,7 @@ int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p) {
 int begin_call(mshqc_cd_ctx* ctx) {
     if (ctx->call_open) ctx->invalidate_derived();
     ctx->call_open = true;
+    ctx->slices_refused = false;
     CD_ALLOC(ctx->status, sizeof(CallStatus), true);
     return MSHQC_CD_OK;
 }

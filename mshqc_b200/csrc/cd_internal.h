@@ -125,6 +125,7 @@ struct mshqc_cd_ctx {
     mshqc_cd::DevBuf oz_a, oz_b;    // int8 slices of the transform operands (orbitals, vectors)
     mshqc_cd::DevBuf oz_ea, oz_eb;  // their row exponents and digit squares
     mshqc_cd::DevBuf oz_tiles;      // tiles of a sliced FP64 product that the FP64 product computes
+    bool slices_refused = false;    // no room for FP64 slices: not tried again in this call
     mshqc_cd::DevBuf oz_p;          // per-batch FP64 partial products (transposed transforms)
     bool diag_os_valid = false;
     int fixed_point_exact = 1;      // Cauchy-Schwarz bound of the last tensor-core pass held

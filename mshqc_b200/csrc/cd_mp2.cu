@@ -284,7 +284,8 @@ int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
 // at every size.
 constexpr double kSlicedMinFlops = 4e9;
 constexpr int64_t kSlicedMinReuse = 256;
-bool fp64_slices(double flops, double min_flops, int64_t reuse) {
+bool fp64_slices(const mshqc_cd_ctx* ctx, double flops, double min_flops, int64_t reuse) {
+    if (ctx->slices_refused) return false;
     if (const char* env = std::getenv("MSHQC_CD_FP64_SLICES")) {
         if (std::strcmp(env, "off") == 0) return false;
         if (std::strcmp(env, "on") == 0) return true;
@@ -294,10 +295,12 @@ bool fp64_slices(double flops, double min_flops, int64_t reuse) {
 
 // The sliced FP64 products hold their slices next to the operands.  Each of the
 // functions below reserves them before it writes a result, so where the memory
-// does not hold them the FP64 products run instead.
+// does not hold them the FP64 products run instead, for the rest of the call (each
+// attempt frees buffers, which waits for the device).
 bool no_room(mshqc_cd_ctx* ctx, int rc) {
     if (rc != MSHQC_CD_ERR_ALLOC) return false;
     ctx->release_slices();
+    ctx->slices_refused = true;
     return true;
 }
 
@@ -428,7 +431,7 @@ int transform(mshqc_cd_ctx* ctx, int nsp, const int* spins, bool i8) {
             continue;
         }
         const char* tenv = std::getenv("MSHQC_CD_TRANSFORM");   // f64: DMMA for both halves
-        if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
+        if (!(tenv && std::strcmp(tenv, "f64") == 0) && fp64_slices(ctx, 2.0 * v * M * N * ni, kSlicedMinFlops, v)) {
             const int rc = second_half_sliced<ozaki::Full>(ctx, spins[k], lo[k], hi[k]);
             if (!no_room(ctx, rc)) {
                 CD_RC(rc);
@@ -477,7 +480,7 @@ int both_spins_fit(mshqc_cd_ctx* ctx, bool* yes) {
 // work on the slices win.
 constexpr double kSlicedPairFlops = 1.6e10;
 bool sliced_pairs(const mshqc_cd_ctx* ctx, int64_t rows, int64_t cols) {
-    return fp64_slices(2.0 * rows * cols * ctx->Mp, kSlicedPairFlops, ctx->Mp);
+    return fp64_slices(ctx, 2.0 * rows * cols * ctx->Mp, kSlicedPairFlops, ctx->Mp);
 }
 
 // S[(i,a)][(j,b)] = sum_Q X[(i,a)][Q] Y[(j,b)][Q] of a block pair from int8
@@ -1080,7 +1083,7 @@ int virtual_part(mshqc_cd_ctx* ctx, int spin, double scale, double* dC, bool i8)
     const auto& y = ctx->Yr[spin];
     const int64_t v = ctx->N - ctx->spin[spin].nocc;
     const bool full = int8_transform_enabled(ctx) &&
-                      fp64_slices(2.0 * v * ctx->M * ctx->N * (y.hi - y.lo), kSlicedMinFlops, v);
+                      fp64_slices(ctx, 2.0 * v * ctx->M * ctx->N * (y.hi - y.lo), kSlicedMinFlops, v);
     if (full) {   // N = 600, o = 60: the transposed transforms 12.8 -> 8.8 ms; N = 400, o = 40: 2.3 -> 1.9
         const int rc = virtual_part_i8<ozaki::Full>(ctx, spin, scale, dC);
         if (!no_room(ctx, rc)) return rc;
