@@ -291,7 +291,15 @@ int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p) {
 }
 
 int begin_call(mshqc_cd_ctx* ctx) {
-    if (ctx->call_open) ctx->invalidate_derived();
+    if (ctx->call_open) {
+        ctx->invalidate_partial();
+        if (ctx->status.p) {   // what its kernels reported was not read
+            CallStatus st;
+            CD_CUDA(cudaMemcpyAsync(&st, ctx->status.p, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+            CD_CUDA(cudaStreamSynchronize(ctx->stream));
+            if (st.tile_err[0] || st.gamma_err[0] || st.slice_err[0]) ctx->invalidate_derived();
+        }
+    }
     ctx->call_open = true;
     ctx->slices_refused = false;
     CD_ALLOC(ctx->status, sizeof(CallStatus), true);
@@ -318,12 +326,14 @@ int finish_call(mshqc_cd_ctx* ctx, CallStatus* out, const void* dev, size_t extr
                        : st.gamma_err[0] ? "tensor-core backward"
                        : st.slice_err[0] ? "int8 tensor-core product"
                                          : nullptr;
-    if (what)
+    if (what) {
+        ctx->invalidate_derived();
         return set_error(MSHQC_CD_ERR_TIMEOUT,
                          std::string(what) + " gave up waiting (site " +
                              std::to_string(st.tile_err[0] ? st.tile_err[0] : st.gamma_err[0] ? st.gamma_err[0]
                                                                                                : st.slice_err[0]) +
                              ")");
+    }
     ctx->call_open = false;
     return MSHQC_CD_OK;
 }

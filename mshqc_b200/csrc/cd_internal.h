@@ -144,14 +144,21 @@ struct mshqc_cd_ctx {
     bool coll_set = false;
     std::vector<double> pair_energy[3];  // host copies, row-major [i][j]
 
-    // what calls derive from the vectors and orbitals
-    void invalidate_derived() {
+    // what a call that stopped in between may have left half done: all but the MO
+    // vectors, which are marked valid when complete (ranks that share a gradient
+    // gather them together, so all or none form them again)
+    void invalidate_partial() {
         for (auto& s : spin) {
-            s.invalidate();
+            s.B16_valid = false;
             s.norms_pending = false;
         }
         diag_os_valid = false;
         Yr[0].ok = Yr[1].ok = false;
+    }
+    // what calls derive from the vectors and orbitals
+    void invalidate_derived() {
+        invalidate_partial();
+        for (auto& s : spin) s.invalidate();
     }
     void invalidate_all() {
         invalidate_derived();
@@ -302,7 +309,7 @@ struct CallStatus {
 int pinned(mshqc_cd_ctx* ctx, size_t bytes, void** p);
 // Zeroes the status.  A call that stopped in between (an allocation that failed,
 // a kernel that gave up) may have left a buffer half written, or W where Y was:
-// what it had derived is then formed again.
+// that is then formed again.
 int begin_call(mshqc_cd_ctx* ctx);
 // Waits for the call's work, reports kernels that gave up, and copies `extra`
 // bytes from dev to the pinned buffer behind the status (*extra_host).

@@ -78,3 +78,25 @@ def test_energy_after_failed_allocation(inp, kind):
 def test_gradient_after_failed_allocation(inp, kind, precision):
     tol = (1e-12, 1e-10) if precision == capi.FP64 else (1e-9, 1e-9)
     retry(inp, lambda ctx: ctx.mp2_gradient(kind, precision), check_gradient(*tol))
+
+
+def test_complete_vectors_are_kept(inp):
+    """MO vectors that an earlier call completed are not formed again after a call
+    that fails later: ranks that share a gradient gather them together, and a rank
+    that did so alone would wait for the others."""
+    L = torch.from_numpy(inp.L).cuda()
+    with context(inp, L) as ctx:
+        ref = ctx.mp2_gradient(capi.RESTRICTED, capi.FP64)
+    with context(inp, L) as ctx:
+        ctx.mp2_energy(capi.RESTRICTED, capi.FP64)
+        held = fill(8 << 20)
+        try:
+            with pytest.raises(capi.CDError) as ex:
+                ctx.mp2_gradient(capi.RESTRICTED, capi.FP64)
+            assert ex.value.code == capi.ERR_ALLOC
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        g = ctx.mp2_gradient(capi.RESTRICTED, capi.FP64)
+        assert ctx.stage_counts()["transform"] == 0
+        check_gradient(1e-12, 1e-10)(g, ref, 1.0)
