@@ -16,30 +16,31 @@ from oracle import cdmp2_oracle as orc
 pytestmark = pytest.mark.gpu
 
 
-def fragments(n, o, M, coupling, seed):
-    """Two fragments of n functions and o occupied orbitals each."""
+def fragments(n, o, M, coupling, seed, extra=0):
+    """Two fragments of n and n + extra functions, o occupied orbitals each."""
     rng = np.random.default_rng(seed)
-    N = 2 * n
-    side = np.arange(N) // n
+    N = 2 * n + extra
+    side = (np.arange(N) >= n).astype(int)
     L = rng.standard_normal((M, N, N))
     L = 0.05 * (L + L.transpose(0, 2, 1))
     at = np.arange(M) % 2
     big = (side[None, :, None] == at[:, None, None]) & (side[None, None, :] == at[:, None, None])
     L *= np.where(big, 1.0, coupling)
     C = np.zeros((N, N))
-    own = np.concatenate([np.repeat([0, 1], o), np.repeat([0, 1], n - o)])   # fragment of each orbital
+    own = np.concatenate([np.repeat([0, 1], o), np.repeat([0, 1], [n - o, n + extra - o])])   # fragment of each orbital
     for f in (0, 1):
-        q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+        q, _ = np.linalg.qr(rng.standard_normal((np.sum(side == f),) * 2))
         C[np.ix_(side == f, own == f)] = q
     eps = syn.make_orbitals(N, 2 * o, seed).eps
     return L.reshape(M, N * N), C, eps, side, own
 
 
 @pytest.mark.parametrize("slices", ["on", "off"])
-@pytest.mark.parametrize("n,o,M,coupling", [(48, 3, 128, 1e-6), (70, 4, 97, 1e-9), (33, 2, 64, 1e-3)])
-def test_distant_fragments(monkeypatch, slices, n, o, M, coupling):
+@pytest.mark.parametrize("n,o,M,coupling,extra", [(48, 3, 128, 1e-6, 0), (70, 4, 97, 1e-9, 0), (33, 2, 64, 1e-3, 0),
+                                                  (77, 4, 65, 1e-7, 1)])
+def test_distant_fragments(monkeypatch, slices, n, o, M, coupling, extra):
     monkeypatch.setenv("MSHQC_CD_FP64_SLICES", slices)
-    L, C, eps, side, own = fragments(n, o, M, coupling, seed=n)
+    L, C, eps, side, own = fragments(n, o, M, coupling, n, extra)
     oc = 2 * o
     with capi.Context(0) as ctx:
         ctx.set_vectors(L).set_orbitals(capi.ALPHA, C, eps, oc)
