@@ -78,8 +78,8 @@ enum mshqc_cd_precision {
                              int8 slices (5 x 7 bits per operand row) on
                              the tensor cores, about 2^-32 of the row
                              maxima per term (MSHQC_CD_TRANSFORM=f64 in the
-                             environment: those of MSHQC_CD_FP64 for both,
-                             =i8: int8 slices for both at every size)    */
+                             environment: DMMA for both, =i8: int8 slices
+                             for both at every size)                     */
 };
 
 enum mshqc_cd_kind {

@@ -37,8 +37,9 @@
 // (every integral read twice, every 1/D taken twice) and one split per operand
 // the pass took 32.3 ms of the N = 1000, o = 100 restricted mixed backward and
 // 12.9 ms of the N = 600 unrestricted one, now 20.0 and 9.6 (4.1 TB/s at
-// N = 1000); FP64, N = 600, o = 60: 4.8 -> 3.7 ms.  5 CTAs per SM (mixed)
-// measured best of 3, 4, 5, 6 (20.7, 21.3, 19.9, 21.9 ms).
+// N = 1000); FP64, N = 600, o = 60: 4.8 -> 3.7 ms.  The CTAs per SM
+// do not matter: 20.7, 21.3, 19.9, 21.9 ms with 3, 4, 5, 6 (mixed, N = 1000), the
+// spread of one setting.
 #pragma once
 
 #include <cuda_bf16.h>

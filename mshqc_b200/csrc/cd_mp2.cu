@@ -279,7 +279,11 @@ int second_half_sliced(mshqc_cd_ctx* ctx, int spin, int64_t lo, int64_t hi) {
 // FP64 products of at least this many operations run as int8 slices of full
 // accuracy (ozaki::Full) where each sliced element takes part in at least
 // kSlicedMinReuse multiply-adds: slicing costs about 6 ps an element (HBM),
-// the DMMA products 0.06 ps an operation, the sliced ones 0.03.
+// the DMMA products 0.06 ps an operation, the sliced ones 0.03.  Second half
+// transforms and virtual products of the gradient at M = 4 N, o = N / 10, DMMA
+// and sliced (stage times, ms): N = 203 (1.3e9 operations, v = 183) 0.17 and 0.18,
+// 0.26 and 0.37; N = 300 (9.7e9, v = 270) 0.50 and 0.48, 0.84 and 0.84; N = 360
+// 1.18 and 1.10, 1.88 and 1.77; N = 400 1.56 and 1.49, 2.35 and 2.17.
 // MSHQC_CD_FP64_SLICES=off keeps every FP64 product on the DMMA pipe, =on slices
 // at every size.
 constexpr double kSlicedMinFlops = 4e9;
@@ -474,10 +478,12 @@ int both_spins_fit(mshqc_cd_ctx* ctx, bool* yes) {
 }
 
 // Whether the FP64 integral and Gamma products of blocks of `rows` x `cols`
-// composite virtual rows run as int8 slices of full accuracy.  N = 161 (17
-// occupied): the products 0.19 ms each against 0.16 (half of the tiles) and
-// 0.31 ms DMMA, but the slicing passes take what is gained; from twice that
-// work on the slices win.
+// composite virtual rows run as int8 slices of full accuracy.  Whole calls at
+// M = 4 N, o = N / 10, DMMA and sliced (energy; gradient, ms): N = 128 (2.4e9
+// operations) 0.28 and 0.32; 0.69 and 0.87.  N = 161 (1.2e10) 0.55 and 0.44; 1.50
+// and 1.22.  N = 180 (2.1e10) 0.66 and 0.51; 1.73 and 1.44.  N = 245 2.03 and 1.05;
+// 5.05 and 3.06.  N = 161 with M = 403, o = 17 (8.9e9): equal.  So the two cross
+// between 2.4e9 and 1.2e10; the line lies above, on the DMMA side.
 constexpr double kSlicedPairFlops = 1.6e10;
 bool sliced_pairs(const mshqc_cd_ctx* ctx, int64_t rows, int64_t cols) {
     return fp64_slices(ctx, 2.0 * rows * cols * ctx->Mp, kSlicedPairFlops, ctx->Mp);

@@ -25,8 +25,11 @@
 // in order, the core orbitals' columns of the amplitudes, small for every row,
 // kept the Gamma tiles of N = 600 undecided for 2300 terms (6.9 ms of a 27 ms
 // product).  A tile that has not passed after 8 such steps, or a sixteenth of K,
-// is left out: a step costs about as much as the FP64 product of it.  BF16 squares, FP32 sums (positive terms: relative error below 2%),
-// m16n8k16 MMAs; 8 warps of 32 x 32 outputs.
+// is left out: deciding it over all of K takes half as long as its FP64 product
+// (two fragments, N = 400, FP64 gradient: 59.9 ms, with the limit 40.3).  BF16
+// squares, FP32 sums (positive terms: relative error below 2%), m16n8k16 MMAs; 8
+// warps of 32 x 32 outputs, 4 CTAs per SM (N = 400 integrals: 163, 137, 116, 204
+// us with 2, 3, 4, 5).
 #pragma once
 
 #include <cuda_bf16.h>

@@ -6,8 +6,8 @@
 // j), every tile computed once;
 // X and Y are the MO vectors of one spin (restricted, same spin) or of the
 // two spins (opposite spin: X alpha, Y beta).
-// Operands are the exact fixed-point hi/lo of split_bf16.cuh in its 256-row
-// blocked layout over the composite rows (i, a) and (j, b), packed at v rounded
+// Operands are the exact fixed-point hi/lo of split_bf16.cuh in its blocked
+// layout (128-row blocks) over the composite rows (i, a) and (j, b), packed at v rounded
 // to 32 per orbital, so a tile runs across orbitals (padding every orbital's
 // rows to 128 and columns to 256 took 1.66 times the tiles at v = 540).  Tiles
 // lie on the grid of the composite rows; the edge tiles of a block store only
@@ -23,7 +23,7 @@
 //   (ia|jb) = u_ia u_jb (hh + x / 256)
 // in FP64, substitutes the exact (ia|ia) for i = j, a = b when X = Y, and
 // stores it rounded to FP32 into the row-major staging matrix S (row length
-// nbj * VS).  amp_elem.cuh turns S into amplitudes.
+// nbj * RSy).  amp_elem.cuh turns S into amplitudes.
 //
 // Warp roles (576 threads): warp 0 producer, warp 1 MMA issuer and TMEM
 // owner, warps 2..17 epilogue (TMEM lane quadrant warp % 4, column quarter
