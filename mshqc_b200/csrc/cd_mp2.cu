@@ -183,9 +183,11 @@ template <class C>
 OzakiOperand oz_operand(int64_t rows, int64_t K, bool as_a, int64_t batch) {
     return ozaki_operand(rows, K, as_a ? ozaki::BM : C::BN, (int)batch);
 }
+// an operand's digits and, behind them, the squares that the guard samples
 template <class C>
 size_t oz_bytes(const OzakiOperand& op) {
-    return ozaki::operand_bytes<C>(op.Rp, op.Kp) * (size_t)op.batch;
+    return (ozaki::operand_bytes<C>(op.Rp, op.Kp) +
+            (C::GUARD ? sizeof(uint32_t) * ozaki::SAMPLE_WORDS * (size_t)op.Rp : 0)) * (size_t)op.batch;
 }
 int* slice_err(mshqc_cd_ctx* ctx) { return ctx->status.as<CallStatus>()->slice_err; }
 // One sliced product; A has the 128-row blocks.  With C::GUARD its accuracy is
@@ -245,6 +247,8 @@ int oz_reserve(mshqc_cd_ctx* ctx, DevBuf& q, DevBuf& e, size_t bytes, OzakiOpera
     CD_ALLOC(e, op.row_bytes(C::GUARD), false);
     op.q = q.as<int8_t>();
     op.e = e.as<int>();
+    if (C::GUARD)
+        op.smp = reinterpret_cast<uint32_t*>(op.q + ozaki::operand_bytes<C>(op.Rp, op.Kp) * (size_t)op.batch);
     return MSHQC_CD_OK;
 }
 // the rows of Y that hold a spin's half-transformed vectors

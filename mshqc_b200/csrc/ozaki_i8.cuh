@@ -718,7 +718,8 @@ static __global__ void __launch_bounds__(ozaki::THREADS, 1) ozaki_gemm_kernel(Oz
 // (padded to Kp), `batch` copies.
 struct OzakiOperand {
     int8_t* q = nullptr;
-    int* e = nullptr;           // row exponents and, behind them, what the guard needs (row_bytes)
+    int* e = nullptr;           // row exponents and, behind them, the digits' squares (row_bytes)
+    uint32_t* smp = nullptr;    // sampled squares, SAMPLE_WORDS a row (C::GUARD)
     long long R = 0, Rp = 0, K = 0, Kp = 0;
     int BR = 0;
     int batch = 1;
@@ -728,10 +729,7 @@ struct OzakiOperand {
     long long ld = 0, sb = 0;
     bool t = false;
     unsigned* sq() const { return reinterpret_cast<unsigned*>(e + Rp * batch); }
-    uint32_t* sample() const { return reinterpret_cast<uint32_t*>(e + 2 * Rp * batch); }
-    size_t row_bytes(bool guard) const {
-        return sizeof(int) * (size_t)(Rp * batch) * (guard ? 2 + ozaki::SAMPLE_WORDS : 1);
-    }
+    size_t row_bytes(bool guard) const { return sizeof(int) * (size_t)(Rp * batch) * (guard ? 2 : 1); }
 };
 
 inline OzakiOperand ozaki_operand(long long R, long long K, int tile, int batch) {
@@ -758,11 +756,11 @@ inline cudaError_t ozaki_slice_br(const double* src, long long ld, long long src
         if (v2)                                                                                                     \
             ozaki_slice_kernel<C, BR, H, true><<<grid, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K,      \
                                                                      (int)op.Rp, (int)op.Kp, op.q, op.e, op.sq(),   \
-                                                                     op.sample());                                  \
+                                                                     op.smp);                                  \
         else                                                                                                        \
             ozaki_slice_kernel<C, BR, H, false><<<grid, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K,     \
                                                                       (int)op.Rp, (int)op.Kp, op.q, op.e, op.sq(),  \
-                                                                      op.sample());                                 \
+                                                                      op.smp);                                 \
     } while (0)
     if (nkc <= 16)
         MSHQC_SLICE(2);
@@ -806,10 +804,10 @@ inline cudaError_t ozaki_slice_t(const double* src, long long ld, long long src_
     dim3 g2((unsigned)(op.Rp / 32), (unsigned)((op.Kp + 127) / 128), (unsigned)op.batch);
     if (op.BR == BM)
         ozaki_slice_t_kernel<C, BM><<<g2, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K, (int)op.Rp,
-                                                        (int)op.Kp, op.e, op.q, op.sq(), op.sample());
+                                                        (int)op.Kp, op.e, op.q, op.sq(), op.smp);
     else
         ozaki_slice_t_kernel<C, C::BN><<<g2, 256, 0, st>>>(src, ld, src_batch, (int)op.R, (int)op.K, (int)op.Rp,
-                                                           (int)op.Kp, op.e, op.q, op.sq(), op.sample());
+                                                           (int)op.Kp, op.e, op.q, op.sq(), op.smp);
     return cudaGetLastError();
 }
 

@@ -234,7 +234,7 @@ inline cudaError_t guard_slices(const OzakiOperand& A, const OzakiOperand& B, co
     auto side = [](const OzakiOperand& x, bool shared) {
         SliceGuardArgs::Side s{};
         s.src = x.src;  s.ld = x.ld;  s.sb = shared ? 0 : x.sb;
-        s.e = x.e;  s.sq = x.sq();  s.sample = x.sample();
+        s.e = x.e;  s.sq = x.sq();  s.sample = x.smp;
         s.eb = shared ? 0 : x.Rp;
         s.R = (int)x.R;  s.t = x.t ? 1 : 0;
         return s;
